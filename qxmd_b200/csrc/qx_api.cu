@@ -158,9 +158,10 @@ struct qx_ctx {
   // real-space table builder (qx_set_kb_r_builder, qx_build_kb_r)
   KbrGeom kbr_geom = {};
   int kbr_ntype = 0, kbr_mxnl = 0, kbr_natom = 0, kbr_lmx = 4;
+  long kbr_slabs = 0;   // (atom, z plane of the search box) counts held by d_kbr_cnt, d_kbr_soff
   long kbr_cap = 0;
   double *d_kbr_dl = nullptr, *d_kbr_rcut = nullptr, *d_kbr_tab = nullptr, *d_kbr_satm = nullptr;
-  int *d_kbr_poly = nullptr, *d_kbr_ityp = nullptr, *d_kbr_cnt = nullptr, *d_kbr_off = nullptr,
+  int *d_kbr_poly = nullptr, *d_kbr_ityp = nullptr, *d_kbr_cnt = nullptr, *d_kbr_soff = nullptr, *d_kbr_off = nullptr,
       *d_kbr_mesh = nullptr, *d_kbr_ptatom = nullptr, *d_kbr_lcnt = nullptr, *d_kbr_loff = nullptr,
       *d_kbr_cursor = nullptr;
   int4 *d_kbr_lent = nullptr;
@@ -1066,13 +1067,18 @@ extern "C" int qx_build_kb_r(qx_ctx *c, int natom, const int *ityp, const double
   if (natom != c->kbr_natom) {
     TRY(dregrow(c, &c->d_kbr_ityp, sizeof(int) * natom));
     TRY(dregrow(c, &c->d_kbr_satm, sizeof(double) * 3 * natom));
-    TRY(dregrow(c, &c->d_kbr_cnt, sizeof(int) * natom));
     TRY(dregrow(c, &c->d_kbr_off, sizeof(int) * (natom + 1)));
     TRY(dregrow(c, &c->d_kbr_sumr, 2 * ts * (size_t)pl.chunk * natom * c->kbr_lmx));
     c->kbr_natom = natom;
     moved = true;
   }
   if (!c->d_kbr_loff) {
+  const long slabs = (long)natom * (2 * c->kbr_geom.nd[2] + 1);
+  if (slabs != c->kbr_slabs) {
+    TRY(dregrow(c, &c->d_kbr_cnt, sizeof(int) * slabs));
+    TRY(dregrow(c, &c->d_kbr_soff, sizeof(int) * (slabs + 1)));
+    c->kbr_slabs = slabs;
+  }
     TRY(dalloc(c, &c->d_kbr_lcnt, sizeof(int) * nlines));
     TRY(dalloc(c, &c->d_kbr_loff, sizeof(int) * (nlines + 1)));
     TRY(dalloc(c, &c->d_kbr_cursor, sizeof(int) * nlines));
@@ -1082,7 +1088,8 @@ extern "C" int qx_build_kb_r(qx_ctx *c, int natom, const int *ityp, const double
   CK(cudaMemcpyAsync(c->d_kbr_ityp, ityp, sizeof(int) * natom, cudaMemcpyHostToDevice, c->st));
   CK(cudaMemcpyAsync(c->d_kbr_satm, satm, sizeof(double) * 3 * natom, cudaMemcpyHostToDevice, c->st));
   const KbrGeom &G = c->kbr_geom;
-  kbr_count(G, natom, c->d_kbr_ityp, c->d_kbr_satm, c->d_kbr_rcut, c->d_kbr_cnt, c->d_kbr_off, c->st);
+  kbr_count(G, natom, c->d_kbr_ityp, c->d_kbr_satm, c->d_kbr_rcut, c->d_kbr_cnt, c->d_kbr_soff, c->d_kbr_off,
+            c->st);
   int total = 0;
   CK(cudaMemcpyAsync(&total, c->d_kbr_off + natom, sizeof(int), cudaMemcpyDeviceToHost, c->st));
   CK(cudaStreamSynchronize(c->st));
@@ -1101,11 +1108,11 @@ extern "C" int qx_build_kb_r(qx_ctx *c, int natom, const int *ityp, const double
   }
   if (c->prec == QX_PREC_FP64)
     kbr_fill<double>(G, natom, c->kbr_lmx, c->d_kbr_ityp, c->d_kbr_satm, c->d_kbr_rcut, c->d_kbr_rcl, c->d_kbr_dl, c->d_kbr_tab,
-                     c->d_kbr_dtab, c->kbr_mxnl, c->d_kbr_poly, c->d_kbr_off, c->kbr_cap, c->d_kbr_mesh,
+                     c->d_kbr_dtab, c->kbr_mxnl, c->d_kbr_poly, c->d_kbr_soff, c->kbr_cap, c->d_kbr_mesh,
                      c->d_kbr_ptatom, (double *)c->d_kbr_vnl, (double *)c->d_kbr_dvnl, c->st);
   else
     kbr_fill<float>(G, natom, c->kbr_lmx, c->d_kbr_ityp, c->d_kbr_satm, c->d_kbr_rcut, c->d_kbr_rcl, c->d_kbr_dl, c->d_kbr_tab,
-                    c->d_kbr_dtab, c->kbr_mxnl, c->d_kbr_poly, c->d_kbr_off, c->kbr_cap, c->d_kbr_mesh,
+                    c->d_kbr_dtab, c->kbr_mxnl, c->d_kbr_poly, c->d_kbr_soff, c->kbr_cap, c->d_kbr_mesh,
                     c->d_kbr_ptatom, (float *)c->d_kbr_vnl, (float *)c->d_kbr_dvnl, c->st);
   if (kbr_lines(c->d_kbr_off, natom, c->d_kbr_mesh, c->d_kbr_ptatom, pl.k1, nlines, c->d_kbr_lcnt, c->d_kbr_loff,
                 c->d_kbr_cursor, c->d_kbr_lent, c->st)) {
@@ -2439,7 +2446,7 @@ extern "C" int qx_set_force_tables(qx_ctx *c, int natom, int ntype, const int *i
     TRY(dalloc(c, &c->d_svco, sizeof(double) * (size_t)n5 * ntype));
     TRY(dalloc(c, &c->d_dcq, sizeof(double) * (size_t)natom * ktot));
     TRY(dalloc(c, &c->d_dsq, sizeof(double) * (size_t)natom * ktot));
-    TRY(dalloc(c, &c->d_force, sizeof(double) * 6 * natom));
+    TRY(dalloc(c, &c->d_force, sizeof(double) * (6 + 3 * floc_slices(natom)) * natom));
   }
   if (!c->d_gw) TRY(dalloc(c, &c->d_gw, sizeof(double) * 3 * (size_t)(ne / 2)));
   if (!c->dtab) {
@@ -2481,7 +2488,7 @@ static int forces_impl(qx_ctx *c, double *floc, double *fnl) {
   real_to_cplx(c->d_rho_out, nullptr, c->d_zg, n, c->st);
   TRY(launch_full_fft<double>(c->pl, c->d_zg, -1, 1.0 / (double)n, c->st));
   floc_g(natom, c->f_n5, c->d_ijk5, c->d_ngabc, c->d_gvec5, c->d_svco, c->d_ityp, c->d_zg, c->d_dcq, c->d_dsq,
-         c->f_km[0], c->f_km[1], c->f_km[2], c->f_ktot, c->d_force, c->st);
+         c->f_km[0], c->f_km[1], c->f_km[2], c->f_ktot, c->d_force + 6 * natom, c->d_force, c->st);
   CKL();
   const Bufs<T> &b = c->pl.bufs<T>();
   T *P = (T *)c->proj, *D = (T *)c->dproj;

@@ -9,6 +9,8 @@
 //    both as contractions over the half sphere (D through derivative tables
 //    d(2g) = -G beta(2g+1), d(2g+1) = G beta(2g), built once per geometry).
 // All sums in FP64 in a fixed order.
+#include <algorithm>
+
 #include "qx_internal.h"
 
 namespace qx {
@@ -44,17 +46,20 @@ __global__ void k_phase_tables(int natom, const double *__restrict__ satm, int k
 
 // vlocal_g (nlkbpp.f90:862-1036): V(G) = (1/Omega) sum_a svco(G, type of a)
 // (cos G.R_a, -sin G.R_a) on the density half sphere, written at +G and, as
-// its conjugate, at -G of the full complex grid (zeroed before); one thread
-// per G, atoms summed in order.
-__global__ void k_vloc_g(int n5, int natom, const int *__restrict__ ijk5, const int *__restrict__ ngabc,
+// its conjugate, at -G of the full complex grid (zeroed before).  VLS lanes a
+// G, each summing every VLS-th atom; their sums meet in shuffles.  Latency of
+// the phase gathers bounds it: at Si64 (37 k G) one thread a G left eight
+// warps a SM.
+constexpr int VLS = 8;
+__global__ void __launch_bounds__(256) k_vloc_g(int n5, int natom, const int *__restrict__ ijk5, const int *__restrict__ ngabc,
                          const double *__restrict__ svco, const int *__restrict__ ityp, const double *__restrict__ dcq,
                          const double *__restrict__ dsq, int km1, int km2, int km3, int ktot, double rvolr, int k1n,
                          int k2n, int k3n, double2 *__restrict__ zg) {
-  const int g = blockIdx.x * blockDim.x + threadIdx.x;
-  if (g >= n5) return;
+  const int gq = (int)((blockIdx.x * (long)blockDim.x + threadIdx.x) / VLS), sub = threadIdx.x % VLS;
+  const int g = min(gq, n5 - 1);   // whole warps run the shuffles
   const int k1 = ngabc[3 * g], k2 = ngabc[3 * g + 1], k3 = ngabc[3 * g + 2];
   double re = 0.0, im = 0.0;
-  for (int a = 0; a < natom; ++a) {
+  for (int a = sub; a < natom; a += VLS) {
     const double *c1 = dcq + (long)a * ktot + km1, *s1 = dsq + (long)a * ktot + km1;
     const double *c2 = dcq + (long)a * ktot + 2 * km1 + 1 + km2, *s2 = dsq + (long)a * ktot + 2 * km1 + 1 + km2;
     const double *c3 = dcq + (long)a * ktot + 2 * km1 + 2 * km2 + 2 + km3,
@@ -67,6 +72,12 @@ __global__ void k_vloc_g(int n5, int natom, const int *__restrict__ ijk5, const 
     re += sv * zc;
     im -= sv * zs;
   }
+#pragma unroll
+  for (int o = VLS / 2; o > 0; o >>= 1) {
+    re += __shfl_xor_sync(0xffffffffu, re, o);
+    im += __shfl_xor_sync(0xffffffffu, im, o);
+  }
+  if (gq >= n5 || sub) return;
   zg[ijk5[g]] = make_double2(re, im);
   if (g > 0) {
     const int m1 = (k1n - k1 % k1n) % k1n, m2 = (k2n - k2 % k2n) % k2n, m3 = (k3n - k3 % k3n) % k3n;
@@ -87,17 +98,20 @@ void real_part(const double2 *z, double *out, long n, cudaStream_t st) {
 void vloc_g(int n5, int natom, const int *ijk5, const int *ngabc, const double *svco, const int *ityp,
             const double *dcq, const double *dsq, int km1, int km2, int km3, int ktot, double rvol, int k1, int k2,
             int k3, double2 *zg, cudaStream_t st) {
-  k_vloc_g<<<(n5 + 255) / 256, 256, 0, st>>>(n5, natom, ijk5, ngabc, svco, ityp, dcq, dsq, km1, km2, km3, ktot,
+  k_vloc_g<<<(unsigned)(((long)n5 * VLS + 255) / 256), 256, 0, st>>>(n5, natom, ijk5, ngabc, svco, ityp, dcq, dsq, km1, km2, km3, ktot,
                                              1.0 / rvol, k1, k2, k3, zg);
   note_launch();
 }
 
-// One block per atom: the three components of floc, G = 0 excluded.
+// Blocks (atom, slice of the half sphere): the three components of floc over
+// the slice, G = 0 excluded, in part[(slice * natom + atom) * 3 + dim]; the
+// slices are added in order by k_floc_sum.  One block an atom left a 64-atom
+// cell on 64 SMs: 197 us at Si64, gathers in flight being the bound.
 __global__ void __launch_bounds__(FT) k_floc(int n5, const int *__restrict__ ijk5, const int *__restrict__ ngabc,
                                              const double *__restrict__ gvec5, const double *__restrict__ svco,
                                              const int *__restrict__ ityp, const double2 *__restrict__ rhog,
                                              const double *__restrict__ dcq, const double *__restrict__ dsq,
-                                             int km1, int km2, int km3, int ktot, double *__restrict__ floc) {
+                                             int km1, int km2, int km3, int ktot, double *__restrict__ part) {
   __shared__ double red[FT / 32];
   const int a = blockIdx.x;
   const double *c1 = dcq + (long)a * ktot + km1, *s1 = dsq + (long)a * ktot + km1;
@@ -106,7 +120,7 @@ __global__ void __launch_bounds__(FT) k_floc(int n5, const int *__restrict__ ijk
                *s3 = dsq + (long)a * ktot + 2 * km1 + 2 * km2 + 2 + km3;
   const double *sv = svco + (long)ityp[a] * n5;
   double fx = 0.0, fy = 0.0, fz = 0.0;
-  for (int g = 1 + threadIdx.x; g < n5; g += FT) {
+  for (int g = 1 + blockIdx.y * FT + threadIdx.x; g < n5; g += FT * gridDim.y) {
     const int k1 = ngabc[3 * g], k2 = ngabc[3 * g + 1], k3 = ngabc[3 * g + 2];
     const double cc12 = c1[k1] * c2[k2] - s1[k1] * s2[k2];
     const double sc12 = s1[k1] * c2[k2] + c1[k1] * s2[k2];
@@ -122,11 +136,23 @@ __global__ void __launch_bounds__(FT) k_floc(int n5, const int *__restrict__ ijk
   fy = block_sum(fy, red);
   fz = block_sum(fz, red);
   if (threadIdx.x == 0) {
-    floc[3 * a] = 2.0 * fx;
-    floc[3 * a + 1] = 2.0 * fy;
-    floc[3 * a + 2] = 2.0 * fz;
+    double *o = part + ((long)blockIdx.y * gridDim.x + a) * 3;
+    o[0] = fx;
+    o[1] = fy;
+    o[2] = fz;
   }
 }
+
+__global__ void k_floc_sum(int n3, int slices, const double *__restrict__ part, double *__restrict__ floc) {
+  const int q = blockIdx.x * blockDim.x + threadIdx.x;
+  if (q >= n3) return;
+  double s = 0.0;
+  for (int i = 0; i < slices; ++i) s += part[(long)i * n3 + q];
+  floc[q] = 2.0 * s;
+}
+
+// Slices of the half sphere for natom atoms: about eight blocks a SM.
+int floc_slices(int natom) { return std::max(1, std::min(32, 8 * 148 / natom)); }
 
 // Derivative tables dtab[dim][j][.] from kbg[j][.] (both [nproj][nplwex]):
 // entries of G index g >= 1: d(2g) = -G_dim(g) beta(2g+1), d(2g+1) = G_dim(g) beta(2g); G = 0 gives 0.
@@ -178,8 +204,12 @@ void phase_tables(int natom, const double *satm, int km1, int km2, int km3, int 
 }
 void floc_g(int natom, int n5, const int *ijk5, const int *ngabc, const double *gvec5, const double *svco,
             const int *ityp, const double2 *rhog, const double *dcq, const double *dsq, int km1, int km2, int km3,
-            int ktot, double *floc, cudaStream_t st) {
-  k_floc<<<natom, FT, 0, st>>>(n5, ijk5, ngabc, gvec5, svco, ityp, rhog, dcq, dsq, km1, km2, km3, ktot, floc);
+            int ktot, double *part, double *floc, cudaStream_t st) {
+  const int ns = floc_slices(natom);
+  k_floc<<<dim3(natom, ns), FT, 0, st>>>(n5, ijk5, ngabc, gvec5, svco, ityp, rhog, dcq, dsq, km1, km2, km3, ktot,
+                                         part);
+  note_launch();
+  k_floc_sum<<<(3 * natom + 127) / 128, 128, 0, st>>>(3 * natom, ns, part, floc);
   note_launch();
 }
 template <typename T>

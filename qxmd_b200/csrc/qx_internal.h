@@ -186,7 +186,8 @@ void phase_tables(int natom, const double *satm, int km1, int km2, int km3, int 
                   cudaStream_t st);
 void floc_g(int natom, int n5, const int *ijk5, const int *ngabc, const double *gvec5, const double *svco,
             const int *ityp, const double2 *rhog, const double *dcq, const double *dsq, int km1, int km2, int km3,
-            int ktot, double *floc, cudaStream_t st);
+            int ktot, double *part, double *floc, cudaStream_t st);   // part: 3 * natom * floc_slices(natom)
+int floc_slices(int natom);
 void real_part(const double2 *z, double *out, long n, cudaStream_t st);
 void vloc_g(int n5, int natom, const int *ijk5, const int *ngabc, const double *svco, const int *ityp,
             const double *dcq, const double *dsq, int km1, int km2, int km3, int ktot, double rvol, int k1, int k2,
@@ -211,12 +212,14 @@ struct KbrGeom {
   int nd[3];       // box half-widths in grid points
 };
 void kbr_count(const KbrGeom &G, int natom, const int *ityp, const double *satm, const double *rcut, int *cnt,
-               int *off, cudaStream_t st);
+               int *soff, int *off, cudaStream_t st);
 template <typename T>
 void kbr_fill(const KbrGeom &G, int natom, int lmx, const int *ityp, const double *satm, const double *rcut,
               const double *rcl, const double *dltnl, const double *tabnl, const double *dtabnl, int mxnl,
-              const int *poly, const int *off, long cap, int *mesh, int *ptatom, T *vnl, T *dvnl, cudaStream_t st);
+              const int *poly, const int *soff, long cap, int *mesh, int *ptatom, T *vnl, T *dvnl, cudaStream_t st);
 int kbr_lines(const int *off, int natom, const int *mesh, const int *ptatom, int k1, long nlines, int *lcnt,
               int *loff, int *cursor, int4 *lent, cudaStream_t st);
 
 }  // namespace qx
+// Points of every (atom, z plane of its box) and their running offsets: cnt
+// (natom * w3), soff (natom * w3 + 1), off (natom + 1), w3 = 2 nd[2] + 1.

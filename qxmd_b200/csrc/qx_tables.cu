@@ -111,20 +111,64 @@ __device__ __forceinline__ int kbr_wrap(int n, int k) {
   return n < 0 ? n + k : n;
 }
 
-// Box point q of atom a: wrapped grid index and displacement r - R_a (bohr).
-__device__ __forceinline__ void kbr_point(const KbrGeom &G, const double *s, long q, int &mesh, double &dx,
-                                          double &dy, double &dz) {
-  const int w1 = 2 * G.nd[0] + 1, w2 = 2 * G.nd[1] + 1;
-  const int o1 = (int)(q % w1) - G.nd[0];
-  const int o2 = (int)((q / w1) % w2) - G.nd[1];
-  const int o3 = (int)(q / ((long)w1 * w2)) - G.nd[2];
-  const int n1 = (int)floor(s[0] * G.k[0] + 0.5) + o1, n2 = (int)floor(s[1] * G.k[1] + 0.5) + o2,
-            n3 = (int)floor(s[2] * G.k[2] + 0.5) + o3;
-  const double f1 = (double)n1 / G.k[0] - s[0], f2 = (double)n2 / G.k[1] - s[1], f3 = (double)n3 / G.k[2] - s[2];
+// The points of one (atom, z plane o3) of the search box.  The fractional
+// displacements f1, f2 and the wrapped indices of the plane's columns and
+// rows are formed once per block (they hold the divisions); a point then
+// costs the three displacement components.
+struct KbrPlane {
+  double *f1, *f2;   // shared: w1, w2
+  int *i1, *i2;      // shared: w1, w2 (i2 already times k1)
+  double f3;
+  int i3, w1, w2;    // i3 already times k1 * k2
+};
+constexpr int KBR_T = 256;
+
+__device__ __forceinline__ KbrPlane kbr_plane(const KbrGeom &G, const double *s, int q3, double *smem) {
+  KbrPlane B;
+  B.w1 = 2 * G.nd[0] + 1;
+  B.w2 = 2 * G.nd[1] + 1;
+  B.f1 = smem;
+  B.f2 = smem + B.w1;
+  B.i1 = reinterpret_cast<int *>(B.f2 + B.w2);
+  B.i2 = B.i1 + B.w1;
+  for (int q = threadIdx.x; q < B.w1 + B.w2; q += blockDim.x) {
+    const int d = q < B.w1 ? 0 : 1, o = (d ? q - B.w1 : q) - G.nd[d];
+    const int n = (int)floor(s[d] * G.k[d] + 0.5) + o;
+    const double f = (double)n / G.k[d] - s[d];
+    if (d == 0) {
+      B.f1[q] = f;
+      B.i1[q] = kbr_wrap(n, G.k[0]);
+    } else {
+      B.f2[q - B.w1] = f;
+      B.i2[q - B.w1] = G.k[0] * kbr_wrap(n, G.k[1]);
+    }
+  }
+  const int n3 = (int)floor(s[2] * G.k[2] + 0.5) + q3 - G.nd[2];
+  B.f3 = (double)n3 / G.k[2] - s[2];
+  B.i3 = G.k[0] * G.k[1] * kbr_wrap(n3, G.k[2]);
+  __syncthreads();
+  return B;
+}
+
+// Point q of the plane (x fastest): displacement r - R_a (bohr), grid index.
+__device__ __forceinline__ int kbr_point(const KbrGeom &G, const KbrPlane &B, int q, double &dx, double &dy,
+                                         double &dz) {
+  const int o2 = q / B.w1, o1 = q - o2 * B.w1;
+  const double f1 = B.f1[o1], f2 = B.f2[o2], f3 = B.f3;
   dx = G.rba[0] * f1 + G.rba[1] * f2 + G.rba[2] * f3;
   dy = G.rba[3] * f1 + G.rba[4] * f2 + G.rba[5] * f3;
   dz = G.rba[6] * f1 + G.rba[7] * f2 + G.rba[8] * f3;
-  mesh = kbr_wrap(n1, G.k[0]) + G.k[0] * (kbr_wrap(n2, G.k[1]) + G.k[1] * kbr_wrap(n3, G.k[2]));
+  return B.i1[o1] + B.i2[o2] + B.i3;
+}
+
+// Shared memory of a plane's columns and rows; boxes beyond the default
+// limit (more than 4096 columns and rows) opt in (at most 117 KB: no axis is
+// longer than 4900).
+template <typename K>
+static size_t kbr_smem(const KbrGeom &G, K *kernel) {
+  const size_t sm = (sizeof(double) + sizeof(int)) * (size_t)(2 * G.nd[0] + 1 + 2 * G.nd[1] + 1);
+  if (sm > 48 * 1024) cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+  return sm;
 }
 
 // real solid-harmonic polynomials of degree <= 2 (normalisation in the table)
@@ -142,17 +186,20 @@ __device__ __forceinline__ double kbr_poly(int c, double x, double y, double z) 
   }
 }
 
-__global__ void k_kbr_count(KbrGeom G, const int *__restrict__ ityp, const double *__restrict__ satm,
-                            const double *__restrict__ rcut, int *__restrict__ cnt) {
-  const int a = blockIdx.x;
-  const double *s = satm + 3 * a;
+// One block per (z plane of the box, atom).  The search is arithmetic on
+// registers, so the number of busy SMs bounds it: one block an atom kept a
+// 64-atom cell on 64 SMs (count 49 us, fill 198 us at Si64).
+__global__ void __launch_bounds__(KBR_T) k_kbr_count(KbrGeom G, const int *__restrict__ ityp,
+                                                     const double *__restrict__ satm,
+                                                     const double *__restrict__ rcut, int *__restrict__ cnt) {
+  extern __shared__ double kbr_sm[];
+  const int a = blockIdx.y;
+  const KbrPlane B = kbr_plane(G, satm + 3 * a, blockIdx.x, kbr_sm);
   const double rc2 = rcut[ityp[a]] * rcut[ityp[a]];
-  const long nbox = (long)(2 * G.nd[0] + 1) * (2 * G.nd[1] + 1) * (2 * G.nd[2] + 1);
   int c = 0;
-  for (long q = threadIdx.x; q < nbox; q += blockDim.x) {
-    int m;
+  for (int q = threadIdx.x; q < B.w1 * B.w2; q += blockDim.x) {
     double dx, dy, dz;
-    kbr_point(G, s, q, m, dx, dy, dz);
+    kbr_point(G, B, q, dx, dy, dz);
     c += (dx * dx + dy * dy + dz * dz <= rc2) ? 1 : 0;
   }
   __shared__ int red[32];
@@ -162,8 +209,14 @@ __global__ void k_kbr_count(KbrGeom G, const int *__restrict__ ityp, const doubl
   if (threadIdx.x == 0) {
     int t = 0;
     for (int w = 0; w < (int)(blockDim.x >> 5); ++w) t += red[w];
-    cnt[a] = t;
+    cnt[(long)a * gridDim.x + blockIdx.x] = t;
   }
+}
+
+// off[a] = soff[a * w3]: the atoms' offsets from the planes'.
+__global__ void k_kbr_off(int natom, int w3, const int *__restrict__ soff, int *__restrict__ off) {
+  const int a = blockIdx.x * blockDim.x + threadIdx.x;
+  if (a <= natom) off[a] = soff[(long)a * w3];
 }
 
 // Exclusive scan of n counts by one block of 1024 threads: out[0..n],
@@ -223,30 +276,30 @@ __device__ __forceinline__ double kbr_interp(const double *tb, int mm, double d)
 // gradient, at the points beyond its own channel's radius, so each channel
 // sums over exactly the points of its own list in setnlc.
 template <typename T>
-__global__ void k_kbr_fill(KbrGeom G, int lmx, const int *__restrict__ ityp, const double *__restrict__ satm,
+__global__ void __launch_bounds__(KBR_T) k_kbr_fill(KbrGeom G, int lmx, const int *__restrict__ ityp, const double *__restrict__ satm,
                            const double *__restrict__ rcut, const double *__restrict__ rcl,
                            const double *__restrict__ dltnl,
                            const double *__restrict__ tabnl, const double *__restrict__ dtabnl, int mxnl,
-                           const int *__restrict__ poly, const int *__restrict__ off, int natom, long cap,
+                           const int *__restrict__ poly, const int *__restrict__ soff, int natom, long cap,
                            int *__restrict__ mesh, int *__restrict__ ptatom, T *__restrict__ vnl,
                            T *__restrict__ dvnl) {
-  if (off[natom] > cap) return;   // the host grows the buffers and launches again
-  const int a = blockIdx.x, it = ityp[a];
-  const double *s = satm + 3 * a;
+  if (soff[(long)natom * gridDim.x] > cap) return;   // the host grows the buffers and launches again
+  extern __shared__ double kbr_sm[];
+  const int a = blockIdx.y, it = ityp[a];
+  const long slab = (long)a * gridDim.x + blockIdx.x;
+  const KbrPlane B = kbr_plane(G, satm + 3 * a, blockIdx.x, kbr_sm);
   const double rc2 = rcut[it] * rcut[it], dl = dltnl[it];
-  const long nbox = (long)(2 * G.nd[0] + 1) * (2 * G.nd[1] + 1) * (2 * G.nd[2] + 1);
+  const int nbox = B.w1 * B.w2, iend = soff[slab + 1];
   __shared__ int wsum[32];
-  __shared__ int base;
-  if (threadIdx.x == 0) base = off[a];
-  __syncthreads();
+  int base = soff[slab];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
-  for (long q0 = 0; q0 < nbox; q0 += blockDim.x) {
-    const long q = q0 + threadIdx.x;
+  for (int q0 = 0; q0 < nbox; q0 += blockDim.x) {
+    const int q = q0 + threadIdx.x;
     int m = 0;
     double dx = 0, dy = 0, dz = 0;
     bool in = false;
     if (q < nbox) {
-      kbr_point(G, s, q, m, dx, dy, dz);
+      m = kbr_point(G, B, q, dx, dy, dz);
       in = dx * dx + dy * dy + dz * dz <= rc2;
     }
     const unsigned bal = __ballot_sync(0xffffffffu, in);
@@ -258,7 +311,7 @@ __global__ void k_kbr_fill(KbrGeom G, int lmx, const int *__restrict__ ityp, con
       tot += wsum[w];
     }
     const long i = base + wo + __popc(bal & ((1u << lane) - 1u));
-    if (in && i < off[a + 1]) {
+    if (in && i < iend) {
       mesh[i] = m;
       ptatom[i] = a;
       const double r = sqrt(dx * dx + dy * dy + dz * dz);
@@ -281,9 +334,8 @@ __global__ void k_kbr_fill(KbrGeom G, int lmx, const int *__restrict__ ityp, con
         }
       }
     }
-    __syncthreads();
-    if (threadIdx.x == 0) base += tot;
-    __syncthreads();
+    base += tot;
+    __syncthreads();   // wsum is rewritten in the next round
   }
 }
 
@@ -341,19 +393,23 @@ __global__ void __launch_bounds__(128) k_kbr_line_sort(const int *__restrict__ l
 }
 
 void kbr_count(const KbrGeom &G, int natom, const int *ityp, const double *satm, const double *rcut, int *cnt,
-               int *off, cudaStream_t st) {
-  k_kbr_count<<<natom, 256, 0, st>>>(G, ityp, satm, rcut, cnt);
+               int *soff, int *off, cudaStream_t st) {
+  const int w3 = 2 * G.nd[2] + 1;
+  k_kbr_count<<<dim3(w3, natom), KBR_T, kbr_smem(G, k_kbr_count), st>>>(G, ityp, satm, rcut, cnt);
   note_launch();
-  k_scan1<<<1, 1024, 0, st>>>(cnt, natom, off, nullptr);
+  k_scan1<<<1, 1024, 0, st>>>(cnt, (long)natom * w3, soff, nullptr);
+  note_launch();
+  k_kbr_off<<<(natom + 1 + 255) / 256, 256, 0, st>>>(natom, w3, soff, off);
   note_launch();
 }
 
 template <typename T>
 void kbr_fill(const KbrGeom &G, int natom, int lmx, const int *ityp, const double *satm, const double *rcut,
               const double *rcl, const double *dltnl, const double *tabnl, const double *dtabnl, int mxnl,
-              const int *poly, const int *off, long cap, int *mesh, int *ptatom, T *vnl, T *dvnl, cudaStream_t st) {
-  k_kbr_fill<T><<<natom, 256, 0, st>>>(G, lmx, ityp, satm, rcut, rcl, dltnl, tabnl, dtabnl, mxnl, poly, off, natom,
-                                       cap, mesh, ptatom, vnl, dtabnl ? dvnl : nullptr);
+              const int *poly, const int *soff, long cap, int *mesh, int *ptatom, T *vnl, T *dvnl, cudaStream_t st) {
+  k_kbr_fill<T><<<dim3(2 * G.nd[2] + 1, natom), KBR_T, kbr_smem(G, k_kbr_fill<T>), st>>>(
+      G, lmx, ityp, satm, rcut, rcl, dltnl, tabnl, dtabnl, mxnl, poly, soff, natom, cap, mesh, ptatom, vnl,
+      dtabnl ? dvnl : nullptr);
   note_launch();
 }
 template void kbr_fill<float>(const KbrGeom &, int, int, const int *, const double *, const double *, const double *,
