@@ -1072,13 +1072,13 @@ extern "C" int qx_build_kb_r(qx_ctx *c, int natom, const int *ityp, const double
     c->kbr_natom = natom;
     moved = true;
   }
-  if (!c->d_kbr_loff) {
   const long slabs = (long)natom * (2 * c->kbr_geom.nd[2] + 1);
   if (slabs != c->kbr_slabs) {
     TRY(dregrow(c, &c->d_kbr_cnt, sizeof(int) * slabs));
     TRY(dregrow(c, &c->d_kbr_soff, sizeof(int) * (slabs + 1)));
     c->kbr_slabs = slabs;
   }
+  if (!c->d_kbr_loff) {
     TRY(dalloc(c, &c->d_kbr_lcnt, sizeof(int) * nlines));
     TRY(dalloc(c, &c->d_kbr_loff, sizeof(int) * (nlines + 1)));
     TRY(dalloc(c, &c->d_kbr_cursor, sizeof(int) * nlines));

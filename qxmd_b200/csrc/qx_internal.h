@@ -211,6 +211,8 @@ struct KbrGeom {
   int k[3];        // FFT grid
   int nd[3];       // box half-widths in grid points
 };
+// Points of every (atom, z plane of its box) and their running offsets: cnt
+// (natom * w3), soff (natom * w3 + 1), off (natom + 1), w3 = 2 nd[2] + 1.
 void kbr_count(const KbrGeom &G, int natom, const int *ityp, const double *satm, const double *rcut, int *cnt,
                int *soff, int *off, cudaStream_t st);
 template <typename T>
@@ -221,5 +223,3 @@ int kbr_lines(const int *off, int natom, const int *mesh, const int *ptatom, int
               int *loff, int *cursor, int4 *lent, cudaStream_t st);
 
 }  // namespace qx
-// Points of every (atom, z plane of its box) and their running offsets: cnt
-// (natom * w3), soff (natom * w3 + 1), off (natom + 1), w3 = 2 nd[2] + 1.
