@@ -165,6 +165,8 @@ struct qx_ctx {
       *d_kbr_mesh = nullptr, *d_kbr_ptatom = nullptr, *d_kbr_lcnt = nullptr, *d_kbr_loff = nullptr,
       *d_kbr_cursor = nullptr;
   int4 *d_kbr_lent = nullptr;
+  int *d_kbr_ptoff = nullptr;
+  int2 *d_kbr_ptent = nullptr;
   void *d_kbr_vnl = nullptr, *d_kbr_sumr = nullptr, *d_kbr_bufR = nullptr;
   double *d_kbr_rcl = nullptr;    // radius of each projector's channel (lmx * ntype)
   std::vector<double> kbr_rcut_h; // species radii (the largest channel's)
@@ -912,25 +914,24 @@ extern "C" int qx_set_kb_r(qx_ctx *c, int natom, int lmx, const int *off, const 
     if (off[a + 1] < off[a]) { set_error("qx_set_kb_r: off not ascending"); return QX_ERR_ARG; }
   for (int i = 0; i < npts; ++i)
     if (mesh[i] < 0 || mesh[i] >= pl.n) { set_error("qx_set_kb_r: mesh index out of range"); return QX_ERR_ARG; }
-  // line CSR: the projector points that fall on each x line (i3*k2 + i2)
-  const long nlines = (long)pl.k2 * pl.k3;
-  std::vector<int> loff(nlines + 1, 0);
-  for (int i = 0; i < npts; ++i) loff[mesh[i] / pl.k1 + 1]++;
-  for (long l = 0; l < nlines; ++l) loff[l + 1] += loff[l];
-  std::vector<int4> lent(std::max(npts, 1));
-  std::vector<int> fill(loff.begin(), loff.end() - 1);
+  // the projector points at each grid point, in point order
+  std::vector<int> poff(pl.n + 1, 0);
+  for (int i = 0; i < npts; ++i) poff[mesh[i] + 1]++;
+  for (long g = 0; g < pl.n; ++g) poff[g + 1] += poff[g];
+  std::vector<int2> pent(std::max(npts, 1));
+  std::vector<int> fill(poff.begin(), poff.end() - 1);
   for (int a = 0; a < natom; ++a)
-    for (int i = off[a]; i < off[a + 1]; ++i) lent[fill[mesh[i] / pl.k1]++] = make_int4(mesh[i] % pl.k1, i, a, 0);
+    for (int i = off[a]; i < off[a + 1]; ++i) pent[fill[mesh[i]]++] = make_int2(i, a);
   TRY(dalloc(c, &pl.d_kb_off, sizeof(int) * (natom + 1)));
   TRY(dalloc(c, &pl.d_kb_mesh, sizeof(int) * std::max(npts, 1)));
   TRY(dalloc(c, &pl.d_kb_clalp, sizeof(double) * lmx));
-  TRY(dalloc(c, &pl.d_line_off, sizeof(int) * (nlines + 1)));
-  TRY(dalloc(c, &pl.d_line_ent, sizeof(int4) * lent.size()));
+  TRY(dalloc(c, &pl.d_pt_off, sizeof(int) * poff.size()));
+  TRY(dalloc(c, &pl.d_pt_ent, sizeof(int2) * pent.size()));
   CK(cudaMemcpy(pl.d_kb_off, off, sizeof(int) * (natom + 1), cudaMemcpyHostToDevice));
   CK(cudaMemcpy(pl.d_kb_mesh, mesh, sizeof(int) * npts, cudaMemcpyHostToDevice));
   CK(cudaMemcpy(pl.d_kb_clalp, clalp, sizeof(double) * lmx, cudaMemcpyHostToDevice));
-  CK(cudaMemcpy(pl.d_line_off, loff.data(), sizeof(int) * (nlines + 1), cudaMemcpyHostToDevice));
-  CK(cudaMemcpy(pl.d_line_ent, lent.data(), sizeof(int4) * lent.size(), cudaMemcpyHostToDevice));
+  CK(cudaMemcpy(pl.d_pt_off, poff.data(), sizeof(int) * poff.size(), cudaMemcpyHostToDevice));
+  CK(cudaMemcpy(pl.d_pt_ent, pent.data(), sizeof(int2) * pent.size(), cudaMemcpyHostToDevice));
   void *v = nullptr;
   TRY(dalloc(c, &v, c->tsize() * (size_t)npts * lmx));
   TRY(up(c, v, vnl, (long)npts * lmx));
@@ -1082,6 +1083,7 @@ extern "C" int qx_build_kb_r(qx_ctx *c, int natom, const int *ityp, const double
     TRY(dalloc(c, &c->d_kbr_lcnt, sizeof(int) * nlines));
     TRY(dalloc(c, &c->d_kbr_loff, sizeof(int) * (nlines + 1)));
     TRY(dalloc(c, &c->d_kbr_cursor, sizeof(int) * nlines));
+    TRY(dalloc(c, &c->d_kbr_ptoff, sizeof(int) * (pl.n + 1)));
     TRY(dalloc(c, &c->d_kbr_bufR, 2 * ts * (size_t)pl.chunk * pl.n));
     moved = true;
   }
@@ -1098,6 +1100,7 @@ extern "C" int qx_build_kb_r(qx_ctx *c, int natom, const int *ityp, const double
     TRY(dregrow(c, &c->d_kbr_mesh, sizeof(int) * cap));
     TRY(dregrow(c, &c->d_kbr_ptatom, sizeof(int) * cap));
     TRY(dregrow(c, &c->d_kbr_lent, sizeof(int4) * cap));
+    TRY(dregrow(c, &c->d_kbr_ptent, sizeof(int2) * cap));
     TRY(dregrow(c, &c->d_kbr_vnl, ts * c->kbr_lmx * (size_t)cap));
     c->kbr_cap = cap;
     moved = true;
@@ -1115,18 +1118,18 @@ extern "C" int qx_build_kb_r(qx_ctx *c, int natom, const int *ityp, const double
                     c->d_kbr_dtab, c->kbr_mxnl, c->d_kbr_poly, c->d_kbr_soff, c->kbr_cap, c->d_kbr_mesh,
                     c->d_kbr_ptatom, (float *)c->d_kbr_vnl, (float *)c->d_kbr_dvnl, c->st);
   if (kbr_lines(c->d_kbr_off, natom, c->d_kbr_mesh, c->d_kbr_ptatom, pl.k1, nlines, c->d_kbr_lcnt, c->d_kbr_loff,
-                c->d_kbr_cursor, c->d_kbr_lent, c->st)) {
+                c->d_kbr_cursor, c->d_kbr_lent, c->d_kbr_ptoff, c->d_kbr_ptent, c->st)) {
     set_error("qx_build_kb_r: memset failed");
     return QX_ERR_CUDA;
   }
   CKL();
-  if (pl.d_kb_off != c->d_kbr_off || pl.d_kb_mesh != c->d_kbr_mesh || pl.d_line_off != c->d_kbr_loff ||
-      pl.d_line_ent != c->d_kbr_lent)
+  if (pl.d_kb_off != c->d_kbr_off || pl.d_kb_mesh != c->d_kbr_mesh || pl.d_pt_off != c->d_kbr_ptoff ||
+      pl.d_pt_ent != c->d_kbr_ptent)
     moved = true;
   pl.d_kb_off = c->d_kbr_off;
   pl.d_kb_mesh = c->d_kbr_mesh;
-  pl.d_line_off = c->d_kbr_loff;
-  pl.d_line_ent = c->d_kbr_lent;
+  pl.d_pt_off = c->d_kbr_ptoff;
+  pl.d_pt_ent = c->d_kbr_ptent;
   if (c->prec == QX_PREC_FP64) {
     moved |= pl.b64.kb_vnl != (double *)c->d_kbr_vnl || pl.b64.sumr != (double2 *)c->d_kbr_sumr;
     pl.b64.kb_vnl = (double *)c->d_kbr_vnl;

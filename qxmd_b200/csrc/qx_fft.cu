@@ -22,6 +22,7 @@
 #include <cstdlib>
 
 #include <mutex>
+#include <type_traits>
 
 #include "qx_internal.h"
 
@@ -475,83 +476,129 @@ __global__ void __launch_bounds__(QX_THREADS) k_xinv_r(PipeParams P, const typen
   }
 }
 
-// Real-space KB force of one (atom, band pair) (fnnlcl2, nlkbppr.f90:2024-3120):
-// for each band b of the pair, P_l = rdelv sum_points vnl_l psi_b and
-// D_l = rdelv sum_points grad vnl_l psi_b (gradient with respect to the
-// point), then F_a += 2 occ_b / Omega sum_l clalp_l P_l D_l; one partial per
-// pair in fpart[(pair * natom + atom) * 3 + dim] (summed over pairs in a
-// fixed order afterwards).  wocc = occ / Omega.  lmx <= ML projectors per
-// point (ML = 4: s, p; ML = 9: s, p, d).
-template <typename T, int ML>
-__global__ void __launch_bounds__(QX_THREADS) k_fnl_r(PipeParams P, const typename c2t<T>::type *__restrict__ R,
+// Sums over an atom's projector points as FP64 tensor-core contractions
+// (mma m8n8k4): D(row, band) = sum_points tab(row, point) psi_band(point).  A
+// CTA takes one atom and NT * 8 bands; its warps take the points four at a
+// time in turn, UN of them in flight, straight from global memory (a lane's
+// fragment element is one table value or one component of psi at a point),
+// and their sums are added in warp order.  Rows 0 .. lmx - 1 are the
+// projector values; with FORCE the rows lmx + 3 l + d are their gradients.
+//   FORCE = false: sumr(l, atom) = rdelv clalp_l D(l, band), the projections
+//     of calnlc;
+//   FORCE = true: the real-space KB force partials (fnnlcl2,
+//     nlkbppr.f90:2024-3120) of each band pair, F = sum_b 2 occ_b / Omega
+//     rdelv^2 sum_l clalp_l P_l D_l in fpart[(pair * natom + atom) * 3 + dim]
+//     (added over pairs in a fixed order afterwards); wocc = occ / Omega.
+// The gathers of psi (32-byte sectors of L2) bound it.  One thread per point
+// and pair, as before, was bound by FP32 to FP64 conversions and by re-reading
+// the table for every pair; at Si64, 160 bands: projections 133 -> 98 us,
+// forces 506 -> 228 us.
+template <typename T, int MT, int NT, bool FORCE>
+__global__ void __launch_bounds__(QX_THREADS) k_ptsum(PipeParams P, const typename c2t<T>::type *__restrict__ R,
                                                        const int *__restrict__ off, const int *__restrict__ mesh,
                                                        const T *__restrict__ vnl, const T *__restrict__ dvnl,
                                                        const double *__restrict__ clalp, double rdelv, int natom,
-                                                       int lmx, const double *__restrict__ wocc, int npl, int ppb,
+                                                       int lmx, int npl, const double *__restrict__ wocc,
+                                                       typename c2t<T>::type *__restrict__ sumr,
                                                        double *__restrict__ fpart) {
-  typedef typename c2t<T>::type C;
-  constexpr int NQ = 8 * ML;   // P[band][l] (2 ML), then D[band][l][dim] (6 ML)
-  const int at = blockIdx.x;
-  // ppb pairs of the chunk per block, one after another, so that the atom's
-  // table slice is read from cache after the first
-  const int pend = min(npl, (int)(blockIdx.y + 1) * ppb);
-  for (int pl = blockIdx.y * ppb; pl < pend; ++pl) {
-  const int p = P.pair0 + pl;
-  if (p >= pair_count(P)) break;   // uniform across the block
+  constexpr int NW = QX_THREADS / 32, UN = MT * NT <= 8 ? 4 : 2;
+  const int at = blockIdx.x, pg = blockIdx.y * (NT * 4);   // first pair of the CTA
+  const int np = min(npl, pair_count(P) - P.pair0);
+  if (pg >= np) return;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int row = lane >> 2, kk = lane & 3;                // fragment row (band) and point of this lane
+  const int rows = FORCE ? 4 * lmx : lmx;
   const long n = (long)P.k1 * P.k2 * P.k3;
-  const C *Rp = R + (long)pl * n;
-  double acc[NQ];
+  const int p0 = off[at], cnt = off[at + 1] - p0;
+  double acc[MT][NT][2];
 #pragma unroll
-  for (int q = 0; q < NQ; ++q) acc[q] = 0.0;
-  for (int mm = off[at] + threadIdx.x; mm < off[at + 1]; mm += blockDim.x) {
-    const C z = Rp[mesh[mm]];
+  for (int m = 0; m < MT; ++m)
 #pragma unroll
-    for (int l = 0; l < ML; ++l) {
-      if (l >= lmx) break;   // uniform
-      const double v = (double)vnl[(long)mm * lmx + l];
-      acc[l] += v * (double)z.x;
-      acc[ML + l] += v * (double)z.y;
+    for (int q = 0; q < NT; ++q) acc[m][q][0] = acc[m][q][1] = 0.0;
+  // band nt * 8 + row: pair pg + 4 nt + row / 2, component row & 1 (clamped address, zeroed past the last pair)
+  const T *Rb[NT];
+  bool bon[NT];
 #pragma unroll
-      for (int d = 0; d < 3; ++d) {
-        const double g = (double)dvnl[((long)mm * lmx + l) * 3 + d];
-        acc[2 * ML + l * 3 + d] += g * (double)z.x;
-        acc[5 * ML + l * 3 + d] += g * (double)z.y;
+  for (int q = 0; q < NT; ++q) {
+    const int pl = pg + 4 * q + (row >> 1);
+    bon[q] = pl < np;
+    Rb[q] = reinterpret_cast<const T *>(R + (long)min(pl, np - 1) * n) + (row & 1);
+  }
+  for (int k0 = 4 * warp; k0 < cnt; k0 += 4 * NW * UN) {
+    T av[UN][MT], bv[UN][NT];
+#pragma unroll
+    for (int u = 0; u < UN; ++u) {
+      const int k = k0 + 4 * NW * u + kk;
+      const bool on = k < cnt;
+      const long pt = p0 + min(k, cnt - 1);
+      const long m = mesh[pt];
+#pragma unroll
+      for (int i = 0; i < MT; ++i) {
+        const int r = i * 8 + row;
+        T v = 0;
+        if (on && r < rows) v = (!FORCE || r < lmx) ? vnl[pt * lmx + r] : dvnl[pt * 3 * lmx + (r - lmx)];
+        av[u][i] = v;
+      }
+#pragma unroll
+      for (int q = 0; q < NT; ++q) {
+        const T v = Rb[q][2 * m];
+        bv[u][q] = (on && bon[q]) ? v : (T)0;
       }
     }
-  }
-  // the NQ sums: warp shuffles, then one pass over the warps' partials
-  __shared__ double red[QX_THREADS / 32][NQ];
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
 #pragma unroll
-  for (int q = 0; q < NQ; ++q) {
-    double v = acc[q];
+    for (int u = 0; u < UN; ++u)
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-    if (lane == 0) red[warp][q] = v;
+      for (int i = 0; i < MT; ++i)
+#pragma unroll
+        for (int q = 0; q < NT; ++q) {
+          const double a = (double)av[u][i], b = (double)bv[u][q];
+          asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1}, {%2}, {%3}, {%0,%1};\n"
+                       : "+d"(acc[i][q][0]), "+d"(acc[i][q][1])
+                       : "d"(a), "d"(b));
+        }
   }
+  // D(row, band) of every warp, added in warp order
+  constexpr int NQ = MT * 8 * NT * 8;
+  __shared__ double red[NW][NQ];
+#pragma unroll
+  for (int i = 0; i < MT; ++i)
+#pragma unroll
+    for (int q = 0; q < NT; ++q) {
+      double *d = &red[warp][(i * 8 + row) * (NT * 8) + q * 8 + 2 * kk];
+      d[0] = acc[i][q][0];
+      d[1] = acc[i][q][1];
+    }
   __syncthreads();
-  for (int q = threadIdx.x; q < NQ; q += blockDim.x) {
+  for (int q = threadIdx.x; q < NQ; q += QX_THREADS) {
     double v = 0.0;
-    for (int w = 0; w < (int)(blockDim.x >> 5); ++w) v += red[w][q];
+#pragma unroll
+    for (int w = 0; w < NW; ++w) v += red[w][q];
     red[0][q] = v;
   }
   __syncthreads();
-  if (threadIdx.x == 0) {
-    const double *s = red[0];
-    const int b[2] = {P.pairs[2 * p], P.pairs[2 * p + 1]};
-    double f[3] = {0.0, 0.0, 0.0};
-    for (int h = 0; h < 2; ++h) {
-      if (b[h] < 0) continue;
-      const double w = 2.0 * wocc[b[h]] * rdelv * rdelv;
-      for (int l = 0; l < lmx; ++l)
-        for (int d = 0; d < 3; ++d) f[d] += w * clalp[l] * s[h * ML + l] * s[2 * ML + 3 * ML * h + l * 3 + d];
+  const double *s = red[0];
+  if constexpr (!FORCE) {
+    for (int q = threadIdx.x; q < lmx * NT * 4; q += QX_THREADS) {
+      const int l = q / (NT * 4), pl = q - l * (NT * 4);
+      if (pg + pl >= np) continue;
+      const double f = rdelv * clalp[l];
+      const double *d = s + l * (NT * 8) + 2 * pl;
+      sumr[((long)(pg + pl) * natom + at) * lmx + l] = mk2<T>((T)(d[0] * f), (T)(d[1] * f));
     }
-    double *o = fpart + ((long)p * natom + at) * 3;
-    o[0] = f[0];
-    o[1] = f[1];
-    o[2] = f[2];
-  }
-  __syncthreads();
+  } else {
+    for (int q = threadIdx.x; q < 3 * NT * 4; q += QX_THREADS) {
+      const int pl = q / 3, d = q - 3 * pl, p = P.pair0 + pg + pl;
+      if (pg + pl >= np) continue;
+      double f = 0.0;
+      for (int h = 0; h < 2; ++h) {
+        const int b = P.pairs[2 * p + h];
+        if (b < 0) continue;
+        const double w = 2.0 * wocc[b] * rdelv * rdelv;
+        const double *x = s + 2 * pl + h;
+        for (int l = 0; l < lmx; ++l) f += w * clalp[l] * x[l * (NT * 8)] * x[(lmx + 3 * l + d) * (NT * 8)];
+      }
+      fpart[((long)p * natom + at) * 3 + d] = f;
+    }
   }
 }
 
@@ -564,101 +611,52 @@ __global__ void k_fnl_r_sum(const double *__restrict__ fpart, int npair, int nat
   fnl[q] = s;
 }
 
-// sumr(l, atom) = rdelv * clalp_l * sum_points vnl_l * psi(point), both bands
-// of the pair at once (real part band A, imaginary part band B); lmx <= ML
-// projectors per point.
-template <typename T, int ML>
-__global__ void __launch_bounds__(QX_THREADS) k_nlproj(PipeParams P, const typename c2t<T>::type *__restrict__ R,
-                                                        const int *__restrict__ off, const int *__restrict__ mesh,
-                                                        const T *__restrict__ vnl, const double *__restrict__ clalp,
-                                                        double rdelv, int natom, int lmx,
-                                                        typename c2t<T>::type *__restrict__ sumr) {
-  typedef typename c2t<T>::type C;
-  const int at = blockIdx.x;
-  const int pl = blockIdx.y, p = P.pair0 + pl;
-  if (p >= pair_count(P)) return;
-  const long n = (long)P.k1 * P.k2 * P.k3;
-  const C *Rp = R + (long)pl * n;
-  double acc[2 * ML];
-#pragma unroll
-  for (int q = 0; q < 2 * ML; ++q) acc[q] = 0.0;
-  for (int mm = off[at] + threadIdx.x; mm < off[at + 1]; mm += blockDim.x) {
-    const C z = Rp[mesh[mm]];
-#pragma unroll
-    for (int l = 0; l < ML; ++l) {
-      if (l >= lmx) break;   // uniform
-      const double v = (double)vnl[(long)mm * lmx + l];
-      acc[2 * l] += v * (double)z.x;
-      acc[2 * l + 1] += v * (double)z.y;
-    }
-  }
-  __shared__ double red[QX_THREADS / 32];
-  for (int l = 0; l < 2 * lmx; ++l) {
-    const double s = block_sum(acc[l], red);
-    if (threadIdx.x == 0) acc[l] = s;
-  }
-  if (threadIdx.x == 0) {
-    C *o = sumr + ((long)pl * natom + at) * lmx;
-    for (int l = 0; l < lmx; ++l) {
-      const double f = rdelv * clalp[l];
-      o[l] = mk2<T>((T)(acc[2 * l] * f), (T)(acc[2 * l + 1] * f));
-    }
-  }
-}
-
 // Forward x pass for the real-space KB mode: V*psi + sum vnl*sumr, forward
-// x-FFT, keep the pruned part.  Line CSR `loff/lent` lists the projector
-// points of each line (i3*k2 + i2): {i1, point index, atom}.
-template <typename T, int ML>
+// x-FFT, keep the pruned part.  A thread adds the projector points of its own
+// grid points (NlPoints) in a fixed order.
+template <typename T>
 __global__ void __launch_bounds__(QX_THREADS) k_xfwd_r(PipeParams P, const typename c2t<T>::type *__restrict__ R,
                                                         typename c2t<T>::type *__restrict__ bufB,
-                                                        const T *__restrict__ vloc, const int *__restrict__ loff,
-                                                        const int4 *__restrict__ lent, const T *__restrict__ vnl,
-                                                        const typename c2t<T>::type *__restrict__ sumr, int natom,
-                                                        int lmx, int nlines, int nchunk,
-                                                        FftTabs<T> gt1) {
+                                                        const T *__restrict__ vloc, qx::NlPoints<T> nl, int nlines,
+                                                        int nchunk, FftTabs<T> gt1) {
   typedef typename c2t<T>::type C;
   const int i3 = blockIdx.x / nchunk, ch = blockIdx.x - i3 * nchunk;
   const int pl = blockIdx.y, p = P.pair0 + pl;
   if (p >= pair_count(P)) return;
   const int k1 = P.k1, k2 = P.k2, P1 = P.P1;
-  const int i20 = ch * nlines, nl = min(nlines, k2 - i20), ld = nl | 1;
+  const int i20 = ch * nlines, nln = min(nlines, k2 - i20), ld = nln | 1;
   extern __shared__ unsigned char smraw[];
   SmTabs<T> tb = load_tabs<T>(smraw, P.L1, gt1);
   C *t0 = tb.tiles;
   C *t1 = t0 + k1 * ld;
   const C *src = R + (((long)pl * P.k3 + i3) * k2 + i20) * k1;
-  const T *V = vloc + ((long)i3 * k2 + i20) * k1;
-  for (int i = threadIdx.x; i < nl * k1; i += blockDim.x) {
+  const long g0 = ((long)i3 * k2 + i20) * k1;
+  const T *V = vloc + g0;
+  const C *S = nl.sumr + (long)pl * nl.natom * nl.lmx;
+  for (int i = threadIdx.x; i < nln * k1; i += blockDim.x) {
     const int l = i / k1, i1 = i - l * k1;
+    const int e0 = nl.off[g0 + i], e1 = nl.off[g0 + i + 1];
     C z = src[i];
     const T v = V[i];
     z.x *= v; z.y *= v;
+    for (int e = e0; e < e1; ++e) {
+      const int2 en = nl.ent[e];
+      const C *s = S + (long)en.y * nl.lmx;
+      const T *w = nl.vnl + (long)en.x * nl.lmx;
+      T ar = 0, ai = 0;
+      for (int q = 0; q < nl.lmx; ++q) {
+        ar += w[q] * s[q].x;
+        ai += w[q] * s[q].y;
+      }
+      z.x += ar;
+      z.y += ai;
+    }
     t0[i1 * ld + l] = z;
   }
   __syncthreads();
-  const C *S = sumr + (long)pl * natom * lmx;
-  const int line0 = i3 * k2 + i20;
-  for (int l = 0; l < nl; ++l) {
-    for (int e = loff[line0 + l] + threadIdx.x; e < loff[line0 + l + 1]; e += blockDim.x) {
-      const int4 en = lent[e];
-      const C *s = S + (long)en.z * lmx;
-      const T *v = vnl + (long)en.y * lmx;
-      T ar = 0, ai = 0;
-#pragma unroll
-      for (int q = 0; q < ML; ++q) {
-        if (q >= lmx) break;   // uniform
-        ar += v[q] * s[q].x;
-        ai += v[q] * s[q].y;
-      }
-      atomicAdd(&t0[en.x * ld + l].x, ar);
-      atomicAdd(&t0[en.x * ld + l].y, ai);
-    }
-  }
-  __syncthreads();
-  C *res = smem_fft<T, -1>(t0, t1, nl, ld, P.L1, tb.tw, tb.stw, tb.sob);
+  C *res = smem_fft<T, -1>(t0, t1, nln, ld, P.L1, tb.tw, tb.stw, tb.sob);
   C *B = bufB + (((long)pl * P.k3 + i3) * k2 + i20) * P1;
-  for (int i = threadIdx.x; i < nl * P1; i += blockDim.x) {
+  for (int i = threadIdx.x; i < nln * P1; i += blockDim.x) {
     const int l = i / P1, a = i - l * P1;
     B[i] = res[a_to_i1(a, P.m1, k1) * ld + l];
   }
@@ -821,6 +819,33 @@ static bool zcols_fwd_enabled(int k3) {
   return k3 <= 32;
 }
 
+// The projections of the chunk's pairs on every atom's projectors.  16 bands
+// a CTA where that fills the GPU, 8 otherwise.
+template <typename T, bool FORCE>
+static void launch_ptsum(const Plan &pl, const PipeParams &P, int npl, const T *dvnl, const double *wocc,
+                         double *fpart, cudaStream_t st) {
+  Bufs<T> &bf = pl.bufs<T>();
+  auto go = [&](auto mt, auto nt) {
+    constexpr int MT = decltype(mt)::value, NT = decltype(nt)::value;
+    k_ptsum<T, MT, NT, FORCE><<<dim3(pl.natom, (npl + NT * 4 - 1) / (NT * 4)), QX_THREADS, 0, st>>>(
+        P, bf.bufR, pl.d_kb_off, pl.d_kb_mesh, bf.kb_vnl, dvnl, pl.d_kb_clalp, pl.rdelv, pl.natom, pl.kb_lmx, npl,
+        wocc, bf.sumr, fpart);
+    note_launch();
+  };
+  using std::integral_constant;
+  const bool wide = (long)pl.natom * ((npl + 7) / 8) >= 148;
+  const int rows = FORCE ? 4 * pl.kb_lmx : pl.kb_lmx;   // at most 36
+  if (rows <= 8) {
+    if (wide) go(integral_constant<int, 1>(), integral_constant<int, 2>());
+    else go(integral_constant<int, 1>(), integral_constant<int, 1>());
+  } else if (rows <= 16) {
+    if (wide) go(integral_constant<int, 2>(), integral_constant<int, 2>());
+    else go(integral_constant<int, 2>(), integral_constant<int, 1>());
+  } else if constexpr (FORCE) {
+    go(integral_constant<int, 5>(), integral_constant<int, 1>());
+  }
+}
+
 template <typename T>
 int launch_hpsi_chunk(const Plan &pl, const PipeParams &P, int npl, const T *cin, long ldc, T *out, long ldo,
                       const double *dk, int accumulate, int nlmode, cudaStream_t st, cudaEvent_t before_unpack) {
@@ -849,6 +874,20 @@ int launch_hpsi_chunk(const Plan &pl, const PipeParams &P, int npl, const T *cin
     k_unpack<T><<<gu, 128, 0, st>>>(P, bf.zsph, cin, ldc, out, ldo, dk, accumulate); note_launch();
     return 0;
   }
+  const NlPoints<T> nl{pl.d_pt_off, pl.d_pt_ent, bf.kb_vnl, bf.sumr, pl.natom, pl.kb_lmx};
+  if constexpr (sizeof(T) == sizeof(float)) {
+    if (nlmode == 2 && pl.use_plane && plane_enabled() &&
+        launch_plane_r_f32(P, npl, bf.bufA, bf.bufR, bf.vloc, nullptr, st) == 0) {
+      launch_ptsum<T, false>(pl, P, npl, nullptr, nullptr, nullptr, st);
+      launch_plane_r_f32(P, npl, bf.bufA, bf.bufR, bf.vloc, &nl, st);
+      zfwd();
+      if (before_unpack) cudaStreamWaitEvent(st, before_unpack, 0);
+      k_unpack<T><<<dim3((P.nplw + 1 + 127) / 128, npl), 128, 0, st>>>(P, bf.zsph, cin, ldc, out, ldo, dk,
+                                                                      accumulate);
+      note_launch();
+      return 0;
+    }
+  }
   k_ypass<T, +1><<<gy, QX_THREADS, smy, st>>>(P, bf.bufA, bf.bufB, g2); note_launch();
   const int nlines = pl.xlines<T>();
   const int nch = (P.k2 + nlines - 1) / nlines;
@@ -856,20 +895,8 @@ int launch_hpsi_chunk(const Plan &pl, const PipeParams &P, int npl, const T *cin
   const size_t smx = fft_smem(P.L1, nlines | 1, cs);
   if (nlmode == 2) {
     k_xinv_r<T><<<gx, QX_THREADS, smx, st>>>(P, bf.bufB, bf.bufR, nlines, nch, g1); note_launch();
-    dim3 ga(pl.natom, npl);
-    if (pl.kb_lmx <= 4) {
-      k_nlproj<T, 4><<<ga, QX_THREADS, 0, st>>>(P, bf.bufR, pl.d_kb_off, pl.d_kb_mesh, bf.kb_vnl, pl.d_kb_clalp,
-                                                pl.rdelv, pl.natom, pl.kb_lmx, bf.sumr); note_launch();
-      k_xfwd_r<T, 4><<<gx, QX_THREADS, smx, st>>>(P, bf.bufR, bf.bufB, bf.vloc, pl.d_line_off, pl.d_line_ent,
-                                                  bf.kb_vnl, bf.sumr, pl.natom, pl.kb_lmx, nlines, nch, g1);
-      note_launch();
-    } else {
-      k_nlproj<T, 9><<<ga, QX_THREADS, 0, st>>>(P, bf.bufR, pl.d_kb_off, pl.d_kb_mesh, bf.kb_vnl, pl.d_kb_clalp,
-                                                pl.rdelv, pl.natom, pl.kb_lmx, bf.sumr); note_launch();
-      k_xfwd_r<T, 9><<<gx, QX_THREADS, smx, st>>>(P, bf.bufR, bf.bufB, bf.vloc, pl.d_line_off, pl.d_line_ent,
-                                                  bf.kb_vnl, bf.sumr, pl.natom, pl.kb_lmx, nlines, nch, g1);
-      note_launch();
-    }
+    launch_ptsum<T, false>(pl, P, npl, nullptr, nullptr, nullptr, st);
+    k_xfwd_r<T><<<gx, QX_THREADS, smx, st>>>(P, bf.bufR, bf.bufB, bf.vloc, nl, nlines, nch, g1); note_launch();
   } else {
     k_xvx<T><<<gx, QX_THREADS, smx, st>>>(P, bf.bufB, bf.vloc, nlines, nch, g1); note_launch();
   }
@@ -919,24 +946,20 @@ int launch_fnl_r_chunk(const Plan &pl, const PipeParams &P, int npl, const T *ci
         launch_zcols_inv_f32(P, npl, (const float *)cin, ldc, (float2 *)bf.bufA, st) == 0)) {
     k_zinv<T><<<gz, QX_THREADS, fft_smem(P.L3, P.P1 | 1, cs), st>>>(P, cin, ldc, bf.bufA, g3); note_launch();
   }
-  dim3 gy(P.k3, npl);
-  k_ypass<T, +1><<<gy, QX_THREADS, fft_smem(P.L2, P.P1, cs), st>>>(P, bf.bufA, bf.bufB, g2); note_launch();
-  const int nlines = pl.xlines<T>();
-  const int nch = (P.k2 + nlines - 1) / nlines;
-  dim3 gx(P.k3 * nch, npl);
-  k_xinv_r<T><<<gx, QX_THREADS, fft_smem(P.L1, nlines | 1, cs), st>>>(P, bf.bufB, bf.bufR, nlines, nch, g1);
-  note_launch();
-  // about four blocks per SM: pairs split over gy groups of ppb
-  const int gyf = std::max(1, std::min(npl, (4 * 148 + pl.natom - 1) / pl.natom));
-  const int ppb = (npl + gyf - 1) / gyf;
-  dim3 ga(pl.natom, (npl + ppb - 1) / ppb);
-  if (pl.kb_lmx <= 4)
-    k_fnl_r<T, 4><<<ga, QX_THREADS, 0, st>>>(P, bf.bufR, pl.d_kb_off, pl.d_kb_mesh, bf.kb_vnl, dvnl, pl.d_kb_clalp,
-                                             pl.rdelv, pl.natom, pl.kb_lmx, wocc, npl, ppb, fpart);
-  else
-    k_fnl_r<T, 9><<<ga, QX_THREADS, 0, st>>>(P, bf.bufR, pl.d_kb_off, pl.d_kb_mesh, bf.kb_vnl, dvnl, pl.d_kb_clalp,
-                                             pl.rdelv, pl.natom, pl.kb_lmx, wocc, npl, ppb, fpart);
-  note_launch();
+  bool plane = false;
+  if constexpr (sizeof(T) == sizeof(float))
+    plane = pl.use_plane && plane_enabled() &&
+            launch_plane_r_f32(P, npl, bf.bufA, bf.bufR, bf.vloc, nullptr, st) == 0;
+  if (!plane) {
+    k_ypass<T, +1><<<dim3(P.k3, npl), QX_THREADS, fft_smem(P.L2, P.P1, cs), st>>>(P, bf.bufA, bf.bufB, g2);
+    note_launch();
+    const int nlines = pl.xlines<T>();
+    const int nch = (P.k2 + nlines - 1) / nlines;
+    k_xinv_r<T><<<dim3(P.k3 * nch, npl), QX_THREADS, fft_smem(P.L1, nlines | 1, cs), st>>>(P, bf.bufB, bf.bufR, nlines,
+                                                                                          nch, g1);
+    note_launch();
+  }
+  launch_ptsum<T, true>(pl, P, npl, dvnl, wocc, fpart, st);
   return 0;
 }
 
@@ -1022,8 +1045,7 @@ void set_fft_smem_limits(size_t bytes) {
   cudaFuncSetAttribute(k_xvx<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
   cudaFuncSetAttribute(k_zfwd<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
   cudaFuncSetAttribute(k_xinv_r<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
-  cudaFuncSetAttribute(k_xfwd_r<T, 4>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
-  cudaFuncSetAttribute(k_xfwd_r<T, 9>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+  cudaFuncSetAttribute(k_xfwd_r<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
   cudaFuncSetAttribute(k_xrho<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
   cudaFuncSetAttribute(k_full_z<T, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
   cudaFuncSetAttribute(k_full_z<T, -1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);

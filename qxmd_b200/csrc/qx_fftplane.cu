@@ -95,4 +95,18 @@ int launch_plane_f32(const PipeParams &P, int npl, float2 *bufA, const float *vl
   }
 }
 
+// The plane passes around the real-space projectors (see k_plane_inv_r);
+// -1 when the grid has no kernel of one line a thread.
+int launch_plane_r_f32(const PipeParams &P, int npl, float2 *bufA, float2 *R, const float *vloc,
+                       const NlPoints<float> *nl, cudaStream_t st) {
+  if (P.P1 > P.k1 || P.P2 > P.k2) return -1;
+  switch (plane_grid_key(P.k1, P.k2)) {
+#define QX_CASE(NX, NY) \
+  case plane_grid_key(NX, NY): return plane_r_launch<NX, NY>(P, npl, bufA, R, vloc, nl, st);
+    QX_PLANE_GRIDS(QX_CASE)
+#undef QX_CASE
+    default: return -1;
+  }
+}
+
 }  // namespace qx

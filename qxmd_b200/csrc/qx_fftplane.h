@@ -12,6 +12,11 @@ namespace qx {
 // most 64), z columns of N = k3 points.
 template <int NX, int NY>
 int plane_launch(const PipeParams &P, int npl, float2 *bufA, const float *vloc, cudaStream_t st);
+// the passes around the real-space projectors: backward into R (nl null),
+// forward from R with the projectors' part (nl)
+template <int NX, int NY>
+int plane_r_launch(const PipeParams &P, int npl, float2 *bufA, float2 *R, const float *vloc,
+                   const NlPoints<float> *nl, cudaStream_t st);
 template <int NX, int NY>
 int rho_launch(const PipeParams &P, int npl, const float2 *bufA, const double *wocc, double *part, double *rho,
                int accumulate, cudaStream_t st);

@@ -254,6 +254,185 @@ __global__ void __launch_bounds__(2 * N) k_plane2(PipeParams P, float2 *__restri
 }
 
 // ---------------------------------------------------------------------------
+// The y and x passes around the real-space projectors, which need psi(r) of
+// the whole cell between the backward and the forward transforms: two band
+// pairs of one z plane a CTA, 64 threads a pair, the planes in shared memory
+// as NY x (NX | 1) complex values.
+//   k_plane_inv_r: backward y and x, the planes stored to R (coalesced);
+//   k_plane_fwd_r: V psi plus the projectors' part, forward x and y back to
+//     bufA.  A grid point's projector points come from the point index
+//     (pt_off, pt_ent), so each thread sums its own points in a fixed order,
+//     for both pairs of the CTA from one read of the projector values.
+// Latency and the L2 traffic of the projector values bound the second (24
+// bytes an entry and CTA, 313 k entries at Si64), hence two pairs a CTA and
+// four grid points in flight a thread.  Against the shared-memory stage
+// kernels and the scatter by float atomics in shared memory that these
+// replace, per 160-band pass at Si64: y and x backward 118 -> 55 us, forward
+// 366 -> 145 us.
+template <int NX, int NY>
+__global__ void __launch_bounds__(128, plane_minb(NX > NY ? NX : NY) > 1 ? 4 : 1)
+    k_plane_inv_r(PipeParams P, const float2 *__restrict__ bufA, float2 *__restrict__ R, int npl) {
+  using rf::out_pos;
+  constexpr int LD = NX | 1;
+  const int i3 = blockIdx.x, h = threadIdx.x >> 6, u = threadIdx.x & 63;
+  const int pl = blockIdx.y * 2 + h, np = P.npair_dev ? *P.npair_dev : P.npair;
+  if (P.pair0 + (int)blockIdx.y * 2 >= np) return;
+  const bool on = pl < npl && P.pair0 + pl < np;
+  const int P1 = P.P1, P2 = P.P2, m1 = P.m1, m2 = P.m2;
+  extern __shared__ float2 T[];
+  float2 *Tp = T + h * (NY * LD);
+  const float2 zero = make_float2(0.f, 0.f);
+  if (on && u < P1) {
+    const float2 *A = bufA + ((long)pl * P.k3 + i3) * P2 * P1;
+    const int xi = u >= m1 ? u - m1 : u - m1 + NX;
+    float2 x[NY];
+#pragma unroll
+    for (int i2 = 0; i2 < NY; ++i2) {
+      const int j2 = (i2 <= m2) ? i2 + m2 : ((i2 >= NY - m2) ? i2 - NY + m2 : -1);
+      float2 v = zero;
+      if (j2 >= 0 && u >= P.row_lo[j2] && u <= P.row_hi[j2]) v = A[j2 * P1 + u];
+      x[i2] = v;
+    }
+    rf::fft<float, +1, NY>(x);
+    rf::static_for<0, NY>([&](auto ic) {
+      constexpr int i2 = decltype(ic)::value, q = out_pos(NY, i2);
+      Tp[i2 * LD + xi] = x[q];
+    });
+  }
+  __syncthreads();
+  if (on && u < NY) {
+    float2 x[NX];
+    float2 *row = Tp + u * LD;
+#pragma unroll
+    for (int i1 = 0; i1 < NX; ++i1) x[i1] = (i1 <= m1 || i1 >= NX - m1) ? row[i1] : zero;
+    rf::fft<float, +1, NX>(x);
+    rf::static_for<0, NX>([&](auto ic) {
+      constexpr int i1 = decltype(ic)::value, q = out_pos(NX, i1);
+      row[i1] = x[q];
+    });
+  }
+  __syncthreads();
+  if (on) {
+    float2 *dst = R + ((long)pl * P.k3 + i3) * (NX * NY);
+#pragma unroll 4
+    for (int i = u; i < NX * NY; i += 64) dst[i] = Tp[(i / NX) * LD + i % NX];
+  }
+}
+
+template <int NX, int NY>
+__global__ void __launch_bounds__(128, plane_minb(NX > NY ? NX : NY) > 1 ? 4 : 1)
+    k_plane_fwd_r(PipeParams P, const float2 *__restrict__ R, float2 *__restrict__ bufA,
+                  const float *__restrict__ vloc, NlPoints<float> nl, int npl) {
+  using rf::out_pos;
+  constexpr int LD = NX | 1, NP = NX * NY, UN = 4;
+  const int i3 = blockIdx.x, t = threadIdx.x, h = t >> 6, u = t & 63;
+  const int pl0 = blockIdx.y * 2, np = P.npair_dev ? *P.npair_dev : P.npair;
+  if (P.pair0 + pl0 >= np) return;
+  const bool two = pl0 + 1 < npl && P.pair0 + pl0 + 1 < np;
+  const int P1 = P.P1, P2 = P.P2, m1 = P.m1, m2 = P.m2;
+  extern __shared__ float2 T[];
+  const float2 zero = make_float2(0.f, 0.f);
+  {
+    const long g0 = (long)i3 * NP;
+    const float2 *R0 = R + (long)pl0 * P.k3 * NP + g0, *R1 = two ? R0 + (long)P.k3 * NP : R0;
+    const float *V = vloc + g0;
+    const int *off = nl.off + g0;
+    const float2 *S0 = nl.sumr + (long)pl0 * nl.natom * nl.lmx, *S1 = two ? S0 + (long)nl.natom * nl.lmx : S0;
+    for (int ib = t; ib < NP; ib += 128 * UN) {
+      float2 z0[UN], z1[UN];
+      int e0[UN], e1[UN];
+#pragma unroll
+      for (int q = 0; q < UN; ++q) {
+        const int i = min(ib + 128 * q, NP - 1);
+        e0[q] = off[i];
+        e1[q] = off[i + 1];
+        const float v = V[i];
+        const float2 a = R0[i], b = R1[i];
+        z0[q] = make_float2(a.x * v, a.y * v);
+        z1[q] = make_float2(b.x * v, b.y * v);
+      }
+      if (nl.lmx == 4) {
+        // the UN points' entries side by side, so that their loads overlap
+        int more = 0;
+#pragma unroll
+        for (int q = 0; q < UN; ++q) more = max(more, e1[q] - e0[q]);
+        for (int k = 0; k < more; ++k) {
+          int2 en[UN];
+          float4 v[UN];
+#pragma unroll
+          for (int q = 0; q < UN; ++q) en[q] = e0[q] + k < e1[q] ? nl.ent[e0[q] + k] : make_int2(-1, 0);
+#pragma unroll
+          for (int q = 0; q < UN; ++q)
+            v[q] = en[q].x >= 0 ? *reinterpret_cast<const float4 *>(nl.vnl + 4L * en[q].x)
+                                : make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+          for (int q = 0; q < UN; ++q) {
+            if (en[q].x < 0) continue;
+            const float4 *a = reinterpret_cast<const float4 *>(S0 + 4L * en[q].y);
+            const float4 *b = reinterpret_cast<const float4 *>(S1 + 4L * en[q].y);
+            const float4 a0 = a[0], a1 = a[1], b0 = b[0], b1 = b[1], w = v[q];
+            z0[q].x += w.x * a0.x + w.y * a0.z + w.z * a1.x + w.w * a1.z;
+            z0[q].y += w.x * a0.y + w.y * a0.w + w.z * a1.y + w.w * a1.w;
+            z1[q].x += w.x * b0.x + w.y * b0.z + w.z * b1.x + w.w * b1.z;
+            z1[q].y += w.x * b0.y + w.y * b0.w + w.z * b1.y + w.w * b1.w;
+          }
+        }
+      } else {
+#pragma unroll
+        for (int q = 0; q < UN; ++q)
+          for (int e = e0[q]; e < e1[q]; ++e) {
+            const int2 en = nl.ent[e];
+            for (int l = 0; l < nl.lmx; ++l) {
+              const float v = nl.vnl[(long)nl.lmx * en.x + l];
+              const float2 a = S0[(long)nl.lmx * en.y + l], b = S1[(long)nl.lmx * en.y + l];
+              z0[q].x += v * a.x;
+              z0[q].y += v * a.y;
+              z1[q].x += v * b.x;
+              z1[q].y += v * b.y;
+            }
+          }
+      }
+#pragma unroll
+      for (int q = 0; q < UN; ++q) {
+        const int i = ib + 128 * q;
+        if (i >= NP) break;
+        const int o = (i / NX) * LD + i % NX;
+        T[o] = z0[q];
+        T[NY * LD + o] = z1[q];
+      }
+    }
+  }
+  __syncthreads();
+  float2 *Tp = T + h * (NY * LD);
+  const bool on = h == 0 || two;
+  if (on && u < NY) {
+    float2 x[NX];
+    float2 *row = Tp + u * LD;
+#pragma unroll
+    for (int i1 = 0; i1 < NX; ++i1) x[i1] = row[i1];
+    rf::fft<float, -1, NX>(x);
+    rf::static_for<0, NX>([&](auto ic) {
+      constexpr int i1 = decltype(ic)::value, q = out_pos(NX, i1);
+      if (i1 <= m1 || i1 >= NX - m1) row[i1] = x[q];
+    });
+  }
+  __syncthreads();
+  if (on && u < P1) {
+    const int xi = u >= m1 ? u - m1 : u - m1 + NX;
+    float2 *A = bufA + ((long)(pl0 + h) * P.k3 + i3) * P2 * P1;
+    float2 x[NY];
+#pragma unroll
+    for (int i2 = 0; i2 < NY; ++i2) x[i2] = Tp[i2 * LD + xi];
+    rf::fft<float, -1, NY>(x);
+    rf::static_for<0, NY>([&](auto ic) {
+      constexpr int i2 = decltype(ic)::value, q = out_pos(NY, i2);
+      const int j2 = (i2 <= m2) ? i2 + m2 : ((i2 >= NY - m2) ? i2 - NY + m2 : -1);
+      if (j2 >= 0 && u >= P.row_lo[j2] && u <= P.row_hi[j2]) A[j2 * P1 + u] = x[q];
+    });
+  }
+}
+
+// ---------------------------------------------------------------------------
 // The z transforms of the FP32 pipeline, one sphere z-column (j2, a) of one
 // band pair per thread with the whole line in registers (replacing the
 // shared-memory k_zinv / k_zfwd for the specialised lengths).  The column's
@@ -609,6 +788,25 @@ int plane_launch(const PipeParams &P, int npl, float2 *bufA, const float *vloc, 
   return 0;
 }
 
+template <int NX, int NY>
+int plane_r_launch(const PipeParams &P, int npl, float2 *bufA, float2 *R, const float *vloc,
+                   const NlPoints<float> *nl, cudaStream_t st) {
+  const size_t sm = sizeof(float2) * 2 * (size_t)NY * (NX | 1);
+  static bool attr = false;
+  if (!attr) {
+    cudaFuncSetAttribute(k_plane_inv_r<NX, NY>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+    cudaFuncSetAttribute(k_plane_fwd_r<NX, NY>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+    attr = true;
+  }
+  dim3 g(P.k3, (npl + 1) / 2);
+  if (nl)
+    k_plane_fwd_r<NX, NY><<<g, 128, sm, st>>>(P, R, bufA, vloc, *nl, npl);
+  else
+    k_plane_inv_r<NX, NY><<<g, 128, sm, st>>>(P, bufA, R, npl);
+  note_launch();
+  return 0;
+}
+
 template <int N>
 int plane2_launch(const PipeParams &P, int npl, float2 *bufA, const float *vloc, cudaStream_t st) {
   const size_t sm = sizeof(float2) * (size_t)N * P.P1;
@@ -627,6 +825,8 @@ int plane2_launch(const PipeParams &P, int npl, float2 *bufA, const float *vloc,
 // Explicit instantiation of the launchers of one k1 x k2 plane shape.
 #define QX_PLANE_GRID(NX, NY)                                                                                    \
   template int plane_launch<NX, NY>(const PipeParams &, int, float2 *, const float *, cudaStream_t);             \
+  template int plane_r_launch<NX, NY>(const PipeParams &, int, float2 *, float2 *, const float *,                \
+                                      const NlPoints<float> *, cudaStream_t);                                    \
   template int rho_launch<NX, NY>(const PipeParams &, int, const float2 *, const double *, double *, double *,   \
                                   int, cudaStream_t);
 // ... and of the z-column launcher of one k3.

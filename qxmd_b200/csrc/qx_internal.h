@@ -52,6 +52,17 @@ struct Bufs {
   double *rho_part = nullptr;   // RHO_GROUPS partial density planes (plane-kernel grids)
 };
 
+// Real-space projectors by grid point (Plan::d_pt_off, d_pt_ent), their
+// values and the projections <beta|psi> D of the chunk's band pairs.
+template <typename T>
+struct NlPoints {
+  const int *off;
+  const int2 *ent;
+  const T *vnl;
+  const typename c2t<T>::type *sumr;
+  int natom, lmx;
+};
+
 struct Plan {
   int k1 = 0, k2 = 0, k3 = 0;
   long n = 0;
@@ -74,8 +85,8 @@ struct Plan {
   int *d_kb_off = nullptr, *d_kb_mesh = nullptr;
   double *d_kb_clalp = nullptr;
   double rdelv = 0.0;
-  int *d_line_off = nullptr;
-  int4 *d_line_ent = nullptr;
+  int *d_pt_off = nullptr;    // kfft0 + 1: the projector points at each grid point ...
+  int2 *d_pt_ent = nullptr;   // ... as (point index, atom), ordered by point index
   // G-space KB
   int nproj = 0;
   bool use_plane = true;   // FP32 fused plane kernels where supported (the autotuner may turn them off)
@@ -113,6 +124,10 @@ template <typename T> void set_fft_smem_limits(size_t bytes);
 // qx_fftplane.cu: fused y-x-y pass (FP32, k1 x k2 planes of a specialised
 // shape, QX_PLANE_GRIDS); returns -1 when the grid is not covered.
 int launch_plane_f32(const PipeParams &P, int npl, float2 *bufA, const float *vloc, cudaStream_t st);
+// The same passes split around the real-space projectors: nl null, backward
+// into R; else forward from R.  -1 when the grid is not covered.
+int launch_plane_r_f32(const PipeParams &P, int npl, float2 *bufA, float2 *R, const float *vloc,
+                       const NlPoints<float> *nl, cudaStream_t st);
 // Density through the plane kernel: groups of pairs per z plane, partial
 // planes in part (RHO_GROUPS * kfft0 doubles) summed in a fixed order.
 constexpr int RHO_GROUPS = 16;
@@ -220,6 +235,6 @@ void kbr_fill(const KbrGeom &G, int natom, int lmx, const int *ityp, const doubl
               const double *rcl, const double *dltnl, const double *tabnl, const double *dtabnl, int mxnl,
               const int *poly, const int *soff, long cap, int *mesh, int *ptatom, T *vnl, T *dvnl, cudaStream_t st);
 int kbr_lines(const int *off, int natom, const int *mesh, const int *ptatom, int k1, long nlines, int *lcnt,
-              int *loff, int *cursor, int4 *lent, cudaStream_t st);
+              int *loff, int *cursor, int4 *lent, int *ptoff, int2 *ptent, cudaStream_t st);
 
 }  // namespace qx

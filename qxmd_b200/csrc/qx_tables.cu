@@ -19,9 +19,9 @@
 //    grid points around the atom's nearest grid point, periodic wrap), in
 //    box order (x fastest), with the projector values interpolated from the
 //    radial table by the same three-point formula times a real solid
-//    harmonic polynomial of the displacement, then the x-line index (points
-//    of each grid line, ordered by point) that the real-space KB kernels of
-//    the FFT pipeline read.
+//    harmonic polynomial of the displacement, then the grid-point index (the
+//    projector points at each grid point, ordered by point) that the
+//    real-space KB kernels of the FFT pipeline read.
 #include "qx_internal.h"
 
 namespace qx {
@@ -357,38 +357,65 @@ __global__ void k_kbr_line_fill(const int *__restrict__ off, int natom, const in
   }
 }
 
-// One block per line: entries ordered by point index.  Up to LSORT_MAX
-// entries go to shared memory and each lands at its rank (the count of
-// smaller point indices; indices are unique); a longer line is sorted by one
-// thread in place (insertion sort).
+// One block per x line: its entries to their places in the grid-point index,
+// ordered by x and then by point index, and the offsets of the line's grid
+// points.  Lines of up to LSORT_MAX entries by a counting sort over x in
+// shared memory (k1 counters), then the rank among the few entries of the
+// same x; longer ones by ranking every entry against the line in global
+// memory.
 constexpr int LSORT_MAX = 1024;
-__global__ void __launch_bounds__(128) k_kbr_line_sort(const int *__restrict__ loff, long nlines,
-                                                       int4 *__restrict__ lent) {
-  __shared__ int4 e[LSORT_MAX];
+__global__ void __launch_bounds__(128) k_kbr_line_sort(const int *__restrict__ loff, long nlines, int k1,
+                                                       const int4 *__restrict__ lent, int *__restrict__ ptoff,
+                                                       int2 *__restrict__ ptent) {
+  extern __shared__ int start[];   // k1 + 1 offsets, then k1 cursors
+  int *cursor = start + k1 + 1;
+  __shared__ int2 sorted[LSORT_MAX];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  if (blockIdx.x == 0 && threadIdx.x == 0) ptoff[nlines * k1] = loff[nlines];
   for (long l = blockIdx.x; l < nlines; l += gridDim.x) {
-    const int lo = loff[l], hi = loff[l + 1], m = hi - lo;
-    if (m <= 1) continue;   // uniform across the block
+    const int lo = loff[l], m = loff[l + 1] - lo;
+    const int4 *e = lent + lo;
+    for (int x = threadIdx.x; x < k1; x += blockDim.x) cursor[x] = 0;
+    __syncthreads();
+    for (int i = threadIdx.x; i < m; i += blockDim.x) atomicAdd(&cursor[e[i].x], 1);
+    __syncthreads();
+    if (warp == 0) {   // exclusive scan of the counts
+      int run = 0;
+      for (int x0 = 0; x0 < k1; x0 += 32) {
+        const int x = x0 + lane, c = x < k1 ? cursor[x] : 0;
+        int v = c;
+        for (int o = 1; o < 32; o <<= 1) {
+          const int u = __shfl_up_sync(0xffffffffu, v, o);
+          if (lane >= o) v += u;
+        }
+        if (x < k1) start[x] = cursor[x] = run + v - c;
+        run += __shfl_sync(0xffffffffu, v, 31);
+      }
+      if (lane == 0) start[k1] = run;
+    }
+    __syncthreads();
+    for (int x = threadIdx.x; x < k1; x += blockDim.x) ptoff[l * k1 + x] = lo + start[x];
     if (m <= LSORT_MAX) {
-      for (int i = threadIdx.x; i < m; i += blockDim.x) e[i] = lent[lo + i];
+      for (int i = threadIdx.x; i < m; i += blockDim.x) {
+        const int4 v = e[i];
+        sorted[atomicAdd(&cursor[v.x], 1)] = make_int2(v.y, v.z);
+      }
       __syncthreads();
       for (int i = threadIdx.x; i < m; i += blockDim.x) {
-        const int key = e[i].y;
-        int r = 0;
-        for (int j = 0; j < m; ++j) r += e[j].y < key ? 1 : 0;
-        lent[lo + r] = e[i];
+        const int4 v = e[i];
+        int r = start[v.x];
+        for (int j = start[v.x]; j < start[v.x + 1]; ++j) r += sorted[j].x < v.y ? 1 : 0;
+        ptent[lo + r] = make_int2(v.y, v.z);
       }
-      __syncthreads();
-    } else if (threadIdx.x == 0) {
-      for (int i = lo + 1; i < hi; ++i) {
-        const int4 v = lent[i];
-        int j = i - 1;
-        while (j >= lo && lent[j].y > v.y) {
-          lent[j + 1] = lent[j];
-          --j;
-        }
-        lent[j + 1] = v;
+    } else {
+      for (int i = threadIdx.x; i < m; i += blockDim.x) {
+        const int4 v = e[i];
+        int r = start[v.x];
+        for (int j = 0; j < m; ++j) r += (e[j].x == v.x && e[j].y < v.y) ? 1 : 0;
+        ptent[lo + r] = make_int2(v.y, v.z);
       }
     }
+    __syncthreads();
   }
 }
 
@@ -420,7 +447,7 @@ template void kbr_fill<double>(const KbrGeom &, int, int, const int *, const dou
                                int *, int *, double *, double *, cudaStream_t);
 
 int kbr_lines(const int *off, int natom, const int *mesh, const int *ptatom, int k1, long nlines, int *lcnt,
-              int *loff, int *cursor, int4 *lent, cudaStream_t st) {
+              int *loff, int *cursor, int4 *lent, int *ptoff, int2 *ptent, cudaStream_t st) {
   if (cudaMemsetAsync(lcnt, 0, sizeof(int) * nlines, st) != cudaSuccess) return 1;
   k_kbr_line_count<<<148 * 4, 256, 0, st>>>(off, natom, mesh, k1, lcnt);
   note_launch();
@@ -428,7 +455,8 @@ int kbr_lines(const int *off, int natom, const int *mesh, const int *ptatom, int
   note_launch();
   k_kbr_line_fill<<<148 * 4, 256, 0, st>>>(off, natom, mesh, ptatom, k1, cursor, lent);
   note_launch();
-  k_kbr_line_sort<<<(unsigned)std::min<long>(148 * 16, nlines), 128, 0, st>>>(loff, nlines, lent);
+  k_kbr_line_sort<<<(unsigned)std::min<long>(148 * 16, nlines), 128, sizeof(int) * (2 * k1 + 1), st>>>(loff, nlines, k1, lent, ptoff,
+                                                                                                         ptent);
   note_launch();
   return 0;
 }
