@@ -103,7 +103,7 @@ struct qx_ctx {
   bool scf_ready = false;
   // sequential CG: device band cursor, dot-product buffer and the captured
   // while-loop graph (rebuilt when its buffers or parameters change)
-  int *d_seqi = nullptr;   // cur, pairs[2], list[1]
+  int *d_seqi = nullptr;   // cur, pairs[2]
   double *d_seqw = nullptr;
   int seqw_len = 0;
   cudaStream_t cap_st = nullptr;
@@ -1543,30 +1543,39 @@ static int eigen_impl(qx_ctx *c, const qx_cgparm *p, int *nriter, int *nhpsi_out
   c->have_hsub = false;
   return 0;
 }
-// One CG step of band *cur (the body of the sequential loop): preconditioned
-// direction, subgs3 against the snapshot of the bands below (already final),
-// subgs4, H|h> of this one band, BKL update and, once the band stops, the
-// move to the next band.
+// One CG step of band *cur (the body of the sequential loop, see qx_cg.cu):
+// the direction projected on the snapshot of the bands below (already final)
+// and on the band itself, H|h> of this one band, the BKL update and, once the
+// band stops, the move to the next one.
 template <typename T>
 static int seq_body(qx_ctx *c, const CgParm &pm, const SeqArgs &q) {
-  const int nb = c->nb, ne = c->ne;
+  const int ne = c->ne;
   T *x = (T *)c->psi, *hx = (T *)c->hpsi, *g = (T *)c->g, *h = (T *)c->h, *gh = (T *)c->gh;
-  const T *snap = (const T *)c->snap;
   const CgState &s = c->cg;
-  cg_prec<T>(nb, ne, ne, g, h, c->d_dk, s, c->st, q.cur);
-  seq_dots<T>(nb, q.cur, ne, snap, ne, h, ne, q.cur, 1, nullptr, c->d_seqw, c->st);
-  seq_axpy<T>(nb, q.cur, ne, snap, ne, c->d_seqw, -1.0, h, ne, q.cur, c->st);
-  cg_orth<T>(nb, ne, ne, x, hx, h, s, c->st, q.cur);
+  const int off = std::max(c->nb, c->pl.nproj);   // d_seqw: p and q of the projections, then the KB coefficients
+  seq_project<T>(ne, ne, x, g, h, s, q, c->d_seqw, c->d_seqw + off, c->st);
   CKL();
-  const int fl = QX_HPSI_KINETIC | (c->nlmode == QX_NL_RSPACE ? QX_HPSI_NONLOCAL : 0);
-  TRY(hpsi_impl<T>(c, h, gh, q.pairs, nullptr, 1, nullptr, nullptr, 1, fl));
-  if (c->nlmode == QX_NL_GSPACE) {
+  const bool kb = c->nlmode == QX_NL_GSPACE;
+  const bool side = kb && kb_side_stream_enabled();
+  if (kb) {
     const Bufs<T> &b = c->pl.bufs<T>();
-    const int np = c->pl.nproj;
-    seq_dots<T>(np, nullptr, ne, b.kbg, ne, h, ne, q.cur, 2, b.vclalp, c->d_seqw, c->st);
-    seq_axpy<T>(np, nullptr, ne, b.kbg, ne, c->d_seqw, 1.0, gh, ne, q.cur, c->st);
+    cudaStream_t kst = c->st;
+    if (side) {
+      CK(cudaEventRecord(c->ev_fork, c->st));
+      CK(cudaStreamWaitEvent(c->st2, c->ev_fork, 0));
+      kst = c->st2;
+    }
+    seq_kb<T>(c->pl.nproj, ne, b.kbg, b.vclalp, h, gh, ne, q.cur, c->d_seqw + 2 * off, kst);
+    CKL();
+    if (side) CK(cudaEventRecord(c->ev_join, c->st2));
   }
-  cg_update_seq<T>(ne, ne, x, hx, g, h, gh, s, pm, q, c->st);
+  PipeParams P = base_params(c);
+  P.pairs = q.pairs;
+  P.npair = 1;
+  TRY(launch_hpsi_chunk<T>(c->pl, P, 1, h, ne, gh, ne, c->d_dk, kb ? 1 : 0, c->nlmode == QX_NL_RSPACE ? 2 : 0, c->st,
+                           side ? c->ev_join : nullptr));
+  CKL();
+  seq_update<T>(ne, ne, x, hx, g, h, gh, c->d_dk, s, pm, q, c->st);
   CKL();
   return 0;
 }
@@ -1601,7 +1610,7 @@ static int seq_graph(qx_ctx *c, const qx_cgparm *p, const CgParm &pm) {
   cudaGraphNode_t node;
   CK(cudaGraphAddNode(&node, g, nullptr, 0, &np));
   cudaGraph_t body = np.conditional.phGraph_out[0];
-  SeqArgs q{c->d_seqi, c->d_seqi + 1, c->d_seqi + 3, c->snap, c->nb,
+  SeqArgs q{c->d_seqi, c->d_seqi + 1, c->snap, c->nb,
             (sizeof(T) == sizeof(double) && p->ccreal4) ? 1 : 0, hd};
   CK(cudaStreamBeginCaptureToGraph(c->cap_st, body, nullptr, nullptr, 0, cudaStreamCaptureModeThreadLocal));
   cudaStream_t user = c->st;
@@ -1627,7 +1636,8 @@ static int eigen_seq_impl(qx_ctx *c, const qx_cgparm *p, int *nriter, int *nhpsi
   const int nb = c->nb, ne = c->ne;
   CgParm pm{p->itermx, p->iteremx, p->noband, p->tolera, p->roughfzan, p->roughfeig, p->threinn, p->wdinner};
   T *x = (T *)c->psi, *hx = (T *)c->hpsi, *g = (T *)c->g;
-  const int need = std::max(nb, c->pl.nproj);
+  if (!c->have_glocal) { set_error("hpsi: glocal not set"); return QX_ERR_STATE; }
+  const int need = 3 * std::max(nb, c->pl.nproj);
   if (c->seqw_len < need) {
     TRY(dalloc(c, &c->d_seqw, sizeof(double) * need));
     c->seqw_len = need;
@@ -1635,11 +1645,10 @@ static int eigen_seq_impl(qx_ctx *c, const qx_cgparm *p, int *nriter, int *nhpsi
   if (!c->d_seqi) TRY(dalloc(c, &c->d_seqi, sizeof(int) * 4));
   // No entry snapshot: band ib reads the columns of bands < ib only, and each
   // of those is written with its final vector before band ib starts.
-  cg_init<T>(nb, ne, ne, x, hx, g, c->cg, c->st);
-  CKL();
+  TRY(side_stream(c));
   TRY(seq_graph<T>(c, p, pm));
-  SeqArgs q{c->d_seqi, c->d_seqi + 1, c->d_seqi + 3, c->snap, nb, 0, 0};
-  seq_reset(q, c->st);
+  SeqArgs q{c->d_seqi, c->d_seqi + 1, c->snap, nb, 0, 0};
+  seq_init<T>(nb, ne, ne, x, hx, g, c->d_dk, c->cg, q, c->st);
   CKL();
   CK(cudaGraphLaunch(c->seq_exec, c->st));
   CK(cudaMemcpyAsync(c->d_eig, c->cg.eig, sizeof(double) * nb, cudaMemcpyDeviceToDevice, c->st));

@@ -5,10 +5,13 @@
 // the reference's result with one band per rank.  One CTA per band; every
 // reduction is accumulated in FP64.  Per-band state lives on the device, so a
 // CG sweep needs no host round trip.
+#include <cooperative_groups.h>
+
 #include "qx_internal.h"
 #include "qx_cg.h"
 
 namespace qx {
+namespace cg = cooperative_groups;
 
 // One CTA per band; 1024 threads give each SM enough loads in flight for
 // these bandwidth-bound sweeps over a band.
@@ -58,23 +61,26 @@ __global__ void __launch_bounds__(CGT) k_cg_init(int ne, long ldx, const T *__re
   }
 }
 
+// prpcg (eigen.f90:1093-1113), e15 = 1.5 ekib.
+__device__ __forceinline__ double prpcg(double dk, double e15) {
+  const double x = dk / e15;
+  const double t = 27.0 + x * (18.0 + x * (12.0 + 8.0 * x));
+  const double x2 = x * x, x4 = x2 * x2;
+  return t / (t + 16.0 * x4) * 2.0 / e15;
+}
+
 // g <- prcd * g; zansap = <g|g>; h <- g + beta*h (h <- g on reset).
 template <typename T>
 __global__ void __launch_bounds__(CGT) k_cg_prec(int ne, long ldx, T *__restrict__ g, T *__restrict__ h,
-                                                         const double *__restrict__ dk, CgState s,
-                                                         const int *__restrict__ cur, int nb) {
+                                                         const double *__restrict__ dk, CgState s) {
   __shared__ double red[CGT / 32];
-  const int b = cur ? *cur : blockIdx.x;
-  if (b >= nb || !s.active[b]) return;
+  const int b = blockIdx.x;
+  if (!s.active[b]) return;
   T *gb = g + b * ldx, *hb = h + b * ldx;
   const double e15 = 1.5 * s.ekib[b];
   double z = 0.0;
   for (int i = threadIdx.x; i < ne; i += blockDim.x) {
-    const double x = dk[i] / e15;
-    double t = 27.0 + x * (18.0 + x * (12.0 + 8.0 * x));
-    const double x2 = x * x, x4 = x2 * x2;
-    t = t / (t + 16.0 * x4);
-    const T v = (T)((double)gb[i] * (t * 2.0 / e15));
+    const T v = (T)((double)gb[i] * prpcg(dk[i], e15));
     gb[i] = v;
     z += (double)v * (double)v;
   }
@@ -106,11 +112,10 @@ __global__ void k_cg_mask(int nb, T *__restrict__ Pm, CgState s) {
 // subgs4: h -= <x|h> x; cai = <h|hx>.
 template <typename T>
 __global__ void __launch_bounds__(CGT) k_cg_orth(int ne, long ldx, const T *__restrict__ x,
-                                                         const T *__restrict__ hx, T *__restrict__ h, CgState s,
-                                                         const int *__restrict__ cur, int nb) {
+                                                         const T *__restrict__ hx, T *__restrict__ h, CgState s) {
   __shared__ double red[CGT / 32];
-  const int b = cur ? *cur : blockIdx.x;
-  if (b >= nb || !s.active[b]) return;
+  const int b = blockIdx.x;
+  if (!s.active[b]) return;
   const T *xb = x + b * ldx, *hxb = hx + b * ldx;
   T *hb = h + b * ldx;
   const double hhx = bdot(xb, (const T *)hb, ne, red);
@@ -147,26 +152,72 @@ __global__ void k_cg_list(int nb, CgState s) {
   }
 }
 
-// BKL 2x2 step (eigen.f90:593-622), line minimisation fallback (624-695),
-// x/hx update (698-709), residual and convergence test (731-764).
-// SEQ: one CTA on band *q.cur; when the band stops, its final vector becomes
-// its snapshot column (cgjr(:,ib) = gdcr(:,ibb), eigen.f90:699, real*4 when
-// q.ccreal4) and the next band starts.
-// All bands at once: two CTAs per SM (at most 32 registers), so that 160
-// bands fit one wave on 148 SMs.
-template <typename T, bool SEQ>
-__global__ void __launch_bounds__(CGT, SEQ ? 1 : 2) k_cg_update(int ne, long ldx, T *__restrict__ x, T *__restrict__ hx,
-                                                           T *__restrict__ g, const T *__restrict__ h,
-                                                           const T *__restrict__ gh, CgState s, CgParm pm,
-                                                           SeqArgs q) {
-  __shared__ double red[CGT / 32];
-  __shared__ int stop_sh;
-  const int b = SEQ ? *q.cur : blockIdx.x;
-  if (SEQ && b >= q.nb) {
-    if (threadIdx.x == 0) cudaGraphSetConditional(q.handle, 0);
-    return;
+// BKL 2x2 step (eigen.f90:593-622): the new eigenvalue e, the step dtnew
+// along h and the normalisation alpsq, from cai = <h|hx>, cbi = <h|gh>,
+// hhi = <h|h> > 0.
+__device__ __forceinline__ void bkl_step(double cai, double cbi, double hhi, double &e, double &dtnew,
+                                         double &alpsq) {
+  const double h11 = e, h12 = cai / sqrt(hhi), h21 = h12, h22 = cbi / hhi;
+  const double enew = 0.5 * (h11 + h22 - sqrt((h11 + h22) * (h11 + h22) - 4.0 * (h11 * h22 - h12 * h21)));
+  dtnew = (enew - h11) / h12 / sqrt(hhi);
+  alpsq = sqrt(1.0 / (1.0 + dtnew * (0.0 + dtnew * hhi)));
+  e = enew;
+}
+
+// Line minimisation (eigen.f90:624-695) for hhi = 0, with hhx = <h|x>; *dmax
+// receives a larger inner product than dinx.
+__device__ __forceinline__ void bkl_line(double cai, double cbi, double hhi, double hhx, double dinx,
+                                         const CgParm &pm, double *dmax, bool writer, double &e, double &dtnew,
+                                         double &alpsq) {
+  const double c0 = e, c1 = cai, c2 = cbi, c3 = hhi, c4 = 2.0 * hhx;
+  const double s0 = c0 * c4 - c1, s1 = c0 * c3 - c2, s2 = c1 * c3 - c2 * c4;
+  const double sr = s1 * s1 - s2 * s0;
+  dtnew = (sr > 0.0) ? (-s1 - sqrt(sr)) / s2 : -1.0;
+  if (dtnew > 0.0) {
+    const double dinner = sqrt(1.0 / (1.0 + dtnew * dtnew * hhi));
+    if (dinner < pm.threinn) dtnew = 0.0;
+    if (dinner < dinx * pm.wdinner) dtnew = 0.0;
+    if (writer && dinner > dinx) *dmax = dinner;
   }
-  if (!SEQ && !s.active[b]) return;
+  const double d2 = dtnew * dtnew;
+  const double alpsq2 = 1.0 / (1.0 + dtnew * c4 + d2 * c3);
+  e = (c0 + dtnew * c1 + d2 * c2) * alpsq2;
+  alpsq = sqrt(alpsq2);
+}
+
+// Convergence test of band b after step `iter` (eigen.f90:731-764) and its
+// state for the next one; true when the band stops.
+__device__ __forceinline__ bool bkl_stop(const CgState &s, const CgParm &pm, int b, int iter, double e,
+                                         double zansa) {
+  const double de = fabs(s.eigb[b] - e);
+  const bool stop = (b < pm.noband && iter >= pm.itermx) || (b >= pm.noband && iter >= pm.iteremx) ||
+                    zansa < pm.tolera || de < pm.tolera || zansa < s.z000re[b] * pm.roughfzan ||
+                    (iter > 1 && de < s.x000re[b] * pm.roughfeig);
+  s.eig[b] = e;
+  s.zansa[b] = zansa;
+  if (stop) {
+    s.active[b] = 0;
+  } else {
+    if (iter == 1) s.x000re[b] = de;
+    if (zansa > s.zansab[b]) {
+      if (++s.izcnt[b] > 20) { s.izcnt[b] = 0; s.lreset[b] = 1; }
+    }
+    s.zansab[b] = zansa;
+    s.eigb[b] = e;
+  }
+  return stop;
+}
+
+// x/hx update (eigen.f90:698-709), residual and convergence test of every
+// active band.  Two CTAs per SM (at most 32 registers), so that 160 bands fit
+// one wave on 148 SMs.
+template <typename T>
+__global__ void __launch_bounds__(CGT, 2) k_cg_update(int ne, long ldx, T *__restrict__ x, T *__restrict__ hx,
+                                                      T *__restrict__ g, const T *__restrict__ h,
+                                                      const T *__restrict__ gh, CgState s, CgParm pm) {
+  __shared__ double red[CGT / 32];
+  const int b = blockIdx.x;
+  if (!s.active[b]) return;
   T *xb = x + b * ldx, *hxb = hx + b * ldx, *gb = g + b * ldx;
   const T *hb = h + b * ldx, *ghb = gh + b * ldx;
   const double dinx = s.dinnerx[b];   // read before thread 0 may update it
@@ -185,31 +236,12 @@ __global__ void __launch_bounds__(CGT, SEQ ? 1 : 2) k_cg_update(int ne, long ldx
   double e = s.eig[b];
   double dtnew, alpsq;
   if (hhi > 0.0) {
-    const double h11 = e, h12 = cai / sqrt(hhi), h21 = h12, h22 = cbi / hhi;
-    const double enew = 0.5 * (h11 + h22 - sqrt((h11 + h22) * (h11 + h22) - 4.0 * (h11 * h22 - h12 * h21)));
-    dtnew = (enew - h11) / h12 / sqrt(hhi);
-    const double alpsq2 = 1.0 / (1.0 + dtnew * (0.0 + dtnew * hhi));
-    alpsq = sqrt(alpsq2);
-    e = enew;
+    bkl_step(cai, cbi, hhi, e, dtnew, alpsq);
   } else {
     double hx2 = 0.0;
     for (int i = threadIdx.x; i < ne; i += blockDim.x) hx2 += (double)hb[i] * (double)xb[i];
     hx2 = block_sum(hx2, red);
-    const double hhx = 2.0 * hx2 - h0 * ld(xb, 0);
-    const double c0 = e, c1 = cai, c2 = cbi, c3 = hhi, c4 = 2.0 * hhx;
-    const double s0 = c0 * c4 - c1, s1 = c0 * c3 - c2, s2 = c1 * c3 - c2 * c4;
-    const double sr = s1 * s1 - s2 * s0;
-    dtnew = (sr > 0.0) ? (-s1 - sqrt(sr)) / s2 : -1.0;
-    if (dtnew > 0.0) {
-      const double dinner = sqrt(1.0 / (1.0 + dtnew * dtnew * hhi));
-      if (dinner < pm.threinn) dtnew = 0.0;
-      if (dinner < dinx * pm.wdinner) dtnew = 0.0;
-      if (threadIdx.x == 0 && dinner > dinx) s.dinnerx[b] = dinner;
-    }
-    const double d2 = dtnew * dtnew;
-    const double alpsq2 = 1.0 / (1.0 + dtnew * c4 + d2 * c3);
-    e = (c0 + dtnew * c1 + d2 * c2) * alpsq2;
-    alpsq = sqrt(alpsq2);
+    bkl_line(cai, cbi, hhi, 2.0 * hx2 - h0 * ld(xb, 0), dinx, pm, &s.dinnerx[b], threadIdx.x == 0, e, dtnew, alpsq);
   }
   const T a = (T)alpsq, dt = (T)dtnew, et = (T)e;
   double z = 0.0;
@@ -224,45 +256,64 @@ __global__ void __launch_bounds__(CGT, SEQ ? 1 : 2) k_cg_update(int ne, long ldx
   }
   z = block_sum(z, red);
   const double zansa = 2.0 * z - ld(gb, 0) * ld(gb, 0);
-  if (threadIdx.x == 0) {
-    const int iter = s.iter[b];
-    const double eigb = s.eigb[b];
-    const double de = fabs(eigb - e);
-    const int stop = (b < pm.noband && iter >= pm.itermx) || (b >= pm.noband && iter >= pm.iteremx) ||
-                     zansa < pm.tolera || de < pm.tolera || zansa < s.z000re[b] * pm.roughfzan ||
-                     (iter > 1 && de < s.x000re[b] * pm.roughfeig);
-    s.eig[b] = e;
-    s.zansa[b] = zansa;
-    if (stop) {
-      s.active[b] = 0;
-    } else {
-      if (iter == 1) s.x000re[b] = de;
-      if (zansa > s.zansab[b]) {
-        if (++s.izcnt[b] > 20) { s.izcnt[b] = 0; s.lreset[b] = 1; }
-      }
-      s.zansab[b] = zansa;
-      s.eigb[b] = e;
-    }
-    stop_sh = stop;
+  if (threadIdx.x == 0) bkl_stop(s, pm, b, s.iter[b], e, zansa);
+}
+
+// ---- the one-rank band order ------------------------------------------------
+// A CG step of band *cur is a chain of kernels in a graph loop, so its length
+// in kernels and the slowest of them bound it.  The step is arranged so that
+// every sweep over the band runs on many CTAs and every reduction ends in the
+// kernel that needs it:
+//   * g is kept preconditioned (g <- prcd (e x - hx), with zp = <g|g>), so
+//     h = g + beta h (beta = zp / zp of the previous step) is formed where it
+//     is read;
+//   * k_seq_dots: p_j = <s_j|h> and q_j = <s_j|x> for the snapshot columns
+//     s_j of the bands below, and <x|h>;
+//   * k_seq_axpy_h: subgs3 and subgs4 in one pass, h <- h - sum_j p_j s_j -
+//     hhx x with hhx = <x|h> - sum_j p_j q_j = <x|h - sum_j p_j s_j>;
+//   * H|h>: the FFT pipeline beside the two KB kernels;
+//   * k_seq_update, one cluster of CTAs: <h|hx>, <h|gh>, <h|h>, the BKL step,
+//     x, hx, g, the residual and the next band.
+// Before this the step ran thirteen kernels in a row, four of them (g and h,
+// the projection on x, the update) sweeping the band on one SM.
+// One sweep at Si64 (FP64, 160 bands): 25.6 -> 16.2 ms.
+
+// g = prcd (e x - hx) of every band at entry, with its <g|g> before (z) and
+// after (zp, in s.cai) the preconditioner.
+template <typename T>
+__global__ void __launch_bounds__(CGT) k_seq_init(int ne, long ldx, const T *__restrict__ x,
+                                                  const T *__restrict__ hx, T *__restrict__ g,
+                                                  const double *__restrict__ dk, CgState s) {
+  __shared__ double red[CGT / 32];
+  const int b = blockIdx.x;
+  const T *xb = x + b * ldx, *hb = hx + b * ldx;
+  T *gb = g + b * ldx;
+  const double e = bdot(xb, hb, ne, red), e15 = 1.5 * s.ekib[b];
+  double z = 0.0, zp = 0.0;
+  for (int i = threadIdx.x; i < ne; i += blockDim.x) {
+    const T v = (T)e * xb[i] - hb[i];
+    const T w = (T)((double)v * prpcg(dk[i], e15));
+    gb[i] = w;
+    const double f = i == 0 ? 1.0 : 2.0;
+    z += f * (double)v * (double)v;
+    zp += f * (double)w * (double)w;
   }
-  if constexpr (SEQ) {
-    __syncthreads();
-    if (stop_sh) {
-      // each thread reads back the elements of x it wrote above
-      T *sb = (T *)q.snap + b * ldx;
-      for (int i = threadIdx.x; i < ne; i += blockDim.x) {
-        const T v = xb[i];
-        sb[i] = q.ccreal4 ? (T)(float)v : v;
-      }
-      if (threadIdx.x == 0) {
-        const int nx = b + 1;
-        *q.cur = nx;
-        q.pairs[0] = nx;
-        q.pairs[1] = -1;
-        q.list[0] = nx;
-        if (nx >= q.nb) cudaGraphSetConditional(q.handle, 0);
-      }
-    }
+  z = block_sum(z, red);
+  zp = block_sum(zp, red);
+  if (threadIdx.x == 0) {
+    s.eig[b] = e;
+    s.zansa[b] = z;
+    s.zansab[b] = z;
+    s.z000re[b] = z;
+    s.x000re[b] = 1.0e10;
+    s.eigb[b] = e;
+    s.dinnerx[b] = 0.0;
+    s.betk[b] = 0.0;
+    s.cai[b] = zp;
+    s.izcnt[b] = 0;
+    s.lreset[b] = 1;
+    s.iter[b] = 0;
+    s.active[b] = 1;
   }
 }
 
@@ -270,43 +321,232 @@ __global__ void k_seq_reset(SeqArgs q) {
   *q.cur = 0;
   q.pairs[0] = 0;
   q.pairs[1] = -1;
-  q.list[0] = 0;
 }
 
-// Band-space dot products against band *cur: one CTA per vector j.
+// h of band b before the projections (the previous h does not enter after a reset).
 template <typename T>
-__global__ void __launch_bounds__(256) k_seq_dots(int nmax, const int *__restrict__ n_dev, int ne,
-                                                  const T *__restrict__ V, long ldv, const T *__restrict__ Y, long ldy,
-                                                  const int *__restrict__ cur, int gamma, const T *__restrict__ scale,
-                                                  double *__restrict__ out) {
-  __shared__ double red[8];
-  const int j = blockIdx.x;
-  const int n = n_dev ? min(nmax, *n_dev) : nmax;
-  if (j >= n) return;
-  const T *v = V + j * ldv, *y = Y + (long)*cur * ldy;
-  double sum = 0.0;
-  for (int i = threadIdx.x; i < ne; i += blockDim.x) sum += (double)v[i] * (double)y[i];
-  sum = block_sum(sum, red);
-  if (threadIdx.x == 0) {
-    double r = 2.0 * sum - (double)v[0] * (double)y[0];
-    if (gamma == 2) r -= 2.0 * (double)v[1] * (double)y[1];
-    if (scale) r *= (double)scale[j];
-    out[j] = r;
+__device__ __forceinline__ T seq_h(const T *gb, const T *hb, int i, T beta, bool reset) {
+  return reset ? gb[i] : gb[i] + beta * hb[i];
+}
+
+// CTA j < b: p[j], q[j]; CTA b: p[b] = <x|h>.
+constexpr int SQD_T = 512;
+template <typename T>
+__global__ void __launch_bounds__(SQD_T) k_seq_dots(int ne, long ldx, const T *__restrict__ snap,
+                                                    const T *__restrict__ x, const T *__restrict__ g,
+                                                    const T *__restrict__ h, CgState s,
+                                                    const int *__restrict__ cur, int nb, double *__restrict__ p,
+                                                    double *__restrict__ q) {
+  __shared__ double red[2][SQD_T / 32];
+  const int b = *cur, j = blockIdx.x;
+  if (b >= nb || j > b) return;
+  const T *xb = x + b * ldx, *gb = g + b * ldx, *hb = h + b * ldx;
+  const T *v = j < b ? snap + j * ldx : xb;
+  const bool reset = s.lreset[b];
+  const T beta = reset ? (T)0 : (T)(s.cai[b] / s.betk[b]);
+  double sh = 0.0, sx = 0.0;
+#pragma unroll 4
+  for (int i = threadIdx.x; i < ne; i += SQD_T) {
+    const double f = i == 0 ? 1.0 : 2.0, a = f * (double)v[i];
+    sh += a * (double)seq_h(gb, hb, i, beta, reset);
+    sx += a * (double)xb[i];
+  }
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    sh += __shfl_xor_sync(0xffffffffu, sh, o);
+    sx += __shfl_xor_sync(0xffffffffu, sx, o);
+  }
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  if (lane == 0) { red[0][warp] = sh; red[1][warp] = sx; }
+  __syncthreads();
+  if (warp < 2) {
+    double r = lane < SQD_T / 32 ? red[warp][lane] : 0.0;
+#pragma unroll
+    for (int o = 8; o > 0; o >>= 1) r += __shfl_xor_sync(0xffffffffu, r, o);
+    if (lane == 0) {
+      if (warp == 0) p[j] = r;
+      else if (j < b) q[j] = r;
+    }
   }
 }
 
-// Y_cur[i] += sign * sum_j coef[j] V_j[i]: a CTA owns 32 consecutive rows (one
-// per lane); warp w takes j = w, w+8, ..., and the eight partial sums are added
+// h <- h - sum_{j<b} p_j s_j - hhx x: a CTA owns 32 consecutive rows (one per
+// lane); warp w takes j = w, w + 8, ..., and the eight partial sums are added
 // in a fixed order.
 template <typename T>
-__global__ void __launch_bounds__(256) k_seq_axpy(int nmax, const int *__restrict__ n_dev, int ne,
-                                                  const T *__restrict__ V, long ldv, const double *__restrict__ coef,
-                                                  double sign, T *__restrict__ Y, long ldy,
-                                                  const int *__restrict__ cur) {
+__global__ void __launch_bounds__(256) k_seq_axpy_h(int ne, long ldx, const T *__restrict__ snap,
+                                                    const T *__restrict__ x, const T *__restrict__ g,
+                                                    T *__restrict__ h, CgState s, const int *__restrict__ cur,
+                                                    int nb, const double *__restrict__ p,
+                                                    const double *__restrict__ q) {
+  __shared__ double part[8][33];
+  __shared__ double pq[8];
+  const int b = *cur;
+  if (b >= nb) return;
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  const int i = blockIdx.x * 32 + lane;
+  double acc = 0.0, c = 0.0;
+  if (i < ne) {
+    int j = w;
+    for (; j + 24 < b; j += 32) {
+      const T a0 = snap[j * ldx + i], a1 = snap[(j + 8) * ldx + i];
+      const T a2 = snap[(j + 16) * ldx + i], a3 = snap[(j + 24) * ldx + i];
+      acc += p[j] * (double)a0;
+      acc += p[j + 8] * (double)a1;
+      acc += p[j + 16] * (double)a2;
+      acc += p[j + 24] * (double)a3;
+    }
+    for (; j < b; j += 8) acc += p[j] * (double)snap[j * ldx + i];
+  }
+  for (int j = threadIdx.x; j < b; j += 256) c += p[j] * q[j];
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) c += __shfl_xor_sync(0xffffffffu, c, o);
+  part[w][lane] = acc;
+  if (lane == 0) pq[w] = c;
+  __syncthreads();
+  if (w == 0 && i < ne) {
+    double t = 0.0, d = 0.0;
+#pragma unroll
+    for (int u = 0; u < 8; ++u) {
+      t += part[u][lane];
+      d += pq[u];
+    }
+    const bool reset = s.lreset[b];
+    const T beta = reset ? (T)0 : (T)(s.cai[b] / s.betk[b]);
+    T *hb = h + b * ldx;
+    const double hv = (double)seq_h(g + b * ldx, (const T *)hb, i, beta, reset);
+    hb[i] = (T)(hv - t - (p[b] - d) * (double)x[b * ldx + i]);
+  }
+}
+
+// Sum of NV values over the CTAs of a cluster, the same in every thread: each
+// CTA leaves its sums in its own shared memory (slot `ph`, used once), and
+// after the cluster barrier every warp reads all of them, rank by rank.
+constexpr int SQU_C = 8;   // CTAs of the update's cluster (the portable limit)
+template <int NV>
+__device__ __forceinline__ void cluster_sums(double (&v)[NV], double (*red)[32], double *slot) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
+#pragma unroll
+  for (int k = 0; k < NV; ++k) {
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) v[k] += __shfl_xor_sync(0xffffffffu, v[k], o);
+    if (lane == 0) red[k][warp] = v[k];
+  }
+  __syncthreads();
+  if (warp < NV) {
+    double r = lane < nw ? red[warp][lane] : 0.0;
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) r += __shfl_xor_sync(0xffffffffu, r, o);
+    if (lane == 0) slot[warp] = r;
+  }
+  cg::cluster_group cl = cg::this_cluster();
+  cl.sync();
+#pragma unroll
+  for (int k = 0; k < NV; ++k) {
+    double r = lane < SQU_C ? cl.map_shared_rank(slot, lane & (SQU_C - 1))[k] : 0.0;
+#pragma unroll
+    for (int o = SQU_C / 2; o > 0; o >>= 1) r += __shfl_xor_sync(0xffffffffu, r, o);
+    v[k] = __shfl_sync(0xffffffffu, r, 0);
+  }
+}
+
+// The update of band *cur by one cluster; when the band stops, its final
+// vector has become its snapshot column (cgjr(:,ib) = gdcr(:,ibb),
+// eigen.f90:699, real*4 when q.ccreal4) and the next band starts.
+template <typename T>
+__global__ void __cluster_dims__(SQU_C, 1, 1) __launch_bounds__(CGT)
+    k_seq_update(int ne, long ldx, T *__restrict__ x, T *__restrict__ hx, T *__restrict__ g, const T *__restrict__ h,
+                 const T *__restrict__ gh, const double *__restrict__ dk, CgState s, CgParm pm, SeqArgs q) {
+  __shared__ double red[3][32];
+  __shared__ double slot[3][4];
+  cg::cluster_group cl = cg::this_cluster();
+  const int b = *q.cur;   // every CTA reads it before the first cluster barrier
+  const bool first = blockIdx.x == 0 && threadIdx.x == 0;
+  if (b >= q.nb) {        // the same in every CTA
+    if (first) cudaGraphSetConditional(q.handle, 0);
+    return;
+  }
+  T *xb = x + b * ldx, *hxb = hx + b * ldx, *gb = g + b * ldx, *sb = (T *)q.snap + b * ldx;
+  const T *hb = h + b * ldx, *ghb = gh + b * ldx;
+  const double dinx = s.dinnerx[b], e15 = 1.5 * s.ekib[b];
+  double e = s.eig[b], dtnew, alpsq;
+  const int i0 = blockIdx.x * CGT + threadIdx.x, step = SQU_C * CGT;
+  double v[3] = {0.0, 0.0, 0.0};
+  for (int i = i0; i < ne; i += step) {
+    const double f = i == 0 ? 1.0 : 2.0, hv = (double)hb[i];
+    v[0] += f * hv * (double)hxb[i];
+    v[1] += f * hv * (double)ghb[i];
+    v[2] += f * hv * hv;
+  }
+  cluster_sums<3>(v, red, slot[0]);
+  if (v[2] > 0.0) {
+    bkl_step(v[0], v[1], v[2], e, dtnew, alpsq);
+  } else {                // the same in every thread of the cluster
+    double w[1] = {0.0};
+    for (int i = i0; i < ne; i += step) w[0] += (i == 0 ? 1.0 : 2.0) * (double)hb[i] * (double)xb[i];
+    __syncthreads();
+    cluster_sums<1>(w, red, slot[1]);
+    bkl_line(v[0], v[1], v[2], w[0], dinx, pm, &s.dinnerx[b], first, e, dtnew, alpsq);
+  }
+  const T a = (T)alpsq, dt = (T)dtnew, et = (T)e;
+  double z[2] = {0.0, 0.0};
+  for (int i = i0; i < ne; i += step) {
+    const T xn = a * (xb[i] + dt * hb[i]);
+    const T hn = a * (hxb[i] + dt * ghb[i]);
+    xb[i] = xn;
+    hxb[i] = hn;
+    sb[i] = q.ccreal4 ? (T)(float)xn : xn;
+    const T gv = et * xn - hn;
+    const T gp = (T)((double)gv * prpcg(dk[i], e15));
+    gb[i] = gp;
+    const double f = i == 0 ? 1.0 : 2.0;
+    z[0] += f * (double)gv * (double)gv;
+    z[1] += f * (double)gp * (double)gp;
+  }
+  __syncthreads();
+  cluster_sums<2>(z, red, slot[2]);
+  if (first) {
+    const int iter = s.iter[b] + 1;
+    s.iter[b] = iter;
+    s.lreset[b] = 0;
+    s.betk[b] = s.cai[b];
+    s.cai[b] = z[1];
+    if (bkl_stop(s, pm, b, iter, e, z[0])) {
+      const int nx = b + 1;
+      *q.cur = nx;
+      q.pairs[0] = nx;
+      q.pairs[1] = -1;
+      if (nx >= q.nb) cudaGraphSetConditional(q.handle, 0);
+    }
+  }
+  cl.sync();   // no CTA leaves while another still reads its sums
+}
+
+// KB projections of band *cur: out[j] = scale_j (2 sum B_j y - B_j(0) y(0) -
+// 2 B_j(1) y(1)), one CTA per projector j.
+template <typename T>
+__global__ void __launch_bounds__(256) k_seq_kb_dots(int ne, const T *__restrict__ V, long ldv,
+                                                     const T *__restrict__ Y, long ldy, const int *__restrict__ cur,
+                                                     const T *__restrict__ scale, double *__restrict__ out) {
+  __shared__ double red[8];
+  const int j = blockIdx.x;
+  const T *v = V + j * ldv, *y = Y + (long)*cur * ldy;
+  double sum = 0.0;
+#pragma unroll 4
+  for (int i = threadIdx.x; i < ne; i += 256) sum += (double)v[i] * (double)y[i];
+  sum = block_sum(sum, red);
+  if (threadIdx.x == 0)
+    out[j] = (2.0 * sum - (double)v[0] * (double)y[0] - 2.0 * (double)v[1] * (double)y[1]) * (double)scale[j];
+}
+
+// Y_cur(i) = sum_j coef_j B_j(i) (rows and order as in k_seq_axpy_h).
+template <typename T>
+__global__ void __launch_bounds__(256) k_seq_kb_axpy(int n, int ne, const T *__restrict__ V, long ldv,
+                                                     const double *__restrict__ coef, T *__restrict__ Y, long ldy,
+                                                     const int *__restrict__ cur) {
   __shared__ double part[8][33];
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   const int i = blockIdx.x * 32 + lane;
-  const int n = n_dev ? min(nmax, *n_dev) : nmax;
   double acc = 0.0;
   if (i < ne) {
     int j = w;
@@ -325,9 +565,8 @@ __global__ void __launch_bounds__(256) k_seq_axpy(int nmax, const int *__restric
   if (w == 0 && i < ne) {
     double t = 0.0;
 #pragma unroll
-    for (int q = 0; q < 8; ++q) t += part[q][lane];
-    T *y = Y + (long)*cur * ldy;
-    y[i] = (T)((double)y[i] + sign * t);
+    for (int u = 0; u < 8; ++u) t += part[u][lane];
+    Y[(long)*cur * ldy + i] = (T)t;
   }
 }
 
@@ -407,17 +646,15 @@ __global__ void k_scale_rows(int nproj, int ncol, T *__restrict__ P, long ldp, c
 template <typename T> void cg_init(int nb, int ne, long ldx, const T *x, const T *hx, T *g, const CgState &s, cudaStream_t st) {
   k_cg_init<T><<<nb, CGT, 0, st>>>(ne, ldx, x, hx, g, s); note_launch();
 }
-template <typename T> void cg_prec(int nb, int ne, long ldx, T *g, T *h, const double *dk, const CgState &s, cudaStream_t st,
-                                   const int *cur) {
-  k_cg_prec<T><<<cur ? 1 : nb, CGT, 0, st>>>(ne, ldx, g, h, dk, s, cur, nb); note_launch();
+template <typename T> void cg_prec(int nb, int ne, long ldx, T *g, T *h, const double *dk, const CgState &s, cudaStream_t st) {
+  k_cg_prec<T><<<nb, CGT, 0, st>>>(ne, ldx, g, h, dk, s); note_launch();
 }
 template <typename T> void cg_mask(int nb, T *Pm, const CgState &s, cudaStream_t st) {
   const long nn = (long)nb * nb;
   k_cg_mask<T><<<(int)((nn + 255) / 256), 256, 0, st>>>(nb, Pm, s); note_launch();
 }
-template <typename T> void cg_orth(int nb, int ne, long ldx, const T *x, const T *hx, T *h, const CgState &s, cudaStream_t st,
-                                   const int *cur) {
-  k_cg_orth<T><<<cur ? 1 : nb, CGT, 0, st>>>(ne, ldx, x, hx, h, s, cur, nb); note_launch();
+template <typename T> void cg_orth(int nb, int ne, long ldx, const T *x, const T *hx, T *h, const CgState &s, cudaStream_t st) {
+  k_cg_orth<T><<<nb, CGT, 0, st>>>(ne, ldx, x, hx, h, s); note_launch();
 }
 void cg_list(int nb, const CgState &s, cudaStream_t st) { k_cg_list<<<1, 32, 0, st>>>(nb, s); note_launch(); }
 void gradres_stats(const double *prod, const double *occ, int nb, double *out, cudaStream_t st) {
@@ -426,21 +663,27 @@ void gradres_stats(const double *prod, const double *occ, int nb, double *out, c
 void iter_sum(const int *iter, int nb, int *out, cudaStream_t st) { k_iter_sum<<<1, 32, 0, st>>>(iter, nb, out); note_launch(); }
 template <typename T> void cg_update(int nb, int ne, long ldx, T *x, T *hx, T *g, const T *h, const T *gh,
                                      const CgState &s, const CgParm &pm, cudaStream_t st) {
-  k_cg_update<T, false><<<nb, CGT, 0, st>>>(ne, ldx, x, hx, g, h, gh, s, pm, SeqArgs{}); note_launch();
+  k_cg_update<T><<<nb, CGT, 0, st>>>(ne, ldx, x, hx, g, h, gh, s, pm); note_launch();
 }
-template <typename T> void cg_update_seq(int ne, long ldx, T *x, T *hx, T *g, const T *h, const T *gh, const CgState &s,
-                                         const CgParm &pm, const SeqArgs &q, cudaStream_t st) {
-  k_cg_update<T, true><<<1, CGT, 0, st>>>(ne, ldx, x, hx, g, h, gh, s, pm, q); note_launch();
+template <typename T> void seq_init(int nb, int ne, long ldx, const T *x, const T *hx, T *g, const double *dk,
+                                    const CgState &s, const SeqArgs &q, cudaStream_t st) {
+  k_seq_init<T><<<nb, CGT, 0, st>>>(ne, ldx, x, hx, g, dk, s); note_launch();
+  k_seq_reset<<<1, 1, 0, st>>>(q); note_launch();
 }
-void seq_reset(const SeqArgs &q, cudaStream_t st) { k_seq_reset<<<1, 1, 0, st>>>(q); note_launch(); }
-template <typename T> void seq_dots(int nmax, const int *n_dev, int ne, const T *V, long ldv, const T *Y, long ldy,
-                                    const int *cur, int gamma, const T *scale, double *out, cudaStream_t st) {
-  if (nmax <= 0) return;
-  k_seq_dots<T><<<nmax, 256, 0, st>>>(nmax, n_dev, ne, V, ldv, Y, ldy, cur, gamma, scale, out); note_launch();
+template <typename T> void seq_project(int ne, long ldx, const T *x, const T *g, T *h, const CgState &s,
+                                       const SeqArgs &q, double *p, double *w, cudaStream_t st) {
+  k_seq_dots<T><<<q.nb, SQD_T, 0, st>>>(ne, ldx, (const T *)q.snap, x, g, h, s, q.cur, q.nb, p, w); note_launch();
+  k_seq_axpy_h<T><<<(ne + 31) / 32, 256, 0, st>>>(ne, ldx, (const T *)q.snap, x, g, h, s, q.cur, q.nb, p, w);
+  note_launch();
 }
-template <typename T> void seq_axpy(int nmax, const int *n_dev, int ne, const T *V, long ldv, const double *coef,
-                                    double sign, T *Y, long ldy, const int *cur, cudaStream_t st) {
-  k_seq_axpy<T><<<(ne + 31) / 32, 256, 0, st>>>(nmax, n_dev, ne, V, ldv, coef, sign, Y, ldy, cur); note_launch();
+template <typename T> void seq_kb(int np, int ne, const T *kbg, const T *scale, const T *h, T *gh, long ldx,
+                                  const int *cur, double *coef, cudaStream_t st) {
+  k_seq_kb_dots<T><<<np, 256, 0, st>>>(ne, kbg, ne, h, ldx, cur, scale, coef); note_launch();
+  k_seq_kb_axpy<T><<<(ne + 31) / 32, 256, 0, st>>>(np, ne, kbg, ne, coef, gh, ldx, cur); note_launch();
+}
+template <typename T> void seq_update(int ne, long ldx, T *x, T *hx, T *g, const T *h, const T *gh, const double *dk,
+                                      const CgState &s, const CgParm &pm, const SeqArgs &q, cudaStream_t st) {
+  k_seq_update<T><<<SQU_C, CGT, 0, st>>>(ne, ldx, x, hx, g, h, gh, dk, s, pm, q); note_launch();
 }
 template <typename T> void ekin(int nb, int ne, long ldx, const T *x, const double *dk, double *ekib, cudaStream_t st) {
   k_ekin<T><<<nb, CGT, 0, st>>>(ne, ldx, x, dk, ekib); note_launch();
@@ -457,17 +700,17 @@ template <typename T> void scale_rows(int nproj, int ncol, T *P, long ldp, const
 
 #define QX_INST(T)                                                                                          \
   template void cg_init<T>(int, int, long, const T *, const T *, T *, const CgState &, cudaStream_t);        \
-  template void cg_prec<T>(int, int, long, T *, T *, const double *, const CgState &, cudaStream_t,          \
-                           const int *);                                                                    \
+  template void cg_prec<T>(int, int, long, T *, T *, const double *, const CgState &, cudaStream_t);         \
   template void cg_mask<T>(int, T *, const CgState &, cudaStream_t);                                         \
-  template void cg_orth<T>(int, int, long, const T *, const T *, T *, const CgState &, cudaStream_t,         \
-                           const int *);                                                                    \
-  template void cg_update_seq<T>(int, long, T *, T *, T *, const T *, const T *, const CgState &,            \
-                                 const CgParm &, const SeqArgs &, cudaStream_t);                            \
-  template void seq_dots<T>(int, const int *, int, const T *, long, const T *, long, const int *, int,      \
-                            const T *, double *, cudaStream_t);                                             \
-  template void seq_axpy<T>(int, const int *, int, const T *, long, const double *, double, T *, long,      \
-                            const int *, cudaStream_t);                                                     \
+  template void cg_orth<T>(int, int, long, const T *, const T *, T *, const CgState &, cudaStream_t);        \
+  template void seq_init<T>(int, int, long, const T *, const T *, T *, const double *, const CgState &,      \
+                            const SeqArgs &, cudaStream_t);                                                 \
+  template void seq_project<T>(int, long, const T *, const T *, T *, const CgState &, const SeqArgs &,       \
+                               double *, double *, cudaStream_t);                                           \
+  template void seq_kb<T>(int, int, const T *, const T *, const T *, T *, long, const int *, double *,       \
+                          cudaStream_t);                                                                    \
+  template void seq_update<T>(int, long, T *, T *, T *, const T *, const T *, const double *,                \
+                              const CgState &, const CgParm &, const SeqArgs &, cudaStream_t);              \
   template void cg_update<T>(int, int, long, T *, T *, T *, const T *, const T *, const CgState &,            \
                              const CgParm &, cudaStream_t);                                                  \
   template void ekin<T>(int, int, long, const T *, const double *, double *, cudaStream_t);                  \
