@@ -84,7 +84,6 @@ __device__ __forceinline__ bool grid_barrier(unsigned *bar, unsigned nblk, int *
 constexpr int CB = 32;
 constexpr int CHT = 256;            // threads of k_cholinv (8 warps)
 constexpr int DLD = CB + 1;         // leading dimension of the 32 x 32 temporary
-constexpr size_t CH_SMEM_MAX = 220 * 1024;
 
 // 1/sqrt(x): the hardware's approximate reciprocal square root refined by
 // two Newton-Raphson steps y <- y (3 - x y^2) / 2, each doubling the number
@@ -165,24 +164,18 @@ __device__ __forceinline__ void warp_trinv(const double *L, int ldl, const doubl
   __syncwarp();
 }
 
-// USE_SMEM: the matrix lives in shared memory, and the compiler sees that
-// every access to it is a shared-memory access (no generic addressing).
-template <bool USE_SMEM>
+// The matrix in global memory: sizes beyond one SM's shared memory where the
+// cooperative kernel cannot be launched.
 __global__ void __launch_bounds__(CHT) k_cholinv(double *__restrict__ Sg, int n, double *__restrict__ work,
                                                   int *__restrict__ info) {
-  constexpr bool use_smem = USE_SMEM;
-  extern __shared__ double sm[];
   __shared__ int bad;
-  const int ld = use_smem ? (n | 1) : n;
-  double *A = use_smem ? sm : Sg;
-  double *T = use_smem ? sm + (long)ld * n : work;   // CB x DLD temporary
+  const int ld = n;
+  double *A = Sg;
+  double *T = work;                                  // CB x DLD temporary
   double *rd = T + CB * DLD;                         // n reciprocal pivots
   __shared__ double cb[CB];                          // column broadcast of warp_chol
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nw = CHT / 32;
 #define A_(i, j) A[(long)(j) * ld + (i)]
-  if (use_smem)
-    for (int j = warp; j < n; j += nw)
-      for (int i = lane; i < n; i += 32) A_(i, j) = Sg[(long)j * n + i];
   if (tid == 0) bad = 0;
   __syncthreads();
   const int nblk = (n + CB - 1) / CB;
@@ -291,414 +284,193 @@ __global__ void __launch_bounds__(CHT) k_cholinv(double *__restrict__ Sg, int n,
       __syncthreads();
     }
   }
-  if (use_smem)
-    for (int j = warp; j < n; j += nw)
-      for (int i = lane; i < n; i += 32) Sg[(long)j * n + i] = A_(i, j);
 #undef A_
   if (tid == 0) *info = 0;
 }
 
 // --------------------------------------------------------------------------
-// The same result for n <= CP_MAXN (and within shared memory), 12 warps, one
-// n x n shared-memory matrix (odd leading dimension) holding L in the lower
-// triangle and X^T = (L^-1)^T strictly above it (X's diagonal apart):
-//  * Cholesky right-looking in panels of PB = 8 columns: warp 0 factors the
-//    panel in registers (rows lane + 32 q, column values by shuffle, no CTA
-//    barrier inside the panel) and copies it row-major to Pr; all warps then
-//    apply the rank-8 update to the trailing lower triangle;
-//  * inverse in 32 x 32 blocks: the diagonal blocks inverted side by side
-//    (one warp each); M_IK = -X_II L_IK in place of L_IK (all blocks at
-//    once); X_IJ = sum_{K=J}^{I-1} M_IK X_KJ by block diagonals d = I - J
-//    (the blocks of one diagonal at once, two warps a block).  Every inner
-//    loop runs over compile-time indices into registers.
-constexpr int CPT = 384, CPW = CPT / 32, PB = 8, CP_MQ = 6;
-constexpr int CP_MAXN = 32 * CP_MQ;   // also bounded by shared memory
-
-__global__ void __launch_bounds__(CPT) k_cholinv_sm(double *__restrict__ Sg, int n, int *__restrict__ info) {
-  extern __shared__ double smf[];
-  __shared__ int bad;
-  const int ld = n | 1;
-  double *A = smf, *xd = A + (long)ld * n, *rd = xd + n, *Pr = rd + n;   // Pr: PB * n
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-#define AA(i, j) A[(j) * ld + (i)]
-  if (tid == 0) bad = 0;
-  for (int j = warp; j < n; j += CPW)
-    for (int i = j + lane; i < n; i += 32) AA(i, j) = Sg[(long)j * n + i];
-  __syncthreads();
-  // ---------------- Cholesky ----------------
-  for (int j0 = 0; j0 < n; j0 += PB) {
-    const int pb = min(PB, n - j0);
-    if (warp == 0) {
-      double a[CP_MQ][PB];
-#pragma unroll
-      for (int q = 0; q < CP_MQ; ++q) {
-        const int r = j0 + lane + 32 * q, rr = min(r, n - 1);
-#pragma unroll
-        for (int c = 0; c < PB; ++c) {
-          const double v = AA(rr, min(j0 + c, n - 1));   // clamped address, then selection
-          a[q][c] = (c < pb && r < n && r >= j0 + c) ? v : 0.0;
-        }
-      }
-      int b = 0;
-#pragma unroll
-      for (int c = 0; c < PB; ++c) {
-        if (c < pb && b == 0) {   // uniform
-          const double piv = __shfl_sync(0xffffffffu, a[0][c], c);   // row j0 + c: lane c, q 0
-          if (!(piv > 1.0e-30)) {   // uniform; also catches NaN
-            b = 1 + j0 + c;
-          } else {
-            const double rs = rsqrt_nr(piv);
-#pragma unroll
-            for (int q = 0; q < CP_MQ; ++q) {
-              const int r = j0 + lane + 32 * q;
-              a[q][c] = (r == j0 + c) ? piv * rs : a[q][c] * rs;
-            }
-            if (lane == 0) rd[j0 + c] = rs;
-            // columns c2 > c; rows above row j0 + c2 pick up values that are
-            // never read (only rows >= j0 + c2 of column c2 are stored)
-#pragma unroll
-            for (int c2 = c + 1; c2 < PB; ++c2) {
-              const double l = __shfl_sync(0xffffffffu, a[0][c], c2);   // L(j0 + c2, j0 + c)
-#pragma unroll
-              for (int q = 0; q < CP_MQ; ++q) a[q][c2] -= a[q][c] * l;
-            }
-          }
-        }
-      }
-      if (b) {
-        if (lane == 0) bad = b;
-      } else {
-#pragma unroll
-        for (int q = 0; q < CP_MQ; ++q) {
-          const int r = j0 + lane + 32 * q;
-          if (r < n) {
-#pragma unroll
-            for (int c = 0; c < PB; ++c) {
-              if (c < pb && r >= j0 + c) AA(r, j0 + c) = a[q][c];
-              Pr[r * PB + c] = (c < pb) ? a[q][c] : 0.0;   // zero above the diagonal
-            }
-          }
-        }
-      }
-    }
-    __syncthreads();
-    if (bad) break;   // uniform
-    // trailing update: A(i, j) -= sum_c L(i, j0+c) L(j, j0+c), j0+pb <= j <= i;
-    // rows by lane in 32-row chunks, columns by warp, four columns at a time
-    const int t0 = j0 + pb;
-    if (t0 < n) {
-      const int nch = (n - t0 + 31) / 32;
-#pragma unroll 1
-      for (int ch = 0; ch < nch; ++ch) {
-        const int i = t0 + ch * 32 + lane;
-        const bool rowok = i < n;
-        double li[PB];
-#pragma unroll
-        for (int c = 0; c < PB; ++c) {
-          const double v = Pr[min(i, n - 1) * PB + c];
-          li[c] = rowok ? v : 0.0;
-        }
-        const int jend = min(n, t0 + ch * 32 + 32);   // columns up to this chunk's last row
-#pragma unroll 1
-        for (int jb = t0 + 4 * warp; jb < jend; jb += 4 * CPW) {
-          double acc[4];
-#pragma unroll
-          for (int u = 0; u < 4; ++u) {
-            const int j = min(jb + u, n - 1);
-            double s0 = 0.0, s1 = 0.0;
-#pragma unroll
-            for (int c = 0; c < PB; c += 2) {
-              s0 += li[c] * Pr[j * PB + c];
-              s1 += li[c + 1] * Pr[j * PB + c + 1];
-            }
-            acc[u] = s0 + s1;
-          }
-#pragma unroll
-          for (int u = 0; u < 4; ++u) {
-            const int j = jb + u;
-            if (rowok && j < jend && i >= j) AA(i, j) -= acc[u];
-          }
-        }
-      }
-    }
-    __syncthreads();
-  }
-  if (bad) {
-    if (tid == 0) *info = bad;
-    return;
-  }
-  // ---------------- inverse ----------------
-  const int nblk = (n + 31) / 32;
-  // diagonal blocks: lane = column c of X_JJ, forward substitution down the
-  // rows; X(r, c), r > c, goes to A(c, r), the diagonal to xd
-  for (int J = warp; J < nblk; J += CPW) {
-    const int j0 = J * 32, bs = min(32, n - j0);
-    // rows past the matrix (last block) read row n - 1 and are zeroed
-    double x[32];
-#pragma unroll
-    for (int r = 0; r < 32; ++r) {
-      const int rr = min(j0 + r, n - 1);
-      double sum = (r == lane) ? 1.0 : 0.0;
-#pragma unroll
-      for (int k = 0; k < r; ++k) sum -= AA(rr, min(j0 + k, n - 1)) * x[k];
-      x[r] = (r < bs) ? sum * rd[rr] : 0.0;
-    }
-    if (lane < bs) {
-#pragma unroll
-      for (int r = 0; r < 32; ++r) {
-        if (r < bs && r > lane) AA(j0 + lane, j0 + r) = x[r];
-        if (r == lane) xd[j0 + lane] = x[r];
-      }
-    }
-  }
-  __syncthreads();
-  // M_IK = -X_II L_IK in place of L_IK, one warp per block; lane = row i,
-  // which holds row i of X_II in registers
-  for (int pair = warp; pair < nblk * (nblk - 1) / 2; pair += CPW) {
-    int I = 1;
-    while (I * (I + 1) / 2 <= pair) ++I;
-    const int K = pair - I * (I - 1) / 2;
-    const int i0 = I * 32, k0 = K * 32, bi = min(32, n - i0);
-    const bool rowok = lane < bi;
-    // row i of X_II (zero past the diagonal and for rows past the matrix);
-    // loads from clamped addresses, selection after the load
-    const int ir = min(i0 + lane, n - 1);
-    double xr[32];
-#pragma unroll
-    for (int k = 0; k < 32; ++k) {
-      const int kr = min(i0 + k, n - 1);
-      const double v = AA(kr, ir), dv = xd[kr];
-      xr[k] = (!rowok || k > lane || k >= bi) ? 0.0 : (k == lane ? dv : v);
-    }
-#pragma unroll 1
-    for (int c = 0; c < 32; ++c) {   // the columns of block K are full (K < I)
-      const double *col = &AA(0, k0 + c);
-      double s0 = 0.0, s1 = 0.0;
-#pragma unroll
-      for (int k = 0; k < 32; k += 2) {
-        s0 += xr[k] * col[min(i0 + k, n - 1)];
-        s1 += xr[k + 1] * col[min(i0 + k + 1, n - 1)];
-      }
-      __syncwarp();
-      if (rowok) AA(i0 + lane, k0 + c) = -(s0 + s1);
-      __syncwarp();
-    }
-  }
-  __syncthreads();
-  // X_IJ = sum_{K=J}^{I-1} M_IK X_KJ by block diagonals; two warps a block
-  // (16 columns each), lane = row i; X(k, c) for k > c read from A(c, k)
-  for (int d = 1; d < nblk; ++d) {
-    const int nb_d = nblk - d;
-    for (int task = warp; task < nb_d * 2; task += CPW) {
-      const int J = task >> 1, half = task & 1, I = J + d;
-      const int i0 = I * 32, j0 = J * 32, bi = min(32, n - i0);
-      const int cb = j0 + 16 * half;
-      const int i = i0 + lane;
-      const bool rowok = lane < bi;
-      const int ir = min(i, n - 1);
-      double acc[16], xdv[16];
-#pragma unroll
-      for (int u = 0; u < 16; ++u) {
-        acc[u] = 0.0;
-        xdv[u] = xd[cb + u];
-      }
-#pragma unroll 1
-      for (int K = J; K < I; ++K) {
-        const int k0 = K * 32;
-#pragma unroll 1
-        for (int kk = 0; kk < 32; ++kk) {
-          const int k = k0 + kk;
-          const double mv = AA(ir, k);
-          const double m = rowok ? mv : 0.0;
-          const double *xrow = &AA(cb, k);   // X(k, cb + u) = A(cb + u, k) for k > cb + u
-#pragma unroll
-          for (int u = 0; u < 16; ++u) {
-            const int c = cb + u;
-            const double xu = xrow[u];
-            const double xv = (k > c) ? xu : ((k == c) ? xdv[u] : 0.0);
-            acc[u] += m * xv;
-          }
-        }
-      }
-      if (rowok) {
-#pragma unroll
-        for (int u = 0; u < 16; ++u) AA(cb + u, i) = acc[u];   // X(i, c) to A(c, i)
-      }
-    }
-    __syncthreads();
-  }
-  // out: X in the lower triangle, zeros above
-  for (int j = warp; j < n; j += CPW)
-    for (int i = lane; i < n; i += 32) Sg[(long)j * n + i] = (i > j) ? AA(j, i) : ((i == j) ? xd[j] : 0.0);
-#undef AA
-  if (tid == 0) *info = 0;
+// Cholesky and L^-1 in one CTA for n <= CM_MAXN, by 16-column blocks with the
+// FP64 tensor cores (mma m8n8k4).  X = L^-1 comes from the same elimination:
+// the matrix [S | I] is reduced block by block, and as S's columns are
+// consumed their place is taken by X's (both are lower triangular), so one
+// lower triangle holds the state.  Block k (rows and columns 16k .. 16k + 15):
+//   (A) warp 0 reduces the 16 x 16 diagonal block beside the identity in
+//       registers (lane = column): X_D = L_D^-1;
+//   (B) the panel P(i, :), by warps of 8 columns i: S(i, blk) X_D^T = L(i,
+//       blk) below the block, X_D R(blk, i) = X(blk, i) left of it (final,
+//       stored) and X_D's columns inside it;
+//   (C) every 8 x 8 tile (I, J <= I) below the block: A -= P(I) P(J)^T, the
+//       block's own columns starting from zero.
+// Warp 0 updates the next diagonal block first and goes on to its (A) while
+// the other warps finish (C), so the chain of 16 pivots a block runs beside
+// the products: two barriers a block.  Tiles are stored one after another
+// with their pairs of columns swizzled by row, so that fragment accesses and
+// the column-wise transfers from and to global memory meet few bank
+// conflicts.  Rows past n are an identity.
+// What bounds it: the pivot chain (about 150 cycles a column) and the FP64
+// rate of one SM for n^3 / 3 products.  At n = 160: 142 us with the matrix in
+// registers and one rank-2 update and barrier per column pair, 56 us so.
+// info: 0, or 1 + the first row whose pivot is not > 1e-30 (S then left as it was).
+constexpr int CMT = 512, CMW = CMT / 32, CM_MAXN = 208, CM_LD = 20;
+constexpr int cm_tiles(int n) { const int nt = 2 * ((n + 15) / 16); return nt * (nt + 1) / 2; }
+constexpr size_t cm_smem(int n) {
+  return sizeof(double) * ((size_t)cm_tiles(n) * 64 + (size_t)16 * ((n + 15) / 16) * CM_LD + 16 * CM_LD);
+}
+__device__ __forceinline__ int cm_tile(int I, int J) { return (I * (I + 1) / 2 + J) * 64; }
+// position of element (r, c) in a tile, and of its column pair c & ~1
+__device__ __forceinline__ int cm_pos(int r, int c) { return r * 8 + 2 * ((c >> 1) ^ ((r >> 1) & 3)) + (c & 1); }
+__device__ __forceinline__ void cm_mma(double (&d)[2], double a, double b) {
+  asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1}, {%2}, {%3}, {%0,%1};\n"
+               : "+d"(d[0]), "+d"(d[1])
+               : "d"(a), "d"(b));
 }
 
-// Cholesky and L^-1 together with the matrix in registers (n <= W NR and
-// n <= 32 NC; one CTA of W warps; thread (w, l) keeps rows NR w .. NR w + NR - 1
-// of the columns l + 32 c).  X = L^-1 is found by rows (X L = I top down)
-// with running right-hand sides R (R(i,:) = e_i at the start), stored where L
-// was consumed.  Columns go two at a time (k, k + 1; NR even, so rows k and
-// k + 1 sit in one warp): columns k and k + 1 (the Schur complement) are
-// published and replaced by e_k, e_(k+1), which start R's columns; rows k
-// and k + 1 (R(k, :), R(k+1, :)) are published; one barrier.  Then
-// L(k,k) = sqrt(piv0), l = L(k+1,k), L(k+1,k+1) = sqrt(piv1 - l^2),
-// m0_i = L(i,k), m1_i = L(i,k+1) and y0, y1 (the rows of X for the columns
-// <= k + 1, the L columns beyond) give every row below k one rank-2 update
-// a(i,:) -= m0_i y0 + m1_i y1: the Cholesky update of the columns > k + 1 and
-// the forward-substitution update of the columns <= k + 1 (y0 is 0 at k + 1:
-// that part of the Schur update is folded into piv1).  Rows k and k + 1 are
-// final from then on and are scaled by their 1 / L(i,i) when written out.
-// The gathered columns and rows alternate by parity, so one barrier a step
-// suffices.  The matrix is staged through shared memory on the way in (the
-// lower triangle, as rsdecmp reads it) and out (coalesced column-major
-// stores).  info as k_cholinv_sm; S is left as it was on failure.
-template <int W, int NR, int NC>
-__global__ void __launch_bounds__(W * 32, 1) k_cholinv_rg(double *__restrict__ Sg, int n, int *__restrict__ info) {
-  constexpr int NROW = W * NR, NCOL = 32 * NC;
-  constexpr int NX = NROW > NCOL ? NROW : NCOL;
-  static_assert(NR <= 32 && NR % 2 == 0, "lane r of a warp keeps m of row r; row pairs stay in one warp");
-  extern __shared__ double stg[];   // n x (n | 1) staging
-  __shared__ __align__(16) double xcol[2][2][NX];
-  __shared__ __align__(16) double xrow[2][2][NX];
-  __shared__ double rsv[NX];
-  __shared__ double2 mw[W][NR];     // m0, m1 of each warp's rows (read back as broadcasts)
-  const int ld = n | 1;
+// (A): the diagonal block k of T to X_D (xd, row-major, zeros above the
+// diagonal); returns 0 or 1 + the first bad row.  One whole warp.
+__device__ __forceinline__ int cm_diag(const double *T, int k, double *xd, int lane) {
+  double a[16];
+#pragma unroll
+  for (int r = 0; r < 16; ++r) {
+    // lane < 16: column lane of S, by symmetry from the lower triangle
+    const int c = lane & 15, hi = max(r, c), lo = min(r, c);
+    const double v = T[cm_tile(2 * k + (hi >> 3), 2 * k + (lo >> 3)) + cm_pos(hi & 7, lo & 7)];
+    a[r] = lane < 16 ? v : (r == c ? 1.0 : 0.0);
+  }
+  int bad = 0;
+#pragma unroll
+  for (int s = 0; s < 16; ++s) {
+    const double piv = __shfl_sync(0xffffffffu, a[s], s);
+    if (bad == 0 && !(piv > 1.0e-30)) bad = 1 + 16 * k + s;   // uniform; also catches NaN
+    const double rs = rsqrt_nr(piv);
+    const double y = a[s] * rs;
+    a[s] = y;
+#pragma unroll
+    for (int r = s + 1; r < 16; ++r) a[r] = fma(-(__shfl_sync(0xffffffffu, a[r], s) * rs), y, a[r]);
+  }
+  if (lane >= 16) {
+    const int c = lane - 16;
+#pragma unroll
+    for (int r = 0; r < 16; ++r) xd[r * CM_LD + c] = r >= c ? a[r] : 0.0;
+  }
+  return bad;
+}
+
+// (C) for one tile: C = (from ? A : 0) - P(I) P(J)^T.
+__device__ __forceinline__ void cm_update(double *T, const double *P, int I, int J, bool from, const double (&af)[4],
+                                          int lane) {
+  const int row = lane >> 2, kk = lane & 3;
+  double2 *cp = reinterpret_cast<double2 *>(T + cm_tile(I, J) + cm_pos(row, 2 * kk));
+  const double2 c0 = *cp;
+  double d[2] = {from ? c0.x : 0.0, from ? c0.y : 0.0};
+  const double *pj = P + (J * 8 + row) * CM_LD + kk;
+#pragma unroll
+  for (int s = 0; s < 4; ++s) cm_mma(d, af[s], pj[4 * s]);
+  *cp = make_double2(d[0], d[1]);
+}
+__device__ __forceinline__ void cm_load_a(const double *P, int I, double (&af)[4], int lane) {
+  const double *pi = P + (I * 8 + (lane >> 2)) * CM_LD + (lane & 3);
+#pragma unroll
+  for (int s = 0; s < 4; ++s) af[s] = -pi[4 * s];
+}
+
+__global__ void __launch_bounds__(CMT, 1) k_cholinv_mm(double *__restrict__ Sg, int n, int *__restrict__ info) {
+  extern __shared__ double cm_sm[];
+  __shared__ int bad;
+  __shared__ unsigned char ti[cm_tiles(CM_MAXN)];   // row of tile q
+  const int nb = (n + 15) / 16, nt = 2 * nb, np = 16 * nb;
+  double *T = cm_sm, *P = T + (long)cm_tiles(n) * 64, *xd = P + np * CM_LD;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const int r0 = warp * NR;
-  // global to shared by cp.async: every copy of a thread in flight at once,
-  // none through registers; element q = j n + i, stepped by the block size
-  // without a division
-  {
-    int j = tid / n, i = tid - j * n;
-    for (long q = tid; q < (long)n * n; q += W * 32) {
-      const unsigned sa = (unsigned)__cvta_generic_to_shared(stg + (long)j * ld + i);
-      asm volatile("cp.async.ca.shared.global [%0], [%1], 8;\n" ::"r"(sa), "l"(Sg + q) : "memory");
-      i += W * 32;
-      while (i >= n) {
-        i -= n;
-        ++j;
-      }
+  const int row = lane >> 2, kk = lane & 3;
+  if (tid == 0) bad = 0;
+  for (int I = warp; I < nt; I += CMW)
+    for (int J = lane; J <= I; J += 32) ti[I * (I + 1) / 2 + J] = (unsigned char)I;
+  // the lower triangle, column by column (rows along the lanes); the part of
+  // a diagonal tile above the diagonal is never read
+  for (int j = warp; j < np; j += CMW)
+    for (int i = j + lane; i < np; i += 32) {
+      const double v = (i < n && j < n) ? Sg[(long)j * n + i] : (i == j ? 1.0 : 0.0);
+      T[cm_tile(i >> 3, j >> 3) + cm_pos(i & 7, j & 7)] = v;
     }
-    asm volatile("cp.async.wait_all;\n" ::: "memory");
+  __syncthreads();
+  if (warp == 0) {
+    const int b = cm_diag(T, 0, xd, lane);
+    if (b && lane == 0) bad = b;
   }
   __syncthreads();
-  double a[NR][NC];
-#pragma unroll
-  for (int r = 0; r < NR; ++r)
-#pragma unroll
-    for (int c = 0; c < NC; ++c) {
-      const int row = r0 + r, col = lane + 32 * c;
-      const int hi = row > col ? row : col, lo = row > col ? col : row;
-      const double v = stg[(long)min(lo, n - 1) * ld + min(hi, n - 1)];   // S(hi, lo), clamped address
-      a[r][c] = (row < n && col < n) ? v : 0.0;
-    }
-  for (int k = 0; k < n; k += 2) {
-    const int b = (k >> 1) & 1, kc = k >> 5, kl = k & 31;   // k even: k and k + 1 share slot kc
-    const bool two = k + 1 < n;
-    if (lane == kl || (two && lane == kl + 1)) {   // columns k, k + 1 out, e_k, e_(k+1) in
-      const int h = lane - kl, col = k + h;
-      dense_static_for<0, NC>([&](auto cc) {
-        constexpr int C = decltype(cc)::value;
-        if (C == kc) {
-#pragma unroll
-          for (int r = 0; r < NR; r += 2) {
-            *reinterpret_cast<double2 *>(&xcol[b][h][r0 + r]) = make_double2(a[r][C], a[r + 1][C]);
-            a[r][C] = (r0 + r == col) ? 1.0 : 0.0;
-            a[r + 1][C] = (r0 + r + 1 == col) ? 1.0 : 0.0;
-          }
-        }
-      });
-    }
-    if (warp == k / NR) {     // rows k, k + 1 out
-      const int kr = k - r0;
-      dense_static_for<0, NR / 2>([&](auto rr) {
-        constexpr int R = 2 * decltype(rr)::value;
-        if (R == kr) {
-#pragma unroll
-          for (int c = 0; c < NC; ++c) {
-            xrow[b][0][lane + 32 * c] = a[R][c];
-            xrow[b][1][lane + 32 * c] = a[R + 1][c];
-          }
-        }
-      });
-    }
-    __syncthreads();
-    const double *x0 = xcol[b][0], *x1 = xcol[b][1], *w0 = xrow[b][0], *w1 = xrow[b][1];
-    const double piv0 = x0[k];
-    if (!(piv0 > 1.0e-30)) {   // the same in every thread; also catches NaN
-      if (tid == 0) *info = 1 + k;
+  for (int k = 0; k < nb; ++k) {
+    if (bad) {   // uniform: written before the barrier
+      if (tid == 0) *info = bad;
       return;
     }
-    const double rs0 = rsqrt_nr(piv0);   // 1 / L(k,k)
-    const double l10 = two ? x0[k + 1] * rs0 : 0.0;
-    double rs1 = 0.0;
-    if (two) {
-      const double piv1 = x1[k + 1] - l10 * l10;
-      if (!(piv1 > 1.0e-30)) {
-        if (tid == 0) *info = 2 + k;
-        return;
-      }
-      rs1 = rsqrt_nr(piv1);
-    }
-    if (tid == 0) {
-      rsv[k] = rs0;
-      if (two) rsv[k + 1] = rs1;
-    }
-    // lane r < NR: m0, m1 of row r0 + r (0 where the row takes no update)
-    const int ri = r0 + lane, rc = min(ri, NX - 1);
-    const double m0row = (lane < NR && ri > k && ri < n) ? x0[rc] * rs0 : 0.0;
-    const double m1row = (two && lane < NR && ri > k + 1 && ri < n) ? (x1[rc] - m0row * l10) * rs1 : 0.0;
-    if (lane < NR) mw[warp][lane] = make_double2(m0row, m1row);
-    __syncwarp();
-    if (r0 + NR > k + 1) {    // rows below k in this warp
-      double y0[NC], y1[NC];
+    // (B)
+    for (int I = warp; I < nt; I += CMW) {
+      double b[4], d[2][2] = {{0.0, 0.0}, {0.0, 0.0}};
+      const bool left = I < 2 * k, in = (I >> 1) == k;
 #pragma unroll
-      for (int c = 0; c < NC; ++c) {
-        const int col = lane + 32 * c, cc = min(col, NX - 1);
-        const double s0 = (col <= k) ? w0[cc] : x0[cc];
-        const double s1 = (col <= k + 1) ? w1[cc] : x1[cc];
-        y0[c] = (col == k + 1 || col >= n) ? 0.0 : s0 * rs0;
-        y1[c] = (two && col < n) ? (s1 - l10 * y0[c]) * rs1 : 0.0;
+      for (int s = 0; s < 4; ++s) {
+        const int c = 4 * s + kk;   // column of the block; the operand element is (row 8 I + row, c) or its transpose
+        if (in) b[s] = (I & 1) * 8 + row == c ? 1.0 : 0.0;
+        else if (left) b[s] = T[cm_tile(2 * k + (c >> 3), I) + cm_pos(c & 7, row)];
+        else b[s] = T[cm_tile(I, 2 * k + (c >> 3)) + cm_pos(row, c & 7)];
       }
 #pragma unroll
-      for (int r = 0; r < NR; ++r) {
-        const double2 mi = mw[warp][r];
+      for (int s = 0; s < 4; ++s) {
+        if (s < 2) cm_mma(d[0], xd[row * CM_LD + 4 * s + kk], b[s]);   // X_D is lower triangular
+        cm_mma(d[1], xd[(8 + row) * CM_LD + 4 * s + kk], b[s]);
+      }
+      __syncwarp();   // the tile is rewritten below
 #pragma unroll
-        for (int c = 0; c < NC; ++c) a[r][c] = fma(-mi.y, y1[c], fma(-mi.x, y0[c], a[r][c]));
+      for (int m = 0; m < 2; ++m)
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+          const int c = 8 * m + row, i = 2 * kk + h;   // P(8 I + i, c)
+          P[(I * 8 + i) * CM_LD + c] = d[m][h];
+          if (left) T[cm_tile(2 * k + m, I) + cm_pos(row, i)] = d[m][h];
+        }
+    }
+    __syncthreads();
+    // X_D is final; its block is not read again before the way out
+    if (warp == CMW - 1)
+      for (int q = lane; q < 256; q += 32) {
+        const int r = q >> 4, c = q & 15;
+        if (r >= c) T[cm_tile(2 * k + (r >> 3), 2 * k + (c >> 3)) + cm_pos(r & 7, c & 7)] = P[(16 * k + c) * CM_LD + r];
+      }
+    if (k + 1 == nb) break;
+    // (C), warp 0 with the next (A)
+    const int q0 = (2 * k + 2) * (2 * k + 3) / 2, q1 = nt * (nt + 1) / 2;
+    double af[4];
+    if (warp == 0) {
+      cm_load_a(P, 2 * k + 2, af, lane);
+      cm_update(T, P, 2 * k + 2, 2 * k + 2, true, af, lane);
+      cm_load_a(P, 2 * k + 3, af, lane);
+      cm_update(T, P, 2 * k + 3, 2 * k + 2, true, af, lane);
+      cm_update(T, P, 2 * k + 3, 2 * k + 3, true, af, lane);
+      __syncwarp();
+      const int b = cm_diag(T, k + 1, xd, lane);
+      if (b && lane == 0) bad = b;
+    } else {
+      const int per = (q1 - q0 + CMW - 2) / (CMW - 1), qa = q0 + (warp - 1) * per, qe = min(q1, qa + per);
+      int last = -1;
+      for (int q = qa; q < qe; ++q) {
+        const int I = ti[q], J = q - I * (I + 1) / 2;
+        if (I <= 2 * k + 3 && J >= 2 * k + 2) continue;   // warp 0's
+        if (I != last) cm_load_a(P, I, af, lane);
+        last = I;
+        cm_update(T, P, I, J, (J >> 1) != k, af, lane);
       }
     }
-    __syncwarp();   // mw is rewritten in the next step
+    __syncthreads();
   }
   __syncthreads();
-  // X to the staging area (lower triangle, zeros above), then out column-major
-#pragma unroll
-  for (int r = 0; r < NR; ++r) {
-    const int row = r0 + r;
-    const double sc = rsv[min(row, NX - 1)];
-#pragma unroll
-    for (int c = 0; c < NC; ++c) {
-      const int col = lane + 32 * c;
-      if (row < n && col < n) stg[(long)col * ld + row] = (row >= col) ? a[r][c] * sc : 0.0;
-    }
-  }
-  __syncthreads();
-  {
-    int j = tid / n, i = tid - j * n;
-    for (long q = tid; q < (long)n * n; q += W * 32) {
-      Sg[q] = stg[(long)j * ld + i];
-      i += W * 32;
-      while (i >= n) {
-        i -= n;
-        ++j;
-      }
-    }
-  }
+  // X, column-major with zeros above the diagonal
+  for (int j = warp; j < n; j += CMW)
+    for (int i = lane; i < n; i += 32)
+      Sg[(long)j * n + i] = i >= j ? T[cm_tile(i >> 3, j >> 3) + cm_pos(i & 7, j & 7)] : 0.0;
   if (tid == 0) *info = 0;
 }
 
 // Cholesky and L^-1 over the whole GPU for large n (one cooperative launch of
-// G CTAs; the algorithm of k_cholinv_rg, one rank-1 update a column): CTA c
+// G CTAs; the algorithm of k_cholinv_mm, one rank-1 update a column): CTA c
 // keeps the columns j = c + G q in shared memory.  Step k: the owner of column
 // k publishes it (the Schur complement) and replaces it by e_k; every CTA
 // publishes its entries of row k (R(k, .) left of k); one grid barrier; then
@@ -707,7 +479,7 @@ __global__ void __launch_bounds__(W * 32, 1) k_cholinv_rg(double *__restrict__ S
 // columns.  Row k is final from then on and is scaled by rs when written out.
 // The published column and row alternate by parity.  gs: 5n doubles of
 // global scratch (column, row, 1/L(k,k)); bar: two zeroed unsigned ints.
-// info as k_cholinv_sm (S left as it was on a bad pivot); -1 on a barrier
+// info as k_cholinv_mm (S left as it was on a bad pivot); -1 on a barrier
 // time-out.
 constexpr int CHG_T = 256;
 
@@ -822,63 +594,27 @@ static bool cholinv_grid(double *S, int n, double *work, int *d_info, cudaStream
   return true;
 }
 
-// QX_CHOLINV_REG=0 keeps the shared-memory kernels at every size (read at
-// every call).
-static bool cholinv_registers_enabled() {
-  const char *v = getenv("QX_CHOLINV_REG");
-  return !(v && v[0] == '0');
-}
-
-// S: n x n column-major.  When S does not fit shared memory the kernel works
-// in S itself (L2-resident) and uses work (>= CB*DLD + n doubles) as temporary.
 int cholinv(double *S, int n, double *work, int *d_info, cudaStream_t st) {
   if (n > 8192) { set_error("cholinv: n=%d too large", n); return 1; }
-  const size_t bytes = sizeof(double) * ((size_t)(n | 1) * n + CB * DLD + n);
-  const int use = bytes <= CH_SMEM_MAX;
-  static bool attr = false;
-  if (!attr) {
-    cudaFuncSetAttribute(k_cholinv<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)CH_SMEM_MAX);
-    attr = true;
-  }
-  if (!use && !work) { set_error("cholinv: n=%d needs a work buffer", n); return 1; }
-  const size_t pbytes = sizeof(double) * ((size_t)(n | 1) * n + 2 * (size_t)n + (size_t)PB * n);
-  const size_t rbytes = sizeof(double) * (size_t)(n | 1) * n;
-  if (n <= 160 && cholinv_registers_enabled()) {
-    // per process, only ever raised; the first call always sets it (the
-    // kernels' static shared buffers count against the 48 KB default, so a
-    // dynamic size below 48 KB can still need the opt-in)
-    static size_t rset = 0;
-    if (rbytes > rset) {
-      // exactly what this size needs: with the kernels' static buffers the
-      // opt-in ceiling is below the 227 KB of a CTA
-      const cudaError_t e1 = cudaFuncSetAttribute(k_cholinv_rg<8, 10, 3>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                                  (int)rbytes);
-      const cudaError_t e2 = cudaFuncSetAttribute(k_cholinv_rg<8, 20, 5>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                                  (int)rbytes);
-      if (e1 != cudaSuccess || e2 != cudaSuccess) {
-        set_error("cholinv: n=%d: shared-memory opt-in failed: %s", n, cudaGetErrorString(e1 ? e1 : e2));
+  if (n <= CM_MAXN) {
+    // one CTA as long as the triangle fits its shared memory
+    static bool attr = false;
+    if (!attr) {
+      const cudaError_t e = cudaFuncSetAttribute(k_cholinv_mm, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                                 (int)cm_smem(CM_MAXN));
+      if (e != cudaSuccess) {
+        set_error("cholinv: n=%d: shared-memory opt-in failed: %s", n, cudaGetErrorString(e));
         return 1;
       }
-      rset = rbytes;
+      attr = true;
     }
-    if (n <= 80) k_cholinv_rg<8, 10, 3><<<1, 8 * 32, rbytes, st>>>(S, n, d_info);
-    else k_cholinv_rg<8, 20, 5><<<1, 8 * 32, rbytes, st>>>(S, n, d_info);
+    k_cholinv_mm<<<1, CMT, cm_smem(n), st>>>(S, n, d_info);
     note_launch();
     return 0;
   }
-  if (n > 192 && cholinv_grid(S, n, work, d_info, st)) return 0;
-  if (n <= CP_MAXN && pbytes <= CH_SMEM_MAX) {
-    static bool pattr = false;
-    if (!pattr) {
-      cudaFuncSetAttribute(k_cholinv_sm, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)CH_SMEM_MAX);
-      pattr = true;
-    }
-    k_cholinv_sm<<<1, CPT, pbytes, st>>>(S, n, d_info);
-    note_launch();
-    return 0;
-  }
-  if (use) k_cholinv<true><<<1, CHT, bytes, st>>>(S, n, work, d_info);
-  else k_cholinv<false><<<1, CHT, 0, st>>>(S, n, work, d_info);
+  if (!work) { set_error("cholinv: n=%d needs a work buffer", n); return 1; }
+  if (cholinv_grid(S, n, work, d_info, st)) return 0;
+  k_cholinv<<<1, CHT, 0, st>>>(S, n, work, d_info);
   note_launch();
   return 0;
 }
