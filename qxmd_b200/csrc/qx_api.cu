@@ -1518,8 +1518,7 @@ static int eigen_impl(qx_ctx *c, const qx_cgparm *p, int *nriter, int *nhpsi_out
     TRY(gemm<T>(true, false, nb, nb, ne, (T)1, snap, ne, h, ne, (T)0, pm_t, nb, 1, nullptr, nullptr, c->st, c->gws, c->gws_bytes, nullptr, c->tcpad, c->tcpad_bytes));
     cg_mask<T>(nb, pm_t, s, c->st);
     TRY(gemm<T>(false, false, ne, nb, nb, (T)-1, snap, ne, pm_t, nb, (T)1, h, ne, 0, nullptr, nullptr, c->st, nullptr, 0, nullptr, c->tcpad, c->tcpad_bytes));
-    cg_orth<T>(nb, ne, ne, x, hx, h, s, c->st);
-    cg_list(nb, s, c->st);
+    cg_orth<T>(nb, ne, ne, x, h, s, c->st);
     CKL();
     TRY(hpsi_impl<T>(c, h, gh, s.pairs, s.npair, c->npair_all, s.list, s.nact, nb,
                      QX_HPSI_KINETIC | QX_HPSI_NONLOCAL));

@@ -35,8 +35,9 @@ struct SeqArgs {
 
 template <typename T> void cg_init(int nb, int ne, long ldx, const T *x, const T *hx, T *g, const CgState &s, cudaStream_t st);
 template <typename T> void cg_prec(int nb, int ne, long ldx, T *g, T *h, const double *dk, const CgState &s, cudaStream_t st);
+// the subgs3 mask, and the active-band list and pairs
 template <typename T> void cg_mask(int nb, T *Pm, const CgState &s, cudaStream_t st);
-template <typename T> void cg_orth(int nb, int ne, long ldx, const T *x, const T *hx, T *h, const CgState &s, cudaStream_t st);
+template <typename T> void cg_orth(int nb, int ne, long ldx, const T *x, T *h, const CgState &s, cudaStream_t st);
 // Entry state of every band (g preconditioned) and band 0 as the current one.
 template <typename T> void seq_init(int nb, int ne, long ldx, const T *x, const T *hx, T *g, const double *dk,
                                     const CgState &s, const SeqArgs &q, cudaStream_t st);
@@ -49,7 +50,6 @@ template <typename T> void seq_kb(int np, int ne, const T *kbg, const T *scale, 
                                   const int *cur, double *coef, cudaStream_t st);
 template <typename T> void seq_update(int ne, long ldx, T *x, T *hx, T *g, const T *h, const T *gh, const double *dk,
                                       const CgState &s, const CgParm &pm, const SeqArgs &q, cudaStream_t st);
-void cg_list(int nb, const CgState &s, cudaStream_t st);
 void gradres_stats(const double *prod, const double *occ, int nb, double *out, cudaStream_t st);
 void iter_sum(const int *iter, int nb, int *out, cudaStream_t st);
 template <typename T> void cg_update(int nb, int ne, long ldx, T *x, T *hx, T *g, const T *h, const T *gh,
