@@ -491,8 +491,8 @@ __global__ void __launch_bounds__(QX_THREADS) k_xinv_r(PipeParams P, const typen
 //     (added over pairs in a fixed order afterwards); wocc = occ / Omega.
 // The gathers of psi (32-byte sectors of L2) bound it.  One thread per point
 // and pair, as before, was bound by FP32 to FP64 conversions and by re-reading
-// the table for every pair; at Si64, 160 bands: projections 133 -> 98 us,
-// forces 506 -> 228 us.
+// the table for every pair; at Si64, 160 bands: projections 133 -> 78 us,
+// forces 506 -> 187 us.
 template <typename T, int MT, int NT, bool FORCE>
 __global__ void __launch_bounds__(QX_THREADS) k_ptsum(PipeParams P, const typename c2t<T>::type *__restrict__ R,
                                                        const int *__restrict__ off, const int *__restrict__ mesh,
@@ -524,11 +524,12 @@ __global__ void __launch_bounds__(QX_THREADS) k_ptsum(PipeParams P, const typena
     bon[q] = pl < np;
     Rb[q] = reinterpret_cast<const T *>(R + (long)min(pl, np - 1) * n) + (row & 1);
   }
-  for (int k0 = 4 * warp; k0 < cnt; k0 += 4 * NW * UN) {
+  // a warp's UN quads are consecutive points, so that they share sectors of psi
+  for (int k0 = 4 * UN * warp; k0 < cnt; k0 += 4 * NW * UN) {
     T av[UN][MT], bv[UN][NT];
 #pragma unroll
     for (int u = 0; u < UN; ++u) {
-      const int k = k0 + 4 * NW * u + kk;
+      const int k = k0 + 4 * u + kk;
       const bool on = k < cnt;
       const long pt = p0 + min(k, cnt - 1);
       const long m = mesh[pt];
@@ -819,8 +820,9 @@ static bool zcols_fwd_enabled(int k3) {
   return k3 <= 32;
 }
 
-// The projections of the chunk's pairs on every atom's projectors.  16 bands
-// a CTA where that fills the GPU, 8 otherwise.
+// The sums of the chunk's pairs over every atom's points.  Where that fills
+// the GPU a CTA takes 16 bands (projections) or 32 (forces, whose table rows
+// are four times as many; at Si64 16 bands measured 228 us against 198), else 8.
 template <typename T, bool FORCE>
 static void launch_ptsum(const Plan &pl, const PipeParams &P, int npl, const T *dvnl, const double *wocc,
                          double *fpart, cudaStream_t st) {
@@ -833,13 +835,14 @@ static void launch_ptsum(const Plan &pl, const PipeParams &P, int npl, const T *
     note_launch();
   };
   using std::integral_constant;
-  const bool wide = (long)pl.natom * ((npl + 7) / 8) >= 148;
+  constexpr int NT = FORCE ? 4 : 2;
+  const bool wide = (long)pl.natom * ((npl + 4 * NT - 1) / (4 * NT)) >= 148;
   const int rows = FORCE ? 4 * pl.kb_lmx : pl.kb_lmx;   // at most 36
   if (rows <= 8) {
-    if (wide) go(integral_constant<int, 1>(), integral_constant<int, 2>());
+    if (wide) go(integral_constant<int, 1>(), integral_constant<int, NT>());
     else go(integral_constant<int, 1>(), integral_constant<int, 1>());
   } else if (rows <= 16) {
-    if (wide) go(integral_constant<int, 2>(), integral_constant<int, 2>());
+    if (wide) go(integral_constant<int, 2>(), integral_constant<int, NT>());
     else go(integral_constant<int, 2>(), integral_constant<int, 1>());
   } else if constexpr (FORCE) {
     go(integral_constant<int, 5>(), integral_constant<int, 1>());
