@@ -8,6 +8,7 @@
 // 2*sum - x(1)*y(1) is applied in the epilogue.
 #include <algorithm>
 #include <atomic>
+#include <cmath>
 
 #include "qx_internal.h"
 #include "qx_cg.h"
@@ -531,7 +532,8 @@ __global__ void __launch_bounds__(256) k_sgemm(int M, int N, int K, float alpha,
                                                const float *__restrict__ B, long ldb, float beta,
                                                float *__restrict__ Cm, long ldc, int gamma,
                                                const int *__restrict__ colmap, const int *__restrict__ ncol_dev,
-                                               int kchunk, float *__restrict__ W, int *__restrict__ cnt) {
+                                               const float *__restrict__ rowscale, int kchunk, float *__restrict__ W,
+                                               int *__restrict__ cnt) {
   constexpr int TMM = 16 * MT, TNN = 16 * NT, PA = TMM + 1, PB = TNN + 1;
   constexpr int SA = SBK * PA, SSZ = SA + SBK * PB;
   extern __shared__ __align__(16) float ssm[];
@@ -634,7 +636,8 @@ __global__ void __launch_bounds__(256) k_sgemm(int M, int N, int K, float alpha,
     for (int i = 0; i < MT; ++i)
 #pragma unroll
       for (int j = 0; j < NT; ++j) acc[i][j] = 0.f;
-    for (int z = 0; z < (int)gridDim.z; ++z)
+#pragma unroll 4
+    for (int z = 0; z < (int)gridDim.z; ++z)   // unrolled: four partials' loads in flight
 #pragma unroll
       for (int i = 0; i < MT; ++i)
 #pragma unroll
@@ -662,7 +665,8 @@ __global__ void __launch_bounds__(256) k_sgemm(int M, int N, int K, float alpha,
         }
       }
       float *c = Cm + cn * ldc + gm;
-      *c = (beta == 0.f) ? alpha * v : alpha * v + beta * *c;
+      v = (beta == 0.f) ? alpha * v : alpha * v + beta * *c;
+      *c = rowscale ? v * rowscale[gm] : v;
     }
   }
 }
@@ -684,40 +688,37 @@ static int sgemm_rows(int n) {
 
 template <bool TA, bool TB, bool SPLIT, int MT, int NT>
 static void sgemm_go(dim3 g, int M, int N, int K, float alpha, const float *A, long lda, const float *B, long ldb,
-                     float beta, float *C, long ldc, int gamma, const int *colmap, const int *ncol_dev, int kchunk,
-                     float *W, int *cnt, cudaStream_t st) {
+                     float beta, float *C, long ldc, int gamma, const int *colmap, const int *ncol_dev,
+                     const float *rowscale, int kchunk, float *W, int *cnt, cudaStream_t st) {
   constexpr size_t sm = sgemm_smem<MT, NT>();
   static_assert(sm <= 48 * 1024, "stages fit the default shared-memory limit");
   k_sgemm<TA, TB, SPLIT, MT, NT><<<g, 256, sm, st>>>(M, N, K, alpha, A, lda, B, ldb, beta, C, ldc, gamma, colmap,
-                                                     ncol_dev, kchunk, W, cnt);
+                                                     ncol_dev, rowscale, kchunk, W, cnt);
   note_launch();
 }
 
 // One shape's launch: tile rows MT x NT from the extents (k-contiguous A:
-// both from the band-sized extents; otherwise 64-row tiles down M), K split
-// as k_gemm's, the partials summed by the last CTA of each tile (cnt: one
-// zeroed counter per tile).
+// both from the band-sized extents; otherwise 64-row tiles down M), and K
+// split to shorten the chain of one CTA: a k-block of 16 costs about 0.5 us
+// and a partial tile summed by the last CTA about 0.1 us (cnt: one zeroed
+// counter per tile), so K / (32 z) + z / 10 us is least at z = sqrt(K / 3),
+// as far as two CTAs a SM hold the splits.  At Si8 (32 x 16 x 738) the one
+// CTA of the unsplit call ran 24.8 us.
 template <bool TA, bool TB>
 static void sgemm_launch(int M, int N, int K, float alpha, const float *A, long lda, const float *B, long ldb,
-                         float beta, float *C, long ldc, int gamma, const int *colmap, const int *ncol_dev, void *ws,
-                         size_t ws_bytes, int *cnt, cudaStream_t st) {
+                         float beta, float *C, long ldc, int gamma, const int *colmap, const int *ncol_dev,
+                         const float *rowscale, void *ws, size_t ws_bytes, int *cnt, cudaStream_t st) {
   const int mt = TA ? sgemm_rows(M) : 4, nt = sgemm_rows(N);
   dim3 g((M + 16 * mt - 1) / (16 * mt), (N + 16 * nt - 1) / (16 * nt));
   const long tiles = (long)g.x * g.y;
   const size_t part = sizeof(float) * (size_t)tiles * 256 * mt * nt;   // one split's partial tiles
   int nsplit = 1, kchunk = K;
-  if (ws && cnt && tiles <= GEMM_TILE_COUNTERS && tiles < 2 * 148 && K >= 4 * 256) {
-    nsplit = (int)std::min<long>((2 * 148 + tiles - 1) / tiles, (K + 255) / 256);
+  if (ws && cnt && tiles <= GEMM_TILE_COUNTERS && tiles < 2 * 148 && K >= 256) {
+    nsplit = (int)std::min<long>((2 * 148 + tiles - 1) / tiles, (long)std::sqrt(K / 3.0));
+    nsplit = (int)std::min<size_t>(nsplit, ws_bytes / part);
+    if (nsplit < 2) nsplit = 1;
     kchunk = ((K + nsplit - 1) / nsplit + SBK - 1) / SBK * SBK;
     nsplit = (K + kchunk - 1) / kchunk;
-    if ((size_t)nsplit * part > ws_bytes) {
-      nsplit = (int)(ws_bytes / part);
-      if (nsplit < 2) nsplit = 1;
-      else {
-        kchunk = ((K + nsplit - 1) / nsplit + SBK - 1) / SBK * SBK;
-        nsplit = (K + kchunk - 1) / kchunk;
-      }
-    }
   }
   if (nsplit <= 1) kchunk = K;
   g.z = nsplit;
@@ -726,9 +727,9 @@ static void sgemm_launch(int M, int N, int K, float alpha, const float *A, long 
 #define QX_SG(MT_, NT_)                                                                                              \
   if (mt == MT_ && nt == NT_) {                                                                                      \
     if (split) sgemm_go<TA, TB, true, MT_, NT_>(g, M, N, K, alpha, A, lda, B, ldb, beta, C, ldc, gamma, colmap,     \
-                                                ncol_dev, kchunk, W, cnt, st);                                       \
+                                                ncol_dev, rowscale, kchunk, W, cnt, st);                                       \
     else sgemm_go<TA, TB, false, MT_, NT_>(g, M, N, K, alpha, A, lda, B, ldb, beta, C, ldc, gamma, colmap, ncol_dev, \
-                                           kchunk, W, nullptr, st);                                                  \
+                                           rowscale, kchunk, W, nullptr, st);                                                  \
   }
   if (TA) {
     QX_SG(2, 2) else QX_SG(2, 3) else QX_SG(2, 4) else QX_SG(2, 5)
@@ -799,18 +800,17 @@ int gemm(bool ta, bool tb, int M, int N, int K, T alpha, const T *A, long lda, c
     return 0;
   }
   if (sizeof(T) == sizeof(float) && !(ta && tb) && sgemm_enabled()) {
-    const float *Af = (const float *)A, *Bf = (const float *)B;
+    const float *Af = (const float *)A, *Bf = (const float *)B, *rs = (const float *)rowscale;
     float *Cf = (float *)C;
     if (ta)
       sgemm_launch<true, false>(M, N, K, (float)alpha, Af, lda, Bf, ldb, (float)beta, Cf, ldc, gamma, colmap, ncol_dev,
-                                ws, ws_bytes, cnt, st);
+                                rs, ws, ws_bytes, cnt, st);
     else if (tb)
       sgemm_launch<false, true>(M, N, K, (float)alpha, Af, lda, Bf, ldb, (float)beta, Cf, ldc, gamma, colmap, ncol_dev,
-                                ws, ws_bytes, cnt, st);
+                                rs, ws, ws_bytes, cnt, st);
     else
       sgemm_launch<false, false>(M, N, K, (float)alpha, Af, lda, Bf, ldb, (float)beta, Cf, ldc, gamma, colmap,
-                                 ncol_dev, ws, ws_bytes, cnt, st);
-    if (rowscale) scale_rows<T>(M, N, C, ldc, rowscale, colmap, ncol_dev, st);
+                                 ncol_dev, rs, ws, ws_bytes, cnt, st);
     return 0;
   }
   dim3 g((M + BM - 1) / BM, (N + BN - 1) / BN);
