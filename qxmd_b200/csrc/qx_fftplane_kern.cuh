@@ -36,21 +36,29 @@ struct PlaneRows {
   __device__ static int row(int t) { return both ? (t & 31) : t; }
 };
 
-template <int NX, int NY, int PL>
-__global__ void __launch_bounds__(64, plane_minb(NX > NY ? NX : NY))
-    k_plane(PipeParams P, float2 *__restrict__ bufA, const float *__restrict__ vloc) {
+// U units a CTA: U band pairs of the same planes on 64 threads each, whose
+// phases the CTA's barriers keep together.  The unrolled transforms are some
+// tens of kilobytes of code that every unit runs once, so units in step share
+// its instruction fetches: two at 54 x 54 (Si64, 160 bands, whole H|psi>) 163
+// -> 147 us, four the same, eight 158 us.
+template <int NX, int NY, int PL, int U>
+__global__ void __launch_bounds__(64 * U, (plane_minb(NX > NY ? NX : NY) + U - 1) / U)
+    k_plane(PipeParams P, float2 *__restrict__ bufA, const float *__restrict__ vloc, int npl) {
   using rf::out_pos;
   using Rows = PlaneRows<NY, PL>;
   // PL = 2: the CTA takes planes i3 and i3 + 1; the y phases give warp w the
   // columns of plane w (P1 <= 32).  PL = 1: one plane, the columns on
   // threads 0 .. P1 - 1.  NX = k1 (x, the sphere's P1 columns), NY = k2.
   const int i3b = blockIdx.x * PL;
-  const int pl = blockIdx.y, p = P.pair0 + pl;
-  if (p >= (P.npair_dev ? *P.npair_dev : P.npair)) return;
+  const int np = P.npair_dev ? *P.npair_dev : P.npair;
+  if (P.pair0 + (int)blockIdx.y * U >= np) return;
+  const int pl = blockIdx.y * U + (threadIdx.x >> 6);
+  const bool live = pl < npl && P.pair0 + pl < np;
   const int P1 = P.P1, P2 = P.P2, m1 = P.m1, m2 = P.m2;
-  const int npl_here = min(PL, P.k3 - i3b);   // planes this CTA owns (uniform)
-  extern __shared__ float2 T[];   // [PL][NY][P1]
-  const int t = threadIdx.x;
+  const int npl_here = live ? min(PL, P.k3 - i3b) : 0;   // planes of this unit
+  extern __shared__ float2 Tu[];   // [U][PL][NY][P1]
+  float2 *T = Tu + (threadIdx.x >> 6) * (PL * NY * P1);
+  const int t = threadIdx.x & 63;
   const float2 zero = make_float2(0.f, 0.f);
   // column phases: plane and column of this thread
   const int cpl = (PL == 2) ? (t >> 5) : 0, col = (PL == 2) ? (t & 31) : t;
@@ -769,20 +777,19 @@ int rho2_launch(const PipeParams &P, int npl, const float2 *bufA, const double *
 
 template <int NX, int NY>
 int plane_launch(const PipeParams &P, int npl, float2 *bufA, const float *vloc, cudaStream_t st) {
+  constexpr int U = 2;
   static bool attr = false;
   if (!attr) {
-    cudaFuncSetAttribute(k_plane<NX, NY, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, 64 * 1024);
-    cudaFuncSetAttribute(k_plane<NX, NY, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, 64 * 1024);
+    cudaFuncSetAttribute(k_plane<NX, NY, 1, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, 64 * 1024);
+    cudaFuncSetAttribute(k_plane<NX, NY, 2, U>, cudaFuncAttributeMaxDynamicSharedMemorySize, 80 * 1024);
     attr = true;
   }
-  if (P.P1 <= 32 && plane_pairs_enabled()) {   // two planes a CTA: warp w takes plane w's columns
-    const size_t sm = sizeof(float2) * 2 * (size_t)NY * P.P1;
-    dim3 g((P.k3 + 1) / 2, npl);
-    k_plane<NX, NY, 2><<<g, 64, sm, st>>>(P, bufA, vloc);
+  if (P.P1 <= 32 && plane_pairs_enabled()) {   // two planes a unit: warp w takes plane w's columns
+    const size_t sm = sizeof(float2) * 2 * U * (size_t)NY * P.P1;
+    k_plane<NX, NY, 2, U><<<dim3((P.k3 + 1) / 2, (npl + U - 1) / U), 64 * U, sm, st>>>(P, bufA, vloc, npl);
   } else {
     const size_t sm = sizeof(float2) * (size_t)NY * P.P1;
-    dim3 g(P.k3, npl);
-    k_plane<NX, NY, 1><<<g, 64, sm, st>>>(P, bufA, vloc);
+    k_plane<NX, NY, 1, 1><<<dim3(P.k3, npl), 64, sm, st>>>(P, bufA, vloc, npl);
   }
   note_launch();
   return 0;
