@@ -368,6 +368,9 @@ static int alloc_pipe(qx_ctx *c) {
   const double mb = env ? atof(env) : 160.0;
   long ch = (long)(mb * 1048576.0 / (sizeof(C) * (double)per_pair));
   ch = std::max(1L, std::min(ch, (long)c->npair_all));
+  // equal chunks: 80 pairs that fit 75 run as 40 + 40, not 75 + 5
+  const long nch = (c->npair_all + ch - 1) / ch;
+  ch = (c->npair_all + nch - 1) / nch;
   pl.chunk = (int)ch;
   TRY(dalloc(c, &b.bufA, sizeof(C) * ch * pl.k3 * pl.P2 * pl.P1));
   TRY(dalloc(c, &b.bufB, sizeof(C) * ch * pl.k3 * pl.k2 * pl.P1));

@@ -1,6 +1,7 @@
-// Dispatch of the fused FFT plane passes of the FP32 H|psi> pipeline on the
-// grid length: the kernels are in qx_fftplane_kern.cuh, their launchers are
-// instantiated per length in the qx_fftplane_*.cu files.
+// Dispatch of the fused FFT plane passes of the H|psi> pipeline on the grid
+// length: the kernels are in qx_fftplane_kern.cuh (FP32) and
+// qx_fftplane64_kern.cuh (FP64), their launchers are instantiated per length
+// in the qx_fftplane_*.cu and qx_fftplane64_*.cu files.
 #include "qx_fftplane.h"
 
 namespace qx {
@@ -83,7 +84,7 @@ bool plane_length_supported(int k1, int k2) {
 }
 
 // Launch the fused pass if this grid has a specialised length; -1 otherwise.
-int launch_plane_f32(const PipeParams &P, int npl, float2 *bufA, const float *vloc, cudaStream_t st) {
+int launch_plane(const PipeParams &P, int npl, float2 *bufA, const float *vloc, cudaStream_t st) {
   if (P.P1 > P.k1 || P.P2 > P.k2) return -1;
   switch (plane_grid_key(P.k1, P.k2)) {
 #define QX_CASE(NX, NY) \
@@ -91,6 +92,17 @@ int launch_plane_f32(const PipeParams &P, int npl, float2 *bufA, const float *vl
     QX_PLANE_GRIDS(QX_CASE)
 #undef QX_CASE
     case plane_grid_key(96, 96): return plane2_launch<96>(P, npl, bufA, vloc, st);
+    default: return -1;
+  }
+}
+
+int launch_plane(const PipeParams &P, int npl, double2 *bufA, const double *vloc, cudaStream_t st) {
+  if (P.P1 > P.k1 || P.P2 > P.k2) return -1;
+  switch (plane_grid_key(P.k1, P.k2)) {
+#define QX_CASE(NX, NY) \
+  case plane_grid_key(NX, NY): return plane64_launch<NX, NY>(P, npl, bufA, vloc, st);
+    QX_PLANE64_GRIDS(QX_CASE)
+#undef QX_CASE
     default: return -1;
   }
 }

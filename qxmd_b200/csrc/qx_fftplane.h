@@ -47,6 +47,15 @@ int zcols2_launch(const PipeParams &P, int npl, const float *cin, long ldc, floa
 #define QX_ZCOLS_LENGTHS(X) \
   X(20) X(21) X(24) X(25) X(27) X(30) X(32) X(36) X(40) X(42) X(45) X(48) X(49) X(54) X(60) X(64)
 
+// FP64 (qx_fftplane64_kern.cuh): the plane shapes whose lines are even, or odd
+// and at most 32 points.
+#define QX_PLANE64_GRIDS(X)                                                                            \
+  X(20, 20) X(21, 21) X(24, 24) X(25, 25) X(27, 27) X(30, 30) X(32, 32) X(36, 36) X(40, 40) X(42, 42) \
+  X(48, 48) X(54, 54) X(60, 60) X(64, 64)                                                             \
+  X(24, 25) X(25, 24) X(25, 27) X(27, 25) X(42, 21) X(54, 24) X(54, 25) X(54, 27)
+template <int NX, int NY>
+int plane64_launch(const PipeParams &P, int npl, double2 *bufA, const double *vloc, cudaStream_t st);
+
 constexpr int plane_grid_key(int k1, int k2) { return k1 * 1024 + k2; }
 
 // QX_PLANE_PAIRS=0 keeps one z plane a CTA (read at every call).

@@ -121,9 +121,10 @@ int launch_full_fft(const Plan &pl, typename c2t<T>::type *g, int sign, double s
 // length has no kernel.
 int launch_full_lines_f64(double2 *g, int k1, int k2, int k3, int axis, int sign, double scale, cudaStream_t st);
 template <typename T> void set_fft_smem_limits(size_t bytes);
-// qx_fftplane.cu: fused y-x-y pass (FP32, k1 x k2 planes of a specialised
-// shape, QX_PLANE_GRIDS); returns -1 when the grid is not covered.
-int launch_plane_f32(const PipeParams &P, int npl, float2 *bufA, const float *vloc, cudaStream_t st);
+// qx_fftplane.cu: fused y-x-y pass (k1 x k2 planes of a specialised shape,
+// QX_PLANE_GRIDS, QX_PLANE64_GRIDS); returns -1 when the grid is not covered.
+int launch_plane(const PipeParams &P, int npl, float2 *bufA, const float *vloc, cudaStream_t st);
+int launch_plane(const PipeParams &P, int npl, double2 *bufA, const double *vloc, cudaStream_t st);
 // The same passes split around the real-space projectors: nl null, backward
 // into R; else forward from R.  -1 when the grid is not covered.
 int launch_plane_r_f32(const PipeParams &P, int npl, float2 *bufA, float2 *R, const float *vloc,
