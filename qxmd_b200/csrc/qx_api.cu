@@ -512,6 +512,13 @@ extern "C" int qx_create(qx_ctx **out, int precision, int k1, int k2, int k3, in
   pl.ncol = (int)col_ja.size();
   std::vector<int> col_ig((size_t)k3 * std::max(1, pl.ncol), 0);
   for (auto &e : ents) col_ig[(size_t)e.i3 * pl.ncol + colq[(size_t)e.j2 * pl.P1 + e.a]] = e.sgn > 0 ? e.ig + 1 : -(e.ig + 1);
+  std::vector<uint2> col_mask(pl.P1, make_uint2(0u, 0u));
+  for (int j = 0; j < pl.P2; ++j)
+    for (int a = lo[j]; a <= hi[j]; ++a) {
+      const int k = j - m2;
+      if (k >= 0 && k < 32) col_mask[a].x |= 1u << k;
+      if (k <= 0 && k > -32) col_mask[a].y |= 1u << -k;
+    }
   int rc = 0;
 #define FAIL(x) do { rc = (x); if (rc) { qx_destroy(c); return rc; } } while (0)
   FAIL(dalloc(c, &pl.d_row_lo, sizeof(int) * pl.P2));
@@ -520,7 +527,9 @@ extern "C" int qx_create(qx_ctx **out, int precision, int k1, int k2, int k3, in
   FAIL(dalloc(c, &pl.d_row_ent, sizeof(int4) * rent.size()));
   FAIL(dalloc(c, &pl.d_col_ja, sizeof(int) * std::max<size_t>(1, col_ja.size())));
   FAIL(dalloc(c, &pl.d_col_ig, sizeof(int) * col_ig.size()));
-  if (cudaMemcpy(pl.d_row_lo, lo.data(), sizeof(int) * pl.P2, cudaMemcpyHostToDevice) ||
+  FAIL(dalloc(c, &pl.d_col_mask, sizeof(uint2) * col_mask.size()));
+  if (cudaMemcpy(pl.d_col_mask, col_mask.data(), sizeof(uint2) * col_mask.size(), cudaMemcpyHostToDevice) ||
+      cudaMemcpy(pl.d_row_lo, lo.data(), sizeof(int) * pl.P2, cudaMemcpyHostToDevice) ||
       cudaMemcpy(pl.d_row_hi, hi.data(), sizeof(int) * pl.P2, cudaMemcpyHostToDevice) ||
       cudaMemcpy(pl.d_row_off, cnt.data(), sizeof(int) * (pl.P2 + 1), cudaMemcpyHostToDevice) ||
       cudaMemcpy(pl.d_row_ent, rent.data(), sizeof(int4) * rent.size(), cudaMemcpyHostToDevice) ||
@@ -1258,11 +1267,11 @@ static PipeParams base_params(const qx_ctx *c) {
   const Plan &pl = c->pl;
   PipeParams P;
   P.k1 = pl.k1; P.k2 = pl.k2; P.k3 = pl.k3;
-  P.m1 = pl.m1; P.m2 = pl.m2; P.P1 = pl.P1; P.P2 = pl.P2;
+  P.m1 = pl.m1; P.m2 = pl.m2; P.m3 = pl.m3; P.P1 = pl.P1; P.P2 = pl.P2;
   P.nplw = pl.nplw;
   P.L1 = pl.L[0]; P.L2 = pl.L[1]; P.L3 = pl.L[2];
   P.row_lo = pl.d_row_lo; P.row_hi = pl.d_row_hi; P.row_off = pl.d_row_off; P.row_ent = pl.d_row_ent;
-  P.col_ja = pl.d_col_ja; P.col_ig = pl.d_col_ig; P.ncol = pl.ncol;
+  P.col_ja = pl.d_col_ja; P.col_ig = pl.d_col_ig; P.ncol = pl.ncol; P.col_mask = pl.d_col_mask;
   P.pairs = c->d_allpairs;
   P.npair_dev = nullptr;
   P.npair = c->npair_all;

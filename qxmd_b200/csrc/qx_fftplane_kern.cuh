@@ -36,51 +36,95 @@ struct PlaneRows {
   __device__ static int row(int t) { return both ? (t & 31) : t; }
 };
 
+// The line of N points whose samples MB < i < N - MB are zero: MB = (N - 1) / 4
+// wherever the density cutoff is at least four times the wavefunction's
+// (then the wavefunction sphere spans half the grid), (N - 1) / 2 otherwise.
+template <int N, bool HALF> constexpr int line_mb() { return HALF ? (N - 1) / 4 : (N - 1) / 2; }
+
+// Backward y transform of sphere column a of a plane (A: its [P2][P1] rows)
+// into column c of a tile with `ld` columns.
+template <int NY, int MB>
+__device__ __forceinline__ void plane_y_back(const PipeParams &P, const float2 *A, int a, float2 *Tc, int ld) {
+  const uint2 in = P.col_mask[a];
+  const int P1 = P.P1;
+  const float2 *A0 = A + P.m2 * P1 + a;
+  const float2 zero = make_float2(0.f, 0.f);
+  float2 x[NY];
+  rf::static_for<0, MB + 1>([&](auto kc) {
+    constexpr int k = decltype(kc)::value;
+    x[k] = (in.x >> k) & 1u ? A0[k * P1] : zero;
+    if constexpr (k > 0) x[NY - k] = (in.y >> k) & 1u ? A0[-k * P1] : zero;
+  });
+  if constexpr (2 * MB + 1 < NY) rf::fft_nz<float, +1, NY, MB>(x);
+  else {
+    if constexpr (2 * MB + 2 == NY) x[MB + 1] = zero;
+    rf::fft<float, +1, NY>(x);
+  }
+  rf::static_for<0, NY>([&](auto ic) {
+    constexpr int i2 = decltype(ic)::value, q = rf::out_pos(NY, i2);
+    Tc[i2 * ld] = x[q];
+  });
+}
+
+// Backward x transform of a tile row: column MB + k holds sample k (|k| <= MB).
+template <int NX, int MB>
+__device__ __forceinline__ void plane_x_back(const float2 *row, float2 (&x)[NX]) {
+  rf::static_for<0, MB + 1>([&](auto kc) {
+    constexpr int k = decltype(kc)::value;
+    x[k] = row[MB + k];
+    if constexpr (k > 0) x[NX - k] = row[MB - k];
+  });
+  if constexpr (2 * MB + 1 < NX && 2 * MB + 2 != NX) rf::fft_nz<float, +1, NX, MB>(x);
+  else {
+    if constexpr (2 * MB + 2 == NX) x[MB + 1] = make_float2(0.f, 0.f);
+    rf::fft<float, +1, NX>(x);
+  }
+}
+
 // U units a CTA: U band pairs of the same planes on 64 threads each, whose
 // phases the CTA's barriers keep together.  The unrolled transforms are some
 // tens of kilobytes of code that every unit runs once, so units in step share
 // its instruction fetches: two at 54 x 54 (Si64, 160 bands, whole H|psi>) 163
 // -> 147 us, four the same, eight 158 us.
-template <int NX, int NY, int PL, int U>
+// HALF: the sphere spans at most half of either axis (line_mb), so that the
+// zero samples' loads and butterflies and the outputs beyond the sphere are
+// left out at compile time; the tile then has 2 MBX + 1 columns, those beyond
+// the sphere zero.  At Si64 (54 x 54, 160 bands): 88 -> 49 us the pass, and the
+// outputs are the same bit for bit.
+template <int NX, int NY, int PL, int U, bool HALF>
 __global__ void __launch_bounds__(64 * U, (plane_minb(NX > NY ? NX : NY) + U - 1) / U)
     k_plane(PipeParams P, float2 *__restrict__ bufA, const float *__restrict__ vloc, int npl) {
   using rf::out_pos;
   using Rows = PlaneRows<NY, PL>;
-  // PL = 2: the CTA takes planes i3 and i3 + 1; the y phases give warp w the
-  // columns of plane w (P1 <= 32).  PL = 1: one plane, the columns on
-  // threads 0 .. P1 - 1.  NX = k1 (x, the sphere's P1 columns), NY = k2.
+  constexpr int MBX = line_mb<NX, HALF>(), MBY = line_mb<NY, HALF>(), PB = 2 * MBX + 1;
+  // PL = 2: the unit takes planes i3 and i3 + 1; the y phases give warp w the
+  // columns of plane w (PB <= 32).  PL = 1: one plane, the columns on
+  // threads 0 .. PB - 1.  NX = k1 (x, the sphere's P1 columns), NY = k2.
   const int i3b = blockIdx.x * PL;
   const int np = P.npair_dev ? *P.npair_dev : P.npair;
   if (P.pair0 + (int)blockIdx.y * U >= np) return;
   const int pl = blockIdx.y * U + (threadIdx.x >> 6);
   const bool live = pl < npl && P.pair0 + pl < np;
-  const int P1 = P.P1, P2 = P.P2, m1 = P.m1, m2 = P.m2;
+  const int P1 = P.P1, P2 = P.P2, m1 = P.m1;
   const int npl_here = live ? min(PL, P.k3 - i3b) : 0;   // planes of this unit
-  extern __shared__ float2 Tu[];   // [U][PL][NY][P1]
-  float2 *T = Tu + (threadIdx.x >> 6) * (PL * NY * P1);
+  extern __shared__ float2 Tu[];   // [U][PL][NY][PB]
+  float2 *T = Tu + (threadIdx.x >> 6) * (PL * NY * PB);
   const int t = threadIdx.x & 63;
-  const float2 zero = make_float2(0.f, 0.f);
-  // column phases: plane and column of this thread
+  // column phases: plane and tile column of this thread
   const int cpl = (PL == 2) ? (t >> 5) : 0, col = (PL == 2) ? (t & 31) : t;
-  const bool col_on = col < P1 && cpl < npl_here;
+  const bool col_on = col < PB && cpl < npl_here;
+  const int a = col - (MBX - m1);   // sphere column
+  const bool in_sphere = a >= 0 && a < P1;
   float2 *A = bufA + ((long)pl * P.k3 + i3b + cpl) * P2 * P1;
-  float2 *Tc = T + (long)cpl * NY * P1;
+  float2 *Tc = T + cpl * (NY * PB) + col;
 
-  // (1) y backward, thread = sphere column a of its plane
+  // (1) y backward, thread = column of its plane
   if (col_on) {
-    float2 x[NY];
-#pragma unroll
-    for (int i2 = 0; i2 < NY; ++i2) {
-      const int j2 = (i2 <= m2) ? i2 + m2 : ((i2 >= NY - m2) ? i2 - NY + m2 : -1);
-      float2 v = zero;
-      if (j2 >= 0 && col >= P.row_lo[j2] && col <= P.row_hi[j2]) v = A[j2 * P1 + col];
-      x[i2] = v;
+    if (in_sphere) {
+      plane_y_back<NY, MBY>(P, A, a, Tc, PB);
+    } else {
+      for (int i = 0; i < NY; ++i) Tc[i * PB] = make_float2(0.f, 0.f);
     }
-    rf::fft<float, +1, NY>(x);
-    rf::static_for<0, NY>([&](auto ic) {
-      constexpr int i2 = decltype(ic)::value, q = out_pos(NY, i2);
-      Tc[i2 * P1 + col] = x[q];
-    });
   }
   __syncthreads();
   // (2) x backward, * V, x forward; thread = grid row r of plane rp
@@ -89,41 +133,46 @@ __global__ void __launch_bounds__(64 * U, (plane_minb(NX > NY ? NX : NY) + U - 1
     const int rp = Rows::plane(t, pass);
     if (r < NY && rp < npl_here) {
       float2 x[NX];
-      float2 *row = T + ((long)rp * NY + r) * P1;
-#pragma unroll
-      for (int i1 = 0; i1 < NX; ++i1) {
-        float2 v = zero;
-        if (i1 <= m1) v = row[i1 + m1];
-        else if (i1 >= NX - m1) v = row[i1 - NX + m1];
-        x[i1] = v;
-      }
-      rf::fft<float, +1, NX>(x);
+      float2 *row = T + (rp * NY + r) * PB;
+      plane_x_back<NX, MBX>(row, x);
       const float *V = vloc + ((long)(i3b + rp) * NY + r) * NX;
       float2 y[NX];
-      rf::static_for<0, NX>([&](auto ic) {
-        constexpr int i1 = decltype(ic)::value, q = out_pos(NX, i1);
-        const float vv = V[i1];
-        y[i1] = make_float2(x[q].x * vv, x[q].y * vv);
-      });
+      if constexpr (NX % 2 == 0) {   // rows start on 8 bytes
+        rf::static_for<0, NX / 2>([&](auto ic) {
+          constexpr int i1 = 2 * decltype(ic)::value, q0 = out_pos(NX, i1), q1 = out_pos(NX, i1 + 1);
+          const float2 vv = *reinterpret_cast<const float2 *>(V + i1);
+          y[i1] = make_float2(x[q0].x * vv.x, x[q0].y * vv.x);
+          y[i1 + 1] = make_float2(x[q1].x * vv.y, x[q1].y * vv.y);
+        });
+      } else {
+        rf::static_for<0, NX>([&](auto ic) {
+          constexpr int i1 = decltype(ic)::value, q = out_pos(NX, i1);
+          const float vv = V[i1];
+          y[i1] = make_float2(x[q].x * vv, x[q].y * vv);
+        });
+      }
       rf::fft<float, -1, NX>(y);
-      rf::static_for<0, NX>([&](auto ic) {
-        constexpr int i1 = decltype(ic)::value, q = out_pos(NX, i1);
-        if (i1 <= m1) row[i1 + m1] = y[q];
-        else if (i1 >= NX - m1) row[i1 - NX + m1] = y[q];
+      rf::static_for<0, MBX + 1>([&](auto kc) {
+        constexpr int k = decltype(kc)::value;
+        row[MBX + k] = y[out_pos(NX, k)];
+        if constexpr (k > 0) row[MBX - k] = y[out_pos(NX, NX - k)];
       });
     }
   }
   __syncthreads();
-  // (3) y forward, thread = sphere column a of its plane; only rows inside the sphere are kept
-  if (col_on) {
+  // (3) y forward, thread = column of its plane; only rows inside the sphere are kept
+  if (col_on && in_sphere) {
+    const uint2 in = P.col_mask[a];
     float2 x[NY];
 #pragma unroll
-    for (int i2 = 0; i2 < NY; ++i2) x[i2] = Tc[i2 * P1 + col];
+    for (int i2 = 0; i2 < NY; ++i2) x[i2] = Tc[i2 * PB];
     rf::fft<float, -1, NY>(x);
-    rf::static_for<0, NY>([&](auto ic) {
-      constexpr int i2 = decltype(ic)::value, q = out_pos(NY, i2);
-      const int j2 = (i2 <= m2) ? i2 + m2 : ((i2 >= NY - m2) ? i2 - NY + m2 : -1);
-      if (j2 >= 0 && col >= P.row_lo[j2] && col <= P.row_hi[j2]) A[j2 * P1 + col] = x[q];
+    float2 *A0 = A + P.m2 * P1 + a;
+    rf::static_for<0, MBY + 1>([&](auto kc) {
+      constexpr int k = decltype(kc)::value;
+      if ((in.x >> k) & 1u) A0[k * P1] = x[out_pos(NY, k)];
+      if constexpr (k > 0)
+        if ((in.y >> k) & 1u) A0[-k * P1] = x[out_pos(NY, NY - k)];
     });
   }
 }
@@ -277,43 +326,36 @@ __global__ void __launch_bounds__(2 * N) k_plane2(PipeParams P, float2 *__restri
 // kernels and the scatter by float atomics in shared memory that these
 // replace, per 160-band pass at Si64: y and x backward 118 -> 55 us, forward
 // 366 -> 145 us.
-template <int NX, int NY>
+template <int NX, int NY, bool HALF>
 __global__ void __launch_bounds__(128, plane_minb(NX > NY ? NX : NY) > 1 ? 4 : 1)
     k_plane_inv_r(PipeParams P, const float2 *__restrict__ bufA, float2 *__restrict__ R, int npl) {
   using rf::out_pos;
-  constexpr int LD = NX | 1;
+  constexpr int LD = NX | 1, MBX = line_mb<NX, HALF>(), MBY = line_mb<NY, HALF>();
   const int i3 = blockIdx.x, h = threadIdx.x >> 6, u = threadIdx.x & 63;
   const int pl = blockIdx.y * 2 + h, np = P.npair_dev ? *P.npair_dev : P.npair;
   if (P.pair0 + (int)blockIdx.y * 2 >= np) return;
   const bool on = pl < npl && P.pair0 + pl < np;
-  const int P1 = P.P1, P2 = P.P2, m1 = P.m1, m2 = P.m2;
   extern __shared__ float2 T[];
   float2 *Tp = T + h * (NY * LD);
-  const float2 zero = make_float2(0.f, 0.f);
-  if (on && u < P1) {
-    const float2 *A = bufA + ((long)pl * P.k3 + i3) * P2 * P1;
-    const int xi = u >= m1 ? u - m1 : u - m1 + NX;
-    float2 x[NY];
-#pragma unroll
-    for (int i2 = 0; i2 < NY; ++i2) {
-      const int j2 = (i2 <= m2) ? i2 + m2 : ((i2 >= NY - m2) ? i2 - NY + m2 : -1);
-      float2 v = zero;
-      if (j2 >= 0 && u >= P.row_lo[j2] && u <= P.row_hi[j2]) v = A[j2 * P1 + u];
-      x[i2] = v;
+  if (on && u < 2 * MBX + 1) {   // x sample k = u - MBX, at position k or NX + k of the rows
+    const int k = u - MBX, a = k + P.m1;
+    float2 *Tc = Tp + (k >= 0 ? k : NX + k);
+    if (a >= 0 && a < P.P1) {
+      plane_y_back<NY, MBY>(P, bufA + ((long)pl * P.k3 + i3) * P.P2 * P.P1, a, Tc, LD);
+    } else {
+      for (int i = 0; i < NY; ++i) Tc[i * LD] = make_float2(0.f, 0.f);
     }
-    rf::fft<float, +1, NY>(x);
-    rf::static_for<0, NY>([&](auto ic) {
-      constexpr int i2 = decltype(ic)::value, q = out_pos(NY, i2);
-      Tp[i2 * LD + xi] = x[q];
-    });
   }
   __syncthreads();
   if (on && u < NY) {
     float2 x[NX];
     float2 *row = Tp + u * LD;
-#pragma unroll
-    for (int i1 = 0; i1 < NX; ++i1) x[i1] = (i1 <= m1 || i1 >= NX - m1) ? row[i1] : zero;
-    rf::fft<float, +1, NX>(x);
+    rf::static_for<0, MBX + 1>([&](auto kc) {
+      constexpr int k = decltype(kc)::value;
+      x[k] = row[k];
+      if constexpr (k > 0) x[NX - k] = row[NX - k];
+    });
+    rf::fft_nz<float, +1, NX, MBX>(x);
     rf::static_for<0, NX>([&](auto ic) {
       constexpr int i1 = decltype(ic)::value, q = out_pos(NX, i1);
       row[i1] = x[q];
@@ -327,19 +369,18 @@ __global__ void __launch_bounds__(128, plane_minb(NX > NY ? NX : NY) > 1 ? 4 : 1
   }
 }
 
-template <int NX, int NY>
+template <int NX, int NY, bool HALF>
 __global__ void __launch_bounds__(128, plane_minb(NX > NY ? NX : NY) > 1 ? 4 : 1)
     k_plane_fwd_r(PipeParams P, const float2 *__restrict__ R, float2 *__restrict__ bufA,
                   const float *__restrict__ vloc, NlPoints<float> nl, int npl) {
   using rf::out_pos;
-  constexpr int LD = NX | 1, NP = NX * NY, UN = 4;
+  constexpr int LD = NX | 1, NP = NX * NY, UN = 4, MBX = line_mb<NX, HALF>(), MBY = line_mb<NY, HALF>();
   const int i3 = blockIdx.x, t = threadIdx.x, h = t >> 6, u = t & 63;
   const int pl0 = blockIdx.y * 2, np = P.npair_dev ? *P.npair_dev : P.npair;
   if (P.pair0 + pl0 >= np) return;
   const bool two = pl0 + 1 < npl && P.pair0 + pl0 + 1 < np;
-  const int P1 = P.P1, P2 = P.P2, m1 = P.m1, m2 = P.m2;
+  const int P1 = P.P1;
   extern __shared__ float2 T[];
-  const float2 zero = make_float2(0.f, 0.f);
   {
     const long g0 = (long)i3 * NP;
     const float2 *R0 = R + (long)pl0 * P.k3 * NP + g0, *R1 = two ? R0 + (long)P.k3 * NP : R0;
@@ -419,23 +460,27 @@ __global__ void __launch_bounds__(128, plane_minb(NX > NY ? NX : NY) > 1 ? 4 : 1
 #pragma unroll
     for (int i1 = 0; i1 < NX; ++i1) x[i1] = row[i1];
     rf::fft<float, -1, NX>(x);
-    rf::static_for<0, NX>([&](auto ic) {
-      constexpr int i1 = decltype(ic)::value, q = out_pos(NX, i1);
-      if (i1 <= m1 || i1 >= NX - m1) row[i1] = x[q];
+    rf::static_for<0, MBX + 1>([&](auto kc) {
+      constexpr int k = decltype(kc)::value;
+      row[k] = x[out_pos(NX, k)];
+      if constexpr (k > 0) row[NX - k] = x[out_pos(NX, NX - k)];
     });
   }
   __syncthreads();
   if (on && u < P1) {
-    const int xi = u >= m1 ? u - m1 : u - m1 + NX;
-    float2 *A = bufA + ((long)(pl0 + h) * P.k3 + i3) * P2 * P1;
+    const int k1 = u - P.m1;
+    const uint2 in = P.col_mask[u];
+    const float2 *Tc = Tp + (k1 >= 0 ? k1 : NX + k1);
+    float2 *A0 = bufA + ((long)(pl0 + h) * P.k3 + i3) * P.P2 * P1 + P.m2 * P1 + u;
     float2 x[NY];
 #pragma unroll
-    for (int i2 = 0; i2 < NY; ++i2) x[i2] = Tp[i2 * LD + xi];
+    for (int i2 = 0; i2 < NY; ++i2) x[i2] = Tc[i2 * LD];
     rf::fft<float, -1, NY>(x);
-    rf::static_for<0, NY>([&](auto ic) {
-      constexpr int i2 = decltype(ic)::value, q = out_pos(NY, i2);
-      const int j2 = (i2 <= m2) ? i2 + m2 : ((i2 >= NY - m2) ? i2 - NY + m2 : -1);
-      if (j2 >= 0 && u >= P.row_lo[j2] && u <= P.row_hi[j2]) A[j2 * P1 + u] = x[q];
+    rf::static_for<0, MBY + 1>([&](auto kc) {
+      constexpr int k = decltype(kc)::value;
+      if ((in.x >> k) & 1u) A0[k * P1] = x[out_pos(NY, k)];
+      if constexpr (k > 0)
+        if ((in.y >> k) & 1u) A0[-k * P1] = x[out_pos(NY, NY - k)];
     });
   }
 }
@@ -452,7 +497,7 @@ __global__ void __launch_bounds__(128, plane_minb(NX > NY ? NX : NY) > 1 ? 4 : 1
 //            scatter to zsph as k_zfwd does.
 constexpr int ZC_T = 64;
 
-template <int N>
+template <int N, bool HALF>
 __global__ void __launch_bounds__(ZC_T) k_zcols_inv(PipeParams P, const float *__restrict__ cin, long ldc,
                                                      float2 *__restrict__ bufA) {
   using rf::out_pos;
@@ -462,9 +507,9 @@ __global__ void __launch_bounds__(ZC_T) k_zcols_inv(PipeParams P, const float *_
   const int bA = P.pairs[2 * p], bB = P.pairs[2 * p + 1];
   const float *cA = cin + (long)bA * ldc;
   const float *cB = bB >= 0 ? cin + (long)bB * ldc : nullptr;
+  constexpr int MB = line_mb<N, HALF>();   // samples beyond it are zero
   float2 x[N];
-#pragma unroll
-  for (int i3 = 0; i3 < N; ++i3) {
+  auto load = [&](int i3) {
     const int code = P.col_ig[i3 * P.ncol + q];
     float2 z = make_float2(0.f, 0.f);
     if (code != 0) {
@@ -474,9 +519,14 @@ __global__ void __launch_bounds__(ZC_T) k_zcols_inv(PipeParams P, const float *_
       if (code > 0) { z.x = ra - ib; z.y = ia + rb; }
       else          { z.x = ra + ib; z.y = rb - ia; }
     }
-    x[i3] = z;
-  }
-  rf::fft<float, +1, N>(x);
+    return z;
+  };
+  rf::static_for<0, MB + 1>([&](auto kc) {
+    constexpr int k = decltype(kc)::value;
+    x[k] = load(k);
+    if constexpr (k > 0) x[N - k] = load(N - k);
+  });
+  rf::fft_nz<float, +1, N, MB>(x);
   float2 *dst = bufA + (long)pl * N * P.P2 * P.P1 + P.col_ja[q];
   rf::static_for<0, N>([&](auto ic) {
     constexpr int i3 = decltype(ic)::value;
@@ -484,7 +534,7 @@ __global__ void __launch_bounds__(ZC_T) k_zcols_inv(PipeParams P, const float *_
   });
 }
 
-template <int N>
+template <int N, bool HALF>
 __global__ void __launch_bounds__(ZC_T) k_zcols_fwd(PipeParams P, const float2 *__restrict__ bufA,
                                                      float2 *__restrict__ zsph) {
   using rf::out_pos;
@@ -498,7 +548,7 @@ __global__ void __launch_bounds__(ZC_T) k_zcols_fwd(PipeParams P, const float2 *
   rf::fft<float, -1, N>(x);
   const float s = (float)P.inv_n;
   float2 *Z = zsph + (long)pl * (P.nplw + 1) * 2;
-  rf::static_for<0, N>([&](auto ic) {
+  auto store = [&](auto ic) {
     constexpr int i3 = decltype(ic)::value;
     const int code = P.col_ig[i3 * P.ncol + q];
     if (code != 0) {
@@ -513,8 +563,14 @@ __global__ void __launch_bounds__(ZC_T) k_zcols_fwd(PipeParams P, const float2 *
         Z[2 * (-code - 1) + 1] = z;
       }
     }
+  };
+  rf::static_for<0, line_mb<N, HALF>() + 1>([&](auto kc) {
+    constexpr int k = decltype(kc)::value;
+    store(rf::IC<k>{});
+    if constexpr (k > 0) store(rf::IC<N - k>{});
   });
 }
+
 
 // The inverse z pass for the two-lanes-a-line lengths (N = 2H > 64): lanes
 // 2c and 2c + 1 own sphere z-column c, each gathers the coefficients of the
@@ -573,8 +629,13 @@ template <int N>
 int zcols_launch(const PipeParams &P, int npl, const float *cin, long ldc, float2 *bufA, const float2 *src,
                         float2 *zsph, bool inv, cudaStream_t st) {
   dim3 g((P.ncol + ZC_T - 1) / ZC_T, npl);
-  if (inv) k_zcols_inv<N><<<g, ZC_T, 0, st>>>(P, cin, ldc, bufA);
-  else k_zcols_fwd<N><<<g, ZC_T, 0, st>>>(P, src, zsph);
+  if (P.m3 <= line_mb<N, true>()) {
+    if (inv) k_zcols_inv<N, true><<<g, ZC_T, 0, st>>>(P, cin, ldc, bufA);
+    else k_zcols_fwd<N, true><<<g, ZC_T, 0, st>>>(P, src, zsph);
+  } else {
+    if (inv) k_zcols_inv<N, false><<<g, ZC_T, 0, st>>>(P, cin, ldc, bufA);
+    else k_zcols_fwd<N, false><<<g, ZC_T, 0, st>>>(P, src, zsph);
+  }
   note_launch();
   return 0;
 }
@@ -586,7 +647,7 @@ int zcols_launch(const PipeParams &P, int npl, const float *cin, long ldc, float
 // owns one grid row).  The group's partial plane goes to part[group]; a
 // second kernel sums the groups in a fixed order, so the result is the same
 // from run to run.
-template <int NX, int NY, int PL>
+template <int NX, int NY, int PL, bool HALF>
 __global__ void __launch_bounds__(64) k_rho_plane(PipeParams P, const float2 *__restrict__ bufA,
                                                   const double *__restrict__ wocc, double *__restrict__ part,
                                                   int npl, int per_group) {
@@ -595,38 +656,28 @@ __global__ void __launch_bounds__(64) k_rho_plane(PipeParams P, const float2 *__
   // PL = 2: planes i3 and i3 + 1, warp w taking plane w's columns in the y
   // phase (P1 <= 32); the x phase as in k_plane.
   const int i3b = blockIdx.x * PL, grp = blockIdx.y;
-  const int P1 = P.P1, P2 = P.P2, m1 = P.m1, m2 = P.m2;
+  constexpr int MBX = line_mb<NX, HALF>(), MBY = line_mb<NY, HALF>(), PB = 2 * MBX + 1, LA = NX | 1;
   const int npl_here = min(PL, P.k3 - i3b);
   constexpr int NP = NX * NY;
-  extern __shared__ double accs[];            // [PL][NY][NX] FP64, then the [PL][NY][P1] complex tiles
-  float2 *T = reinterpret_cast<float2 *>(accs + PL * NP);
+  // [PL][NY][LA] FP64 (a row's pitch keeps the rows of a warp in different
+  // banks), then the [PL][NY][PB] complex tiles
+  extern __shared__ double accs[];
+  float2 *T = reinterpret_cast<float2 *>(accs + PL * NY * LA);
   const int t = threadIdx.x;
-  const float2 zero = make_float2(0.f, 0.f);
   const int cpl = (PL == 2) ? (t >> 5) : 0, col = (PL == 2) ? (t & 31) : t;
-  const bool col_on = col < P1 && cpl < npl_here;
-  float2 *Tc = T + (long)cpl * NY * P1;
-  for (int i = t; i < PL * NP; i += blockDim.x) accs[i] = 0.0;
+  const bool col_on = col < PB && cpl < npl_here;
+  const int a0 = col - (MBX - P.m1);   // sphere column
+  float2 *Tc = T + cpl * (NY * PB) + col;
+  for (int i = t; i < PL * NY * LA; i += blockDim.x) accs[i] = 0.0;
+  if (col_on && (a0 < 0 || a0 >= P.P1))
+    for (int i = 0; i < NY; ++i) Tc[i * PB] = make_float2(0.f, 0.f);
   const int np = min(npl, (P.npair_dev ? *P.npair_dev : P.npair) - P.pair0);
   const int pl0 = grp * per_group, pl1 = min(np, pl0 + per_group);
   const int r = Rows::row(t);
   for (int pl = pl0; pl < pl1; ++pl) {
     const int p = P.pair0 + pl;
-    const float2 *A = bufA + ((long)pl * P.k3 + i3b + cpl) * P2 * P1;
-    if (col_on) {
-      float2 x[NY];
-#pragma unroll
-      for (int i2 = 0; i2 < NY; ++i2) {
-        const int j2 = (i2 <= m2) ? i2 + m2 : ((i2 >= NY - m2) ? i2 - NY + m2 : -1);
-        float2 v = zero;
-        if (j2 >= 0 && col >= P.row_lo[j2] && col <= P.row_hi[j2]) v = A[j2 * P1 + col];
-        x[i2] = v;
-      }
-      rf::fft<float, +1, NY>(x);
-      rf::static_for<0, NY>([&](auto ic) {
-        constexpr int i2 = decltype(ic)::value, q = out_pos(NY, i2);
-        Tc[i2 * P1 + col] = x[q];
-      });
-    }
+    if (col_on && a0 >= 0 && a0 < P.P1)
+      plane_y_back<NY, MBY>(P, bufA + ((long)pl * P.k3 + i3b + cpl) * P.P2 * P.P1, a0, Tc, PB);
     __syncthreads();
     const int bA = P.pairs[2 * p], bB = P.pairs[2 * p + 1];
     const double fa = wocc[bA], fb = bB >= 0 ? wocc[bB] : 0.0;
@@ -634,16 +685,8 @@ __global__ void __launch_bounds__(64) k_rho_plane(PipeParams P, const float2 *__
       const int rp = Rows::plane(t, pass);
       if (r < NY && rp < npl_here) {
         float2 x[NX];
-        const float2 *row = T + ((long)rp * NY + r) * P1;
-#pragma unroll
-        for (int i1 = 0; i1 < NX; ++i1) {
-          float2 v = zero;
-          if (i1 <= m1) v = row[i1 + m1];
-          else if (i1 >= NX - m1) v = row[i1 - NX + m1];
-          x[i1] = v;
-        }
-        rf::fft<float, +1, NX>(x);
-        double *a = accs + ((long)rp * NY + r) * NX;
+        plane_x_back<NX, MBX>(T + (rp * NY + r) * PB, x);
+        double *a = accs + (rp * NY + r) * LA;
         rf::static_for<0, NX>([&](auto ic) {
           constexpr int i1 = decltype(ic)::value, q = out_pos(NX, i1);
           const double re = x[q].x, im = x[q].y;
@@ -656,7 +699,7 @@ __global__ void __launch_bounds__(64) k_rho_plane(PipeParams P, const float2 *__
   __syncthreads();
   for (int rp = 0; rp < npl_here; ++rp) {
     double *dst = part + ((long)grp * P.k3 + i3b + rp) * NP;
-    for (int i = t; i < NP; i += blockDim.x) dst[i] = accs[(long)rp * NP + i];
+    for (int i = t; i < NP; i += blockDim.x) dst[i] = accs[(rp * NY + i / NX) * LA + i % NX];
   }
 }
 
@@ -732,27 +775,32 @@ __global__ void __launch_bounds__(2 * N) k_rho_plane2(PipeParams P, const float2
   for (int i = t; i < N * N; i += 2 * N) dst[i] = accs[i];
 }
 
-template <int NX, int NY>
-int rho_launch(const PipeParams &P, int npl, const float2 *bufA, const double *wocc, double *part, double *rho,
-               int accumulate, cudaStream_t st) {
+template <int NX, int NY, int PL, bool HALF>
+static void rho_go(const PipeParams &P, int npl, const float2 *bufA, const double *wocc, double *part,
+                   cudaStream_t st) {
+  constexpr size_t sm = PL * NY * (sizeof(double) * (NX | 1) + sizeof(float2) * (2 * line_mb<NX, HALF>() + 1));
   static bool attr = false;
   if (!attr) {
-    cudaFuncSetAttribute(k_rho_plane<NX, NY, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, 96 * 1024);
-    cudaFuncSetAttribute(k_rho_plane<NX, NY, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, 192 * 1024);
+    cudaFuncSetAttribute(k_rho_plane<NX, NY, PL, HALF>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
     attr = true;
   }
   const int per_group = (npl + RHO_GROUPS - 1) / RHO_GROUPS;
-  const size_t sm1 = sizeof(double) * (size_t)NX * NY + sizeof(float2) * (size_t)NY * P.P1;
-  if (P.P1 <= 32 && plane_pairs_enabled() && 2 * sm1 <= 192 * 1024) {
-    dim3 g((P.k3 + 1) / 2, RHO_GROUPS);
-    k_rho_plane<NX, NY, 2><<<g, 64, 2 * sm1, st>>>(P, bufA, wocc, part, npl, per_group);
+  k_rho_plane<NX, NY, PL, HALF>
+      <<<dim3((P.k3 + PL - 1) / PL, RHO_GROUPS), 64, sm, st>>>(P, bufA, wocc, part, npl, per_group);
+}
+
+template <int NX, int NY>
+int rho_launch(const PipeParams &P, int npl, const float2 *bufA, const double *wocc, double *part, double *rho,
+               int accumulate, cudaStream_t st) {
+  // two planes a CTA where the half sphere fits 32 lanes
+  if (P.m1 <= line_mb<NX, true>() && P.m2 <= line_mb<NY, true>()) {
+    if (plane_pairs_enabled()) rho_go<NX, NY, 2, true>(P, npl, bufA, wocc, part, st);
+    else rho_go<NX, NY, 1, true>(P, npl, bufA, wocc, part, st);
   } else {
-    dim3 g(P.k3, RHO_GROUPS);
-    k_rho_plane<NX, NY, 1><<<g, 64, sm1, st>>>(P, bufA, wocc, part, npl, per_group);
+    rho_go<NX, NY, 1, false>(P, npl, bufA, wocc, part, st);
   }
   note_launch();
-  const long n = (long)P.k1 * P.k2 * P.k3;
-  rho_groups_launch(part, n, rho, accumulate, st);
+  rho_groups_launch(part, (long)P.k1 * P.k2 * P.k3, rho, accumulate, st);
   return 0;
 }
 
@@ -775,41 +823,56 @@ int rho2_launch(const PipeParams &P, int npl, const float2 *bufA, const double *
   return 0;
 }
 
-template <int NX, int NY>
-int plane_launch(const PipeParams &P, int npl, float2 *bufA, const float *vloc, cudaStream_t st) {
-  constexpr int U = 2;
+template <int NX, int NY, int PL, int U, bool HALF>
+static void plane_go(const PipeParams &P, int npl, float2 *bufA, const float *vloc, cudaStream_t st) {
+  constexpr size_t sm = sizeof(float2) * U * PL * NY * (2 * line_mb<NX, HALF>() + 1);
   static bool attr = false;
   if (!attr) {
-    cudaFuncSetAttribute(k_plane<NX, NY, 1, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, 64 * 1024);
-    cudaFuncSetAttribute(k_plane<NX, NY, 2, U>, cudaFuncAttributeMaxDynamicSharedMemorySize, 80 * 1024);
+    cudaFuncSetAttribute(k_plane<NX, NY, PL, U, HALF>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
     attr = true;
   }
-  if (P.P1 <= 32 && plane_pairs_enabled()) {   // two planes a unit: warp w takes plane w's columns
-    const size_t sm = sizeof(float2) * 2 * U * (size_t)NY * P.P1;
-    k_plane<NX, NY, 2, U><<<dim3((P.k3 + 1) / 2, (npl + U - 1) / U), 64 * U, sm, st>>>(P, bufA, vloc, npl);
+  k_plane<NX, NY, PL, U, HALF>
+      <<<dim3((P.k3 + PL - 1) / PL, (npl + U - 1) / U), 64 * U, sm, st>>>(P, bufA, vloc, npl);
+}
+
+template <int NX, int NY>
+int plane_launch(const PipeParams &P, int npl, float2 *bufA, const float *vloc, cudaStream_t st) {
+  const bool half = P.m1 <= line_mb<NX, true>() && P.m2 <= line_mb<NY, true>();
+  if (half) {
+    // two planes a unit (warp w takes plane w's columns) where 32 lanes hold the columns
+    if constexpr (2 * line_mb<NX, true>() + 1 <= 32) {
+      if (plane_pairs_enabled()) plane_go<NX, NY, 2, 2, true>(P, npl, bufA, vloc, st);
+      else plane_go<NX, NY, 1, 1, true>(P, npl, bufA, vloc, st);
+    } else {
+      plane_go<NX, NY, 1, 1, true>(P, npl, bufA, vloc, st);
+    }
   } else {
-    const size_t sm = sizeof(float2) * (size_t)NY * P.P1;
-    k_plane<NX, NY, 1, 1><<<dim3(P.k3, npl), 64, sm, st>>>(P, bufA, vloc, npl);
+    plane_go<NX, NY, 1, 1, false>(P, npl, bufA, vloc, st);
   }
   note_launch();
   return 0;
 }
 
-template <int NX, int NY>
-int plane_r_launch(const PipeParams &P, int npl, float2 *bufA, float2 *R, const float *vloc,
-                   const NlPoints<float> *nl, cudaStream_t st) {
-  const size_t sm = sizeof(float2) * 2 * (size_t)NY * (NX | 1);
+template <int NX, int NY, bool HALF>
+static void plane_r_go(const PipeParams &P, int npl, float2 *bufA, float2 *R, const float *vloc,
+                       const NlPoints<float> *nl, cudaStream_t st) {
+  constexpr size_t sm = sizeof(float2) * 2 * (size_t)NY * (NX | 1);
   static bool attr = false;
   if (!attr) {
-    cudaFuncSetAttribute(k_plane_inv_r<NX, NY>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-    cudaFuncSetAttribute(k_plane_fwd_r<NX, NY>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+    cudaFuncSetAttribute(k_plane_inv_r<NX, NY, HALF>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+    cudaFuncSetAttribute(k_plane_fwd_r<NX, NY, HALF>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
     attr = true;
   }
   dim3 g(P.k3, (npl + 1) / 2);
-  if (nl)
-    k_plane_fwd_r<NX, NY><<<g, 128, sm, st>>>(P, R, bufA, vloc, *nl, npl);
-  else
-    k_plane_inv_r<NX, NY><<<g, 128, sm, st>>>(P, bufA, R, npl);
+  if (nl) k_plane_fwd_r<NX, NY, HALF><<<g, 128, sm, st>>>(P, R, bufA, vloc, *nl, npl);
+  else k_plane_inv_r<NX, NY, HALF><<<g, 128, sm, st>>>(P, bufA, R, npl);
+}
+
+template <int NX, int NY>
+int plane_r_launch(const PipeParams &P, int npl, float2 *bufA, float2 *R, const float *vloc,
+                   const NlPoints<float> *nl, cudaStream_t st) {
+  if (P.m1 <= line_mb<NX, true>() && P.m2 <= line_mb<NY, true>()) plane_r_go<NX, NY, true>(P, npl, bufA, R, vloc, nl, st);
+  else plane_r_go<NX, NY, false>(P, npl, bufA, R, vloc, nl, st);
   note_launch();
   return 0;
 }

@@ -194,8 +194,82 @@ template <typename T, int SIGN, int R> struct LeafPrime {
 template <typename T, int SIGN> struct Leaf<T, SIGN, 5> : LeafPrime<T, SIGN, 5> {};
 template <typename T, int SIGN> struct Leaf<T, SIGN, 7> : LeafPrime<T, SIGN, 7> {};
 
+// The innermost leaves of a transform whose inputs ZM < i < N - ZM are known to
+// be zero (their values are never read): butterflies with the zero terms
+// left out.  NZ: bit r set where input r of the leaf may be nonzero.
+template <bool A, bool B, typename C> QX_HD C addz(C a, C b) {
+  if constexpr (A && B) return add(a, b);
+  else if constexpr (A) return a;
+  else return b;
+}
+template <bool A, bool B, typename C> QX_HD C subz(C a, C b) {
+  if constexpr (A && B) return sub(a, b);
+  else if constexpr (A) return a;
+  else { b.x = -b.x; b.y = -b.y; return b; }
+}
+template <typename T, int SIGN, int R, int NZ, typename C> QX_HD void leaf_nz(C *v) {
+  constexpr int FULL = (1 << R) - 1;
+  if constexpr (NZ == FULL) {
+    Leaf<T, SIGN, R>::run(v);
+  } else {
+    C zero;
+    zero.x = 0;
+    zero.y = 0;
+    if constexpr (NZ == 0) {
+#pragma unroll
+      for (int r = 0; r < R; ++r) v[r] = zero;
+    } else if constexpr (NZ == 1) {
+#pragma unroll
+      for (int r = 1; r < R; ++r) v[r] = v[0];
+    } else if constexpr (R == 2) {   // input 1 alone
+      v[0] = v[1];
+      v[1].x = -v[0].x;
+      v[1].y = -v[0].y;
+    } else if constexpr (R == 3) {
+      constexpr bool n0 = NZ & 1, n1 = NZ & 2, n2 = NZ & 4;
+      constexpr T h = (T)0.86602540378443864676 * (T)SIGN;
+      const C t1 = addz<n1, n2>(v[1], v[2]), d = subz<n1, n2>(v[1], v[2]);
+      C t2, jd;
+      t2.x = (n0 ? v[0].x : (T)0) - (T)0.5 * t1.x;
+      t2.y = (n0 ? v[0].y : (T)0) - (T)0.5 * t1.y;
+      jd.x = -h * d.y;
+      jd.y = h * d.x;
+      v[0] = addz<n0, true>(v[0], t1);
+      v[1] = add(t2, jd);
+      v[2] = sub(t2, jd);
+    } else if constexpr (R == 4) {
+      constexpr bool n0 = NZ & 1, n1 = NZ & 2, n2 = NZ & 4, n3 = NZ & 8;
+      constexpr bool e = n0 || n2, o = n1 || n3;
+      C s0 = zero, d0 = zero, s1 = zero, jd = zero;
+      if constexpr (e) { s0 = addz<n0, n2>(v[0], v[2]); d0 = subz<n0, n2>(v[0], v[2]); }
+      if constexpr (o) {
+        s1 = addz<n1, n3>(v[1], v[3]);
+        const C d1 = subz<n1, n3>(v[1], v[3]);
+        if (SIGN < 0) { jd.x = d1.y; jd.y = -d1.x; } else { jd.x = -d1.y; jd.y = d1.x; }
+      }
+      v[0] = addz<e, o>(s0, s1);
+      v[2] = subz<e, o>(s0, s1);
+      v[1] = addz<e, o>(d0, jd);
+      v[3] = subz<e, o>(d0, jd);
+    } else {                         // the odd radices: zero inputs as values
+#pragma unroll
+      for (int r = 0; r < R; ++r)
+        if (!((NZ >> r) & 1)) v[r] = zero;
+      Leaf<T, SIGN, R>::run(v);
+    }
+  }
+}
+template <int R, int OFF, int STR, int TOT, int ZM> constexpr int leaf_mask() {
+  int m = 0;
+  for (int r = 0; r < R; ++r) {
+    const int i = OFF + STR * r;
+    if (ZM < 0 || i <= ZM || i >= TOT - ZM) m |= 1 << r;
+  }
+  return m;
+}
+
 // Combine step for output group k (template recursion over k).
-template <typename T, int SIGN, int N, int OFF, int STR, int TOT, int K>
+template <typename T, int SIGN, int N, int OFF, int STR, int TOT, int K, int ZM>
 QX_HD void combine(typename C2<T>::t (&x)[TOT]) {
   constexpr int R = leaf_radix(N), M = N / R;
   if constexpr (K < M) {
@@ -209,32 +283,33 @@ QX_HD void combine(typename C2<T>::t (&x)[TOT]) {
     if constexpr (R >= 5) v[4] = twiddle<T, SIGN, 4L * K, N>(x[OFF + STR * (4 + R * PK)]);
     if constexpr (R >= 6) v[5] = twiddle<T, SIGN, 5L * K, N>(x[OFF + STR * (5 + R * PK)]);
     if constexpr (R >= 7) v[6] = twiddle<T, SIGN, 6L * K, N>(x[OFF + STR * (6 + R * PK)]);
-    Leaf<T, SIGN, R>::run(v);
+    if constexpr (M == 1 && ZM >= 0) leaf_nz<T, SIGN, R, leaf_mask<R, OFF, STR, TOT, ZM>()>(v);
+    else Leaf<T, SIGN, R>::run(v);
     // X[K + q M] -> position q + R*PK
 #pragma unroll
     for (int q = 0; q < R; ++q) x[OFF + STR * (q + R * PK)] = v[q];
-    combine<T, SIGN, N, OFF, STR, TOT, K + 1>(x);
+    combine<T, SIGN, N, OFF, STR, TOT, K + 1, ZM>(x);
   }
 }
 
-template <typename T, int SIGN, int N, int OFF, int STR, int TOT>
+template <typename T, int SIGN, int N, int OFF, int STR, int TOT, int ZM>
 QX_HD void rfft(typename C2<T>::t (&x)[TOT]);
 
-template <typename T, int SIGN, int N, int OFF, int STR, int TOT, int Rr>
+template <typename T, int SIGN, int N, int OFF, int STR, int TOT, int Rr, int ZM>
 QX_HD void subffts(typename C2<T>::t (&x)[TOT]) {
   constexpr int R = leaf_radix(N), M = N / R;
   if constexpr (Rr < R) {
-    rfft<T, SIGN, M, OFF + STR * Rr, STR * R, TOT>(x);
-    subffts<T, SIGN, N, OFF, STR, TOT, Rr + 1>(x);
+    rfft<T, SIGN, M, OFF + STR * Rr, STR * R, TOT, ZM>(x);
+    subffts<T, SIGN, N, OFF, STR, TOT, Rr + 1, ZM>(x);
   }
 }
 
-template <typename T, int SIGN, int N, int OFF, int STR, int TOT>
+template <typename T, int SIGN, int N, int OFF, int STR, int TOT, int ZM>
 QX_HD void rfft(typename C2<T>::t (&x)[TOT]) {
   static_assert(leaf_radix(N) <= 7, "lengths must be products of 2, 3, 5, 7");
   if constexpr (N > 1) {
-    subffts<T, SIGN, N, OFF, STR, TOT, 0>(x);
-    combine<T, SIGN, N, OFF, STR, TOT, 0>(x);
+    subffts<T, SIGN, N, OFF, STR, TOT, 0, ZM>(x);
+    combine<T, SIGN, N, OFF, STR, TOT, 0, ZM>(x);
   }
 }
 
@@ -242,7 +317,12 @@ QX_HD void rfft(typename C2<T>::t (&x)[TOT]) {
 // result at positions out_pos(N, k).
 template <typename T, int SIGN, int N>
 QX_HD void fft(typename C2<T>::t (&x)[N]) {
-  rfft<T, SIGN, N, 0, 1, N>(x);
+  rfft<T, SIGN, N, 0, 1, N, -1>(x);
+}
+// The same for inputs that are zero at ZM < j < N - ZM (not read there).
+template <typename T, int SIGN, int N, int ZM>
+QX_HD void fft_nz(typename C2<T>::t (&x)[N]) {
+  rfft<T, SIGN, N, 0, 1, N, (2 * ZM + 1 < N ? ZM : -1)>(x);
 }
 
 }  // namespace rf
