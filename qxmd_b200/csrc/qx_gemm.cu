@@ -8,12 +8,13 @@
 // 2*sum - x(1)*y(1) is applied in the epilogue.
 #include <algorithm>
 #include <atomic>
-#include <cmath>
+#include <cooperative_groups.h>
 
 #include "qx_internal.h"
 #include "qx_cg.h"
 
 namespace qx {
+namespace cg = cooperative_groups;
 
 constexpr int BM = 64, BN = 64, BK = 16;
 
@@ -514,8 +515,9 @@ static double tc_min_flops() {
 // row offsets of what a thread stages are computed once (B through the
 // column map).  Shared layout [k][row] for both operands (pitch rows + 1):
 // in a warp the A reads are two broadcasts and the B reads 16 consecutive
-// words.  Split-K partials and the epilogue as k_gemm's.
+// words.  Split K is summed in clusters (below); the epilogue is k_gemm's.
 constexpr int SBK = 16, SST = 3;
+constexpr int SCL = 8;   // splits of K summed within a cluster
 
 __device__ __forceinline__ void cp_async4(float *sdst, const float *gsrc, bool live) {
   const unsigned sa = (unsigned)__cvta_generic_to_shared(sdst);
@@ -612,62 +614,90 @@ __global__ void __launch_bounds__(256) k_sgemm(int M, int N, int K, float alpha,
     }
   }
   cp_async_wait<0>();
-  if (SPLIT) {
-    // Split K: every CTA stores its partial tile (element e of thread t at
-    // W[((z tiles + tile) MT NT + e) 256 + t], coalesced), counts itself in
-    // for the tile, and the last to arrive sums the partials in z order and
-    // finishes the tile; it then clears the count for the next launch.  No
-    // CTA waits for another.
+  // final value of element (gm, gn): the Gamma metric, alpha, beta and the row scale
+  auto put = [&](int gm, int gn, float v) {
+    if (gm >= M || gn >= Nact) return;
+    const long cn = colmap ? colmap[gn] : gn;
+    if (gamma) {
+      const float a0 = TA ? A[(long)gm * lda] : A[gm];
+      const float b0 = TB ? B[cn] : B[cn * ldb];
+      v = 2.f * v - a0 * b0;
+      if (gamma == 2) {
+        const float a1 = TA ? A[(long)gm * lda + 1] : A[lda + gm];
+        const float b1 = TB ? B[ldb + cn] : B[cn * ldb + 1];
+        v -= 2.f * a1 * b1;
+      }
+    }
+    float *c = Cm + cn * ldc + gm;
+    v = (beta == 0.f) ? alpha * v : alpha * v + beta * *c;
+    *c = rowscale ? v * rowscale[gm] : v;
+  };
+  if constexpr (SPLIT) {
+    // Split K, a cluster of SCL splits at a time: every CTA leaves its partial
+    // tile in shared memory (element e of thread t at e 256 + t), and CTA r of
+    // the cluster sums slice r of the tile over the cluster's CTAs in order.
+    // With more than one cluster a tile the slice sums go to W, counted per
+    // (tile, slice), and the last CTA to arrive for a slice adds the clusters'
+    // sums in order and clears the count for the next launch.  No CTA waits
+    // for one of another cluster.
+    constexpr int E = MT * NT * 256, ES = E / SCL;
+    cg::cluster_group cl = cg::this_cluster();
+    const int r = (int)cl.block_rank(), nz = gridDim.z / SCL, zc = blockIdx.z / SCL;
     const int tile = blockIdx.y * gridDim.x + blockIdx.x;
-    const long zs = (long)gridDim.x * gridDim.y * MT * NT * 256;
-    float *Wt = W + (long)tile * MT * NT * 256 + tid;
+    __syncthreads();   // the last k-block is consumed
 #pragma unroll
     for (int i = 0; i < MT; ++i)
 #pragma unroll
-      for (int j = 0; j < NT; ++j) Wt[blockIdx.z * zs + (i * NT + j) * 256] = acc[i][j];
-    __threadfence();
-    __syncthreads();
-    __shared__ int last;
-    if (tid == 0) last = atomicAdd(cnt + tile, 1) == (int)gridDim.z - 1;
-    __syncthreads();
-    if (!last) return;
-    __threadfence();
+      for (int j = 0; j < NT; ++j) ssm[(i * NT + j) * 256 + tid] = acc[i][j];
+    cl.sync();
+    float s[(ES + 255) / 256];
 #pragma unroll
-    for (int i = 0; i < MT; ++i)
+    for (int u = 0; u < (ES + 255) / 256; ++u) {
+      const int e = tid + 256 * u;
+      s[u] = 0.f;
+      if (e < ES) {
+        float v[SCL];
 #pragma unroll
-      for (int j = 0; j < NT; ++j) acc[i][j] = 0.f;
-#pragma unroll 4
-    for (int z = 0; z < (int)gridDim.z; ++z)   // unrolled: four partials' loads in flight
+        for (int q = 0; q < SCL; ++q) v[q] = cl.map_shared_rank(ssm, q)[r * ES + e];
 #pragma unroll
-      for (int i = 0; i < MT; ++i)
+        for (int q = 0; q < SCL; ++q) s[u] += v[q];
+      }
+    }
+    cl.sync();         // no CTA leaves while another still reads its tile
+    if (nz > 1) {
+      const long zs = (long)gridDim.x * gridDim.y * E;
+      float *Wt = W + (long)tile * E + r * ES;
 #pragma unroll
-        for (int j = 0; j < NT; ++j) acc[i][j] += __ldcg(Wt + z * zs + (i * NT + j) * 256);
-    if (tid == 0) cnt[tile] = 0;
-  }
+      for (int u = 0; u < (ES + 255) / 256; ++u)
+        if (tid + 256 * u < ES) Wt[zc * zs + tid + 256 * u] = s[u];
+      __threadfence();
+      __syncthreads();
+      __shared__ int last;
+      if (tid == 0) last = atomicAdd(cnt + tile * SCL + r, 1) == nz - 1;
+      __syncthreads();
+      if (!last) return;
+      __threadfence();
 #pragma unroll
-  for (int i = 0; i < MT; ++i) {
-    const int gm = m0 + ty + 16 * i;
-    if (gm >= M) continue;
-#pragma unroll
-    for (int j = 0; j < NT; ++j) {
-      const int gn = n0 + tx + 16 * j;
-      if (gn >= Nact) continue;
-      const long cn = colmap ? colmap[gn] : gn;
-      float v = acc[i][j];
-      if (gamma) {
-        const float a0 = TA ? A[(long)gm * lda] : A[gm];
-        const float b0 = TB ? B[cn] : B[cn * ldb];
-        v = 2.f * v - a0 * b0;
-        if (gamma == 2) {
-          const float a1 = TA ? A[(long)gm * lda + 1] : A[lda + gm];
-          const float b1 = TB ? B[ldb + cn] : B[cn * ldb + 1];
-          v -= 2.f * a1 * b1;
+      for (int u = 0; u < (ES + 255) / 256; ++u) {
+        const int e = tid + 256 * u;
+        s[u] = 0.f;
+        if (e < ES) {
+#pragma unroll 8
+          for (int z = 0; z < nz; ++z) s[u] += __ldcg(Wt + z * zs + e);
         }
       }
-      float *c = Cm + cn * ldc + gm;
-      v = (beta == 0.f) ? alpha * v : alpha * v + beta * *c;
-      *c = rowscale ? v * rowscale[gm] : v;
+      if (tid == 0) cnt[tile * SCL + r] = 0;
     }
+#pragma unroll
+    for (int u = 0; u < (ES + 255) / 256; ++u) {
+      const int e = r * ES + tid + 256 * u, ij = e >> 8, t = e & 255;
+      if (tid + 256 * u < ES) put(m0 + (t >> 4) + 16 * (ij / NT), n0 + (t & 15) + 16 * (ij % NT), s[u]);
+    }
+  } else {
+#pragma unroll
+    for (int i = 0; i < MT; ++i)
+#pragma unroll
+      for (int j = 0; j < NT; ++j) put(m0 + ty + 16 * i, n0 + tx + 16 * j, acc[i][j]);
   }
 }
 
@@ -692,33 +722,48 @@ static void sgemm_go(dim3 g, int M, int N, int K, float alpha, const float *A, l
                      const float *rowscale, int kchunk, float *W, int *cnt, cudaStream_t st) {
   constexpr size_t sm = sgemm_smem<MT, NT>();
   static_assert(sm <= 48 * 1024, "stages fit the default shared-memory limit");
-  k_sgemm<TA, TB, SPLIT, MT, NT><<<g, 256, sm, st>>>(M, N, K, alpha, A, lda, B, ldb, beta, C, ldc, gamma, colmap,
-                                                     ncol_dev, rowscale, kchunk, W, cnt);
+  static_assert(sm >= sizeof(float) * 256 * MT * NT, "a partial tile fits the stages");
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = g;
+  cfg.blockDim = dim3(256);
+  cfg.dynamicSmemBytes = sm;
+  cfg.stream = st;
+  cudaLaunchAttribute at = {};
+  at.id = cudaLaunchAttributeClusterDimension;
+  at.val.clusterDim.x = 1;
+  at.val.clusterDim.y = 1;
+  at.val.clusterDim.z = SCL;
+  cfg.attrs = &at;
+  cfg.numAttrs = SPLIT ? 1 : 0;
+  cudaLaunchKernelEx(&cfg, k_sgemm<TA, TB, SPLIT, MT, NT>, M, N, K, alpha, A, lda, B, ldb, beta, C, ldc, gamma, colmap,
+                     ncol_dev, rowscale, kchunk, W, cnt);
   note_launch();
 }
 
 // One shape's launch: tile rows MT x NT from the extents (k-contiguous A:
-// both from the band-sized extents; otherwise 64-row tiles down M), and K
-// split to shorten the chain of one CTA: a k-block of 16 costs about 0.5 us
-// and a partial tile summed by the last CTA about 0.1 us (cnt: one zeroed
-// counter per tile), so K / (32 z) + z / 10 us is least at z = sqrt(K / 3),
-// as far as two CTAs a SM hold the splits.  At Si8 (32 x 16 x 738) the one
-// CTA of the unsplit call ran 24.8 us.
+// both from the band-sized extents; otherwise 64-row tiles down M, or 48- or
+// 32-row ones where 64 leave SMs without a tile (M 4810: 16.2 -> 13.8 us)), and K split to shorten the
+// chain of one CTA: a k-block of 16 costs 0.5 to 1 us, so chunks of about four
+// k-blocks, in whole clusters, as far as two CTAs a SM hold them (cnt: one
+// zeroed counter per tile and slice).  At 65 bands (K 4810) splits summed by
+// the last CTA of a tile cost 30 to 45 us, most of it that CTA's reads;
+// in clusters 19 to 20 us.
 template <bool TA, bool TB>
 static void sgemm_launch(int M, int N, int K, float alpha, const float *A, long lda, const float *B, long ldb,
                          float beta, float *C, long ldc, int gamma, const int *colmap, const int *ncol_dev,
                          const float *rowscale, void *ws, size_t ws_bytes, int *cnt, cudaStream_t st) {
-  const int mt = TA ? sgemm_rows(M) : 4, nt = sgemm_rows(N);
-  dim3 g((M + 16 * mt - 1) / (16 * mt), (N + 16 * nt - 1) / (16 * nt));
+  const int nt = sgemm_rows(N), tn = (N + 16 * nt - 1) / (16 * nt);
+  int mt = TA ? sgemm_rows(M) : 4;
+  if (!TA)
+    while (mt > 2 && (long)((M + 16 * mt - 1) / (16 * mt)) * tn < 148) --mt;
+  dim3 g((M + 16 * mt - 1) / (16 * mt), tn);
   const long tiles = (long)g.x * g.y;
-  const size_t part = sizeof(float) * (size_t)tiles * 256 * mt * nt;   // one split's partial tiles
+  const size_t part = sizeof(float) * (size_t)tiles * 256 * mt * nt;   // one cluster's partial tiles
   int nsplit = 1, kchunk = K;
-  if (ws && cnt && tiles <= GEMM_TILE_COUNTERS && tiles < 2 * 148 && K >= 256) {
-    nsplit = (int)std::min<long>((2 * 148 + tiles - 1) / tiles, (long)std::sqrt(K / 3.0));
-    nsplit = (int)std::min<size_t>(nsplit, ws_bytes / part);
-    if (nsplit < 2) nsplit = 1;
+  if (ws && cnt && tiles * SCL <= GEMM_TILE_COUNTERS && tiles < 2 * 148 / SCL && K >= (TA ? 256 : 1024)) {
+    const long cl = std::min<long>((2 * 148 / SCL + tiles - 1) / tiles, std::max(1, K / (64 * SCL)));
+    nsplit = SCL * (int)std::max<long>(1, std::min<long>(cl, (long)(ws_bytes / part)));
     kchunk = ((K + nsplit - 1) / nsplit + SBK - 1) / SBK * SBK;
-    nsplit = (K + kchunk - 1) / kchunk;
   }
   if (nsplit <= 1) kchunk = K;
   g.z = nsplit;
@@ -737,7 +782,9 @@ static void sgemm_launch(int M, int N, int K, float alpha, const float *A, long 
     else QX_SG(4, 2) else QX_SG(4, 3) else QX_SG(4, 4) else QX_SG(4, 5)
     else QX_SG(5, 2) else QX_SG(5, 3) else QX_SG(5, 4) else QX_SG(5, 5)
   } else {
-    QX_SG(4, 2) else QX_SG(4, 3) else QX_SG(4, 4) else QX_SG(4, 5)
+    QX_SG(2, 2) else QX_SG(2, 3) else QX_SG(2, 4) else QX_SG(2, 5)
+    else QX_SG(3, 2) else QX_SG(3, 3) else QX_SG(3, 4) else QX_SG(3, 5)
+    else QX_SG(4, 2) else QX_SG(4, 3) else QX_SG(4, 4) else QX_SG(4, 5)
   }
 #undef QX_SG
 }
