@@ -671,10 +671,12 @@ int tc_gemm(bool ta, bool tb, int M, int N, int K, float alpha, const float *A, 
   const int tm = (M + BM - 1) / BM, nkb = (K + BK - 1) / BK;
   CUtensorMap ma, mb;
   const bool atm = tc::atmem_enabled();
-  // tile width: 80 for K-major B, 96 (three 32-column chunks) for MN-major
-  // B, unless the autotuner measured another for this shape (A in tensor
-  // memory only)
-  int bn = b_mn ? 96 : 80;
+  // tile width: 80 for K-major B (128 where 80 takes more than one tile a SM:
+  // its epilogue spills, but fewer tiles read A and fill fewer waves; Si512
+  // H|psi>, 1100 bands: 11.83 -> 11.37 ms, 64 wide 12.32), 96 (three 32-column
+  // chunks) for MN-major B, unless the autotuner measured another for this
+  // shape (A in tensor memory only)
+  int bn = b_mn ? 96 : (atm && (long)tm * ((N + 79) / 80) > 148 ? 128 : 80);
   {
     // QX_TC_TILE forces a width for every shape where it is valid (tests)
     const char *env = getenv("QX_TC_TILE");
