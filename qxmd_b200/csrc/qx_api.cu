@@ -512,12 +512,12 @@ extern "C" int qx_create(qx_ctx **out, int precision, int k1, int k2, int k3, in
   pl.ncol = (int)col_ja.size();
   std::vector<int> col_ig((size_t)k3 * std::max(1, pl.ncol), 0);
   for (auto &e : ents) col_ig[(size_t)e.i3 * pl.ncol + colq[(size_t)e.j2 * pl.P1 + e.a]] = e.sgn > 0 ? e.ig + 1 : -(e.ig + 1);
-  std::vector<uint2> col_mask(pl.P1, make_uint2(0u, 0u));
+  std::vector<ulonglong2> col_mask(pl.P1, make_ulonglong2(0ull, 0ull));
   for (int j = 0; j < pl.P2; ++j)
     for (int a = lo[j]; a <= hi[j]; ++a) {
       const int k = j - m2;
-      if (k >= 0 && k < 32) col_mask[a].x |= 1u << k;
-      if (k <= 0 && k > -32) col_mask[a].y |= 1u << -k;
+      if (k >= 0 && k < 64) col_mask[a].x |= 1ull << k;
+      if (k <= 0 && k > -64) col_mask[a].y |= 1ull << -k;
     }
   int rc = 0;
 #define FAIL(x) do { rc = (x); if (rc) { qx_destroy(c); return rc; } } while (0)
@@ -527,8 +527,8 @@ extern "C" int qx_create(qx_ctx **out, int precision, int k1, int k2, int k3, in
   FAIL(dalloc(c, &pl.d_row_ent, sizeof(int4) * rent.size()));
   FAIL(dalloc(c, &pl.d_col_ja, sizeof(int) * std::max<size_t>(1, col_ja.size())));
   FAIL(dalloc(c, &pl.d_col_ig, sizeof(int) * col_ig.size()));
-  FAIL(dalloc(c, &pl.d_col_mask, sizeof(uint2) * col_mask.size()));
-  if (cudaMemcpy(pl.d_col_mask, col_mask.data(), sizeof(uint2) * col_mask.size(), cudaMemcpyHostToDevice) ||
+  FAIL(dalloc(c, &pl.d_col_mask, sizeof(ulonglong2) * col_mask.size()));
+  if (cudaMemcpy(pl.d_col_mask, col_mask.data(), sizeof(ulonglong2) * col_mask.size(), cudaMemcpyHostToDevice) ||
       cudaMemcpy(pl.d_row_lo, lo.data(), sizeof(int) * pl.P2, cudaMemcpyHostToDevice) ||
       cudaMemcpy(pl.d_row_hi, hi.data(), sizeof(int) * pl.P2, cudaMemcpyHostToDevice) ||
       cudaMemcpy(pl.d_row_off, cnt.data(), sizeof(int) * (pl.P2 + 1), cudaMemcpyHostToDevice) ||

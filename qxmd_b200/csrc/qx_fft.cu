@@ -812,12 +812,13 @@ static bool plane_enabled() {
 // Forward z pass one sphere column a thread (k_zcols_fwd) for columns of at
 // most 32 points, where it measured faster than the shared-memory pass (the
 // 48-cell batch, z lengths 21-27: 9365 -> 9735 cell-iter/s); at 54 points
-// (Si64) it measured 2.5 % slower.  QX_ZCOLS_FWD=0 / 1 forces either (read at
+// (Si64) it measured 2.5 % slower.  At 96 (Si512) k_zcols_fwd2 takes 820 us
+// where the shared-memory pass took 960.  QX_ZCOLS_FWD=0 / 1 forces either (read at
 // every call).
 static bool zcols_fwd_enabled(int k3) {
   const char *e = getenv("QX_ZCOLS_FWD");
   if (e && (e[0] == '0' || e[0] == '1')) return e[0] == '1';
-  return k3 <= 32;
+  return k3 <= 32 || k3 == 96;
 }
 
 // The sums of the chunk's pairs over every atom's points.  Where that fills

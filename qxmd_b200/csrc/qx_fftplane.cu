@@ -25,7 +25,7 @@ static int zcols_dispatch(const PipeParams &P, int npl, const float *cin, long l
   case N: return zcols_launch<N>(P, npl, cin, ldc, bufA, src, zsph, inv, st);
     QX_ZCOLS_LENGTHS(QX_CASE)
 #undef QX_CASE
-    case 96: return zcols2_launch<96>(P, npl, cin, ldc, bufA, inv, st);
+    case 96: return zcols2_launch<96>(P, npl, cin, ldc, bufA, src, zsph, inv, st);
     default: return -1;
   }
 }

@@ -31,8 +31,8 @@ template <int N>
 int rho2_launch(const PipeParams &P, int npl, const float2 *bufA, const double *wocc, double *part, double *rho,
                 int accumulate, cudaStream_t st);
 template <int N>
-int zcols2_launch(const PipeParams &P, int npl, const float *cin, long ldc, float2 *bufA, bool inv,
-                  cudaStream_t st);
+int zcols2_launch(const PipeParams &P, int npl, const float *cin, long ldc, float2 *bufA, const float2 *src,
+                  float2 *zsph, bool inv, cudaStream_t st);
 
 // The k1 x k2 plane shapes with register kernels, X(k1, k2): the square
 // grids of 20 to 64 points built from radices 2, 3, 5 and 7, and the
@@ -57,6 +57,24 @@ template <int NX, int NY>
 int plane64_launch(const PipeParams &P, int npl, double2 *bufA, const double *vloc, cudaStream_t st);
 
 constexpr int plane_grid_key(int k1, int k2) { return k1 * 1024 + k2; }
+
+// The line of N points whose samples MB < i < N - MB are zero: MB = (N - 1) / 4
+// wherever the density cutoff is at least four times the wavefunction's
+// (then the wavefunction sphere spans half the grid), (N - 1) / 2 otherwise.
+template <int N, bool HALF> constexpr int line_mb() { return HALF ? (N - 1) / 4 : (N - 1) / 2; }
+
+// Which samples i = 2 j + h of a two-lane line may be nonzero when those at
+// MB < i < N - MB are zero: nothing for either lane, one lane, or both, at
+// the start (sample i) or the end (sample i - N) of the line.
+enum { Z2_NONE, Z2_POS, Z2_POS0, Z2_NEG, Z2_NEG1 };
+template <int N, int MB> constexpr int z2_kind(int j) {
+  return 2 * j + 1 <= MB ? Z2_POS : 2 * j <= MB ? Z2_POS0 : 2 * j >= N - MB ? Z2_NEG : 2 * j + 1 >= N - MB ? Z2_NEG1 : Z2_NONE;
+}
+// the bound of rf::fft_nz on a lane's N / 2 samples
+template <int N, int MB> constexpr int z2_bound() {
+  const int lo = MB / 2, hi = N / 2 - (N - MB) / 2;
+  return lo > hi ? lo : hi;
+}
 
 // QX_PLANE_PAIRS=0 keeps one z plane a CTA (read at every call).
 bool plane_pairs_enabled();

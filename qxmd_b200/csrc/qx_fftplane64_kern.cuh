@@ -10,7 +10,9 @@
 // two passes per stage through shared memory and the round trips of bufB bound
 // them.  Whole pipeline, 160 / 16 / 2 bands: 24^3 81 / 37 / 35 -> 42 / 27 / 27
 // us, 40^3 192 / 49 / 38 -> 124 / 37 / 33, 54^3 392 / 63 / 45 -> 342 / 52 / 45,
-// 60^3 598 / 90 / 51 -> 440 / 77 / 49.  At 54 points registers allow three
+// 60^3 598 / 90 / 51 -> 440 / 77 / 49 with whole lines; leaving out what a
+// sphere of half the grid has zero (HALF) took H|psi> of Si64 (54^3, 160 bands,
+// both projector contractions included) from 410 to 292 us.  At 54 points registers allow three
 // CTAs of 128 threads a SM; the FP64 chains and instruction fetches bound it.
 // The z passes in the same form measured slower than the stage kernels (54^3,
 // 16 bands: 63 -> 69 us) and were left out.
@@ -40,9 +42,10 @@ template <int N>
 struct Line {
   static constexpr int L = lanes(N), M = N / L;
   // x[j] = sample L j + h in; sample k + h M at x[out_pos(M, k)] out
-  template <int SIGN>
+  // (ZM: rf::fft_nz's bound on the lane's samples, (M - 1) / 2 for none zero)
+  template <int SIGN, int ZM = M / 2>
   static __device__ __forceinline__ void dit(double2 (&x)[M], int h) {
-    rf::fft<double, SIGN, M>(x);
+    rf::fft_nz<double, SIGN, M, ZM>(x);
     if constexpr (L == 2) {
       rf::static_for<0, M>([&](auto kc) {
         constexpr int k = decltype(kc)::value, pk = rf::out_pos(M, k);
@@ -72,46 +75,60 @@ struct Line {
 
 constexpr int plane_ld(int p1) { return p1 + (6 - p1 % 4) % 4; }
 
+// z2_kind and z2_bound for a line over one or two lanes
+template <int N, int MB> constexpr int kind(int j) {
+  return lanes(N) == 2 ? z2_kind<N, MB>(j) : (j <= MB ? Z2_POS : j >= N - MB ? Z2_NEG : Z2_NONE);
+}
+template <int N, int MB> constexpr int bound() {
+  return lanes(N) == 2 ? z2_bound<N, MB>() : (2 * MB + 1 < N ? MB : N / 2);
+}
+
 }  // namespace pl64
 
 // One band pair's z plane a CTA; whole warps run each phase (lanes without a
 // line work on zeros and store nothing), so every shuffle has its full mask.
-template <int NX, int NY>
+// HALF, the tile's columns and the sphere's rows as in k_plane.
+template <int NX, int NY, bool HALF>
 __global__ void __launch_bounds__(pl64::plane_threads(NX, NY), pl64::plane_ctas(NX, NY))
     k_plane64(PipeParams P, double2 *__restrict__ bufA, const double *__restrict__ vloc) {
   using rf::out_pos;
   using X = pl64::Line<NX>;
   using Y = pl64::Line<NY>;
-  constexpr int NT = pl64::plane_threads(NX, NY);
+  constexpr int NT = pl64::plane_threads(NX, NY), MBX = line_mb<NX, HALF>(), MBY = line_mb<NY, HALF>();
+  constexpr int PC = 2 * MBX + 1, LD = pl64::plane_ld(PC);
   const int i3 = blockIdx.x;
   const int pl = blockIdx.y, p = P.pair0 + pl;
   if (p >= (P.npair_dev ? *P.npair_dev : P.npair)) return;
-  const int P1 = P.P1, P2 = P.P2, m1 = P.m1, m2 = P.m2, LD = pl64::plane_ld(P1);
+  const int P1 = P.P1, m1 = P.m1;
   extern __shared__ double2 T64[];   // [NY][LD]
   double2 *T = T64;
-  double2 *A = bufA + ((long)pl * P.k3 + i3) * P2 * P1;
+  double2 *A = bufA + ((long)pl * P.k3 + i3) * P.P2 * P1 + P.m2 * P1;   // row m2
   const int t = threadIdx.x;
   const double2 zero = make_double2(0.0, 0.0);
 
-  // (1) y backward, line = sphere column a
-  for (int a0 = 0; a0 < P1; a0 += NT / Y::L) {
-    const int a = a0 + t / Y::L, h = t % Y::L;
-    if (a0 + (t & ~31) / Y::L >= P1) continue;   // uniform in the warp
-    const bool on = a < P1;
+  // (1) y backward, line = tile column c (sphere column c - (MBX - m1))
+  for (int c0 = 0; c0 < PC; c0 += NT / Y::L) {
+    const int c = c0 + t / Y::L, h = t % Y::L, a = c - (MBX - m1);
+    if (c0 + (t & ~31) / Y::L >= PC) continue;   // uniform in the warp
+    const bool in = c < PC && a >= 0 && a < P1;
+    const ulonglong2 m = in ? P.col_mask[a] : make_ulonglong2(0ull, 0ull);
+    const unsigned px = (unsigned)m.x >> h, nx = (unsigned)m.y << h;   // bit L j: row L j + h; bit NY - L j: row -(NY - L j - h)
     double2 x[Y::M];
-#pragma unroll
-    for (int j = 0; j < Y::M; ++j) {
-      const int i2 = Y::L * j + h;
-      const int j2 = (i2 <= m2) ? i2 + m2 : ((i2 >= NY - m2) ? i2 - NY + m2 : -1);
+    rf::static_for<0, Y::M>([&](auto jc) {
+      constexpr int j = decltype(jc)::value, kind = pl64::kind<NY, MBY>(j);
       double2 v = zero;
-      if (on && j2 >= 0 && a >= P.row_lo[j2] && a <= P.row_hi[j2]) v = A[j2 * P1 + a];
+      if constexpr (kind == Z2_POS || kind == Z2_POS0) {
+        if ((px >> (Y::L * j)) & 1u) v = A[(Y::L * j + h) * P1 + a];
+      } else if constexpr (kind == Z2_NEG || kind == Z2_NEG1) {
+        if ((nx >> (NY - Y::L * j)) & 1u) v = A[-(NY - Y::L * j - h) * P1 + a];
+      }
       x[j] = v;
-    }
-    Y::template dit<+1>(x, h);
-    if (on) {
+    });
+    Y::template dit<+1, pl64::bound<NY, MBY>()>(x, h);
+    if (c < PC) {
       rf::static_for<0, Y::M>([&](auto kc) {
         constexpr int k = decltype(kc)::value;
-        T[(k + h * Y::M) * LD + a] = x[out_pos(Y::M, k)];
+        T[(k + h * Y::M) * LD + c] = x[out_pos(Y::M, k)];
       });
     }
   }
@@ -120,17 +137,18 @@ __global__ void __launch_bounds__(pl64::plane_threads(NX, NY), pl64::plane_ctas(
   if ((t & ~31) / X::L < NY) {
     const int r = t / X::L, h = t % X::L;
     const bool on = r < NY;
-    double2 *row = T + (on ? r : NY - 1) * LD;
+    double2 *row = T + (on ? r : NY - 1) * LD + MBX;   // sample k at row[k]
     double2 x[X::M], u[X::M];
-#pragma unroll
-    for (int j = 0; j < X::M; ++j) {
-      const int i1 = X::L * j + h;
+    rf::static_for<0, X::M>([&](auto jc) {
+      constexpr int j = decltype(jc)::value, kind = pl64::kind<NX, MBX>(j);
       double2 v = zero;
-      if (i1 <= m1) v = row[i1 + m1];
-      else if (i1 >= NX - m1) v = row[i1 - NX + m1];
+      if constexpr (kind == Z2_POS) v = row[X::L * j + h];
+      else if constexpr (kind == Z2_POS0) v = h ? zero : row[2 * j];
+      else if constexpr (kind == Z2_NEG) v = row[X::L * j - NX + h];
+      else if constexpr (kind == Z2_NEG1) v = h ? row[2 * j + 1 - NX] : zero;
       x[j] = v;
-    }
-    X::template dit<+1>(x, h);
+    });
+    X::template dit<+1, pl64::bound<NX, MBX>()>(x, h);
     const double *V = vloc + ((long)i3 * NY + (on ? r : NY - 1)) * NX + h * X::M;
     rf::static_for<0, X::M>([&](auto kc) {
       constexpr int k = decltype(kc)::value, pk = out_pos(X::M, k);
@@ -141,44 +159,63 @@ __global__ void __launch_bounds__(pl64::plane_threads(NX, NY), pl64::plane_ctas(
     __syncwarp();   // a row's lanes, in one warp, have read it before either rewrites it
     if (on) {
       rf::static_for<0, X::M>([&](auto jc) {
-        constexpr int j = decltype(jc)::value;
-        const int i1 = X::L * j + h;
-        if (i1 <= m1) row[i1 + m1] = u[out_pos(X::M, j)];
-        else if (i1 >= NX - m1) row[i1 - NX + m1] = u[out_pos(X::M, j)];
+        constexpr int j = decltype(jc)::value, kind = pl64::kind<NX, MBX>(j), q = out_pos(X::M, j);
+        if constexpr (kind == Z2_POS) row[X::L * j + h] = u[q];
+        else if constexpr (kind == Z2_POS0) { if (!h) row[2 * j] = u[q]; }
+        else if constexpr (kind == Z2_NEG) row[X::L * j - NX + h] = u[q];
+        else if constexpr (kind == Z2_NEG1) { if (h) row[2 * j + 1 - NX] = u[q]; }
       });
     }
   }
   __syncthreads();
-  // (3) y forward, line = sphere column a; only rows inside the sphere are kept
-  for (int a0 = 0; a0 < P1; a0 += NT / Y::L) {
-    const int a = a0 + t / Y::L, h = t % Y::L;
-    if (a0 + (t & ~31) / Y::L >= P1) continue;
-    const bool on = a < P1;
+  // (3) y forward, line = tile column c; only rows inside the sphere are kept
+  for (int c0 = 0; c0 < PC; c0 += NT / Y::L) {
+    const int c = c0 + t / Y::L, h = t % Y::L, a = c - (MBX - m1);
+    if (c0 + (t & ~31) / Y::L >= PC) continue;
+    const bool in = c < PC && a >= 0 && a < P1;
+    const ulonglong2 m = in ? P.col_mask[a] : make_ulonglong2(0ull, 0ull);
+    const unsigned inx = (unsigned)m.x, iny = (unsigned)m.y;
     double2 x[Y::M];
 #pragma unroll
-    for (int j = 0; j < Y::M; ++j) x[j] = on ? T[(Y::L * j + h) * LD + a] : zero;
+    for (int j = 0; j < Y::M; ++j) x[j] = c < PC ? T[(Y::L * j + h) * LD + c] : zero;
     Y::template dit<-1>(x, h);
-    if (on) {
+    if constexpr (Y::L == 2) {
+      // lane 0 holds rows k < M, lane 1 rows k - M
       rf::static_for<0, Y::M>([&](auto kc) {
+        constexpr int k = decltype(kc)::value, kn = Y::M - k;
+        if constexpr (k <= MBY || kn <= MBY) {
+          const bool keep = h ? (kn <= MBY && ((iny >> (kn < 32 ? kn : 0)) & 1u)) : (k <= MBY && ((inx >> k) & 1u));
+          if (keep) A[(k - h * Y::M) * P1 + a] = x[out_pos(Y::M, k)];
+        }
+      });
+    } else {
+      rf::static_for<0, MBY + 1>([&](auto kc) {
         constexpr int k = decltype(kc)::value;
-        const int i2 = k + h * Y::M;
-        const int j2 = (i2 <= m2) ? i2 + m2 : ((i2 >= NY - m2) ? i2 - NY + m2 : -1);
-        if (j2 >= 0 && a >= P.row_lo[j2] && a <= P.row_hi[j2]) A[j2 * P1 + a] = x[out_pos(Y::M, k)];
+        if ((inx >> k) & 1u) A[k * P1 + a] = x[out_pos(NY, k)];
+        if constexpr (k > 0)
+          if ((iny >> k) & 1u) A[-k * P1 + a] = x[out_pos(NY, NY - k)];
       });
     }
   }
 }
 
-template <int NX, int NY>
-int plane64_launch(const PipeParams &P, int npl, double2 *bufA, const double *vloc, cudaStream_t st) {
-  const size_t sm = sizeof(double2) * (size_t)NY * pl64::plane_ld(P.P1);
+template <int NX, int NY, bool HALF>
+static void plane64_go(const PipeParams &P, int npl, double2 *bufA, const double *vloc, cudaStream_t st) {
+  constexpr size_t sm = sizeof(double2) * (size_t)NY * pl64::plane_ld(2 * line_mb<NX, HALF>() + 1);
   static bool attr = false;
   if (!attr) {
-    cudaFuncSetAttribute(k_plane64<NX, NY>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                         (int)(sizeof(double2) * NY * pl64::plane_ld(NX)));
+    cudaFuncSetAttribute(k_plane64<NX, NY, HALF>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
     attr = true;
   }
-  k_plane64<NX, NY><<<dim3(P.k3, npl), pl64::plane_threads(NX, NY), sm, st>>>(P, bufA, vloc);
+  k_plane64<NX, NY, HALF><<<dim3(P.k3, npl), pl64::plane_threads(NX, NY), sm, st>>>(P, bufA, vloc);
+}
+
+// Spheres beyond half the grid (a density cutoff below four times the
+// wavefunction's) take the stage kernels.
+template <int NX, int NY>
+int plane64_launch(const PipeParams &P, int npl, double2 *bufA, const double *vloc, cudaStream_t st) {
+  if (P.m1 > line_mb<NX, true>() || P.m2 > line_mb<NY, true>()) return -1;
+  plane64_go<NX, NY, true>(P, npl, bufA, vloc, st);
   note_launch();
   return 0;
 }

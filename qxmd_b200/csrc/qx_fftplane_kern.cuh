@@ -36,16 +36,17 @@ struct PlaneRows {
   __device__ static int row(int t) { return both ? (t & 31) : t; }
 };
 
-// The line of N points whose samples MB < i < N - MB are zero: MB = (N - 1) / 4
-// wherever the density cutoff is at least four times the wavefunction's
-// (then the wavefunction sphere spans half the grid), (N - 1) / 2 otherwise.
-template <int N, bool HALF> constexpr int line_mb() { return HALF ? (N - 1) / 4 : (N - 1) / 2; }
+// the rows of sphere column a as P.col_mask, at most 32 either way
+__device__ __forceinline__ uint2 col_rows(const PipeParams &P, int a) {
+  const ulonglong2 m = P.col_mask[a];
+  return make_uint2((unsigned)m.x, (unsigned)m.y);
+}
 
 // Backward y transform of sphere column a of a plane (A: its [P2][P1] rows)
 // into column c of a tile with `ld` columns.
 template <int NY, int MB>
 __device__ __forceinline__ void plane_y_back(const PipeParams &P, const float2 *A, int a, float2 *Tc, int ld) {
-  const uint2 in = P.col_mask[a];
+  const uint2 in = col_rows(P, a);
   const int P1 = P.P1;
   const float2 *A0 = A + P.m2 * P1 + a;
   const float2 zero = make_float2(0.f, 0.f);
@@ -162,7 +163,7 @@ __global__ void __launch_bounds__(64 * U, (plane_minb(NX > NY ? NX : NY) + U - 1
   __syncthreads();
   // (3) y forward, thread = column of its plane; only rows inside the sphere are kept
   if (col_on && in_sphere) {
-    const uint2 in = P.col_mask[a];
+    const uint2 in = col_rows(P, a);
     float2 x[NY];
 #pragma unroll
     for (int i2 = 0; i2 < NY; ++i2) x[i2] = Tc[i2 * PB];
@@ -222,7 +223,11 @@ __device__ __forceinline__ void dif_split(const float2 (&v)[N / 2], float2 (&u)[
 }
 }  // namespace pl2
 
-template <int N>
+// The tile holds the sphere's columns only: at Si512 (96^3, 1100 bands) the pass
+// took 5950 us with whole lines, 2920 us with HALF (and 2 MB + 1 = 47 columns).
+template <int N, bool HALF> constexpr int plane2_pitch() { return (2 * line_mb<N, HALF>() + 1 + 14) / 16 * 16 + 2; }
+
+template <int N, bool HALF>
 __global__ void __launch_bounds__(2 * N) k_plane2(PipeParams P, float2 *__restrict__ bufA,
                                                  const float *__restrict__ vloc) {
   using rf::out_pos;
@@ -230,31 +235,43 @@ __global__ void __launch_bounds__(2 * N) k_plane2(PipeParams P, float2 *__restri
   const int i3 = blockIdx.x;
   const int pl = blockIdx.y, p = P.pair0 + pl;
   if (p >= (P.npair_dev ? *P.npair_dev : P.npair)) return;
-  const int P1 = P.P1, P2 = P.P2, m1 = P.m1, m2 = P.m2;
-  extern __shared__ float2 T[];   // [N][P1]
-  float2 *A = bufA + ((long)pl * P.k3 + i3) * P2 * P1;
+  // tile columns: sample k of x at column MB + k (zero beyond the sphere); the
+  // pitch PB = 2 modulo 16 puts the eight lines of a half warp, two adjacent
+  // samples each, in different banks
+  constexpr int MB = line_mb<N, HALF>(), PC = 2 * MB + 1, PB = plane2_pitch<N, HALF>();
+  const int P1 = P.P1, m1 = P.m1;
+  extern __shared__ float2 T[];   // [N][PB]
+  float2 *A = bufA + ((long)pl * P.k3 + i3) * P.P2 * P1;
   const int t = threadIdx.x, l = t >> 1, h = t & 1;
-  const bool warp_on_cols = (t & ~31) < 2 * P1;   // some lane of this warp owns a column
+  const bool warp_on_cols = (t & ~31) < 2 * PC;   // some lane of this warp owns a column
   const float2 zero = make_float2(0.f, 0.f);
+  const int a = l - (MB - m1);                    // sphere column of tile column l
+  const bool in_sphere = l < PC && a >= 0 && a < P1;
+  typedef typename std::conditional<(MB < 31), unsigned, unsigned long long>::type Mask;
+  const ulonglong2 in2 = in_sphere ? P.col_mask[a] : make_ulonglong2(0ull, 0ull);
+  const Mask inx = (Mask)in2.x, iny = (Mask)in2.y;
+  float2 *A0 = A + P.m2 * P1 + a;
 
-  // (1) y backward, line = sphere column a = l
+  // (1) y backward, line = tile column l
   if (warp_on_cols) {
-    const bool on = l < P1;
+    const Mask px = inx >> h, nx = iny << h;   // bit 2j: row 2j + h; bit N - 2j: row -(N - 2j - h)
     float2 x[H];
-#pragma unroll
-    for (int j = 0; j < H; ++j) {
-      const int i2 = 2 * j + h;
-      const int j2 = (i2 <= m2) ? i2 + m2 : ((i2 >= N - m2) ? i2 - N + m2 : -1);
+    rf::static_for<0, H>([&](auto jc) {
+      constexpr int j = decltype(jc)::value, kind = z2_kind<N, MB>(j);
       float2 v = zero;
-      if (on && j2 >= 0 && l >= P.row_lo[j2] && l <= P.row_hi[j2]) v = A[j2 * P1 + l];
+      if constexpr (kind == Z2_POS || kind == Z2_POS0) {
+        if ((px >> (2 * j)) & 1) v = A0[(2 * j + h) * P1];
+      } else if constexpr (kind == Z2_NEG || kind == Z2_NEG1) {
+        if ((nx >> (N - 2 * j)) & 1) v = A0[-(N - 2 * j - h) * P1];
+      }
       x[j] = v;
-    }
-    rf::fft<float, +1, H>(x);
+    });
+    rf::fft_nz<float, +1, H, z2_bound<N, MB>()>(x);
     pl2::dit_combine<+1, N>(x, h);
-    if (on) {
+    if (l < PC) {
       rf::static_for<0, H>([&](auto kc) {
         constexpr int k = decltype(kc)::value;
-        T[(k + h * H) * P1 + l] = x[out_pos(H, k)];
+        T[(k + h * H) * PB + l] = x[out_pos(H, k)];
       });
     }
   }
@@ -262,16 +279,17 @@ __global__ void __launch_bounds__(2 * N) k_plane2(PipeParams P, float2 *__restri
   // (2) x backward, * V, x forward; line = grid row i2 = l (every thread has one)
   {
     float2 x[H];
-    float2 *row = T + l * P1;
-#pragma unroll
-    for (int j = 0; j < H; ++j) {
-      const int i1 = 2 * j + h;
+    float2 *row = T + l * PB + MB;   // sample k at row[k]
+    rf::static_for<0, H>([&](auto jc) {
+      constexpr int j = decltype(jc)::value, kind = z2_kind<N, MB>(j);
       float2 v = zero;
-      if (i1 <= m1) v = row[i1 + m1];
-      else if (i1 >= N - m1) v = row[i1 - N + m1];
+      if constexpr (kind == Z2_POS) v = row[2 * j + h];
+      else if constexpr (kind == Z2_POS0) v = h ? zero : row[2 * j];
+      else if constexpr (kind == Z2_NEG) v = row[2 * j - N + h];
+      else if constexpr (kind == Z2_NEG1) v = h ? row[2 * j + 1 - N] : zero;
       x[j] = v;
-    }
-    rf::fft<float, +1, H>(x);
+    });
+    rf::fft_nz<float, +1, H, z2_bound<N, MB>()>(x);
     pl2::dit_combine<+1, N>(x, h);
     const float *V = vloc + ((long)i3 * N + l) * N + h * H;
     rf::static_for<0, H>([&](auto kc) {
@@ -282,31 +300,32 @@ __global__ void __launch_bounds__(2 * N) k_plane2(PipeParams P, float2 *__restri
     float2 u[H];
     pl2::dif_split<-1, N>(x, u, h);
     rf::fft<float, -1, H>(u);
-    __syncthreads();   // every thread has read its row before any row is rewritten
+    __syncwarp();   // a row's two lanes have read it before either rewrites it
     rf::static_for<0, H>([&](auto jc) {
-      constexpr int j = decltype(jc)::value;
-      const int i1 = 2 * j + h;
-      if (i1 <= m1) row[i1 + m1] = u[out_pos(H, j)];
-      else if (i1 >= N - m1) row[i1 - N + m1] = u[out_pos(H, j)];
+      constexpr int j = decltype(jc)::value, kind = z2_kind<N, MB>(j), q = out_pos(H, j);
+      if constexpr (kind == Z2_POS) row[2 * j + h] = u[q];
+      else if constexpr (kind == Z2_POS0) { if (!h) row[2 * j] = u[q]; }
+      else if constexpr (kind == Z2_NEG) row[2 * j - N + h] = u[q];
+      else if constexpr (kind == Z2_NEG1) { if (h) row[2 * j + 1 - N] = u[q]; }
     });
   }
   __syncthreads();
-  // (3) y forward, line = sphere column a = l; only rows inside the sphere are kept
+  // (3) y forward, line = tile column l; only rows inside the sphere are kept
   if (warp_on_cols) {
-    const bool on = l < P1;
     float2 x[H];
 #pragma unroll
-    for (int j = 0; j < H; ++j) x[j] = on ? T[(2 * j + h) * P1 + l] : zero;
+    for (int j = 0; j < H; ++j) x[j] = l < PC ? T[(2 * j + h) * PB + l] : zero;
     rf::fft<float, -1, H>(x);
     pl2::dit_combine<-1, N>(x, h);
-    if (on) {
-      rf::static_for<0, H>([&](auto kc) {
-        constexpr int k = decltype(kc)::value;
-        const int i2 = k + h * H;
-        const int j2 = (i2 <= m2) ? i2 + m2 : ((i2 >= N - m2) ? i2 - N + m2 : -1);
-        if (j2 >= 0 && l >= P.row_lo[j2] && l <= P.row_hi[j2]) A[j2 * P1 + l] = x[out_pos(H, k)];
-      });
-    }
+    // lane 0 holds rows k < H, lane 1 rows k - H
+    rf::static_for<0, H>([&](auto kc) {
+      constexpr int k = decltype(kc)::value;
+      if constexpr (k <= MB || H - k <= MB) {
+        constexpr int kp = k <= MB ? k : 0, kn = H - k <= MB ? H - k : 0;
+        const bool keep = h ? (H - k <= MB && ((iny >> kn) & 1)) : (k <= MB && ((inx >> kp) & 1));
+        if (keep) A0[(k - h * H) * P1] = x[out_pos(H, k)];
+      }
+    });
   }
 }
 
@@ -469,7 +488,7 @@ __global__ void __launch_bounds__(128, plane_minb(NX > NY ? NX : NY) > 1 ? 4 : 1
   __syncthreads();
   if (on && u < P1) {
     const int k1 = u - P.m1;
-    const uint2 in = P.col_mask[u];
+    const uint2 in = col_rows(P, u);
     const float2 *Tc = Tp + (k1 >= 0 ? k1 : NX + k1);
     float2 *A0 = bufA + ((long)(pl0 + h) * P.k3 + i3) * P.P2 * P1 + P.m2 * P1 + u;
     float2 x[NY];
@@ -577,7 +596,7 @@ __global__ void __launch_bounds__(ZC_T) k_zcols_fwd(PipeParams P, const float2 *
 // even or odd i3 and transforms them (H points), and the butterfly exchange
 // of k_plane2 completes the N-point transform.  Whole warps run (lanes past
 // the last column work on zeros and store nothing).
-template <int N>
+template <int N, bool HALF>
 __global__ void __launch_bounds__(ZC_T) k_zcols_inv2(PipeParams P, const float *__restrict__ cin, long ldc,
                                                       float2 *__restrict__ bufA) {
   using rf::out_pos;
@@ -589,22 +608,24 @@ __global__ void __launch_bounds__(ZC_T) k_zcols_inv2(PipeParams P, const float *
   const int bA = P.pairs[2 * p], bB = P.pairs[2 * p + 1];
   const float *cA = cin + (long)bA * ldc;
   const float *cB = bB >= 0 ? cin + (long)bB * ldc : nullptr;
+  constexpr int MB = line_mb<N, HALF>();   // samples beyond it are zero
   float2 x[H];
-#pragma unroll
-  for (int j = 0; j < H; ++j) {
-    const int i3 = 2 * j + h;
-    const int code = on ? P.col_ig[i3 * P.ncol + q] : 0;
+  rf::static_for<0, H>([&](auto jc) {
+    constexpr int j = decltype(jc)::value;
     float2 z = make_float2(0.f, 0.f);
-    if (code != 0) {
-      const int ig = (code > 0 ? code : -code) - 1;
-      const float ra = cA[2 * ig], ia = ig ? cA[2 * ig + 1] : 0.f;
-      const float rb = cB ? cB[2 * ig] : 0.f, ib = (cB && ig) ? cB[2 * ig + 1] : 0.f;
-      if (code > 0) { z.x = ra - ib; z.y = ia + rb; }
-      else          { z.x = ra + ib; z.y = rb - ia; }
+    if constexpr (z2_kind<N, MB>(j) != Z2_NONE) {
+      const int code = on ? P.col_ig[(2 * j + h) * P.ncol + q] : 0;
+      if (code != 0) {
+        const int ig = (code > 0 ? code : -code) - 1;
+        const float ra = cA[2 * ig], ia = ig ? cA[2 * ig + 1] : 0.f;
+        const float rb = cB ? cB[2 * ig] : 0.f, ib = (cB && ig) ? cB[2 * ig + 1] : 0.f;
+        if (code > 0) { z.x = ra - ib; z.y = ia + rb; }
+        else          { z.x = ra + ib; z.y = rb - ia; }
+      }
     }
     x[j] = z;
-  }
-  rf::fft<float, +1, H>(x);
+  });
+  rf::fft_nz<float, +1, H, z2_bound<N, MB>()>(x);
   pl2::dit_combine<+1, N>(x, h);
   if (on) {
     float2 *dst = bufA + (long)pl * N * P.P2 * P.P1 + P.col_ja[q];
@@ -615,12 +636,58 @@ __global__ void __launch_bounds__(ZC_T) k_zcols_inv2(PipeParams P, const float *
   }
 }
 
+// The forward z pass the same way: lane h of a column loads the samples 2j + h
+// of bufA and, after the exchange, scatters the rows k + h H inside the sphere
+// to zsph as k_zfwd does.  At Si512 (96 points, 1100 bands): 960 -> 820 us.
+template <int N, bool HALF>
+__global__ void __launch_bounds__(ZC_T) k_zcols_fwd2(PipeParams P, const float2 *__restrict__ bufA,
+                                                     float2 *__restrict__ zsph) {
+  using rf::out_pos;
+  constexpr int H = N / 2, MB = line_mb<N, HALF>();
+  const int q = (int)((blockIdx.x * ZC_T + threadIdx.x) >> 1), h = threadIdx.x & 1;
+  const int pl = blockIdx.y, p = P.pair0 + pl;
+  if (p >= (P.npair_dev ? *P.npair_dev : P.npair)) return;   // uniform in the block
+  const bool on = q < P.ncol;
+  const float2 *src = bufA + (long)pl * N * P.P2 * P.P1 + (on ? P.col_ja[q] : 0);
+  float2 x[H];
+#pragma unroll
+  for (int j = 0; j < H; ++j) x[j] = on ? src[(long)(2 * j + h) * P.P2 * P.P1] : make_float2(0.f, 0.f);
+  rf::fft<float, -1, H>(x);
+  pl2::dit_combine<-1, N>(x, h);
+  if (!on) return;
+  const float s = (float)P.inv_n;
+  float2 *Z = zsph + (long)pl * (P.nplw + 1) * 2;
+  rf::static_for<0, H>([&](auto kc) {
+    constexpr int k = decltype(kc)::value;
+    if constexpr (k <= MB || H - k <= MB) {
+      const int code = (h ? H - k <= MB : k <= MB) ? P.col_ig[(k + h * H) * P.ncol + q] : 0;
+      if (code != 0) {
+        float2 z = x[out_pos(H, k)];
+        z.x *= s;
+        z.y *= s;
+        if (code > 0) {
+          const int ig = code - 1;
+          Z[2 * ig] = z;
+          if (ig == 0) Z[1] = z;
+        } else {
+          Z[2 * (-code - 1) + 1] = z;
+        }
+      }
+    }
+  });
+}
+
 template <int N>
-int zcols2_launch(const PipeParams &P, int npl, const float *cin, long ldc, float2 *bufA, bool inv,
-                         cudaStream_t st) {
-  if (!inv) return -1;   // the forward z pass stays on the shared-memory kernel
+int zcols2_launch(const PipeParams &P, int npl, const float *cin, long ldc, float2 *bufA, const float2 *src,
+                  float2 *zsph, bool inv, cudaStream_t st) {
   dim3 g((2 * P.ncol + ZC_T - 1) / ZC_T, npl);
-  k_zcols_inv2<N><<<g, ZC_T, 0, st>>>(P, cin, ldc, bufA);
+  if (P.m3 <= line_mb<N, true>()) {
+    if (inv) k_zcols_inv2<N, true><<<g, ZC_T, 0, st>>>(P, cin, ldc, bufA);
+    else k_zcols_fwd2<N, true><<<g, ZC_T, 0, st>>>(P, src, zsph);
+  } else {
+    if (inv) k_zcols_inv2<N, false><<<g, ZC_T, 0, st>>>(P, cin, ldc, bufA);
+    else k_zcols_fwd2<N, false><<<g, ZC_T, 0, st>>>(P, src, zsph);
+  }
   note_launch();
   return 0;
 }
@@ -877,17 +944,20 @@ int plane_r_launch(const PipeParams &P, int npl, float2 *bufA, float2 *R, const 
   return 0;
 }
 
-template <int N>
-int plane2_launch(const PipeParams &P, int npl, float2 *bufA, const float *vloc, cudaStream_t st) {
-  const size_t sm = sizeof(float2) * (size_t)N * P.P1;
-  if (2 * P.P1 > 2 * N || sm > 100 * 1024) return -1;
+template <int N, bool HALF>
+static void plane2_go(const PipeParams &P, int npl, float2 *bufA, const float *vloc, cudaStream_t st) {
+  constexpr size_t sm = sizeof(float2) * (size_t)N * plane2_pitch<N, HALF>();
   static bool attr = false;
   if (!attr) {
-    cudaFuncSetAttribute(k_plane2<N>, cudaFuncAttributeMaxDynamicSharedMemorySize, 100 * 1024);
+    cudaFuncSetAttribute(k_plane2<N, HALF>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
     attr = true;
   }
-  dim3 g(P.k3, npl);
-  k_plane2<N><<<g, 2 * N, sm, st>>>(P, bufA, vloc);
+  k_plane2<N, HALF><<<dim3(P.k3, npl), 2 * N, sm, st>>>(P, bufA, vloc);
+}
+template <int N>
+int plane2_launch(const PipeParams &P, int npl, float2 *bufA, const float *vloc, cudaStream_t st) {
+  if (P.m1 <= line_mb<N, true>() && P.m2 <= line_mb<N, true>()) plane2_go<N, true>(P, npl, bufA, vloc, st);
+  else plane2_go<N, false>(P, npl, bufA, vloc, st);
   note_launch();
   return 0;
 }
@@ -908,6 +978,7 @@ int plane2_launch(const PipeParams &P, int npl, float2 *bufA, const float *vloc,
   template int plane2_launch<N>(const PipeParams &, int, float2 *, const float *, cudaStream_t);                \
   template int rho2_launch<N>(const PipeParams &, int, const float2 *, const double *, double *, double *, int,  \
                               cudaStream_t);                                                                    \
-  template int zcols2_launch<N>(const PipeParams &, int, const float *, long, float2 *, bool, cudaStream_t);
+  template int zcols2_launch<N>(const PipeParams &, int, const float *, long, float2 *, const float2 *, float2 *, \
+                                bool, cudaStream_t);
 
 }  // namespace qx

@@ -22,8 +22,8 @@ struct PipeParams {
   const int *col_ig;
   int ncol;
   // column a of the sphere's x-y shadow: bit k of .x (.y) set where row
-  // j2 = m2 + k (m2 - k) holds it, k < 32
-  const uint2 *col_mask;
+  // j2 = m2 + k (m2 - k) holds it, k < 64
+  const ulonglong2 *col_mask;
   const int *pairs;         // band indices, 2 per pair, -1 = empty slot
   const int *npair_dev;     // number of valid pairs (device), or null
   int npair;                // pair bound when npair_dev is null
@@ -82,7 +82,7 @@ struct Plan {
   int4 *d_row_ent = nullptr;
   // sphere z-columns (see PipeParams)
   int *d_col_ja = nullptr, *d_col_ig = nullptr;
-  uint2 *d_col_mask = nullptr;
+  ulonglong2 *d_col_mask = nullptr;
   int ncol = 0;
   // real-space KB (kb_lmx projectors per point, at most 9: s, p, d)
   int natom = 0, npts = 0, kb_lmx = 4;
