@@ -661,12 +661,15 @@ __device__ __forceinline__ void house(double x0, double sigma, double &tau, doub
     alpha = fabs(x0);
     return;
   }
-  const double s2 = x0 * x0 + sigma;
-  const double mu = s2 * rsqrt_nr(s2);
-  const double v1 = (x0 <= 0.0) ? x0 - mu : -sigma * recip2_nr(x0 + mu);
-  const double v1s = v1 * v1;
-  tau = 2.0 * v1s * recip2_nr(sigma + v1s);
-  rbeta = recip2_nr(v1);
+  // v1 = x0 - mu, formed without cancellation as -t (x0 <= 0) or -sigma / t
+  // with t = |x0| + mu, and tau = 2 v1^2 / (sigma + v1^2) = -v1 / mu since
+  // sigma + v1^2 = -2 mu v1: two dependent approximations, 1 / sigma beside them
+  const double s2 = x0 * x0 + sigma, rsg = recip2_nr(sigma);
+  const double rmu = rsqrt_nr(s2), mu = s2 * rmu;
+  const double t = fabs(x0) + mu, rt = recip2_nr(t);
+  const bool neg = x0 <= 0.0;
+  tau = (neg ? t : sigma * rt) * rmu;
+  rbeta = neg ? -rt : -t * rsg;
   alpha = mu;
 }
 
@@ -817,7 +820,11 @@ __global__ void __launch_bounds__(TRR_W * 32, 1)
   __shared__ double sigp[2][TRR_W];
   __shared__ double part[TRR_W][NCOL];
   __shared__ double ps[NCOL];
-  __shared__ double vsm[TRR_W][NR], wsm[TRR_W][NR];   // v, w of each warp's rows (read back as broadcasts)
+  static_assert(NR % 2 == 0, "rows are read back in pairs");
+  // v, w of each warp's rows, read back as broadcasts of two rows at a time
+  // (one 16-byte load: the loads otherwise take as long as the FMAs)
+  __shared__ __align__(16) double vsm[TRR_W][NR], wsm[TRR_W][NR];
+  __shared__ double vs[NCOL];                         // v, for the columns
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int r0 = warp * NR;
   double a[NR][NC];
@@ -870,7 +877,11 @@ __global__ void __launch_bounds__(TRR_W * 32, 1)
       d[k] = x[k];
       e[k] = al;
     }
-    for (int i = k + 1 + tid; i < n; i += TRR_W * 32) HV[(long)k * n + i] = vof(i);
+    for (int i = tid; i < NCOL; i += TRR_W * 32) {   // read after barrier (2)
+      const double vi = vof(i);
+      vs[i] = vi;
+      if (i > k && i < n) HV[(long)k * n + i] = vi;
+    }
     if (t == 0.0) continue;                                            // same in every thread
     const bool rows_active = r0 + NR > k + 1;                          // uniform in the warp
     // lane r < NR keeps v of row r0 + r; the warp reads it by shuffles
@@ -891,10 +902,10 @@ __global__ void __launch_bounds__(TRR_W * 32, 1)
         for (int c = 0; c < NC; ++c) sc[c] = 0.0;
         if (rows_active) {
 #pragma unroll
-          for (int r = 0; r < NR; ++r) {
-            const double vr = vsm[warp][r];
+          for (int r = 0; r < NR; r += 2) {
+            const double2 vr = *reinterpret_cast<const double2 *>(&vsm[warp][r]);
 #pragma unroll
-            for (int c = P; c < NC; ++c) sc[c] = fma(a[r][c], vr, sc[c]);
+            for (int c = P; c < NC; ++c) sc[c] = fma(a[r + 1][c], vr.y, fma(a[r][c], vr.x, sc[c]));
           }
         }
 #pragma unroll
@@ -910,7 +921,7 @@ __global__ void __launch_bounds__(TRR_W * 32, 1)
       __syncthreads();                                                 // (3)
       double kk = 0.0;
 #pragma unroll
-      for (int c = P; c < NC; ++c) kk = fma(vof(lane + 32 * c), ps[lane + 32 * c], kk);
+      for (int c = P; c < NC; ++c) kk = fma(vs[lane + 32 * c], ps[lane + 32 * c], kk);
       const double K = 0.5 * t * warp_sum(kk);
       // p of rows <= k is zero (ps below slot P is not rewritten in this copy)
       const double prow = (r0 + lane > k) ? ps[min(r0 + lane, NCOL - 1)] : 0.0;
@@ -922,21 +933,27 @@ __global__ void __launch_bounds__(TRR_W * 32, 1)
       if (rows_active) {
         double wc[NC];
 #pragma unroll
-        for (int c = P; c < NC; ++c) wc[c] = fma(-K, vof(lane + 32 * c), ps[lane + 32 * c]);
+        for (int c = P; c < NC; ++c) wc[c] = fma(-K, vs[lane + 32 * c], ps[lane + 32 * c]);
 #pragma unroll
-        for (int r = 0; r < NR; ++r) {
-          const double vi = vsm[warp][r];
+        for (int r = 0; r < NR; r += 2) {
+          const double2 vi = *reinterpret_cast<const double2 *>(&vsm[warp][r]);
 #pragma unroll
-          for (int c = P; c < NC; ++c) a[r][c] = fma(-vi, wc[c], a[r][c]);
+          for (int c = P; c < NC; ++c) {
+            a[r][c] = fma(-vi.x, wc[c], a[r][c]);
+            a[r + 1][c] = fma(-vi.y, wc[c], a[r + 1][c]);
+          }
         }
         double vc[NC];
 #pragma unroll
-        for (int c = P; c < NC; ++c) vc[c] = vof(lane + 32 * c);
+        for (int c = P; c < NC; ++c) vc[c] = vs[lane + 32 * c];
 #pragma unroll
-        for (int r = 0; r < NR; ++r) {
-          const double wi = wsm[warp][r];
+        for (int r = 0; r < NR; r += 2) {
+          const double2 wi = *reinterpret_cast<const double2 *>(&wsm[warp][r]);
 #pragma unroll
-          for (int c = P; c < NC; ++c) a[r][c] = fma(-wi, vc[c], a[r][c]);
+          for (int c = P; c < NC; ++c) {
+            a[r][c] = fma(-wi.x, vc[c], a[r][c]);
+            a[r + 1][c] = fma(-wi.y, vc[c], a[r + 1][c]);
+          }
         }
       }
     };
