@@ -166,7 +166,8 @@ struct qx_ctx {
       *d_kbr_cursor = nullptr;
   int4 *d_kbr_lent = nullptr;
   int *d_kbr_ptoff = nullptr;
-  int2 *d_kbr_ptent = nullptr;
+  int *d_kbr_gpatom = nullptr;
+  void *d_kbr_gpvnl = nullptr;
   void *d_kbr_vnl = nullptr, *d_kbr_sumr = nullptr, *d_kbr_bufR = nullptr;
   double *d_kbr_rcl = nullptr;    // radius of each projector's channel (lmx * ntype)
   std::vector<double> kbr_rcut_h; // species radii (the largest channel's)
@@ -930,23 +931,32 @@ extern "C" int qx_set_kb_r(qx_ctx *c, int natom, int lmx, const int *off, const 
   std::vector<int> poff(pl.n + 1, 0);
   for (int i = 0; i < npts; ++i) poff[mesh[i] + 1]++;
   for (long g = 0; g < pl.n; ++g) poff[g + 1] += poff[g];
-  std::vector<int2> pent(std::max(npts, 1));
+  std::vector<int> patom(std::max(npts, 1));
+  std::vector<double> pvnl((size_t)std::max(npts, 1) * lmx);
   std::vector<int> fill(poff.begin(), poff.end() - 1);
   for (int a = 0; a < natom; ++a)
-    for (int i = off[a]; i < off[a + 1]; ++i) pent[fill[mesh[i]]++] = make_int2(i, a);
+    for (int i = off[a]; i < off[a + 1]; ++i) {
+      const int e = fill[mesh[i]]++;
+      patom[e] = a;
+      std::copy(vnl + (size_t)i * lmx, vnl + (size_t)(i + 1) * lmx, pvnl.begin() + (size_t)e * lmx);
+    }
   TRY(dalloc(c, &pl.d_kb_off, sizeof(int) * (natom + 1)));
   TRY(dalloc(c, &pl.d_kb_mesh, sizeof(int) * std::max(npts, 1)));
   TRY(dalloc(c, &pl.d_kb_clalp, sizeof(double) * lmx));
   TRY(dalloc(c, &pl.d_pt_off, sizeof(int) * poff.size()));
-  TRY(dalloc(c, &pl.d_pt_ent, sizeof(int2) * pent.size()));
+  TRY(dalloc(c, &pl.d_pt_atom, sizeof(int) * patom.size()));
   CK(cudaMemcpy(pl.d_kb_off, off, sizeof(int) * (natom + 1), cudaMemcpyHostToDevice));
   CK(cudaMemcpy(pl.d_kb_mesh, mesh, sizeof(int) * npts, cudaMemcpyHostToDevice));
   CK(cudaMemcpy(pl.d_kb_clalp, clalp, sizeof(double) * lmx, cudaMemcpyHostToDevice));
   CK(cudaMemcpy(pl.d_pt_off, poff.data(), sizeof(int) * poff.size(), cudaMemcpyHostToDevice));
-  CK(cudaMemcpy(pl.d_pt_ent, pent.data(), sizeof(int2) * pent.size(), cudaMemcpyHostToDevice));
+  CK(cudaMemcpy(pl.d_pt_atom, patom.data(), sizeof(int) * patom.size(), cudaMemcpyHostToDevice));
   void *v = nullptr;
   TRY(dalloc(c, &v, c->tsize() * (size_t)npts * lmx));
   TRY(up(c, v, vnl, (long)npts * lmx));
+  void *pv = nullptr;
+  TRY(dalloc(c, &pv, c->tsize() * pvnl.size()));
+  TRY(up(c, pv, pvnl.data(), (long)npts * lmx));
+  CK(cudaStreamSynchronize(c->st));   // pvnl is a host temporary
   pl.natom = natom;
   pl.npts = npts;
   pl.kb_lmx = lmx;
@@ -956,10 +966,12 @@ extern "C" int qx_set_kb_r(qx_ctx *c, int natom, int lmx, const int *off, const 
   const long ch = pl.chunk;
   if (c->prec == QX_PREC_FP64) {
     pl.b64.kb_vnl = (double *)v;
+    pl.b64.kb_pvnl = (double *)pv;
     TRY(dalloc(c, &pl.b64.bufR, sizeof(double2) * ch * pl.n));
     TRY(dalloc(c, &pl.b64.sumr, sizeof(double2) * ch * natom * lmx));
   } else {
     pl.b32.kb_vnl = (float *)v;
+    pl.b32.kb_pvnl = (float *)pv;
     TRY(dalloc(c, &pl.b32.bufR, sizeof(float2) * ch * pl.n));
     TRY(dalloc(c, &pl.b32.sumr, sizeof(float2) * ch * natom * lmx));
   }
@@ -1112,7 +1124,8 @@ extern "C" int qx_build_kb_r(qx_ctx *c, int natom, const int *ityp, const double
     TRY(dregrow(c, &c->d_kbr_mesh, sizeof(int) * cap));
     TRY(dregrow(c, &c->d_kbr_ptatom, sizeof(int) * cap));
     TRY(dregrow(c, &c->d_kbr_lent, sizeof(int4) * cap));
-    TRY(dregrow(c, &c->d_kbr_ptent, sizeof(int2) * cap));
+    TRY(dregrow(c, &c->d_kbr_gpatom, sizeof(int) * cap));
+    TRY(dregrow(c, &c->d_kbr_gpvnl, ts * c->kbr_lmx * (size_t)cap));
     TRY(dregrow(c, &c->d_kbr_vnl, ts * c->kbr_lmx * (size_t)cap));
     c->kbr_cap = cap;
     moved = true;
@@ -1129,27 +1142,33 @@ extern "C" int qx_build_kb_r(qx_ctx *c, int natom, const int *ityp, const double
     kbr_fill<float>(G, natom, c->kbr_lmx, c->d_kbr_ityp, c->d_kbr_satm, c->d_kbr_rcut, c->d_kbr_rcl, c->d_kbr_dl, c->d_kbr_tab,
                     c->d_kbr_dtab, c->kbr_mxnl, c->d_kbr_poly, c->d_kbr_soff, c->kbr_cap, c->d_kbr_mesh,
                     c->d_kbr_ptatom, (float *)c->d_kbr_vnl, (float *)c->d_kbr_dvnl, c->st);
-  if (kbr_lines(c->d_kbr_off, natom, c->d_kbr_mesh, c->d_kbr_ptatom, pl.k1, nlines, c->d_kbr_lcnt, c->d_kbr_loff,
-                c->d_kbr_cursor, c->d_kbr_lent, c->d_kbr_ptoff, c->d_kbr_ptent, c->st)) {
+  auto lines = [&](auto *vnl, auto *gpvnl) {
+    return kbr_lines(c->d_kbr_off, natom, c->d_kbr_mesh, c->d_kbr_ptatom, pl.k1, nlines, c->d_kbr_lcnt, c->d_kbr_loff,
+                     c->d_kbr_cursor, c->d_kbr_lent, c->d_kbr_ptoff, c->d_kbr_gpatom, vnl, c->kbr_lmx, gpvnl, c->st);
+  };
+  if (c->prec == QX_PREC_FP64 ? lines((const double *)c->d_kbr_vnl, (double *)c->d_kbr_gpvnl)
+                              : lines((const float *)c->d_kbr_vnl, (float *)c->d_kbr_gpvnl)) {
     set_error("qx_build_kb_r: memset failed");
     return QX_ERR_CUDA;
   }
   CKL();
   if (pl.d_kb_off != c->d_kbr_off || pl.d_kb_mesh != c->d_kbr_mesh || pl.d_pt_off != c->d_kbr_ptoff ||
-      pl.d_pt_ent != c->d_kbr_ptent)
+      pl.d_pt_atom != c->d_kbr_gpatom)
     moved = true;
   pl.d_kb_off = c->d_kbr_off;
   pl.d_kb_mesh = c->d_kbr_mesh;
   pl.d_pt_off = c->d_kbr_ptoff;
-  pl.d_pt_ent = c->d_kbr_ptent;
+  pl.d_pt_atom = c->d_kbr_gpatom;
   if (c->prec == QX_PREC_FP64) {
-    moved |= pl.b64.kb_vnl != (double *)c->d_kbr_vnl || pl.b64.sumr != (double2 *)c->d_kbr_sumr;
+    moved |= pl.b64.kb_vnl != (double *)c->d_kbr_vnl || pl.b64.kb_pvnl != (double *)c->d_kbr_gpvnl || pl.b64.sumr != (double2 *)c->d_kbr_sumr;
     pl.b64.kb_vnl = (double *)c->d_kbr_vnl;
+    pl.b64.kb_pvnl = (double *)c->d_kbr_gpvnl;
     pl.b64.bufR = (double2 *)c->d_kbr_bufR;
     pl.b64.sumr = (double2 *)c->d_kbr_sumr;
   } else {
-    moved |= pl.b32.kb_vnl != (float *)c->d_kbr_vnl || pl.b32.sumr != (float2 *)c->d_kbr_sumr;
+    moved |= pl.b32.kb_vnl != (float *)c->d_kbr_vnl || pl.b32.kb_pvnl != (float *)c->d_kbr_gpvnl || pl.b32.sumr != (float2 *)c->d_kbr_sumr;
     pl.b32.kb_vnl = (float *)c->d_kbr_vnl;
+    pl.b32.kb_pvnl = (float *)c->d_kbr_gpvnl;
     pl.b32.bufR = (float2 *)c->d_kbr_bufR;
     pl.b32.sumr = (float2 *)c->d_kbr_sumr;
   }

@@ -641,9 +641,8 @@ __global__ void __launch_bounds__(QX_THREADS) k_xfwd_r(PipeParams P, const typen
     const T v = V[i];
     z.x *= v; z.y *= v;
     for (int e = e0; e < e1; ++e) {
-      const int2 en = nl.ent[e];
-      const C *s = S + (long)en.y * nl.lmx;
-      const T *w = nl.vnl + (long)en.x * nl.lmx;
+      const C *s = S + (long)nl.atom[e] * nl.lmx;
+      const T *w = nl.vnl + (long)e * nl.lmx;
       T ar = 0, ai = 0;
       for (int q = 0; q < nl.lmx; ++q) {
         ar += w[q] * s[q].x;
@@ -877,7 +876,7 @@ int launch_hpsi_chunk(const Plan &pl, const PipeParams &P, int npl, const T *cin
     k_unpack<T><<<gu, 128, 0, st>>>(P, bf.zsph, cin, ldc, out, ldo, dk, accumulate); note_launch();
     return 0;
   }
-  const NlPoints<T> nl{pl.d_pt_off, pl.d_pt_ent, bf.kb_vnl, bf.sumr, pl.natom, pl.kb_lmx};
+  const NlPoints<T> nl{pl.d_pt_off, pl.d_pt_atom, bf.kb_pvnl, bf.sumr, pl.natom, pl.kb_lmx};
   if constexpr (sizeof(T) == sizeof(float)) {
     if (nlmode == 2 && pl.use_plane && plane_enabled() &&
         launch_plane_r_f32(P, npl, bf.bufA, bf.bufR, bf.vloc, nullptr, st) == 0) {

@@ -336,8 +336,8 @@ __global__ void __launch_bounds__(2 * N) k_plane2(PipeParams P, float2 *__restri
 // as NY x (NX | 1) complex values.
 //   k_plane_inv_r: backward y and x, the planes stored to R (coalesced);
 //   k_plane_fwd_r: V psi plus the projectors' part, forward x and y back to
-//     bufA.  A grid point's projector points come from the point index
-//     (pt_off, pt_ent), so each thread sums its own points in a fixed order,
+//     bufA.  A grid point's projector points come in grid-point order
+//     (NlPoints), so each thread sums its own points in a fixed order,
 //     for both pairs of the CTA from one read of the projector values.
 // Latency and the L2 traffic of the projector values bound the second (24
 // bytes an entry and CTA, 313 k entries at Si64), hence two pairs a CTA and
@@ -425,19 +425,19 @@ __global__ void __launch_bounds__(128, plane_minb(NX > NY ? NX : NY) > 1 ? 4 : 1
 #pragma unroll
         for (int q = 0; q < UN; ++q) more = max(more, e1[q] - e0[q]);
         for (int k = 0; k < more; ++k) {
-          int2 en[UN];
+          int at[UN];
           float4 v[UN];
 #pragma unroll
-          for (int q = 0; q < UN; ++q) en[q] = e0[q] + k < e1[q] ? nl.ent[e0[q] + k] : make_int2(-1, 0);
-#pragma unroll
-          for (int q = 0; q < UN; ++q)
-            v[q] = en[q].x >= 0 ? *reinterpret_cast<const float4 *>(nl.vnl + 4L * en[q].x)
-                                : make_float4(0.f, 0.f, 0.f, 0.f);
+          for (int q = 0; q < UN; ++q) {
+            const bool in = e0[q] + k < e1[q];
+            at[q] = in ? nl.atom[e0[q] + k] : -1;
+            v[q] = in ? *reinterpret_cast<const float4 *>(nl.vnl + 4L * (e0[q] + k)) : make_float4(0.f, 0.f, 0.f, 0.f);
+          }
 #pragma unroll
           for (int q = 0; q < UN; ++q) {
-            if (en[q].x < 0) continue;
-            const float4 *a = reinterpret_cast<const float4 *>(S0 + 4L * en[q].y);
-            const float4 *b = reinterpret_cast<const float4 *>(S1 + 4L * en[q].y);
+            if (at[q] < 0) continue;
+            const float4 *a = reinterpret_cast<const float4 *>(S0 + 4L * at[q]);
+            const float4 *b = reinterpret_cast<const float4 *>(S1 + 4L * at[q]);
             const float4 a0 = a[0], a1 = a[1], b0 = b[0], b1 = b[1], w = v[q];
             z0[q].x += w.x * a0.x + w.y * a0.z + w.z * a1.x + w.w * a1.z;
             z0[q].y += w.x * a0.y + w.y * a0.w + w.z * a1.y + w.w * a1.w;
@@ -449,10 +449,10 @@ __global__ void __launch_bounds__(128, plane_minb(NX > NY ? NX : NY) > 1 ? 4 : 1
 #pragma unroll
         for (int q = 0; q < UN; ++q)
           for (int e = e0[q]; e < e1[q]; ++e) {
-            const int2 en = nl.ent[e];
+            const long at = (long)nl.lmx * nl.atom[e];
             for (int l = 0; l < nl.lmx; ++l) {
-              const float v = nl.vnl[(long)nl.lmx * en.x + l];
-              const float2 a = S0[(long)nl.lmx * en.y + l], b = S1[(long)nl.lmx * en.y + l];
+              const float v = nl.vnl[(long)nl.lmx * e + l];
+              const float2 a = S0[at + l], b = S1[at + l];
               z0[q].x += v * a.x;
               z0[q].y += v * a.y;
               z1[q].x += v * b.x;

@@ -363,10 +363,17 @@ __global__ void k_kbr_line_fill(const int *__restrict__ off, int natom, const in
 // shared memory (k1 counters), then the rank among the few entries of the
 // same x; longer ones by ranking every entry against the line in global
 // memory.
+// The projector values are copied into that order.
 constexpr int LSORT_MAX = 1024;
+template <typename T>
 __global__ void __launch_bounds__(128) k_kbr_line_sort(const int *__restrict__ loff, long nlines, int k1,
                                                        const int4 *__restrict__ lent, int *__restrict__ ptoff,
-                                                       int2 *__restrict__ ptent) {
+                                                       int *__restrict__ gpatom, const T *__restrict__ vnl, int lmx,
+                                                       T *__restrict__ gpvnl) {
+  auto place = [&](long e, const int4 &v) {
+    gpatom[e] = v.z;
+    for (int l = 0; l < lmx; ++l) gpvnl[e * lmx + l] = vnl[(long)v.y * lmx + l];
+  };
   extern __shared__ int start[];   // k1 + 1 offsets, then k1 cursors
   int *cursor = start + k1 + 1;
   __shared__ int2 sorted[LSORT_MAX];
@@ -405,14 +412,14 @@ __global__ void __launch_bounds__(128) k_kbr_line_sort(const int *__restrict__ l
         const int4 v = e[i];
         int r = start[v.x];
         for (int j = start[v.x]; j < start[v.x + 1]; ++j) r += sorted[j].x < v.y ? 1 : 0;
-        ptent[lo + r] = make_int2(v.y, v.z);
+        place(lo + r, v);
       }
     } else {
       for (int i = threadIdx.x; i < m; i += blockDim.x) {
         const int4 v = e[i];
         int r = start[v.x];
         for (int j = 0; j < m; ++j) r += (e[j].x == v.x && e[j].y < v.y) ? 1 : 0;
-        ptent[lo + r] = make_int2(v.y, v.z);
+        place(lo + r, v);
       }
     }
     __syncthreads();
@@ -446,8 +453,10 @@ template void kbr_fill<double>(const KbrGeom &, int, int, const int *, const dou
                                const double *, const double *, const double *, int, const int *, const int *, long,
                                int *, int *, double *, double *, cudaStream_t);
 
+template <typename T>
 int kbr_lines(const int *off, int natom, const int *mesh, const int *ptatom, int k1, long nlines, int *lcnt,
-              int *loff, int *cursor, int4 *lent, int *ptoff, int2 *ptent, cudaStream_t st) {
+              int *loff, int *cursor, int4 *lent, int *gpoff, int *gpatom, const T *vnl, int lmx, T *gpvnl,
+              cudaStream_t st) {
   if (cudaMemsetAsync(lcnt, 0, sizeof(int) * nlines, st) != cudaSuccess) return 1;
   k_kbr_line_count<<<148 * 4, 256, 0, st>>>(off, natom, mesh, k1, lcnt);
   note_launch();
@@ -455,10 +464,15 @@ int kbr_lines(const int *off, int natom, const int *mesh, const int *ptatom, int
   note_launch();
   k_kbr_line_fill<<<148 * 4, 256, 0, st>>>(off, natom, mesh, ptatom, k1, cursor, lent);
   note_launch();
-  k_kbr_line_sort<<<(unsigned)std::min<long>(148 * 16, nlines), 128, sizeof(int) * (2 * k1 + 1), st>>>(loff, nlines, k1, lent, ptoff,
-                                                                                                         ptent);
+  k_kbr_line_sort<T><<<(unsigned)std::min<long>(148 * 16, nlines), 128, sizeof(int) * (2 * k1 + 1), st>>>(
+      loff, nlines, k1, lent, gpoff, gpatom, vnl, lmx, gpvnl);
   note_launch();
   return 0;
 }
+
+template int kbr_lines<float>(const int *, int, const int *, const int *, int, long, int *, int *, int *, int4 *,
+                              int *, int *, const float *, int, float *, cudaStream_t);
+template int kbr_lines<double>(const int *, int, const int *, const int *, int, long, int *, int *, int *, int4 *,
+                               int *, int *, const double *, int, double *, cudaStream_t);
 
 }  // namespace qx
