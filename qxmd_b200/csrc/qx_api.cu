@@ -1546,8 +1546,8 @@ static int eigen_impl(qx_ctx *c, const qx_cgparm *p, int *nriter, int *nhpsi_out
   for (int it = 0; it < maxit; ++it) {
     cg_prec<T>(nb, ne, ne, g, h, c->d_dk, s, c->st);
     // subgs3: Pm = snap^T h ; Pm masked to j < i, active i ; h -= snap * Pm
-    TRY(gemm<T>(true, false, nb, nb, ne, (T)1, snap, ne, h, ne, (T)0, pm_t, nb, 1, nullptr, nullptr, c->st, c->gws, c->gws_bytes, nullptr, c->tcpad, c->tcpad_bytes));
-    cg_mask<T>(nb, pm_t, s, c->st);
+    TRY(gemm<T>(true, false, nb, nb, ne, (T)1, snap, ne, h, ne, (T)0, pm_t, nb, 1, nullptr, nullptr, c->st, c->gws, c->gws_bytes, nullptr, c->tcpad, c->tcpad_bytes,
+                 s.active));
     TRY(gemm<T>(false, false, ne, nb, nb, (T)-1, snap, ne, pm_t, nb, (T)1, h, ne, 0, nullptr, nullptr, c->st, nullptr, 0, nullptr, c->tcpad, c->tcpad_bytes));
     cg_orth<T>(nb, ne, ne, x, h, s, c->st);
     CKL();

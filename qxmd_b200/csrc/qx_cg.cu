@@ -2,8 +2,8 @@
 // preconditioner prpcg eigen.f90:1093-1113, subgs4 engrad.f90:1196-1248).
 // All bands iterate together; band ib is projected against the entry
 // snapshot of bands < ib (subgs3, done as two GEMMs by the caller), which is
-// the reference's result with one band per rank.  One CTA per band; every
-// reduction is accumulated in FP64.  Per-band state lives on the device, so a
+// the reference's result with one band per rank.  A cluster of CTAs a band (one
+// CTA in k_cg_init); every reduction is accumulated in FP64.  Per-band state lives on the device, so a
 // CG sweep needs no host round trip.
 #include <cooperative_groups.h>
 
@@ -111,13 +111,42 @@ __device__ __forceinline__ void cluster_sums(double (&v)[NV], double (*red)[32],
   }
 }
 
-// g <- prcd * g; zansap = <g|g>; h <- g + beta*h (h <- g on reset).
+// The active-band list and the band pairs of the FFT pipeline, by one warp: 32
+// bands a round with a ballot and a population-count prefix.
+__device__ __forceinline__ void cg_list(int nb, const CgState &s) {
+  const int lane = threadIdx.x;
+  int n = 0;
+  for (int b0 = 0; b0 < nb; b0 += 32) {
+    const int b = b0 + lane;
+    const bool act = (b < nb) && s.active[b];
+    const unsigned m = __ballot_sync(0xffffffffu, act);
+    if (act) s.list[n + __popc(m & ((1u << lane) - 1u))] = b;
+    n += __popc(m);
+  }
+  __syncwarp();
+  for (int p = lane; p < (n + 1) / 2; p += 32) {
+    s.pairs[2 * p] = s.list[2 * p];
+    s.pairs[2 * p + 1] = (2 * p + 1 < n) ? s.list[2 * p + 1] : -1;
+  }
+  if (lane == 0) {
+    *s.nact = n;
+    *s.npair = (n + 1) / 2;
+  }
+}
+
+// g <- prcd * g; zansap = <g|g>; h <- g + beta*h (h <- g on reset).  One more
+// cluster after those of the bands writes the active-band list (the sweep
+// leaves `active` alone), which the H|h> that follows reads.
 template <typename T>
-__global__ void __cluster_dims__(CGC, 1, 1) __launch_bounds__(CGB, 5) k_cg_prec(int ne, long ldx, T *__restrict__ g, T *__restrict__ h,
+__global__ void __cluster_dims__(CGC, 1, 1) __launch_bounds__(CGB, 5) k_cg_prec(int nb, int ne, long ldx, T *__restrict__ g, T *__restrict__ h,
                                                          const double *__restrict__ dk, CgState s) {
   constexpr int U = cgu<T>();
   __shared__ double red[1][32], slot[1];
   const int b = blockIdx.x / CGC;
+  if (b == nb) {
+    if (blockIdx.x % CGC == 0 && threadIdx.x < 32) cg_list(nb, s);
+    return;
+  }
   if (!s.active[b]) return;
   T *gb = g + b * ldx, *hb = h + b * ldx;
   const double e15 = 1.5 * s.ekib[b];
@@ -164,40 +193,6 @@ __global__ void __cluster_dims__(CGC, 1, 1) __launch_bounds__(CGB, 5) k_cg_prec(
     s.betk[b] = z[0];
     s.iter[b] += 1;
   }
-}
-
-// Mask for subgs3: M(j,i) = P(j,i) if j < i and band i is active, else 0.  The
-// last block, in place of a launch of its own, writes the active-band list and the band pairs of the FFT
-// pipeline: its first warp compacts 32 bands per round with a ballot and a
-// population-count prefix.
-template <typename T>
-__global__ void k_cg_mask(int nb, T *__restrict__ Pm, CgState s) {
-  if (blockIdx.x == gridDim.x - 1) {
-    if (threadIdx.x >= 32) return;
-    const int lane = threadIdx.x;
-    int n = 0;
-    for (int b0 = 0; b0 < nb; b0 += 32) {
-      const int b = b0 + lane;
-      const bool act = (b < nb) && s.active[b];
-      const unsigned m = __ballot_sync(0xffffffffu, act);
-      if (act) s.list[n + __popc(m & ((1u << lane) - 1u))] = b;
-      n += __popc(m);
-    }
-    __syncwarp();
-    for (int p = lane; p < (n + 1) / 2; p += 32) {
-      s.pairs[2 * p] = s.list[2 * p];
-      s.pairs[2 * p + 1] = (2 * p + 1 < n) ? s.list[2 * p + 1] : -1;
-    }
-    if (lane == 0) {
-      *s.nact = n;
-      *s.npair = (n + 1) / 2;
-    }
-    return;
-  }
-  const long e = blockIdx.x * (long)blockDim.x + threadIdx.x;
-  if (e >= (long)nb * nb) return;
-  const int i = (int)(e / nb), j = (int)(e - (long)i * nb);
-  if (!(j < i && s.active[i])) Pm[e] = (T)0;
 }
 
 // subgs4: h -= <x|h> x.
@@ -736,11 +731,7 @@ template <typename T> void cg_init(int nb, int ne, long ldx, const T *x, const T
   k_cg_init<T><<<nb, CGT, 0, st>>>(ne, ldx, x, hx, g, s); note_launch();
 }
 template <typename T> void cg_prec(int nb, int ne, long ldx, T *g, T *h, const double *dk, const CgState &s, cudaStream_t st) {
-  k_cg_prec<T><<<nb * CGC, CGB, 0, st>>>(ne, ldx, g, h, dk, s); note_launch();
-}
-template <typename T> void cg_mask(int nb, T *Pm, const CgState &s, cudaStream_t st) {
-  const long nn = (long)nb * nb;
-  k_cg_mask<T><<<(int)((nn + 255) / 256) + 1, 256, 0, st>>>(nb, Pm, s); note_launch();
+  k_cg_prec<T><<<(nb + 1) * CGC, CGB, 0, st>>>(nb, ne, ldx, g, h, dk, s); note_launch();
 }
 template <typename T> void cg_orth(int nb, int ne, long ldx, const T *x, T *h, const CgState &s, cudaStream_t st) {
   k_cg_orth<T><<<nb * CGC, CGB, 0, st>>>(ne, ldx, x, h, s); note_launch();
@@ -789,7 +780,6 @@ template <typename T> void scale_rows(int nproj, int ncol, T *P, long ldp, const
 #define QX_INST(T)                                                                                          \
   template void cg_init<T>(int, int, long, const T *, const T *, T *, const CgState &, cudaStream_t);        \
   template void cg_prec<T>(int, int, long, T *, T *, const double *, const CgState &, cudaStream_t);         \
-  template void cg_mask<T>(int, T *, const CgState &, cudaStream_t);                                         \
   template void cg_orth<T>(int, int, long, const T *, T *, const CgState &, cudaStream_t);                   \
   template void seq_init<T>(int, int, long, const T *, const T *, T *, const double *, const CgState &,      \
                             const SeqArgs &, cudaStream_t);                                                 \

@@ -35,8 +35,6 @@ struct SeqArgs {
 
 template <typename T> void cg_init(int nb, int ne, long ldx, const T *x, const T *hx, T *g, const CgState &s, cudaStream_t st);
 template <typename T> void cg_prec(int nb, int ne, long ldx, T *g, T *h, const double *dk, const CgState &s, cudaStream_t st);
-// the subgs3 mask, and the active-band list and pairs
-template <typename T> void cg_mask(int nb, T *Pm, const CgState &s, cudaStream_t st);
 template <typename T> void cg_orth(int nb, int ne, long ldx, const T *x, T *h, const CgState &s, cudaStream_t st);
 // Entry state of every band (g preconditioned) and band 0 as the current one.
 template <typename T> void seq_init(int nb, int ne, long ldx, const T *x, const T *hx, T *g, const double *dk,

@@ -118,7 +118,8 @@ __global__ void __launch_bounds__(RD_T) k_gemm_reduce(int M, int N, int nsplit, 
                                                       long lda, const T *__restrict__ B, long ldb, T beta,
                                                       T *__restrict__ Cm, long ldc, int gamma,
                                                       const int *__restrict__ colmap, const int *__restrict__ ncol_dev,
-                                                      const T *__restrict__ W, const T *__restrict__ rowscale) {
+                                                      const T *__restrict__ W, const T *__restrict__ rowscale,
+                                                      const int *__restrict__ lower) {
   __shared__ T ws[RD_T / 32][32];
   const int Nact = ncol_dev ? min(N, *ncol_dev) : N;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -158,6 +159,7 @@ __global__ void __launch_bounds__(RD_T) k_gemm_reduce(int M, int N, int nsplit, 
     }
   }
   if (rowscale) v *= rowscale[gm];
+  if (lower && !(gm < gn && lower[gn])) v = 0;
   T *c = Cm + cn * ldc + gm;
   *c = (beta == (T)0) ? alpha * v : alpha * v + beta * *c;
 }
@@ -178,20 +180,35 @@ static void launch(dim3 g, int M, int N, int K, T alpha, const T *A, long lda, c
   note_launch();
   const long mn = (long)M * N;
   k_gemm_reduce<T, TA, TB><<<(int)((mn + 31) / 32), RD_T, 0, st>>>(M, N, nsplit, alpha, A, lda, B, ldb, beta, C, ldc,
-                                                                    gamma, colmap, ncol_dev, W, nullptr);
+                                                                    gamma, colmap, ncol_dev, W, nullptr, nullptr);
+  note_launch();
+}
+
+// C(m, n) = 0 unless m < n and lower[n]: the mask of gemm() where the
+// contraction's own epilogue does not apply it.
+template <typename T>
+__global__ void k_mask_lower(int M, int N, T *__restrict__ C, long ldc, const int *__restrict__ lower) {
+  const long e = blockIdx.x * (long)blockDim.x + threadIdx.x;
+  if (e >= (long)M * N) return;
+  const int n = (int)(e / M), m = (int)(e - (long)n * M);
+  if (!(m < n && lower[n])) C[n * ldc + m] = (T)0;
+}
+template <typename T>
+static void mask_lower(int M, int N, T *C, long ldc, const int *lower, cudaStream_t st) {
+  k_mask_lower<T><<<(int)(((long)M * N + 255) / 256), 256, 0, st>>>(M, N, C, ldc, lower);
   note_launch();
 }
 
 // Finish FP32 split-K partials W[z][n][m] (any producer with that layout).
 void gemm_reduce_f32(bool ta, bool tb, int M, int N, int nsplit, float alpha, const float *A, long lda, const float *B,
                      long ldb, float beta, float *C, long ldc, int gamma, const float *W, cudaStream_t st,
-                     const float *rowscale) {
+                     const float *rowscale, const int *lower) {
   const long mn = (long)M * N;
   const int g = (int)((mn + 31) / 32);
-  if (ta && tb) k_gemm_reduce<float, true, true><<<g, RD_T, 0, st>>>(M, N, nsplit, alpha, A, lda, B, ldb, beta, C, ldc, gamma, nullptr, nullptr, W, rowscale);
-  else if (ta) k_gemm_reduce<float, true, false><<<g, RD_T, 0, st>>>(M, N, nsplit, alpha, A, lda, B, ldb, beta, C, ldc, gamma, nullptr, nullptr, W, rowscale);
-  else if (tb) k_gemm_reduce<float, false, true><<<g, RD_T, 0, st>>>(M, N, nsplit, alpha, A, lda, B, ldb, beta, C, ldc, gamma, nullptr, nullptr, W, rowscale);
-  else k_gemm_reduce<float, false, false><<<g, RD_T, 0, st>>>(M, N, nsplit, alpha, A, lda, B, ldb, beta, C, ldc, gamma, nullptr, nullptr, W, rowscale);
+  if (ta && tb) k_gemm_reduce<float, true, true><<<g, RD_T, 0, st>>>(M, N, nsplit, alpha, A, lda, B, ldb, beta, C, ldc, gamma, nullptr, nullptr, W, rowscale, lower);
+  else if (ta) k_gemm_reduce<float, true, false><<<g, RD_T, 0, st>>>(M, N, nsplit, alpha, A, lda, B, ldb, beta, C, ldc, gamma, nullptr, nullptr, W, rowscale, lower);
+  else if (tb) k_gemm_reduce<float, false, true><<<g, RD_T, 0, st>>>(M, N, nsplit, alpha, A, lda, B, ldb, beta, C, ldc, gamma, nullptr, nullptr, W, rowscale, lower);
+  else k_gemm_reduce<float, false, false><<<g, RD_T, 0, st>>>(M, N, nsplit, alpha, A, lda, B, ldb, beta, C, ldc, gamma, nullptr, nullptr, W, rowscale, lower);
   note_launch();
 }
 
@@ -469,7 +486,7 @@ static int launch_dgemm_tm(int M, int N, int K, double alpha, const double *A, l
   const long mn = (long)M * N;
   k_gemm_reduce<double, TA, TB><<<(int)((mn + 31) / 32), RD_T, 0, st>>>(M, N, nsplit, alpha, A, lda, B, ldb, beta, C,
                                                                        ldc, gamma, colmap, ncol_dev,
-                                                                       (const double *)ws, nullptr);
+                                                                       (const double *)ws, nullptr, nullptr);
   note_launch();
   return 0;
 }
@@ -534,8 +551,8 @@ __global__ void __launch_bounds__(256) k_sgemm(int M, int N, int K, float alpha,
                                                const float *__restrict__ B, long ldb, float beta,
                                                float *__restrict__ Cm, long ldc, int gamma,
                                                const int *__restrict__ colmap, const int *__restrict__ ncol_dev,
-                                               const float *__restrict__ rowscale, int kchunk, float *__restrict__ W,
-                                               int *__restrict__ cnt) {
+                                               const float *__restrict__ rowscale, const int *__restrict__ lower,
+                                               int kchunk, float *__restrict__ W, int *__restrict__ cnt) {
   constexpr int TMM = 16 * MT, TNN = 16 * NT, PA = TMM + 1, PB = TNN + 1;
   constexpr int SA = SBK * PA, SSZ = SA + SBK * PB;
   extern __shared__ __align__(16) float ssm[];
@@ -630,7 +647,8 @@ __global__ void __launch_bounds__(256) k_sgemm(int M, int N, int K, float alpha,
     }
     float *c = Cm + cn * ldc + gm;
     v = (beta == 0.f) ? alpha * v : alpha * v + beta * *c;
-    *c = rowscale ? v * rowscale[gm] : v;
+    if (rowscale) v *= rowscale[gm];
+    *c = lower && !(gm < gn && lower[gn]) ? 0.f : v;
   };
   if constexpr (SPLIT) {
     // Split K, a cluster of SCL splits at a time: every CTA leaves its partial
@@ -719,7 +737,7 @@ static int sgemm_rows(int n) {
 template <bool TA, bool TB, bool SPLIT, int MT, int NT>
 static void sgemm_go(dim3 g, int M, int N, int K, float alpha, const float *A, long lda, const float *B, long ldb,
                      float beta, float *C, long ldc, int gamma, const int *colmap, const int *ncol_dev,
-                     const float *rowscale, int kchunk, float *W, int *cnt, cudaStream_t st) {
+                     const float *rowscale, const int *lower, int kchunk, float *W, int *cnt, cudaStream_t st) {
   constexpr size_t sm = sgemm_smem<MT, NT>();
   static_assert(sm <= 48 * 1024, "stages fit the default shared-memory limit");
   static_assert(sm >= sizeof(float) * 256 * MT * NT, "a partial tile fits the stages");
@@ -736,7 +754,7 @@ static void sgemm_go(dim3 g, int M, int N, int K, float alpha, const float *A, l
   cfg.attrs = &at;
   cfg.numAttrs = SPLIT ? 1 : 0;
   cudaLaunchKernelEx(&cfg, k_sgemm<TA, TB, SPLIT, MT, NT>, M, N, K, alpha, A, lda, B, ldb, beta, C, ldc, gamma, colmap,
-                     ncol_dev, rowscale, kchunk, W, cnt);
+                     ncol_dev, rowscale, lower, kchunk, W, cnt);
   note_launch();
 }
 
@@ -751,7 +769,8 @@ static void sgemm_go(dim3 g, int M, int N, int K, float alpha, const float *A, l
 template <bool TA, bool TB>
 static void sgemm_launch(int M, int N, int K, float alpha, const float *A, long lda, const float *B, long ldb,
                          float beta, float *C, long ldc, int gamma, const int *colmap, const int *ncol_dev,
-                         const float *rowscale, void *ws, size_t ws_bytes, int *cnt, cudaStream_t st) {
+                         const float *rowscale, const int *lower, void *ws, size_t ws_bytes, int *cnt,
+                         cudaStream_t st) {
   const int nt = sgemm_rows(N), tn = (N + 16 * nt - 1) / (16 * nt);
   int mt = TA ? sgemm_rows(M) : 4;
   if (!TA)
@@ -772,9 +791,9 @@ static void sgemm_launch(int M, int N, int K, float alpha, const float *A, long 
 #define QX_SG(MT_, NT_)                                                                                              \
   if (mt == MT_ && nt == NT_) {                                                                                      \
     if (split) sgemm_go<TA, TB, true, MT_, NT_>(g, M, N, K, alpha, A, lda, B, ldb, beta, C, ldc, gamma, colmap,     \
-                                                ncol_dev, rowscale, kchunk, W, cnt, st);                                       \
+                                                ncol_dev, rowscale, lower, kchunk, W, cnt, st);                                       \
     else sgemm_go<TA, TB, false, MT_, NT_>(g, M, N, K, alpha, A, lda, B, ldb, beta, C, ldc, gamma, colmap, ncol_dev, \
-                                           rowscale, kchunk, W, nullptr, st);                                                  \
+                                           rowscale, lower, kchunk, W, nullptr, st);                                                  \
   }
   if (TA) {
     QX_SG(2, 2) else QX_SG(2, 3) else QX_SG(2, 4) else QX_SG(2, 5)
@@ -800,8 +819,9 @@ void fp32_gemm_fallbacks_add(long n) { g_fp32_fallbacks.fetch_add(n); }
 template <typename T>
 int gemm(bool ta, bool tb, int M, int N, int K, T alpha, const T *A, long lda, const T *B, long ldb, T beta, T *C,
          long ldc, int gamma, const int *colmap, const int *ncol_dev, cudaStream_t st, void *ws, size_t ws_bytes,
-         const T *rowscale, void *pad, size_t pad_bytes) {
+         const T *rowscale, void *pad, size_t pad_bytes, const int *lower) {
   if (M <= 0 || N <= 0) return 0;
+  if (lower && (beta != (T)0 || colmap || ncol_dev)) { set_error("gemm: a mask needs beta = 0 and all columns"); return 1; }
   // the workspace opens with the per-tile counters of k_sgemm's split K
   int *cnt = nullptr;
   if (ws && ws_bytes > GEMM_COUNTER_BYTES) {
@@ -818,8 +838,11 @@ int gemm(bool ta, bool tb, int M, int N, int K, T alpha, const T *A, long lda, c
   if (rowscale && beta != (T)0) { set_error("gemm: a row scale needs beta = 0"); return 1; }
   if (sizeof(T) == sizeof(float) && !colmap && !ncol_dev && K > 0 && !small) {
     const int r = tc_gemm(ta, tb, M, N, K, (float)alpha, (const float *)A, lda, (const float *)B, ldb, (float)beta,
-                          (float *)C, ldc, gamma, st, ws, ws_bytes, (const float *)rowscale, pad, pad_bytes);
-    if (r == 0) return 0;
+                          (float *)C, ldc, gamma, st, ws, ws_bytes, (const float *)rowscale, pad, pad_bytes, lower);
+    if (r == 0 || r == -2) {   // -2: launched, the mask not applied
+      if (r) mask_lower(M, N, C, ldc, lower, st);
+      return 0;
+    }
     if (r > 0) {
       set_error("tensor-core GEMM launch failed: %s", cudaGetErrorString(cudaGetLastError()));
       return 2;
@@ -844,6 +867,7 @@ int gemm(bool ta, bool tb, int M, int N, int K, T alpha, const T *A, long lda, c
                                      ws_bytes, st);
     if (r) return r;
     if (rowscale) scale_rows<T>(M, N, C, ldc, rowscale, colmap, ncol_dev, st);
+    if (lower) mask_lower(M, N, C, ldc, lower, st);
     return 0;
   }
   if (sizeof(T) == sizeof(float) && !(ta && tb) && sgemm_enabled()) {
@@ -851,13 +875,13 @@ int gemm(bool ta, bool tb, int M, int N, int K, T alpha, const T *A, long lda, c
     float *Cf = (float *)C;
     if (ta)
       sgemm_launch<true, false>(M, N, K, (float)alpha, Af, lda, Bf, ldb, (float)beta, Cf, ldc, gamma, colmap, ncol_dev,
-                                rs, ws, ws_bytes, cnt, st);
+                                rs, lower, ws, ws_bytes, cnt, st);
     else if (tb)
       sgemm_launch<false, true>(M, N, K, (float)alpha, Af, lda, Bf, ldb, (float)beta, Cf, ldc, gamma, colmap, ncol_dev,
-                                rs, ws, ws_bytes, cnt, st);
+                                rs, lower, ws, ws_bytes, cnt, st);
     else
       sgemm_launch<false, false>(M, N, K, (float)alpha, Af, lda, Bf, ldb, (float)beta, Cf, ldc, gamma, colmap,
-                                 ncol_dev, rs, ws, ws_bytes, cnt, st);
+                                 ncol_dev, rs, lower, ws, ws_bytes, cnt, st);
     return 0;
   }
   dim3 g((M + BM - 1) / BM, (N + BN - 1) / BN);
@@ -882,15 +906,16 @@ int gemm(bool ta, bool tb, int M, int N, int K, T alpha, const T *A, long lda, c
   else if (tb) launch<T, false, true>(g, M, N, K, alpha, A, lda, B, ldb, beta, C, ldc, gamma, colmap, ncol_dev, nsplit, kchunk, W, st);
   else launch<T, false, false>(g, M, N, K, alpha, A, lda, B, ldb, beta, C, ldc, gamma, colmap, ncol_dev, nsplit, kchunk, W, st);
   if (rowscale) scale_rows<T>(M, N, C, ldc, rowscale, colmap, ncol_dev, st);
+  if (lower) mask_lower(M, N, C, ldc, lower, st);
   return 0;
 }
 
 template int gemm<float>(bool, bool, int, int, int, float, const float *, long, const float *, long, float, float *,
                          long, int, const int *, const int *, cudaStream_t, void *, size_t, const float *, void *,
-                         size_t);
+                         size_t, const int *);
 template int gemm<double>(bool, bool, int, int, int, double, const double *, long, const double *, long, double,
                           double *, long, int, const int *, const int *, cudaStream_t, void *, size_t, const double *,
-                          void *, size_t);
+                          void *, size_t, const int *);
 
 }  // namespace qx
 

@@ -162,21 +162,23 @@ constexpr long GEMM_TILE_COUNTERS = GEMM_COUNTER_BYTES / sizeof(int);
 // column n to stored column colmap[n] of B and C; ncol_dev (device,
 // optional) bounds the number of columns.
 // ws/ws_bytes: optional split-K workspace (null: no split).
+// lower (optional, beta = 0): C(m, n) = 0 unless m < n and lower[n] != 0.
 template <typename T>
 int gemm(bool ta, bool tb, int M, int N, int K, T alpha, const T *A, long lda, const T *B, long ldb, T beta, T *C,
          long ldc, int gamma, const int *colmap, const int *ncol_dev, cudaStream_t st, void *ws = nullptr,
-         size_t ws_bytes = 0, const T *rowscale = nullptr, void *pad = nullptr, size_t pad_bytes = 0);
+         size_t ws_bytes = 0, const T *rowscale = nullptr, void *pad = nullptr, size_t pad_bytes = 0,
+         const int *lower = nullptr);
 
 void gemm_reduce_f32(bool ta, bool tb, int M, int N, int nsplit, float alpha, const float *A, long lda, const float *B,
                      long ldb, float beta, float *C, long ldc, int gamma, const float *W, cudaStream_t st,
-                     const float *rowscale = nullptr);
+                     const float *rowscale = nullptr, const int *lower = nullptr);
 
 // qx_tcgemm.cu: tcgen05 3xTF32 GEMM with gemm<float>'s semantics (no column
-// map).  Returns 0 launched, -1 operands unsuitable (use the CUDA-core
-// kernel), > 0 launch error.
+// map).  Returns 0 launched (-2: launched, the mask `lower` left to the
+// caller), -1 operands unsuitable (use the CUDA-core kernel), > 0 launch error.
 int tc_gemm(bool ta, bool tb, int M, int N, int K, float alpha, const float *A, long lda, const float *B, long ldb,
             float beta, float *C, long ldc, int gamma, cudaStream_t st, void *ws, size_t ws_bytes, const float *rowscale = nullptr, void *pad = nullptr,
-            size_t pad_bytes = 0);
+            size_t pad_bytes = 0, const int *lower = nullptr);
 bool tc_enabled();
 // Copies `rows` rows of `inner` floats from stride ld to stride ldp (the
 // tensor maps' 16-byte row-stride rule wants ldp a multiple of four).

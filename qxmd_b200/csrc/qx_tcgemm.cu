@@ -633,13 +633,13 @@ void pad_rows_f32(const float *src, long ld, long inner, long rows, float *dst, 
 }
 
 // Tensor-core FP32 GEMM with the semantics of gemm<float> (no column map).
-// Returns 0 when launched, -1 when the operands do not meet the TMA rules
-// (the caller then uses the CUDA-core kernel), >0 on error.  pad (optional,
+// Returns 0 when launched (-2 with the mask `lower` left to the caller), -1
+// when the operands do not meet the TMA rules (the caller then uses the CUDA-core kernel), >0 on error.  pad (optional,
 // pad_bytes): room to restage an operand whose row stride is not a multiple
 // of four floats (or whose base is not 16-byte aligned) before the launch.
 int tc_gemm(bool ta, bool tb, int M, int N, int K, float alpha, const float *A, long lda, const float *B, long ldb,
             float beta, float *C, long ldc, int gamma, cudaStream_t st, void *ws, size_t ws_bytes,
-            const float *rowscale, void *pad, size_t pad_bytes) {
+            const float *rowscale, void *pad, size_t pad_bytes, const int *lower) {
   using tc::BM;
   using tc::BK;
   if (!tc::enabled() || M <= 0 || N <= 0 || K <= 0) return -1;
@@ -728,8 +728,8 @@ int tc_gemm(bool ta, bool tb, int M, int N, int K, float alpha, const float *A, 
   if (rc) return rc;
   if (nsplit > 1)
     gemm_reduce_f32(ta, tb, M, N, nsplit, alpha, A, lda, B, ldb, beta, C, ldc, gamma, (const float *)ws, st,
-                    rowscale);
-  return 0;
+                    rowscale, lower);
+  return lower && nsplit <= 1 ? -2 : 0;
 }
 
 // Error code recorded by a tensor-core GEMM whose wait timed out (0: none);
