@@ -205,18 +205,29 @@ __device__ __forceinline__ void split1(float x, float &h, float &l) {
   h = tf32_rn(x);
   l = x - h;
 }
+// Every load of a thread goes out before its first store (the compiler cannot
+// move a load above a store to the same tile): one by one, each waited a
+// shared-memory latency, and that chain in the two warps of the B split was
+// what bounded a k-block (Si512, 48424 x 1100 x 2048 and 2048 x 1100 x 48424:
+// 2.04 and 1.80 -> 1.67 and 1.49 ms, with the accumulators out of the split
+// warps' registers).
 template <int N16, int STRIDE>
 __device__ __forceinline__ void split_tf32(float4 *hi, float4 *lo, int t) {
+  constexpr int U = (N16 + STRIDE - 1) / STRIDE;
+  float4 x[U];
 #pragma unroll
-  for (int i = t; i < N16; i += STRIDE) {
-    const float4 x = hi[i];
+  for (int u = 0; u < U; ++u)
+    if (N16 % STRIDE == 0 || t + u * STRIDE < N16) x[u] = hi[t + u * STRIDE];
+#pragma unroll
+  for (int u = 0; u < U; ++u) {
+    if (N16 % STRIDE != 0 && t + u * STRIDE >= N16) break;
     float4 h, l;
-    split1(x.x, h.x, l.x);
-    split1(x.y, h.y, l.y);
-    split1(x.z, h.z, l.z);
-    split1(x.w, h.w, l.w);
-    hi[i] = h;
-    lo[i] = l;
+    split1(x[u].x, h.x, l.x);
+    split1(x[u].y, h.y, l.y);
+    split1(x[u].z, h.z, l.z);
+    split1(x[u].w, h.w, l.w);
+    hi[t + u * STRIDE] = h;
+    lo[t + u * STRIDE] = l;
   }
 }
 
@@ -352,27 +363,6 @@ __global__ void __launch_bounds__(NTHREADS, 1)
     // the drain of accumulator j overlaps the MMAs of k-block j + 1.
     const bool drains = warp < 6;
     const int quad = warp & 3;
-    float acc[BN];
-#pragma unroll
-    for (int j = 0; j < BN; ++j) acc[j] = 0.f;
-    // add the k-block held in accumulator (j & 1) to acc and release it
-    auto drain = [&](int j) {
-      const int ab = j & 1;
-      const bool got = mbar_wait(&accf[ab], (j >> 1) & 1, 5);
-      if (!got) abort_flag = 1;
-      asm volatile("tcgen05.fence::after_thread_sync;");
-      const uint32_t base = tmem + ((uint32_t)(quad * 32) << 16) + (uint32_t)(ab * G::ACC_STRIDE);
-#pragma unroll
-      for (int c = 0; c < BN / 16; ++c) {
-        uint32_t r[16];
-        TMEM_LD16(base + (uint32_t)(c * 16), r);
-        asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-#pragma unroll
-        for (int q = 0; q < 16; ++q) acc[c * 16 + q] += __uint_as_float(r[q]);
-      }
-      asm volatile("tcgen05.fence::before_thread_sync;");
-      mbar_arrive(&acce[ab]);
-    };
     if (!drains && !ATM) {
       const int t = threadIdx.x - 192;   // 0 .. NSPLIT_T - 1 (warps 6-11)
       for (int kb = 0; kb < nkb; ++kb) {
@@ -433,12 +423,41 @@ __global__ void __launch_bounds__(NTHREADS, 1)
         mbar_arrive(&conv[s]);
       }
     } else {
+      // acc only lives in this branch: declared before it, its registers stay
+      // taken in the split warps too, whose loads then spill
+      float acc[BN];
+#pragma unroll
+      for (int j = 0; j < BN; ++j) acc[j] = 0.f;
+      // add the k-block held in accumulator (j & 1) to acc and release it
+      auto drain = [&](int j) {
+        const int ab = j & 1;
+        const bool got = mbar_wait(&accf[ab], (j >> 1) & 1, 5);
+        if (!got) abort_flag = 1;
+        asm volatile("tcgen05.fence::after_thread_sync;");
+        const uint32_t base = tmem + ((uint32_t)(quad * 32) << 16) + (uint32_t)(ab * G::ACC_STRIDE);
+        // two chunks of 16 columns at a time (at 128 columns that would spill)
+        constexpr int CU = BN <= 96 ? 2 : 1;
+#pragma unroll
+        for (int c = 0; c < BN / 16; c += CU) {
+          uint32_t r[CU][16];
+#pragma unroll
+          for (int u = 0; u < CU; ++u)
+            if (c + u < BN / 16) TMEM_LD16(base + (uint32_t)((c + u) * 16), r[u]);
+          asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+          for (int u = 0; u < CU; ++u)
+            if (c + u < BN / 16) {
+#pragma unroll
+              for (int q = 0; q < 16; ++q) acc[(c + u) * 16 + q] += __uint_as_float(r[u][q]);
+            }
+        }
+        asm volatile("tcgen05.fence::before_thread_sync;");
+        mbar_arrive(&acce[ab]);
+      };
       for (int kb = 0; kb < nkb; ++kb) {
         if (__any_sync(0xffffffffu, abort_flag != 0)) break;   // warp-uniform: TMEM loads are .sync.aligned
         drain(kb);
       }
-    }
-    if (drains) {
       // ---------------- epilogue ----------------
       const bool direct = (p.W == nullptr);
       if (direct && p.gamma) {
