@@ -808,16 +808,36 @@ static bool plane_enabled() {
   return !(e && e[0] == '0');
 }
 
-// Forward z pass one sphere column a thread (k_zcols_fwd) for columns of at
-// most 32 points, where it measured faster than the shared-memory pass (the
-// 48-cell batch, z lengths 21-27: 9365 -> 9735 cell-iter/s); at 54 points
-// (Si64) it measured 2.5 % slower.  At 96 (Si512) k_zcols_fwd2 takes 820 us
-// where the shared-memory pass took 960.  QX_ZCOLS_FWD=0 / 1 forces either (read at
-// every call).
-static bool zcols_fwd_enabled(int k3) {
-  const char *e = getenv("QX_ZCOLS_FWD");
-  if (e && (e[0] == '0' || e[0] == '1')) return e[0] == '1';
-  return k3 <= 32 || k3 == 96;
+// The z passes of a chunk of band pairs: a sphere column's line in registers
+// where the length is compiled for (FP64: and the sphere spans half the grid
+// at most), else the shared-memory stages.  In registers against stages, whole
+// H|psi>, 160 / 16 / 2 bands: FP32 forward 27^3 37.0 / 25.8 / 26.3 -> 34.1 /
+// 23.8 / 24.3 us, 40^3 53.6 / 29.3 / 29.3 -> 47.2 / 27.1 / 27.1, 54^3 105 / 58 /
+// 44 -> 99 / 53 / 43, 60^3 123 / 39 / 35 -> 106 / 35 / 32; FP64 both 27^3 54.0
+// / 36.5 / 36.4 -> 43.7 / 36.2 / 36.1, 40^3 111 / 45 / 37 -> 98 / 38 / 36, 54^3
+// 286 / 64 / 57 -> 265 / 64 / 54, 60^3 315 / 62 / 44 -> 268 / 55 / 39.
+template <typename T>
+static void z_backward(const PipeParams &P, int npl, const T *cin, long ldc, const Bufs<T> &bf, const FftTabs<T> &g3,
+                       cudaStream_t st) {
+  if constexpr (sizeof(T) == sizeof(float)) {
+    if (launch_zcols_inv_f32(P, npl, cin, ldc, bf.bufA, st) == 0) return;
+  } else {
+    if (launch_zcols_f64(P, npl, cin, ldc, bf.bufA, nullptr, st) == 0) return;
+  }
+  k_zinv<T><<<dim3(P.P2, npl), QX_THREADS, fft_smem(P.L3, P.P1 | 1, sizeof(typename c2t<T>::type)), st>>>(P, cin, ldc,
+                                                                                                       bf.bufA, g3);
+  note_launch();
+}
+template <typename T>
+static void z_forward(const PipeParams &P, int npl, const Bufs<T> &bf, const FftTabs<T> &g3, cudaStream_t st) {
+  if constexpr (sizeof(T) == sizeof(float)) {
+    if (launch_zcols_fwd_f32(P, npl, bf.bufA, bf.zsph, st) == 0) return;
+  } else {
+    if (launch_zcols_f64(P, npl, nullptr, 0, bf.bufA, bf.zsph, st) == 0) return;
+  }
+  k_zfwd<T><<<dim3(P.P2, npl), QX_THREADS, fft_smem(P.L3, P.P1 | 1, sizeof(typename c2t<T>::type)), st>>>(P, bf.bufA,
+                                                                                                       bf.zsph, g3);
+  note_launch();
 }
 
 // The sums of the chunk's pairs over every atom's points.  Where that fills
@@ -856,17 +876,8 @@ int launch_hpsi_chunk(const Plan &pl, const PipeParams &P, int npl, const T *cin
   const size_t cs = sizeof(C);
   Bufs<T> &bf = pl.bufs<T>();
   const FftTabs<T> g1 = tabs<T>(pl, 0), g2 = tabs<T>(pl, 1), g3 = tabs<T>(pl, 2);
-  dim3 gz(P.P2, npl);
-  const size_t smz = fft_smem(P.L3, P.P1 | 1, cs);
-  const bool zc = sizeof(T) == sizeof(float) &&
-                  launch_zcols_inv_f32(P, npl, (const float *)cin, ldc, (float2 *)bf.bufA, st) == 0;
-  if (!zc) { k_zinv<T><<<gz, QX_THREADS, smz, st>>>(P, cin, ldc, bf.bufA, g3); note_launch(); }
-  auto zfwd = [&]() {
-    if (sizeof(T) == sizeof(float) && zcols_fwd_enabled(P.k3) &&
-        launch_zcols_fwd_f32(P, npl, (const float2 *)bf.bufA, (float2 *)bf.zsph, st) == 0)
-      return;
-    k_zfwd<T><<<gz, QX_THREADS, smz, st>>>(P, bf.bufA, bf.zsph, g3); note_launch();
-  };
+  z_backward(P, npl, cin, ldc, bf, g3, st);
+  auto zfwd = [&]() { z_forward(P, npl, bf, g3, st); };
   dim3 gy(P.k3, npl);
   const size_t smy = fft_smem(P.L2, P.P1, cs);
   if (nlmode != 2 && pl.use_plane && plane_enabled() && launch_plane(P, npl, bf.bufA, bf.vloc, st) == 0) {
@@ -917,11 +928,7 @@ int launch_rho_chunk(const Plan &pl, const PipeParams &P, int npl, const T *cin,
   const size_t cs = sizeof(C);
   Bufs<T> &bf = pl.bufs<T>();
   const FftTabs<T> g1 = tabs<T>(pl, 0), g2 = tabs<T>(pl, 1), g3 = tabs<T>(pl, 2);
-  dim3 gz(P.P2, npl);
-  if (!(sizeof(T) == sizeof(float) &&
-        launch_zcols_inv_f32(P, npl, (const float *)cin, ldc, (float2 *)bf.bufA, st) == 0)) {
-    k_zinv<T><<<gz, QX_THREADS, fft_smem(P.L3, P.P1 | 1, cs), st>>>(P, cin, ldc, bf.bufA, g3); note_launch();
-  }
+  z_backward(P, npl, cin, ldc, bf, g3, st);
   if (sizeof(T) == sizeof(float) && pl.use_plane && plane_enabled() && bf.rho_part &&
       launch_rho_plane_f32(P, npl, (const float2 *)bf.bufA, wocc, bf.rho_part, rho, accumulate, st) == 0)
     return 0;
@@ -943,11 +950,7 @@ int launch_fnl_r_chunk(const Plan &pl, const PipeParams &P, int npl, const T *ci
   const size_t cs = sizeof(C);
   Bufs<T> &bf = pl.bufs<T>();
   const FftTabs<T> g1 = tabs<T>(pl, 0), g2 = tabs<T>(pl, 1), g3 = tabs<T>(pl, 2);
-  dim3 gz(P.P2, npl);
-  if (!(sizeof(T) == sizeof(float) &&
-        launch_zcols_inv_f32(P, npl, (const float *)cin, ldc, (float2 *)bf.bufA, st) == 0)) {
-    k_zinv<T><<<gz, QX_THREADS, fft_smem(P.L3, P.P1 | 1, cs), st>>>(P, cin, ldc, bf.bufA, g3); note_launch();
-  }
+  z_backward(P, npl, cin, ldc, bf, g3, st);
   bool plane = false;
   if constexpr (sizeof(T) == sizeof(float))
     plane = pl.use_plane && plane_enabled() &&

@@ -30,6 +30,18 @@ static int zcols_dispatch(const PipeParams &P, int npl, const float *cin, long l
   }
 }
 
+int launch_zcols_f64(const PipeParams &P, int npl, const double *cin, long ldc, double2 *bufA, double2 *zsph,
+                     cudaStream_t st) {
+  if (!zcols_enabled() || P.ncol <= 0) return -1;
+  switch (P.k3) {
+#define QX_CASE(N) \
+  case N: return zcols64_launch<N>(P, npl, cin, ldc, bufA, zsph, st);
+    QX_ZCOLS64_LENGTHS(QX_CASE)
+#undef QX_CASE
+    default: return -1;
+  }
+}
+
 int launch_zcols_inv_f32(const PipeParams &P, int npl, const float *cin, long ldc, float2 *bufA, cudaStream_t st) {
   return zcols_dispatch(P, npl, cin, ldc, bufA, nullptr, nullptr, true, st);
 }

@@ -53,6 +53,11 @@ int zcols2_launch(const PipeParams &P, int npl, const float *cin, long ldc, floa
   X(20, 20) X(21, 21) X(24, 24) X(25, 25) X(27, 27) X(30, 30) X(32, 32) X(36, 36) X(40, 40) X(42, 42) \
   X(48, 48) X(54, 54) X(60, 60) X(64, 64)                                                             \
   X(24, 25) X(25, 24) X(25, 27) X(27, 25) X(42, 21) X(54, 24) X(54, 25) X(54, 27)
+#define QX_ZCOLS64_LENGTHS(X) X(20) X(21) X(24) X(25) X(27) X(30) X(32) X(36) X(40) X(42) X(48) X(54) X(60) X(64)
+// cin: the backward pass into bufA; null: the forward pass into zsph
+template <int N>
+int zcols64_launch(const PipeParams &P, int npl, const double *cin, long ldc, double2 *bufA, double2 *zsph,
+                   cudaStream_t st);
 template <int NX, int NY>
 int plane64_launch(const PipeParams &P, int npl, double2 *bufA, const double *vloc, cudaStream_t st);
 

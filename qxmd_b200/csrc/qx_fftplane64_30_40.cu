@@ -6,4 +6,8 @@ QX_PLANE64_GRID(30, 30)
 QX_PLANE64_GRID(32, 32)
 QX_PLANE64_GRID(36, 36)
 QX_PLANE64_GRID(40, 40)
+QX_ZCOLS64_LENGTH(30)
+QX_ZCOLS64_LENGTH(32)
+QX_ZCOLS64_LENGTH(36)
+QX_ZCOLS64_LENGTH(40)
 }  // namespace qx

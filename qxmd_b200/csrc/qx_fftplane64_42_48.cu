@@ -5,4 +5,6 @@ namespace qx {
 QX_PLANE64_GRID(42, 42)
 QX_PLANE64_GRID(42, 21)
 QX_PLANE64_GRID(48, 48)
+QX_ZCOLS64_LENGTH(42)
+QX_ZCOLS64_LENGTH(48)
 }  // namespace qx

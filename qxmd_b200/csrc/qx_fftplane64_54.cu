@@ -6,4 +6,5 @@ QX_PLANE64_GRID(54, 54)
 QX_PLANE64_GRID(54, 24)
 QX_PLANE64_GRID(54, 25)
 QX_PLANE64_GRID(54, 27)
+QX_ZCOLS64_LENGTH(54)
 }  // namespace qx

@@ -4,4 +4,6 @@
 namespace qx {
 QX_PLANE64_GRID(60, 60)
 QX_PLANE64_GRID(64, 64)
+QX_ZCOLS64_LENGTH(60)
+QX_ZCOLS64_LENGTH(64)
 }  // namespace qx

@@ -12,13 +12,13 @@
 // us, 40^3 192 / 49 / 38 -> 124 / 37 / 33, 54^3 392 / 63 / 45 -> 342 / 52 / 45,
 // 60^3 598 / 90 / 51 -> 440 / 77 / 49 with whole lines; leaving out what a
 // sphere of half the grid has zero (HALF) took H|psi> of Si64 (54^3, 160 bands,
-// both projector contractions included) from 410 to 292 us.  At 54 points registers allow three
-// CTAs of 128 threads a SM; the FP64 chains and instruction fetches bound it.
-// The z passes in the same form measured slower than the stage kernels (54^3,
-// 16 bands: 63 -> 69 us) and were left out.
+// both projector contractions included) from 410 to 292 us, and the z passes in
+// the same form to 267.  At 54 points registers allow three CTAs of 128 threads
+// a SM; the FP64 chains and instruction fetches bound it.
 #pragma once
 #include "qx_fftplane.h"
 #include "qx_regfft.cuh"
+#include "qx_zlines.cuh"
 
 namespace qx {
 namespace pl64 {
@@ -72,6 +72,8 @@ struct Line {
     rf::fft<double, SIGN, M>(u);
   }
 };
+
+constexpr int z_ctas(int n) { return n / lanes(n) <= 16 ? 8 : 6; }   // of 64 threads
 
 constexpr int plane_ld(int p1) { return p1 + (6 - p1 % 4) % 4; }
 
@@ -199,6 +201,61 @@ __global__ void __launch_bounds__(pl64::plane_threads(NX, NY), pl64::plane_ctas(
   }
 }
 
+// The z passes, one sphere column a line (see k_zcols_inv, k_zcols_fwd).
+constexpr int ZC64_T = 64;
+
+template <int N, bool HALF>
+__global__ void __launch_bounds__(ZC64_T, pl64::z_ctas(N)) k_zcols64_inv(PipeParams P, const double *__restrict__ cin,
+                                                                        long ldc, double2 *__restrict__ bufA) {
+  using Z = pl64::Line<N>;
+  int q = (int)((blockIdx.x * ZC64_T + threadIdx.x) / Z::L);
+  const int h = threadIdx.x % Z::L;
+  const int pl = blockIdx.y, p = P.pair0 + pl;
+  if (p >= (P.npair_dev ? *P.npair_dev : P.npair)) return;   // uniform in the block
+  const bool on = q < P.ncol;
+  q = min(q, P.ncol - 1);
+  const int bA = P.pairs[2 * p], bB = P.pairs[2 * p + 1];
+  const double *cA = cin + (long)bA * ldc;
+  const double *cB = bB >= 0 ? cin + (long)bB * ldc : cA;
+  constexpr int MB = line_mb<N, HALF>();
+  double2 x[Z::M] = {};
+  z_gather<double, Z::M, std::conditional_t<Z::L == 2, ZIn2<N, MB>, ZRows1<N, MB>>>(
+      cA, cB, bB >= 0, [&](auto ic) { return __ldg(P.col_ig + (Z::L * decltype(ic)::value + h) * P.ncol + q); },
+      [&](auto ic, double re, double im) { x[decltype(ic)::value] = make_double2(re, im); });
+  Z::template dit<+1, pl64::bound<N, MB>()>(x, h);
+  if (on) {
+    double2 *dst = bufA + (long)pl * N * P.P2 * P.P1 + P.col_ja[q];
+    rf::static_for<0, Z::M>([&](auto kc) {
+      constexpr int k = decltype(kc)::value;
+      dst[(long)(k + h * Z::M) * P.P2 * P.P1] = x[rf::out_pos(Z::M, k)];
+    });
+  }
+}
+
+template <int N, bool HALF>
+__global__ void __launch_bounds__(ZC64_T, pl64::z_ctas(N)) k_zcols64_fwd(PipeParams P,
+                                                                        const double2 *__restrict__ bufA,
+                                                                        double2 *__restrict__ zsph) {
+  using Z = pl64::Line<N>;
+  int q = (int)((blockIdx.x * ZC64_T + threadIdx.x) / Z::L);
+  const int h = threadIdx.x % Z::L;
+  const int pl = blockIdx.y, p = P.pair0 + pl;
+  if (p >= (P.npair_dev ? *P.npair_dev : P.npair)) return;   // uniform in the block
+  const bool on = q < P.ncol;
+  q = min(q, P.ncol - 1);
+  const double2 *src = bufA + (long)pl * N * P.P2 * P.P1 + P.col_ja[q];
+  double2 x[Z::M];
+#pragma unroll
+  for (int j = 0; j < Z::M; ++j) x[j] = src[(long)(Z::L * j + h) * P.P2 * P.P1];
+  Z::template dit<-1>(x, h);
+  if (!on) return;
+  constexpr int MB = line_mb<N, HALF>(), M = Z::M;
+  z_scatter<double, M, std::conditional_t<Z::L == 2, ZOut2<N, MB>, ZRows1<N, MB>>>(
+      zsph + (long)pl * (P.nplw + 1) * 2, P.inv_n,
+      [&](auto ic) { return __ldg(P.col_ig + (decltype(ic)::value + h * M) * P.ncol + q); },
+      [&](auto ic) { return x[rf::out_pos(M, decltype(ic)::value)]; });
+}
+
 template <int NX, int NY, bool HALF>
 static void plane64_go(const PipeParams &P, int npl, double2 *bufA, const double *vloc, cudaStream_t st) {
   constexpr size_t sm = sizeof(double2) * (size_t)NY * pl64::plane_ld(2 * line_mb<NX, HALF>() + 1);
@@ -220,7 +277,21 @@ int plane64_launch(const PipeParams &P, int npl, double2 *bufA, const double *vl
   return 0;
 }
 
+template <int N>
+int zcols64_launch(const PipeParams &P, int npl, const double *cin, long ldc, double2 *bufA, double2 *zsph,
+                   cudaStream_t st) {
+  if (P.m3 > line_mb<N, true>()) return -1;
+  dim3 g((pl64::lanes(N) * P.ncol + ZC64_T - 1) / ZC64_T, npl);
+  if (cin) k_zcols64_inv<N, true><<<g, ZC64_T, 0, st>>>(P, cin, ldc, bufA);
+  else k_zcols64_fwd<N, true><<<g, ZC64_T, 0, st>>>(P, bufA, zsph);
+  note_launch();
+  return 0;
+}
+
 #define QX_PLANE64_GRID(NX, NY) \
   template int plane64_launch<NX, NY>(const PipeParams &, int, double2 *, const double *, cudaStream_t);
+
+#define QX_ZCOLS64_LENGTH(N) \
+  template int zcols64_launch<N>(const PipeParams &, int, const double *, long, double2 *, double2 *, cudaStream_t);
 
 }  // namespace qx

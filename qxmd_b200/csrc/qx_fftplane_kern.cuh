@@ -18,6 +18,7 @@
 #pragma once
 #include "qx_fftplane.h"
 #include "qx_regfft.cuh"
+#include "qx_zlines.cuh"
 
 namespace qx {
 
@@ -525,26 +526,12 @@ __global__ void __launch_bounds__(ZC_T) k_zcols_inv(PipeParams P, const float *_
   if (p >= (P.npair_dev ? *P.npair_dev : P.npair) || q >= P.ncol) return;
   const int bA = P.pairs[2 * p], bB = P.pairs[2 * p + 1];
   const float *cA = cin + (long)bA * ldc;
-  const float *cB = bB >= 0 ? cin + (long)bB * ldc : nullptr;
+  const float *cB = bB >= 0 ? cin + (long)bB * ldc : cA;
   constexpr int MB = line_mb<N, HALF>();   // samples beyond it are zero
   float2 x[N];
-  auto load = [&](int i3) {
-    const int code = P.col_ig[i3 * P.ncol + q];
-    float2 z = make_float2(0.f, 0.f);
-    if (code != 0) {
-      const int ig = (code > 0 ? code : -code) - 1;
-      const float ra = cA[2 * ig], ia = ig ? cA[2 * ig + 1] : 0.f;
-      const float rb = cB ? cB[2 * ig] : 0.f, ib = (cB && ig) ? cB[2 * ig + 1] : 0.f;
-      if (code > 0) { z.x = ra - ib; z.y = ia + rb; }
-      else          { z.x = ra + ib; z.y = rb - ia; }
-    }
-    return z;
-  };
-  rf::static_for<0, MB + 1>([&](auto kc) {
-    constexpr int k = decltype(kc)::value;
-    x[k] = load(k);
-    if constexpr (k > 0) x[N - k] = load(N - k);
-  });
+  z_gather<float, N, ZRows1<N, MB>>(
+      cA, cB, bB >= 0, [&](auto ic) { return __ldg(P.col_ig + decltype(ic)::value * P.ncol + q); },
+      [&](auto ic, float re, float im) { x[decltype(ic)::value] = make_float2(re, im); });
   rf::fft_nz<float, +1, N, MB>(x);
   float2 *dst = bufA + (long)pl * N * P.P2 * P.P1 + P.col_ja[q];
   rf::static_for<0, N>([&](auto ic) {
@@ -565,29 +552,10 @@ __global__ void __launch_bounds__(ZC_T) k_zcols_fwd(PipeParams P, const float2 *
 #pragma unroll
   for (int i3 = 0; i3 < N; ++i3) x[i3] = src[(long)i3 * P.P2 * P.P1];
   rf::fft<float, -1, N>(x);
-  const float s = (float)P.inv_n;
-  float2 *Z = zsph + (long)pl * (P.nplw + 1) * 2;
-  auto store = [&](auto ic) {
-    constexpr int i3 = decltype(ic)::value;
-    const int code = P.col_ig[i3 * P.ncol + q];
-    if (code != 0) {
-      float2 z = x[out_pos(N, i3)];
-      z.x *= s;
-      z.y *= s;
-      if (code > 0) {
-        const int ig = code - 1;
-        Z[2 * ig] = z;
-        if (ig == 0) Z[1] = z;
-      } else {
-        Z[2 * (-code - 1) + 1] = z;
-      }
-    }
-  };
-  rf::static_for<0, line_mb<N, HALF>() + 1>([&](auto kc) {
-    constexpr int k = decltype(kc)::value;
-    store(rf::IC<k>{});
-    if constexpr (k > 0) store(rf::IC<N - k>{});
-  });
+  z_scatter<float, N, ZRows1<N, line_mb<N, HALF>()>>(
+      zsph + (long)pl * (P.nplw + 1) * 2, (float)P.inv_n,
+      [&](auto ic) { return __ldg(P.col_ig + decltype(ic)::value * P.ncol + q); },
+      [&](auto ic) { return x[out_pos(N, decltype(ic)::value)]; });
 }
 
 
@@ -595,36 +563,26 @@ __global__ void __launch_bounds__(ZC_T) k_zcols_fwd(PipeParams P, const float2 *
 // 2c and 2c + 1 own sphere z-column c, each gathers the coefficients of the
 // even or odd i3 and transforms them (H points), and the butterfly exchange
 // of k_plane2 completes the N-point transform.  Whole warps run (lanes past
-// the last column work on zeros and store nothing).
+// the last column repeat it and store nothing).
 template <int N, bool HALF>
 __global__ void __launch_bounds__(ZC_T) k_zcols_inv2(PipeParams P, const float *__restrict__ cin, long ldc,
                                                       float2 *__restrict__ bufA) {
   using rf::out_pos;
   constexpr int H = N / 2;
-  const int q = (int)((blockIdx.x * ZC_T + threadIdx.x) >> 1), h = threadIdx.x & 1;
+  int q = (int)((blockIdx.x * ZC_T + threadIdx.x) >> 1);
+  const int h = threadIdx.x & 1;
   const int pl = blockIdx.y, p = P.pair0 + pl;
   if (p >= (P.npair_dev ? *P.npair_dev : P.npair)) return;   // uniform in the block
   const bool on = q < P.ncol;
+  q = min(q, P.ncol - 1);
   const int bA = P.pairs[2 * p], bB = P.pairs[2 * p + 1];
   const float *cA = cin + (long)bA * ldc;
-  const float *cB = bB >= 0 ? cin + (long)bB * ldc : nullptr;
+  const float *cB = bB >= 0 ? cin + (long)bB * ldc : cA;
   constexpr int MB = line_mb<N, HALF>();   // samples beyond it are zero
-  float2 x[H];
-  rf::static_for<0, H>([&](auto jc) {
-    constexpr int j = decltype(jc)::value;
-    float2 z = make_float2(0.f, 0.f);
-    if constexpr (z2_kind<N, MB>(j) != Z2_NONE) {
-      const int code = on ? P.col_ig[(2 * j + h) * P.ncol + q] : 0;
-      if (code != 0) {
-        const int ig = (code > 0 ? code : -code) - 1;
-        const float ra = cA[2 * ig], ia = ig ? cA[2 * ig + 1] : 0.f;
-        const float rb = cB ? cB[2 * ig] : 0.f, ib = (cB && ig) ? cB[2 * ig + 1] : 0.f;
-        if (code > 0) { z.x = ra - ib; z.y = ia + rb; }
-        else          { z.x = ra + ib; z.y = rb - ia; }
-      }
-    }
-    x[j] = z;
-  });
+  float2 x[H] = {};
+  z_gather<float, H, ZIn2<N, MB>>(
+      cA, cB, bB >= 0, [&](auto ic) { return __ldg(P.col_ig + (2 * decltype(ic)::value + h) * P.ncol + q); },
+      [&](auto ic, float re, float im) { x[decltype(ic)::value] = make_float2(re, im); });
   rf::fft_nz<float, +1, H, z2_bound<N, MB>()>(x);
   pl2::dit_combine<+1, N>(x, h);
   if (on) {
@@ -638,43 +596,29 @@ __global__ void __launch_bounds__(ZC_T) k_zcols_inv2(PipeParams P, const float *
 
 // The forward z pass the same way: lane h of a column loads the samples 2j + h
 // of bufA and, after the exchange, scatters the rows k + h H inside the sphere
-// to zsph as k_zfwd does.  At Si512 (96 points, 1100 bands): 960 -> 820 us.
+// to zsph as k_zfwd does.
 template <int N, bool HALF>
 __global__ void __launch_bounds__(ZC_T) k_zcols_fwd2(PipeParams P, const float2 *__restrict__ bufA,
                                                      float2 *__restrict__ zsph) {
   using rf::out_pos;
   constexpr int H = N / 2, MB = line_mb<N, HALF>();
-  const int q = (int)((blockIdx.x * ZC_T + threadIdx.x) >> 1), h = threadIdx.x & 1;
+  int q = (int)((blockIdx.x * ZC_T + threadIdx.x) >> 1);
+  const int h = threadIdx.x & 1;
   const int pl = blockIdx.y, p = P.pair0 + pl;
   if (p >= (P.npair_dev ? *P.npair_dev : P.npair)) return;   // uniform in the block
   const bool on = q < P.ncol;
-  const float2 *src = bufA + (long)pl * N * P.P2 * P.P1 + (on ? P.col_ja[q] : 0);
+  q = min(q, P.ncol - 1);
+  const float2 *src = bufA + (long)pl * N * P.P2 * P.P1 + P.col_ja[q];
   float2 x[H];
 #pragma unroll
-  for (int j = 0; j < H; ++j) x[j] = on ? src[(long)(2 * j + h) * P.P2 * P.P1] : make_float2(0.f, 0.f);
+  for (int j = 0; j < H; ++j) x[j] = src[(long)(2 * j + h) * P.P2 * P.P1];
   rf::fft<float, -1, H>(x);
   pl2::dit_combine<-1, N>(x, h);
   if (!on) return;
-  const float s = (float)P.inv_n;
-  float2 *Z = zsph + (long)pl * (P.nplw + 1) * 2;
-  rf::static_for<0, H>([&](auto kc) {
-    constexpr int k = decltype(kc)::value;
-    if constexpr (k <= MB || H - k <= MB) {
-      const int code = (h ? H - k <= MB : k <= MB) ? P.col_ig[(k + h * H) * P.ncol + q] : 0;
-      if (code != 0) {
-        float2 z = x[out_pos(H, k)];
-        z.x *= s;
-        z.y *= s;
-        if (code > 0) {
-          const int ig = code - 1;
-          Z[2 * ig] = z;
-          if (ig == 0) Z[1] = z;
-        } else {
-          Z[2 * (-code - 1) + 1] = z;
-        }
-      }
-    }
-  });
+  z_scatter<float, H, ZOut2<N, MB>>(
+      zsph + (long)pl * (P.nplw + 1) * 2, (float)P.inv_n,
+      [&](auto ic) { return __ldg(P.col_ig + (decltype(ic)::value + h * H) * P.ncol + q); },
+      [&](auto ic) { return x[out_pos(H, decltype(ic)::value)]; });
 }
 
 template <int N>

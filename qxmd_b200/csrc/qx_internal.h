@@ -147,6 +147,9 @@ bool plane_length_supported(int k1, int k2);
 // FFTs of length k3); -1 when k3 has no specialised length.
 int launch_zcols_inv_f32(const PipeParams &P, int npl, const float *cin, long ldc, float2 *bufA, cudaStream_t st);
 int launch_zcols_fwd_f32(const PipeParams &P, int npl, const float2 *bufA, float2 *zsph, cudaStream_t st);
+// FP64: backward into bufA (cin) or forward into zsph (cin null).
+int launch_zcols_f64(const PipeParams &P, int npl, const double *cin, long ldc, double2 *bufA, double2 *zsph,
+                     cudaStream_t st);
 template <typename T> size_t fft_smem_need(const Plan &pl);
 int init_fft_roots();
 
