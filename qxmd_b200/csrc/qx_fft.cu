@@ -984,8 +984,7 @@ int launch_full_fft(const Plan &pl, typename c2t<T>::type *g, int sign, double s
   const int nlines = pl.xlines<T>();
   const int nch = (k2 + nlines - 1) / nlines;
   const FftLen &L1 = pl.L[0], &L2 = pl.L[1], &L3 = pl.L[2];
-  // FP64 lines of at most 32 points: one line per thread in registers (the
-  // x pass applies the scale)
+  // FP64 lines of the compiled lengths in registers (the x pass applies the scale)
   auto lines = [&](int axis) {
     return sizeof(T) == sizeof(double) &&
            launch_full_lines_f64((double2 *)g, k1, k2, k3, axis, sign, scale, st) == 0;
