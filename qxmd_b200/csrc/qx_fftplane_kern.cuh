@@ -293,10 +293,18 @@ __global__ void __launch_bounds__(2 * N) k_plane2(PipeParams P, float2 *__restri
     rf::fft_nz<float, +1, H, z2_bound<N, MB>()>(x);
     pl2::dit_combine<+1, N>(x, h);
     const float *V = vloc + ((long)i3 * N + l) * N + h * H;
-    rf::static_for<0, H>([&](auto kc) {
-      constexpr int k = decltype(kc)::value, pk = out_pos(H, k);
-      const float vv = V[k];
-      x[pk] = make_float2(x[pk].x * vv, x[pk].y * vv);
+    // 16 bytes a load: every lane walks a half row of its own, so each load
+    // touches 32 lines of cache, and value by value they were a seventh of the
+    // pass (Si512: 2885 -> 2480 us)
+    static_assert(H % 4 == 0, "half rows start on 16 bytes");
+    rf::static_for<0, H / 4>([&](auto kc) {
+      constexpr int k = 4 * decltype(kc)::value;
+      constexpr int p0 = out_pos(H, k), p1 = out_pos(H, k + 1), p2 = out_pos(H, k + 2), p3 = out_pos(H, k + 3);
+      const float4 v = *reinterpret_cast<const float4 *>(V + k);
+      x[p0] = make_float2(x[p0].x * v.x, x[p0].y * v.x);
+      x[p1] = make_float2(x[p1].x * v.y, x[p1].y * v.y);
+      x[p2] = make_float2(x[p2].x * v.z, x[p2].y * v.z);
+      x[p3] = make_float2(x[p3].x * v.w, x[p3].y * v.w);
     });
     float2 u[H];
     pl2::dif_split<-1, N>(x, u, h);
