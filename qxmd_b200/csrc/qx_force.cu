@@ -106,7 +106,7 @@ void vloc_g(int n5, int natom, const int *ijk5, const int *ngabc, const double *
 // Blocks (atom, slice of the half sphere): the three components of floc over
 // the slice, G = 0 excluded, in part[(slice * natom + atom) * 3 + dim]; the
 // slices are added in order by k_floc_sum.  One block an atom left a 64-atom
-// cell on 64 SMs: 197 us at Si64, gathers in flight being the bound.
+// cell on 64 SMs: 197 us at Si64, gathers in flight being the bound (now 25).
 __global__ void __launch_bounds__(FT) k_floc(int n5, const int *__restrict__ ijk5, const int *__restrict__ ngabc,
                                              const double *__restrict__ gvec5, const double *__restrict__ svco,
                                              const int *__restrict__ ityp, const double2 *__restrict__ rhog,

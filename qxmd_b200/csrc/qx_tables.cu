@@ -188,7 +188,7 @@ __device__ __forceinline__ double kbr_poly(int c, double x, double y, double z) 
 
 // One block per (z plane of the box, atom).  The search is arithmetic on
 // registers, so the number of busy SMs bounds it: one block an atom kept a
-// 64-atom cell on 64 SMs (count 49 us, fill 198 us at Si64).
+// 64-atom cell on 64 SMs (at Si64 count 49 -> 7 us, fill 198 -> 40 us).
 __global__ void __launch_bounds__(KBR_T) k_kbr_count(KbrGeom G, const int *__restrict__ ityp,
                                                      const double *__restrict__ satm,
                                                      const double *__restrict__ rcut, int *__restrict__ cnt) {
