@@ -378,6 +378,8 @@ static int alloc_pipe(qx_ctx *c) {
   TRY(dalloc(c, &b.zsph, sizeof(C) * ch * (pl.nplw + 1) * 2));
   TRY(dalloc(c, &b.vloc, sizeof(T) * pl.n));
   CK(cudaMemset(b.vloc, 0, sizeof(T) * pl.n));
+  TRY(dalloc(c, &b.vloct, sizeof(T) * pl.n));
+  CK(cudaMemset(b.vloct, 0, sizeof(T) * pl.n));
   if (sizeof(T) == sizeof(float) && plane_length_supported(pl.k1, pl.k2))
     TRY(dalloc(c, &b.rho_part, sizeof(double) * RHO_GROUPS * pl.n));
   TRY(upload_tw<T>(c));
@@ -700,9 +702,9 @@ extern "C" int qx_set_glocal(qx_ctx *c, const double *glocal) {
   if (!c->d_glocal) TRY(dalloc(c, &c->d_glocal, sizeof(double) * c->pl.n));
   CK(cudaMemcpyAsync(c->d_glocal, glocal, sizeof(double) * c->pl.n, cudaMemcpyHostToDevice, c->st));
   if (c->prec == QX_PREC_FP64)
-    convert<double, double>(c->d_glocal, c->pl.b64.vloc, c->pl.n, c->st);
+    glocal_store<double>(c->d_glocal, c->pl.n, c->pl.b64.vloc, c->pl.b64.vloct, c->pl.k1, c->pl.k2, c->st);
   else
-    convert<double, float>(c->d_glocal, c->pl.b32.vloc, c->pl.n, c->st);
+    glocal_store<float>(c->d_glocal, c->pl.n, c->pl.b32.vloc, c->pl.b32.vloct, c->pl.k1, c->pl.k2, c->st);
   CKL();
   c->have_glocal = true;
   return QX_OK;
@@ -1839,11 +1841,11 @@ static int scf_potential(qx_ctx *c) {
   TRY(launch_full_fft<double>(c->pl, c->d_zg, +1, 1.0, c->st));
   const double rdelv = c->rvol / (double)n;
   if (c->prec == QX_PREC_FP64)
-    xc_glocal<double>(c->d_rho_in, c->d_vloc, c->d_zg, n, rdelv, c->d_glocal, c->pl.b64.vloc, c->d_part, c->d_sc + 1,
-                      c->st);
+    xc_glocal<double>(c->d_rho_in, c->d_vloc, c->d_zg, n, rdelv, c->d_glocal, c->pl.b64.vloc, c->pl.b64.vloct,
+                      c->pl.k1, c->pl.k2, c->d_part, c->d_sc + 1, c->st);
   else
-    xc_glocal<float>(c->d_rho_in, c->d_vloc, c->d_zg, n, rdelv, c->d_glocal, c->pl.b32.vloc, c->d_part, c->d_sc + 1,
-                     c->st);
+    xc_glocal<float>(c->d_rho_in, c->d_vloc, c->d_zg, n, rdelv, c->d_glocal, c->pl.b32.vloc, c->pl.b32.vloct,
+                     c->pl.k1, c->pl.k2, c->d_part, c->d_sc + 1, c->st);
   CKL();
   c->have_glocal = true;
   return 0;

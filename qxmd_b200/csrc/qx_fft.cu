@@ -880,7 +880,7 @@ int launch_hpsi_chunk(const Plan &pl, const PipeParams &P, int npl, const T *cin
   auto zfwd = [&]() { z_forward(P, npl, bf, g3, st); };
   dim3 gy(P.k3, npl);
   const size_t smy = fft_smem(P.L2, P.P1, cs);
-  if (nlmode != 2 && pl.use_plane && plane_enabled() && launch_plane(P, npl, bf.bufA, bf.vloc, st) == 0) {
+  if (nlmode != 2 && pl.use_plane && plane_enabled() && launch_plane(P, npl, bf.bufA, bf.vloct, st) == 0) {
     dim3 gu((P.nplw + 1 + 127) / 128, npl);
     zfwd();
     if (before_unpack) cudaStreamWaitEvent(st, before_unpack, 0);

@@ -96,23 +96,23 @@ bool plane_length_supported(int k1, int k2) {
 }
 
 // Launch the fused pass if this grid has a specialised length; -1 otherwise.
-int launch_plane(const PipeParams &P, int npl, float2 *bufA, const float *vloc, cudaStream_t st) {
+int launch_plane(const PipeParams &P, int npl, float2 *bufA, const float *vloct, cudaStream_t st) {
   if (P.P1 > P.k1 || P.P2 > P.k2) return -1;
   switch (plane_grid_key(P.k1, P.k2)) {
 #define QX_CASE(NX, NY) \
-  case plane_grid_key(NX, NY): return plane_launch<NX, NY>(P, npl, bufA, vloc, st);
+  case plane_grid_key(NX, NY): return plane_launch<NX, NY>(P, npl, bufA, vloct, st);
     QX_PLANE_GRIDS(QX_CASE)
 #undef QX_CASE
-    case plane_grid_key(96, 96): return plane2_launch<96>(P, npl, bufA, vloc, st);
+    case plane_grid_key(96, 96): return plane2_launch<96>(P, npl, bufA, vloct, st);
     default: return -1;
   }
 }
 
-int launch_plane(const PipeParams &P, int npl, double2 *bufA, const double *vloc, cudaStream_t st) {
+int launch_plane(const PipeParams &P, int npl, double2 *bufA, const double *vloct, cudaStream_t st) {
   if (P.P1 > P.k1 || P.P2 > P.k2) return -1;
   switch (plane_grid_key(P.k1, P.k2)) {
 #define QX_CASE(NX, NY) \
-  case plane_grid_key(NX, NY): return plane64_launch<NX, NY>(P, npl, bufA, vloc, st);
+  case plane_grid_key(NX, NY): return plane64_launch<NX, NY>(P, npl, bufA, vloct, st);
     QX_PLANE64_GRIDS(QX_CASE)
 #undef QX_CASE
     default: return -1;

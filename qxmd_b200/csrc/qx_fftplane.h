@@ -11,7 +11,7 @@ namespace qx {
 // One grid line per thread: planes of NX = k1 by NY = k2 points (each at
 // most 64), z columns of N = k3 points.
 template <int NX, int NY>
-int plane_launch(const PipeParams &P, int npl, float2 *bufA, const float *vloc, cudaStream_t st);
+int plane_launch(const PipeParams &P, int npl, float2 *bufA, const float *vloct, cudaStream_t st);
 // the passes around the real-space projectors: backward into R (nl null),
 // forward from R with the projectors' part (nl)
 template <int NX, int NY>
@@ -26,7 +26,7 @@ int zcols_launch(const PipeParams &P, int npl, const float *cin, long ldc, float
 
 // Two lanes a line (N = 96).
 template <int N>
-int plane2_launch(const PipeParams &P, int npl, float2 *bufA, const float *vloc, cudaStream_t st);
+int plane2_launch(const PipeParams &P, int npl, float2 *bufA, const float *vloct, cudaStream_t st);
 template <int N>
 int rho2_launch(const PipeParams &P, int npl, const float2 *bufA, const double *wocc, double *part, double *rho,
                 int accumulate, cudaStream_t st);
@@ -59,7 +59,7 @@ template <int N>
 int zcols64_launch(const PipeParams &P, int npl, const double *cin, long ldc, double2 *bufA, double2 *zsph,
                    cudaStream_t st);
 template <int NX, int NY>
-int plane64_launch(const PipeParams &P, int npl, double2 *bufA, const double *vloc, cudaStream_t st);
+int plane64_launch(const PipeParams &P, int npl, double2 *bufA, const double *vloct, cudaStream_t st);
 
 constexpr int plane_grid_key(int k1, int k2) { return k1 * 1024 + k2; }
 

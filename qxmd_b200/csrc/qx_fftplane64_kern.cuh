@@ -92,7 +92,7 @@ template <int N, int MB> constexpr int bound() {
 // HALF, the tile's columns and the sphere's rows as in k_plane.
 template <int NX, int NY, bool HALF>
 __global__ void __launch_bounds__(pl64::plane_threads(NX, NY), pl64::plane_ctas(NX, NY))
-    k_plane64(PipeParams P, double2 *__restrict__ bufA, const double *__restrict__ vloc) {
+    k_plane64(PipeParams P, double2 *__restrict__ bufA, const double *__restrict__ vloct) {
   using rf::out_pos;
   using X = pl64::Line<NX>;
   using Y = pl64::Line<NY>;
@@ -151,10 +151,10 @@ __global__ void __launch_bounds__(pl64::plane_threads(NX, NY), pl64::plane_ctas(
       x[j] = v;
     });
     X::template dit<+1, pl64::bound<NX, MBX>()>(x, h);
-    const double *V = vloc + ((long)i3 * NY + (on ? r : NY - 1)) * NX + h * X::M;
+    const double *V = vloct + ((long)i3 * NX + h * X::M) * NY + (on ? r : NY - 1);   // y fastest (see k_plane)
     rf::static_for<0, X::M>([&](auto kc) {
       constexpr int k = decltype(kc)::value, pk = out_pos(X::M, k);
-      const double vv = V[k];
+      const double vv = V[k * NY];
       x[pk] = make_double2(x[pk].x * vv, x[pk].y * vv);
     });
     X::template dif<-1>(x, u, h);
@@ -257,22 +257,22 @@ __global__ void __launch_bounds__(ZC64_T, pl64::z_ctas(N)) k_zcols64_fwd(PipePar
 }
 
 template <int NX, int NY, bool HALF>
-static void plane64_go(const PipeParams &P, int npl, double2 *bufA, const double *vloc, cudaStream_t st) {
+static void plane64_go(const PipeParams &P, int npl, double2 *bufA, const double *vloct, cudaStream_t st) {
   constexpr size_t sm = sizeof(double2) * (size_t)NY * pl64::plane_ld(2 * line_mb<NX, HALF>() + 1);
   static bool attr = false;
   if (!attr) {
     cudaFuncSetAttribute(k_plane64<NX, NY, HALF>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
     attr = true;
   }
-  k_plane64<NX, NY, HALF><<<dim3(P.k3, npl), pl64::plane_threads(NX, NY), sm, st>>>(P, bufA, vloc);
+  k_plane64<NX, NY, HALF><<<dim3(P.k3, npl), pl64::plane_threads(NX, NY), sm, st>>>(P, bufA, vloct);
 }
 
 // Spheres beyond half the grid (a density cutoff below four times the
 // wavefunction's) take the stage kernels.
 template <int NX, int NY>
-int plane64_launch(const PipeParams &P, int npl, double2 *bufA, const double *vloc, cudaStream_t st) {
+int plane64_launch(const PipeParams &P, int npl, double2 *bufA, const double *vloct, cudaStream_t st) {
   if (P.m1 > line_mb<NX, true>() || P.m2 > line_mb<NY, true>()) return -1;
-  plane64_go<NX, NY, true>(P, npl, bufA, vloc, st);
+  plane64_go<NX, NY, true>(P, npl, bufA, vloct, st);
   note_launch();
   return 0;
 }

@@ -95,7 +95,7 @@ __device__ __forceinline__ void plane_x_back(const float2 *row, float2 (&x)[NX])
 // outputs are the same bit for bit.
 template <int NX, int NY, int PL, int U, bool HALF>
 __global__ void __launch_bounds__(64 * U, (plane_minb(NX > NY ? NX : NY) + U - 1) / U)
-    k_plane(PipeParams P, float2 *__restrict__ bufA, const float *__restrict__ vloc, int npl) {
+    k_plane(PipeParams P, float2 *__restrict__ bufA, const float *__restrict__ vloct, int npl) {
   using rf::out_pos;
   using Rows = PlaneRows<NY, PL>;
   constexpr int MBX = line_mb<NX, HALF>(), MBY = line_mb<NY, HALF>(), PB = 2 * MBX + 1;
@@ -137,22 +137,16 @@ __global__ void __launch_bounds__(64 * U, (plane_minb(NX > NY ? NX : NY) + U - 1
       float2 x[NX];
       float2 *row = T + (rp * NY + r) * PB;
       plane_x_back<NX, MBX>(row, x);
-      const float *V = vloc + ((long)(i3b + rp) * NY + r) * NX;
+      // y fastest, so that the threads of a warp, one row each, read runs: in
+      // the grid's order every load touched 32 lines of cache, 8 cycles each
+      // (H|psi> of Si64: 104.9 -> 101.6 us)
+      const float *V = vloct + (long)(i3b + rp) * NX * NY + r;
       float2 y[NX];
-      if constexpr (NX % 2 == 0) {   // rows start on 8 bytes
-        rf::static_for<0, NX / 2>([&](auto ic) {
-          constexpr int i1 = 2 * decltype(ic)::value, q0 = out_pos(NX, i1), q1 = out_pos(NX, i1 + 1);
-          const float2 vv = *reinterpret_cast<const float2 *>(V + i1);
-          y[i1] = make_float2(x[q0].x * vv.x, x[q0].y * vv.x);
-          y[i1 + 1] = make_float2(x[q1].x * vv.y, x[q1].y * vv.y);
-        });
-      } else {
-        rf::static_for<0, NX>([&](auto ic) {
-          constexpr int i1 = decltype(ic)::value, q = out_pos(NX, i1);
-          const float vv = V[i1];
-          y[i1] = make_float2(x[q].x * vv, x[q].y * vv);
-        });
-      }
+      rf::static_for<0, NX>([&](auto ic) {
+        constexpr int i1 = decltype(ic)::value, q = out_pos(NX, i1);
+        const float vv = V[i1 * NY];
+        y[i1] = make_float2(x[q].x * vv, x[q].y * vv);
+      });
       rf::fft<float, -1, NX>(y);
       rf::static_for<0, MBX + 1>([&](auto kc) {
         constexpr int k = decltype(kc)::value;
@@ -230,7 +224,7 @@ template <int N, bool HALF> constexpr int plane2_pitch() { return (2 * line_mb<N
 
 template <int N, bool HALF>
 __global__ void __launch_bounds__(2 * N) k_plane2(PipeParams P, float2 *__restrict__ bufA,
-                                                 const float *__restrict__ vloc) {
+                                                 const float *__restrict__ vloct) {
   using rf::out_pos;
   constexpr int H = N / 2;
   const int i3 = blockIdx.x;
@@ -292,19 +286,13 @@ __global__ void __launch_bounds__(2 * N) k_plane2(PipeParams P, float2 *__restri
     });
     rf::fft_nz<float, +1, H, z2_bound<N, MB>()>(x);
     pl2::dit_combine<+1, N>(x, h);
-    const float *V = vloc + ((long)i3 * N + l) * N + h * H;
-    // 16 bytes a load: every lane walks a half row of its own, so each load
-    // touches 32 lines of cache, and value by value they were a seventh of the
-    // pass (Si512: 2885 -> 2480 us)
-    static_assert(H % 4 == 0, "half rows start on 16 bytes");
-    rf::static_for<0, H / 4>([&](auto kc) {
-      constexpr int k = 4 * decltype(kc)::value;
-      constexpr int p0 = out_pos(H, k), p1 = out_pos(H, k + 1), p2 = out_pos(H, k + 2), p3 = out_pos(H, k + 3);
-      const float4 v = *reinterpret_cast<const float4 *>(V + k);
-      x[p0] = make_float2(x[p0].x * v.x, x[p0].y * v.x);
-      x[p1] = make_float2(x[p1].x * v.y, x[p1].y * v.y);
-      x[p2] = make_float2(x[p2].x * v.z, x[p2].y * v.z);
-      x[p3] = make_float2(x[p3].x * v.w, x[p3].y * v.w);
+    // y fastest (see k_plane); in the grid's order, value by value, these loads
+    // were a seventh of the pass (Si512: 2885 -> 2480 us)
+    const float *V = vloct + ((long)i3 * N + h * H) * N + l;
+    rf::static_for<0, H>([&](auto kc) {
+      constexpr int k = decltype(kc)::value, pk = out_pos(H, k);
+      const float vv = V[k * N];
+      x[pk] = make_float2(x[pk].x * vv, x[pk].y * vv);
     });
     float2 u[H];
     pl2::dif_split<-1, N>(x, u, h);
@@ -843,7 +831,7 @@ int rho2_launch(const PipeParams &P, int npl, const float2 *bufA, const double *
 }
 
 template <int NX, int NY, int PL, int U, bool HALF>
-static void plane_go(const PipeParams &P, int npl, float2 *bufA, const float *vloc, cudaStream_t st) {
+static void plane_go(const PipeParams &P, int npl, float2 *bufA, const float *vloct, cudaStream_t st) {
   constexpr size_t sm = sizeof(float2) * U * PL * NY * (2 * line_mb<NX, HALF>() + 1);
   static bool attr = false;
   if (!attr) {
@@ -851,22 +839,22 @@ static void plane_go(const PipeParams &P, int npl, float2 *bufA, const float *vl
     attr = true;
   }
   k_plane<NX, NY, PL, U, HALF>
-      <<<dim3((P.k3 + PL - 1) / PL, (npl + U - 1) / U), 64 * U, sm, st>>>(P, bufA, vloc, npl);
+      <<<dim3((P.k3 + PL - 1) / PL, (npl + U - 1) / U), 64 * U, sm, st>>>(P, bufA, vloct, npl);
 }
 
 template <int NX, int NY>
-int plane_launch(const PipeParams &P, int npl, float2 *bufA, const float *vloc, cudaStream_t st) {
+int plane_launch(const PipeParams &P, int npl, float2 *bufA, const float *vloct, cudaStream_t st) {
   const bool half = P.m1 <= line_mb<NX, true>() && P.m2 <= line_mb<NY, true>();
   if (half) {
     // two planes a unit (warp w takes plane w's columns) where 32 lanes hold the columns
     if constexpr (2 * line_mb<NX, true>() + 1 <= 32) {
-      if (plane_pairs_enabled()) plane_go<NX, NY, 2, 2, true>(P, npl, bufA, vloc, st);
-      else plane_go<NX, NY, 1, 1, true>(P, npl, bufA, vloc, st);
+      if (plane_pairs_enabled()) plane_go<NX, NY, 2, 2, true>(P, npl, bufA, vloct, st);
+      else plane_go<NX, NY, 1, 1, true>(P, npl, bufA, vloct, st);
     } else {
-      plane_go<NX, NY, 1, 1, true>(P, npl, bufA, vloc, st);
+      plane_go<NX, NY, 1, 1, true>(P, npl, bufA, vloct, st);
     }
   } else {
-    plane_go<NX, NY, 1, 1, false>(P, npl, bufA, vloc, st);
+    plane_go<NX, NY, 1, 1, false>(P, npl, bufA, vloct, st);
   }
   note_launch();
   return 0;
@@ -897,19 +885,19 @@ int plane_r_launch(const PipeParams &P, int npl, float2 *bufA, float2 *R, const 
 }
 
 template <int N, bool HALF>
-static void plane2_go(const PipeParams &P, int npl, float2 *bufA, const float *vloc, cudaStream_t st) {
+static void plane2_go(const PipeParams &P, int npl, float2 *bufA, const float *vloct, cudaStream_t st) {
   constexpr size_t sm = sizeof(float2) * (size_t)N * plane2_pitch<N, HALF>();
   static bool attr = false;
   if (!attr) {
     cudaFuncSetAttribute(k_plane2<N, HALF>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
     attr = true;
   }
-  k_plane2<N, HALF><<<dim3(P.k3, npl), 2 * N, sm, st>>>(P, bufA, vloc);
+  k_plane2<N, HALF><<<dim3(P.k3, npl), 2 * N, sm, st>>>(P, bufA, vloct);
 }
 template <int N>
-int plane2_launch(const PipeParams &P, int npl, float2 *bufA, const float *vloc, cudaStream_t st) {
-  if (P.m1 <= line_mb<N, true>() && P.m2 <= line_mb<N, true>()) plane2_go<N, true>(P, npl, bufA, vloc, st);
-  else plane2_go<N, false>(P, npl, bufA, vloc, st);
+int plane2_launch(const PipeParams &P, int npl, float2 *bufA, const float *vloct, cudaStream_t st) {
+  if (P.m1 <= line_mb<N, true>() && P.m2 <= line_mb<N, true>()) plane2_go<N, true>(P, npl, bufA, vloct, st);
+  else plane2_go<N, false>(P, npl, bufA, vloct, st);
   note_launch();
   return 0;
 }

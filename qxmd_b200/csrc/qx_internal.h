@@ -49,6 +49,7 @@ struct Bufs {
   C *zsph = nullptr;       // [chunk][nplw+1][2]
   C *sumr = nullptr;       // [chunk][natom][4]
   T *vloc = nullptr;       // glocal(kfft0)
+  T *vloct = nullptr;      // the same with y fastest, [i3][i1][i2]: the plane kernels' threads own rows of x
   T *kb_vnl = nullptr;     // real-space projector values [npts][4]
   T *kb_pvnl = nullptr;    // the same in grid-point order (Plan::d_pt_off)
   T *kbg = nullptr;        // G-space projectors [nproj][nplwex]
@@ -131,8 +132,8 @@ int launch_full_lines_f64(double2 *g, int k1, int k2, int k3, int axis, int sign
 template <typename T> void set_fft_smem_limits(size_t bytes);
 // qx_fftplane.cu: fused y-x-y pass (k1 x k2 planes of a specialised shape,
 // QX_PLANE_GRIDS, QX_PLANE64_GRIDS); returns -1 when the grid is not covered.
-int launch_plane(const PipeParams &P, int npl, float2 *bufA, const float *vloc, cudaStream_t st);
-int launch_plane(const PipeParams &P, int npl, double2 *bufA, const double *vloc, cudaStream_t st);
+int launch_plane(const PipeParams &P, int npl, float2 *bufA, const float *vloct, cudaStream_t st);
+int launch_plane(const PipeParams &P, int npl, double2 *bufA, const double *vloct, cudaStream_t st);
 // The same passes split around the real-space projectors: nl null, backward
 // into R; else forward from R.  -1 when the grid is not covered.
 int launch_plane_r_f32(const PipeParams &P, int npl, float2 *bufA, float2 *R, const float *vloc,

@@ -70,12 +70,36 @@ __global__ void k_kerker(double2 *__restrict__ z, const double *__restrict__ g2,
   }
 }
 
+// Grid point m of the potential in the working precision, in both of its
+// layouts: as the grid is stored, and with y fastest.
+template <typename T>
+__device__ __forceinline__ void put_glocal(long m, T v, T *__restrict__ out, T *__restrict__ out_yt, int k1, int k2) {
+  out[m] = v;
+  const long q = m / k1, i3 = q / k2;
+  const int i1 = (int)(m - q * k1), i2 = (int)(q - i3 * k2);
+  out_yt[(i3 * k1 + i1) * k2 + i2] = v;
+}
+template <typename T>
+__global__ void k_glocal_store(const double *__restrict__ g, long n, T *__restrict__ out, T *__restrict__ out_yt,
+                               int k1, int k2) {
+  for (long m = blockIdx.x * (long)blockDim.x + threadIdx.x; m < n; m += (long)gridDim.x * blockDim.x)
+    put_glocal(m, (T)g[m], out, out_yt, k1, k2);
+}
+template <typename T>
+void glocal_store(const double *g, long n, T *out, T *out_yt, int k1, int k2, cudaStream_t st) {
+  k_glocal_store<T><<<(int)std::min<long>((n + 255) / 256, 148 * 16), 256, 0, st>>>(g, n, out, out_yt, k1, k2);
+  note_launch();
+}
+template void glocal_store<float>(const double *, long, float *, float *, int, int, cudaStream_t);
+template void glocal_store<double>(const double *, long, double *, double *, int, int, cudaStream_t);
+
 // PZ LDA on rho, glocal = vloc + Re(vh) + vxc; partial sums of
 // eps_xc*rho and vxc*rho (times rdelv).
 template <typename T>
 __global__ void __launch_bounds__(RB) k_xc_glocal(const double *__restrict__ rho, const double *__restrict__ vloc,
                                                   const double2 *__restrict__ vh, long n, double rdelv,
                                                   double *__restrict__ glocal, T *__restrict__ glocal_t,
+                                                  T *__restrict__ glocal_yt, int k1, int k2,
                                                   double *__restrict__ part) {
   __shared__ double red[RB / 32];
   const double pi4 = 12.56637061436;
@@ -104,7 +128,7 @@ __global__ void __launch_bounds__(RB) k_xc_glocal(const double *__restrict__ rho
     }
     const double g = vloc[m] + vh[m].x + vexc;
     glocal[m] = g;
-    glocal_t[m] = (T)g;
+    put_glocal(m, (T)g, glocal_t, glocal_yt, k1, k2);
     sx += eexc * rh;
     sv += vexc * rh;
   }
@@ -401,14 +425,14 @@ void kerker(double2 *z, const double *g2, long n, double q02, cudaStream_t st) {
 
 template <typename T>
 void xc_glocal(const double *rho, const double *vloc, const double2 *vh, long n, double rdelv, double *glocal,
-               T *glocal_t, double *part, double *out2, cudaStream_t st) {
-  k_xc_glocal<T><<<SCF_NBLK, RB, 0, st>>>(rho, vloc, vh, n, rdelv, glocal, glocal_t, part); note_launch();
+               T *glocal_t, T *glocal_yt, int k1, int k2, double *part, double *out2, cudaStream_t st) {
+  k_xc_glocal<T><<<SCF_NBLK, RB, 0, st>>>(rho, vloc, vh, n, rdelv, glocal, glocal_t, glocal_yt, k1, k2, part); note_launch();
   k_reduce<<<1, 64, 0, st>>>(part, SCF_NBLK, 2, 2, out2); note_launch();
 }
 template void xc_glocal<float>(const double *, const double *, const double2 *, long, double, double *, float *,
-                               double *, double *, cudaStream_t);
+                               float *, int, int, double *, double *, cudaStream_t);
 template void xc_glocal<double>(const double *, const double *, const double2 *, long, double, double *, double *,
-                                double *, double *, cudaStream_t);
+                                double *, int, int, double *, double *, cudaStream_t);
 
 void mix(double *rho_in, const double *rho_out, const double2 *dfilt, long n, double beta, double rdelv, double *part,
          double *out, cudaStream_t st) {

@@ -35,7 +35,10 @@ void hartree_g(double2 *z, const double *g2, long n, double half_vol, double *pa
 void kerker(double2 *z, const double *g2, long n, double q02, cudaStream_t st);
 template <typename T>
 void xc_glocal(const double *rho, const double *vloc, const double2 *vh, long n, double rdelv, double *glocal,
-               T *glocal_t, double *part, double *out2, cudaStream_t st);
+               T *glocal_t, T *glocal_yt, int k1, int k2, double *part, double *out2, cudaStream_t st);
+// The potential g into both working-precision layouts (Bufs::vloc, vloct).
+template <typename T>
+void glocal_store(const double *g, long n, T *out, T *out_yt, int k1, int k2, cudaStream_t st);
 void mix(double *rho_in, const double *rho_out, const double2 *dfilt, long n, double beta, double rdelv, double *part,
          double *out, cudaStream_t st);
 void band_energy(const double *w, const double *occ, int nb, double *out, cudaStream_t st);
