@@ -47,10 +47,9 @@ HPSI_PASS_DRAM_BYTES = 69974016
 # kernels): its DRAM traffic is a fraction of the algorithmic bytes because
 # the z-transformed planes stay in L2, so it is not HBM-bound; it is bound by
 # latency at low occupancy.
-PIPELINE_LIMITER = ("latency, not HBM: DRAM traffic is 0.17x the algorithmic bytes (the pruned transforms keep "
-                    "only the z-transformed planes); plane pass k_plane (two z planes a CTA) at 22.7% achieved "
-                    "occupancy (128 registers), 41.4% issue active, FMA pipe 36%, stalls led by long scoreboard, "
-                    "instruction fetch and wait")
+PIPELINE_LIMITER = ("instruction issue and fetch, not HBM: DRAM traffic (captured before the half-sphere forms) is "
+                    "0.17x the algorithmic bytes (the pruned transforms keep only the z-transformed planes); plane "
+                    "pass k_plane at 128 registers a thread, 16 warps a SM")
 # FP64 SCF iterations of the refinement sweep after the mixed solution converged
 REFINE_ITERS = 3
 # iteration caps of the Si512 run to self-consistency and of its FP64 sweep
