@@ -963,18 +963,21 @@ __global__ void __launch_bounds__(TRR_W * 32, 1)
     });
     __syncwarp();   // vsm, wsm are rewritten in the next step
   }
-  // the last 2 x 2 block
+  // The last 2 x 2 block, the buffers still by column parity: a last reflector
+  // with tau = 0 skips barriers (2) and (3), so slower warps may still read the
+  // other buffer.
   if (n >= 2) {
-    gather(n - 2, 0);
+    const int b = (n - 2) & 1;
+    gather(n - 2, b);
     __syncthreads();
     if (tid == 0) {
-      d[n - 2] = xs[0][n - 2];
-      e[n - 2] = xs[0][n - 1];
+      d[n - 2] = xs[b][n - 2];
+      e[n - 2] = xs[b][n - 1];
     }
   }
-  gather(n - 1, 1);
+  gather(n - 1, (n - 1) & 1);
   __syncthreads();
-  if (tid == 0) d[n - 1] = xs[1][n - 1];
+  if (tid == 0) d[n - 1] = xs[(n - 1) & 1][n - 1];
 }
 
 // Householder tridiagonalisation over the whole GPU for large n (one
