@@ -204,12 +204,14 @@ static int dalloc(qx_ctx *c, P **p, size_t bytes) {
   return 0;
 }
 
-// Captured SCF-iteration graphs hold the table pointers of their capture:
-// every call that replaces a table buffer drops them (the next iteration
-// captures again).
-static void drop_scf_graphs(qx_ctx *c) {
+// The captured graphs (SCF iterations, the one-rank CG loop) hold the table
+// pointers and sizes of their capture: every call that replaces a table buffer
+// drops them (the next iteration captures again).
+static void drop_graphs(qx_ctx *c) {
   for (auto &g : c->scf_graphs) cudaGraphExecDestroy(g.exec);
   c->scf_graphs.clear();
+  if (c->seq_exec) { cudaGraphExecDestroy(c->seq_exec); c->seq_exec = nullptr; }
+  if (c->seq_graph) { cudaGraphDestroy(c->seq_graph); c->seq_graph = nullptr; }
 }
 
 // Frees a context buffer that a new one replaces (a table that grew, a
@@ -221,9 +223,7 @@ static int dfree(qx_ctx *c, void *p) {
   if (!p) return 0;
   CK(cudaStreamSynchronize(c->st));
   if (c->st2) CK(cudaStreamSynchronize(c->st2));
-  drop_scf_graphs(c);
-  if (c->seq_exec) { cudaGraphExecDestroy(c->seq_exec); c->seq_exec = nullptr; }
-  if (c->seq_graph) { cudaGraphDestroy(c->seq_graph); c->seq_graph = nullptr; }
+  drop_graphs(c);
   auto it = std::find(c->allocs.begin(), c->allocs.end(), p);
   if (it != c->allocs.end()) c->allocs.erase(it);
   CK(cudaFree(p));
@@ -630,9 +630,7 @@ extern "C" int qx_create(qx_ctx **out, int precision, int k1, int k2, int k3, in
 extern "C" int qx_destroy(qx_ctx *c) {
   if (!c) return QX_OK;
   cudaStreamSynchronize(c->st);
-  for (auto &g : c->scf_graphs) cudaGraphExecDestroy(g.exec);
-  if (c->seq_exec) cudaGraphExecDestroy(c->seq_exec);
-  if (c->seq_graph) cudaGraphDestroy(c->seq_graph);
+  drop_graphs(c);
   if (c->cap_st) cudaStreamDestroy(c->cap_st);
   if (c->st2) cudaStreamSynchronize(c->st2);
   if (c->ev_fork) cudaEventDestroy(c->ev_fork);
@@ -739,7 +737,7 @@ extern "C" int qx_set_kb_g(qx_ctx *c, int nproj, const double *eqlmr, const doub
     c->kbgp = nullptr;
     c->kbgp_ld = 0;
     c->pl.nproj = nproj;
-    drop_scf_graphs(c);
+    drop_graphs(c);
     TRY(tcpad_reserve(c, (long)nproj + c->nb));
     if (c->prec == QX_PREC_FP64) { c->pl.b64.kbg = (double *)kbg; c->pl.b64.vclalp = (double *)vcl; }
     else {
@@ -834,7 +832,7 @@ extern "C" int qx_build_kb_g(qx_ctx *c, int natom, const int *ityp, const double
     TRY(dregrow(c, &proj, ts * (size_t)nproj * c->nb));
     TRY(dfree(c, c->kbgp));
     c->pl.nproj = nproj;
-    drop_scf_graphs(c);
+    drop_graphs(c);
     TRY(tcpad_reserve(c, (long)nproj + c->nb));
     c->kbgp = nullptr;
     c->kbgp_ld = 0;
@@ -963,7 +961,7 @@ extern "C" int qx_set_kb_r(qx_ctx *c, int natom, int lmx, const int *off, const 
   pl.npts = npts;
   pl.kb_lmx = lmx;
   pl.rdelv = rdelv;
-  drop_scf_graphs(c);
+  drop_graphs(c);
   // real-space line buffer and projection sums, per chunk
   const long ch = pl.chunk;
   if (c->prec == QX_PREC_FP64) {
@@ -1049,7 +1047,7 @@ extern "C" int qx_set_kb_r_builder(qx_ctx *c, int ntype, int lmx, int mxnl, cons
   }
   CK(cudaMemcpyAsync(c->d_kbr_poly, poly, sizeof(int) * nchan, cudaMemcpyHostToDevice, c->st));
   CK(cudaMemcpyAsync(pl.d_kb_clalp, clalp, sizeof(double) * lmx, cudaMemcpyHostToDevice, c->st));
-  drop_scf_graphs(c);
+  drop_graphs(c);
   c->kbr_geom = G;
   if (lmx != c->kbr_lmx) {   // table buffers sized per projector count: rebuilt at the next build
     c->kbr_cap = 0;
@@ -1177,7 +1175,7 @@ extern "C" int qx_build_kb_r(qx_ctx *c, int natom, const int *ityp, const double
   pl.natom = natom;
   pl.npts = total;
   pl.kb_lmx = c->kbr_lmx;
-  if (moved) drop_scf_graphs(c);
+  if (moved) drop_graphs(c);
   c->have_kbr = true;
   return QX_OK;
 }
@@ -2149,9 +2147,7 @@ static int replan_fft(qx_ctx *c, const FftLen L[3]) {
   }
   TRY(upload_tw<double>(c));
   set_fft_smem_limits<double>(need64);
-  drop_scf_graphs(c);
-  if (c->seq_exec) { cudaGraphExecDestroy(c->seq_exec); c->seq_exec = nullptr; }
-  if (c->seq_graph) { cudaGraphDestroy(c->seq_graph); c->seq_graph = nullptr; }
+  drop_graphs(c);
   CKL();
   return QX_OK;
 }
@@ -2272,8 +2268,7 @@ extern "C" int qx_autotune(qx_ctx *c, char *report, int report_len) {
              ms[1] * 1e3, c->pl.use_plane ? "fused planes" : "y/x passes");
     rep += buf;
   }
-  for (auto &g : c->scf_graphs) cudaGraphExecDestroy(g.exec);
-  c->scf_graphs.clear();
+  drop_graphs(c);
   if (report && report_len > 0) {
     strncpy(report, rep.c_str(), report_len - 1);
     report[report_len - 1] = 0;
