@@ -1310,7 +1310,8 @@ static int side_stream(qx_ctx *c) {
 }
 
 // QX_KB_STREAM=0 keeps the G-space KB contractions behind the FFT pipeline
-// on one stream (read at every call).
+// on one stream (read at every call; an SCF iteration replayed from its graph
+// keeps the setting of its capture).
 static bool kb_side_stream_enabled() {
   const char *v = getenv("QX_KB_STREAM");
   return !(v && v[0] == '0');
@@ -1618,10 +1619,10 @@ template <typename T>
 static int seq_graph(qx_ctx *c, const qx_cgparm *p, const CgParm &pm) {
   const Bufs<T> &b = c->pl.bufs<T>();
   const void *keyp[] = {c->psi, c->hpsi, c->snap, b.kbg, b.vclalp};
-  std::vector<char> key(sizeof(keyp) + sizeof(qx_cgparm) + 2 * sizeof(int));
+  const int extra[3] = {c->nlmode, c->pl.nproj, kb_side_stream_enabled() ? 1 : 0};
+  std::vector<char> key(sizeof(keyp) + sizeof(qx_cgparm) + sizeof(extra));
   memcpy(key.data(), keyp, sizeof(keyp));
   memcpy(key.data() + sizeof(keyp), p, sizeof(qx_cgparm));
-  const int extra[2] = {c->nlmode, c->pl.nproj};
   memcpy(key.data() + sizeof(keyp) + sizeof(qx_cgparm), extra, sizeof(extra));
   if (c->seq_exec && key == c->seq_key) return 0;
   if (c->seq_exec) { cudaGraphExecDestroy(c->seq_exec); c->seq_exec = nullptr; }

@@ -4,7 +4,7 @@ import numpy as np
 import pytest
 
 from qxmd_b200 import cell
-from qxmd_b200.lib import CgParm, Context, QX_NL_RSPACE, QX_PREC_FP64, QX_PREC_MIXED
+from qxmd_b200.lib import CgParm, Context, QX_NL_GSPACE, QX_NL_RSPACE, QX_PREC_FP64, QX_PREC_MIXED
 
 from gpu_util import need_gpu
 
@@ -59,3 +59,19 @@ def test_replaced_tables(si8, si8_psi, prec, how):
     for a, b in zip(got, ref):
         assert np.array_equal(a, b)
     assert not np.allclose(got[2], before[2], rtol=1e-4)
+
+
+def test_stream_switch(monkeypatch, si8, si8_psi):
+    """QX_KB_STREAM between sweeps of one context: the projectors beside the
+    transforms or behind them, to rounding (H psi of the entry sums the two
+    parts in another order)."""
+    need_gpu()
+    ctx = Context(si8, QX_PREC_FP64, QX_NL_GSPACE)
+    out = []
+    for mode in ("1", "0", "1"):
+        monkeypatch.setenv("QX_KB_STREAM", mode)
+        out.append(_sweep(ctx, si8_psi))
+    ctx.close()
+    for r in out[1:]:
+        for a, b in zip(r[:2], out[0][:2]):
+            assert np.max(np.abs(a - b)) < 1e-11
