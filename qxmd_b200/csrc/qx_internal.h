@@ -184,6 +184,7 @@ int tc_gemm(bool ta, bool tb, int M, int N, int K, float alpha, const float *A, 
             float beta, float *C, long ldc, int gamma, cudaStream_t st, void *ws, size_t ws_bytes, const float *rowscale = nullptr, void *pad = nullptr,
             size_t pad_bytes = 0, const int *lower = nullptr);
 bool tc_enabled();
+int tc_tile_default(long tm, int N);   // tm: row tiles of 128
 // Copies `rows` rows of `inner` floats from stride ld to stride ldp (the
 // tensor maps' 16-byte row-stride rule wants ldp a multiple of four).
 void pad_rows_f32(const float *src, long ld, long inner, long rows, float *dst, long ldp, cudaStream_t st);

@@ -619,6 +619,19 @@ bool tc_tile_valid(bool tb, int bn) {
   return tb ? (bn == 64 || bn == 96 || bn == 128) : (bn == 64 || bn == 80 || bn == 128);
 }
 
+// The width for K-major B when nothing was measured: 80, or 128 where that takes
+// at most three quarters of the waves (one CTA a SM, tm row tiles), since a
+// wave of 128 columns costs about 4/3 of one of 80.  Whole H|psi> with 80 / 128
+// columns for K P, by waves: 36 -> 24 (and 2 -> 1 for K^T C: Si512, 1100 bands)
+// 7987 / 6847 us, 4 -> 3 (13572 rows, 350 bands) 1085 / 1079, 3 -> 2 (10252,
+// 256) 202 / 203, 2 -> 1 (9316, 176) 135 / 128; where it saves fewer, 80 is
+// faster: 3 -> 3 (13572, 288) 889 / 896, 2 -> 2 (13134, 160) 164 / 170,
+// (10252, 160) 130 / 133, 1 -> 1 (9316, 160; K^T C too) 113 / 122.
+int tc_tile_default(long tm, int N) {
+  const long w80 = (tm * ((N + 79) / 80) + 147) / 148, w128 = (tm * ((N + 127) / 128) + 147) / 148;
+  return 4 * w128 <= 3 * w80 ? 128 : 80;
+}
+
 namespace tc {
 // Rows of `inner` floats, `ld` apart, copied to rows `ldp` apart (ldp a
 // multiple of 4): an operand whose row stride breaks the 16-byte rule of the
@@ -690,12 +703,10 @@ int tc_gemm(bool ta, bool tb, int M, int N, int K, float alpha, const float *A, 
   const int tm = (M + BM - 1) / BM, nkb = (K + BK - 1) / BK;
   CUtensorMap ma, mb;
   const bool atm = tc::atmem_enabled();
-  // tile width: 80 for K-major B (128 where 80 takes more than one tile a SM:
-  // its epilogue spills, but fewer tiles read A and fill fewer waves; Si512
-  // H|psi>, 1100 bands: 11.83 -> 11.37 ms, 64 wide 12.32), 96 (three 32-column
-  // chunks) for MN-major B, unless the autotuner measured another for this
-  // shape (A in tensor memory only)
-  int bn = b_mn ? 96 : (atm && (long)tm * ((N + 79) / 80) > 148 ? 128 : 80);
+  // tile width: tc_tile_default for K-major B, 96 (three 32-column chunks) for
+  // MN-major B, unless the autotuner measured another for this shape (A in
+  // tensor memory only)
+  int bn = b_mn ? 96 : (atm ? tc_tile_default(tm, N) : 80);
   {
     // QX_TC_TILE forces a width for every shape where it is valid (tests)
     const char *env = getenv("QX_TC_TILE");
