@@ -765,7 +765,10 @@ static void sgemm_go(dim3 g, int M, int N, int K, float alpha, const float *A, l
 // k-blocks, in whole clusters, as far as two CTAs a SM hold them (cnt: one
 // zeroed counter per tile and slice).  At 65 bands (K 4810) splits summed by
 // the last CTA of a tile cost 30 to 45 us, most of it that CTA's reads;
-// in clusters 19 to 20 us.
+// in clusters 19 to 20 us.  One cluster a tile up to two tiles a SM: both
+// projector contractions of 576 x 350 (54 tiles, K 13572) 1036 unsplit, 579 us
+// so, of 1152 x 720 (216 tiles, K 27122) 4344 and 3826 us; the same from K 1066
+// (116 and 82 us) on; beyond 296 tiles not measured.
 template <bool TA, bool TB>
 static void sgemm_launch(int M, int N, int K, float alpha, const float *A, long lda, const float *B, long ldb,
                          float beta, float *C, long ldc, int gamma, const int *colmap, const int *ncol_dev,
@@ -779,7 +782,8 @@ static void sgemm_launch(int M, int N, int K, float alpha, const float *A, long 
   const long tiles = (long)g.x * g.y;
   const size_t part = sizeof(float) * (size_t)tiles * 256 * mt * nt;   // one cluster's partial tiles
   int nsplit = 1, kchunk = K;
-  if (ws && cnt && tiles * SCL <= GEMM_TILE_COUNTERS && tiles < 2 * 148 / SCL && K >= (TA ? 256 : 1024)) {
+  if (ws && cnt && tiles * SCL <= GEMM_TILE_COUNTERS && tiles < 2 * 148 &&
+      K >= (TA && tiles < 2 * 148 / SCL ? 256 : 1024)) {
     const long cl = std::min<long>((2 * 148 / SCL + tiles - 1) / tiles, std::max(1, K / (64 * SCL)));
     nsplit = SCL * (int)std::max<long>(1, std::min<long>(cl, (long)(ws_bytes / part)));
     kchunk = ((K + nsplit - 1) / nsplit + SBK - 1) / SBK * SBK;

@@ -15,6 +15,18 @@ pytestmark = pytest.mark.gpu
 @pytest.mark.parametrize("ecut", [4.0, 6.0, 8.0, 12.0, 30.0])
 @pytest.mark.parametrize("nb", [1, 2, 16, 31, 32, 33, 47, 65, 80, 81, 96])
 def test_hmatrix_split(ecut, nb):
+    _check(ecut, nb)
+
+
+@pytest.mark.parametrize("ecut,nb", [(15.0, 385), (15.5, 384), (15.5, 385), (15.5, 450), (20.0, 1088), (20.0, 1089)])
+def test_many_tiles(monkeypatch, ecut, nb):
+    """36 to 324 output tiles on both sides of the sizes that split K (K of at
+    least 1024, fewer than 296 tiles)."""
+    monkeypatch.setenv("QX_TC_MIN_FLOPS", "1e18")
+    _check(ecut, nb)
+
+
+def _check(ecut, nb):
     need_gpu()
     s = cell.build_system(cell.diamond_si((1, 1, 1), seed=1), ecut, 4 * ecut, nb, with_ewald=False)
     rng = np.random.default_rng(nb)
