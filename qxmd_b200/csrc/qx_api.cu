@@ -155,6 +155,12 @@ struct qx_ctx {
   double *d_kb_zzz = nullptr, *d_kb_vclt = nullptr, *d_kb_dcq = nullptr, *d_kb_dsq = nullptr, *d_kb_satm = nullptr;
   int *d_kb_even = nullptr, *d_kb_ngabc = nullptr, *d_kb_ityp = nullptr;
   bool have_kb_builder = false;
+  // real-space tables uploaded by qx_set_kb_r: atoms, natom * lmx, points and values the buffers hold
+  int kbt_natom = 0;
+  long kbt_nsum = 0, kbt_cap = 0, kbt_vcap = 0;
+  int *d_kbt_off = nullptr, *d_kbt_mesh = nullptr, *d_kbt_perm = nullptr, *d_kbt_ptoff = nullptr, *d_kbt_ptatom = nullptr;
+  double *d_kbt_clalp = nullptr;
+  void *d_kbt_vnl = nullptr, *d_kbt_pvnl = nullptr, *d_kbt_sumr = nullptr;
   // real-space table builder (qx_set_kb_r_builder, qx_build_kb_r)
   KbrGeom kbr_geom = {};
   int kbr_ntype = 0, kbr_mxnl = 0, kbr_natom = 0, kbr_lmx = 4;
@@ -923,58 +929,84 @@ extern "C" int qx_set_kb_r(qx_ctx *c, int natom, int lmx, const int *off, const 
   }
   Plan &pl = c->pl;
   const int npts = off[natom];
+  if (off[0] < 0) { set_error("qx_set_kb_r: off not ascending from 0"); return QX_ERR_ARG; }
   for (int a = 0; a < natom; ++a)
     if (off[a + 1] < off[a]) { set_error("qx_set_kb_r: off not ascending"); return QX_ERR_ARG; }
-  for (int i = 0; i < npts; ++i)
-    if (mesh[i] < 0 || mesh[i] >= pl.n) { set_error("qx_set_kb_r: mesh index out of range"); return QX_ERR_ARG; }
-  // the projector points at each grid point, in point order
+  // the projector points at each grid point, in point order: their indices and
+  // atoms here, their values on the device
   std::vector<int> poff(pl.n + 1, 0);
-  for (int i = 0; i < npts; ++i) poff[mesh[i] + 1]++;
+  for (int i = 0; i < npts; ++i) {
+    if (mesh[i] < 0 || mesh[i] >= pl.n) { set_error("qx_set_kb_r: mesh index out of range"); return QX_ERR_ARG; }
+    poff[mesh[i] + 1]++;
+  }
   for (long g = 0; g < pl.n; ++g) poff[g + 1] += poff[g];
-  std::vector<int> patom(std::max(npts, 1));
-  std::vector<double> pvnl((size_t)std::max(npts, 1) * lmx);
+  std::vector<int> perm(std::max(npts, 1), -1), patom(std::max(npts, 1));
   std::vector<int> fill(poff.begin(), poff.end() - 1);
   for (int a = 0; a < natom; ++a)
     for (int i = off[a]; i < off[a + 1]; ++i) {
       const int e = fill[mesh[i]]++;
+      perm[e] = i;
       patom[e] = a;
-      std::copy(vnl + (size_t)i * lmx, vnl + (size_t)(i + 1) * lmx, pvnl.begin() + (size_t)e * lmx);
     }
-  TRY(dalloc(c, &pl.d_kb_off, sizeof(int) * (natom + 1)));
-  TRY(dalloc(c, &pl.d_kb_mesh, sizeof(int) * std::max(npts, 1)));
-  TRY(dalloc(c, &pl.d_kb_clalp, sizeof(double) * lmx));
-  TRY(dalloc(c, &pl.d_pt_off, sizeof(int) * poff.size()));
-  TRY(dalloc(c, &pl.d_pt_atom, sizeof(int) * patom.size()));
-  CK(cudaMemcpy(pl.d_kb_off, off, sizeof(int) * (natom + 1), cudaMemcpyHostToDevice));
-  CK(cudaMemcpy(pl.d_kb_mesh, mesh, sizeof(int) * npts, cudaMemcpyHostToDevice));
-  CK(cudaMemcpy(pl.d_kb_clalp, clalp, sizeof(double) * lmx, cudaMemcpyHostToDevice));
-  CK(cudaMemcpy(pl.d_pt_off, poff.data(), sizeof(int) * poff.size(), cudaMemcpyHostToDevice));
-  CK(cudaMemcpy(pl.d_pt_atom, patom.data(), sizeof(int) * patom.size(), cudaMemcpyHostToDevice));
-  void *v = nullptr;
-  TRY(dalloc(c, &v, c->tsize() * (size_t)npts * lmx));
-  TRY(up(c, v, vnl, (long)npts * lmx));
-  void *pv = nullptr;
-  TRY(dalloc(c, &pv, c->tsize() * pvnl.size()));
-  TRY(up(c, pv, pvnl.data(), (long)npts * lmx));
-  CK(cudaStreamSynchronize(c->st));   // pvnl is a host temporary
+  // the buffers stay from call to call and grow on need, so uploads go through the stream
+  const size_t ts = c->tsize();
+  c->have_kbr = false;
+  drop_graphs(c);
+  if (natom > c->kbt_natom) {
+    TRY(dregrow(c, &c->d_kbt_off, sizeof(int) * (natom + 1)));
+    c->kbt_natom = natom;
+  }
+  if ((long)natom * lmx > c->kbt_nsum) {
+    TRY(dregrow(c, &c->d_kbt_sumr, 2 * ts * (size_t)pl.chunk * natom * lmx));
+    c->kbt_nsum = (long)natom * lmx;
+  }
+  if (npts > c->kbt_cap || !c->d_kbt_mesh) {
+    const size_t cap = std::max(npts, 1);
+    TRY(dregrow(c, &c->d_kbt_mesh, sizeof(int) * cap));
+    TRY(dregrow(c, &c->d_kbt_perm, sizeof(int) * cap));
+    TRY(dregrow(c, &c->d_kbt_ptatom, sizeof(int) * cap));
+    c->kbt_cap = cap;
+  }
+  if ((long)npts * lmx > c->kbt_vcap || !c->d_kbt_vnl) {
+    const size_t cap = (size_t)std::max(npts, 1) * lmx;
+    TRY(dregrow(c, &c->d_kbt_vnl, ts * cap));
+    TRY(dregrow(c, &c->d_kbt_pvnl, ts * cap));
+    c->kbt_vcap = cap;
+  }
+  if (!c->d_kbt_ptoff) {
+    TRY(dalloc(c, &c->d_kbt_ptoff, sizeof(int) * (pl.n + 1)));
+    TRY(dalloc(c, &c->d_kbt_clalp, sizeof(double) * QX_KBR_MAX_LMX));
+  }
+  if (!c->d_kbr_bufR) TRY(dalloc(c, &c->d_kbr_bufR, 2 * ts * (size_t)pl.chunk * pl.n));
+  CK(cudaMemcpyAsync(c->d_kbt_off, off, sizeof(int) * (natom + 1), cudaMemcpyHostToDevice, c->st));
+  CK(cudaMemcpyAsync(c->d_kbt_mesh, mesh, sizeof(int) * npts, cudaMemcpyHostToDevice, c->st));
+  CK(cudaMemcpyAsync(c->d_kbt_perm, perm.data(), sizeof(int) * npts, cudaMemcpyHostToDevice, c->st));
+  CK(cudaMemcpyAsync(c->d_kbt_ptatom, patom.data(), sizeof(int) * npts, cudaMemcpyHostToDevice, c->st));
+  CK(cudaMemcpyAsync(c->d_kbt_ptoff, poff.data(), sizeof(int) * (pl.n + 1), cudaMemcpyHostToDevice, c->st));
+  CK(cudaMemcpyAsync(c->d_kbt_clalp, clalp, sizeof(double) * lmx, cudaMemcpyHostToDevice, c->st));
+  TRY(up(c, c->d_kbt_vnl, vnl, (long)npts * lmx));
+  auto tables = [&](auto &b, auto *v, auto *pv, auto *r, auto *s) {
+    kbr_by_point(npts, lmx, c->d_kbt_perm, v, pv, c->st);
+    b.kb_vnl = v;
+    b.kb_pvnl = pv;
+    b.bufR = r;
+    b.sumr = s;
+  };
+  if (c->prec == QX_PREC_FP64)
+    tables(pl.b64, (double *)c->d_kbt_vnl, (double *)c->d_kbt_pvnl, (double2 *)c->d_kbr_bufR, (double2 *)c->d_kbt_sumr);
+  else
+    tables(pl.b32, (float *)c->d_kbt_vnl, (float *)c->d_kbt_pvnl, (float2 *)c->d_kbr_bufR, (float2 *)c->d_kbt_sumr);
+  CKL();
+  CK(cudaStreamSynchronize(c->st));   // the lists are host temporaries
+  pl.d_kb_off = c->d_kbt_off;
+  pl.d_kb_mesh = c->d_kbt_mesh;
+  pl.d_pt_off = c->d_kbt_ptoff;
+  pl.d_pt_atom = c->d_kbt_ptatom;
+  pl.d_kb_clalp = c->d_kbt_clalp;
   pl.natom = natom;
   pl.npts = npts;
   pl.kb_lmx = lmx;
   pl.rdelv = rdelv;
-  drop_graphs(c);
-  // real-space line buffer and projection sums, per chunk
-  const long ch = pl.chunk;
-  if (c->prec == QX_PREC_FP64) {
-    pl.b64.kb_vnl = (double *)v;
-    pl.b64.kb_pvnl = (double *)pv;
-    TRY(dalloc(c, &pl.b64.bufR, sizeof(double2) * ch * pl.n));
-    TRY(dalloc(c, &pl.b64.sumr, sizeof(double2) * ch * natom * lmx));
-  } else {
-    pl.b32.kb_vnl = (float *)v;
-    pl.b32.kb_pvnl = (float *)pv;
-    TRY(dalloc(c, &pl.b32.bufR, sizeof(float2) * ch * pl.n));
-    TRY(dalloc(c, &pl.b32.sumr, sizeof(float2) * ch * natom * lmx));
-  }
   c->have_kbr = true;
   return QX_OK;
 }
@@ -1108,9 +1140,9 @@ extern "C" int qx_build_kb_r(qx_ctx *c, int natom, const int *ityp, const double
     TRY(dalloc(c, &c->d_kbr_loff, sizeof(int) * (nlines + 1)));
     TRY(dalloc(c, &c->d_kbr_cursor, sizeof(int) * nlines));
     TRY(dalloc(c, &c->d_kbr_ptoff, sizeof(int) * (pl.n + 1)));
-    TRY(dalloc(c, &c->d_kbr_bufR, 2 * ts * (size_t)pl.chunk * pl.n));
     moved = true;
   }
+  if (!c->d_kbr_bufR) TRY(dalloc(c, &c->d_kbr_bufR, 2 * ts * (size_t)pl.chunk * pl.n));
   CK(cudaMemcpyAsync(c->d_kbr_ityp, ityp, sizeof(int) * natom, cudaMemcpyHostToDevice, c->st));
   CK(cudaMemcpyAsync(c->d_kbr_satm, satm, sizeof(double) * 3 * natom, cudaMemcpyHostToDevice, c->st));
   const KbrGeom &G = c->kbr_geom;
@@ -1329,6 +1361,7 @@ static int hpsi_impl(qx_ctx *c, const T *cin, T *out, const int *pairs, const in
   P.pairs = pairs;
   P.npair_dev = npair_dev;
   const int nlm = (flags & QX_HPSI_NONLOCAL) ? c->nlmode : 0;
+  if (nlm == QX_NL_RSPACE && !c->have_kbr) { set_error("hpsi: real-space tables not set"); return QX_ERR_STATE; }
   const double *dk = (flags & QX_HPSI_KINETIC) ? c->d_dk : nullptr;
   const int acc = (flags & QX_HPSI_ACCUMULATE) ? 1 : 0;
   // G-space KB: out = [out +] beta D <beta|c> on the second stream while the
@@ -1668,6 +1701,7 @@ static int eigen_seq_impl(qx_ctx *c, const qx_cgparm *p, int *nriter, int *nhpsi
   CgParm pm{p->itermx, p->iteremx, p->noband, p->tolera, p->roughfzan, p->roughfeig, p->threinn, p->wdinner};
   T *x = (T *)c->psi, *hx = (T *)c->hpsi, *g = (T *)c->g;
   if (!c->have_glocal) { set_error("hpsi: glocal not set"); return QX_ERR_STATE; }
+  if (c->nlmode == QX_NL_RSPACE && !c->have_kbr) { set_error("hpsi: real-space tables not set"); return QX_ERR_STATE; }
   const int need = 3 * std::max(nb, c->pl.nproj);
   if (c->seqw_len < need) {
     TRY(dalloc(c, &c->d_seqw, sizeof(double) * need));

@@ -250,6 +250,9 @@ template <typename T>
 void kbr_fill(const KbrGeom &G, int natom, int lmx, const int *ityp, const double *satm, const double *rcut,
               const double *rcl, const double *dltnl, const double *tabnl, const double *dtabnl, int mxnl,
               const int *poly, const int *soff, long cap, int *mesh, int *ptatom, T *vnl, T *dvnl, cudaStream_t st);
+// Projector values of uploaded tables in grid-point order: out(e, :) = vnl(perm[e], :).
+template <typename T>
+void kbr_by_point(int npts, int lmx, const int *perm, const T *vnl, T *out, cudaStream_t st);
 template <typename T>
 int kbr_lines(const int *off, int natom, const int *mesh, const int *ptatom, int k1, long nlines, int *lcnt,
               int *loff, int *cursor, int4 *lent, int *gpoff, int *gpatom, const T *vnl, int lmx, T *gpvnl,

@@ -470,6 +470,27 @@ int kbr_lines(const int *off, int natom, const int *mesh, const int *ptatom, int
   return 0;
 }
 
+// out(e, :) = vnl(perm[e], :), zero where perm[e] < 0: the values of uploaded
+// tables in grid-point order.
+template <typename T>
+__global__ void k_kbr_by_point(long n, int lmx, const int *__restrict__ perm, const T *__restrict__ vnl,
+                               T *__restrict__ out) {
+  const long q = blockIdx.x * (long)blockDim.x + threadIdx.x;
+  if (q >= n) return;
+  const long e = q / lmx;
+  const int i = perm[e];
+  out[q] = i >= 0 ? vnl[(long)i * lmx + (q - e * lmx)] : (T)0;
+}
+template <typename T>
+void kbr_by_point(int npts, int lmx, const int *perm, const T *vnl, T *out, cudaStream_t st) {
+  const long n = (long)npts * lmx;
+  if (n <= 0) return;
+  k_kbr_by_point<T><<<(unsigned)((n + 255) / 256), 256, 0, st>>>(n, lmx, perm, vnl, out);
+  note_launch();
+}
+template void kbr_by_point<float>(int, int, const int *, const float *, float *, cudaStream_t);
+template void kbr_by_point<double>(int, int, const int *, const double *, double *, cudaStream_t);
+
 template int kbr_lines<float>(const int *, int, const int *, const int *, int, long, int *, int *, int *, int4 *,
                               int *, int *, const float *, int, float *, cudaStream_t);
 template int kbr_lines<double>(const int *, int, const int *, const int *, int, long, int *, int *, int *, int4 *,
