@@ -183,6 +183,7 @@ struct qx_ctx {
   double *d_kbr_fpart = nullptr, *d_kbr_fout = nullptr;
   long kbr_fpart_n = 0;
   bool have_kbr_builder = false;
+  bool kbr_grad = false;   // the tables of the last qx_build_kb_r came with their gradients (d_kbr_dvnl)
   bool defer = false;
   struct ScfGraph {
     std::vector<char> key;
@@ -1208,6 +1209,7 @@ extern "C" int qx_build_kb_r(qx_ctx *c, int natom, const int *ityp, const double
   pl.npts = total;
   pl.kb_lmx = c->kbr_lmx;
   if (moved) drop_graphs(c);
+  c->kbr_grad = c->d_kbr_dtab != nullptr;
   c->have_kbr = true;
   return QX_OK;
 }
@@ -2619,7 +2621,7 @@ static int fnl_r_impl(qx_ctx *c, double *fnl) {
 extern "C" int qx_forces_nl_r(qx_ctx *c, double *fnl) {
   if (!c || !fnl) { set_error("qx_forces_nl_r: null"); return QX_ERR_ARG; }
   if (!c->have_occ) { set_error("qx_forces_nl_r: occupations not set"); return QX_ERR_STATE; }
-  if (!c->have_kbr || !c->d_kbr_dvnl || c->pl.d_kb_mesh != c->d_kbr_mesh) {
+  if (!c->have_kbr || !c->kbr_grad || c->pl.d_kb_mesh != c->d_kbr_mesh) {
     set_error("qx_forces_nl_r: real-space tables with gradients (qx_set_kb_r_builder with dtabnl, qx_build_kb_r) needed");
     return QX_ERR_STATE;
   }

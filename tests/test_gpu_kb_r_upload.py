@@ -10,7 +10,7 @@ import pytest
 
 import oracle
 from qxmd_b200 import cell
-from qxmd_b200.lib import Context, QX_NL_RSPACE, QX_PREC_FP64, QX_PREC_MIXED
+from qxmd_b200.lib import Context, QxError, QX_NL_RSPACE, QX_PREC_FP64, QX_PREC_MIXED
 
 from gpu_util import need_gpu, relerr
 
@@ -68,3 +68,25 @@ def test_uploads(si8, si8_psi, prec, tol):
     assert one.L.qx_set_kb_r(one.h, si8.cell.natom, 4, bad, np.ascontiguousarray(si8.kb_r.mesh, dtype=np.int32),
                              np.ascontiguousarray(si8.kb_r.vnl), si8.kb_r.clalp, si8.kb_r.rdelv) != 0
     one.close()
+
+
+def test_forces_need_the_gradients_of_their_tables(si8, si8_psi):
+    """Tables built without gradients after others with them: no forces from
+    the gradients of the tables before; the builder alone changes nothing."""
+    need_gpu()
+    b = cell.kbr_builder_tables(si8.gs, si8.cell, si8.pp)
+    plain = {k: v for k, v in b.items() if k != "dtabnl"}
+    ctx = Context(si8, QX_PREC_FP64, QX_NL_RSPACE)
+    ctx.put_psi(si8_psi)
+    ctx.set_kb_r_builder(b)
+    ctx.build_kb_r(b["ityp"], b["satm"])
+    f = ctx.forces_nl_r()
+    ctx.set_kb_r_builder(plain)
+    assert np.array_equal(ctx.forces_nl_r(), f)
+    ctx.build_kb_r(b["ityp"], b["satm"] + 0.01)
+    with pytest.raises(QxError):
+        ctx.forces_nl_r()
+    ctx.set_kb_r_builder(b)
+    ctx.build_kb_r(b["ityp"], b["satm"])
+    assert np.array_equal(ctx.forces_nl_r(), f)
+    ctx.close()
