@@ -953,31 +953,34 @@ extern "C" int qx_set_kb_r(qx_ctx *c, int natom, int lmx, const int *off, const 
   const size_t ts = c->tsize();
   c->have_kbr = false;
   drop_graphs(c);
+  // (a capacity is zero while its buffers grow, so that a growth that failed is tried again)
   if (natom > c->kbt_natom) {
+    c->kbt_natom = 0;
     TRY(dregrow(c, &c->d_kbt_off, sizeof(int) * (natom + 1)));
     c->kbt_natom = natom;
   }
   if ((long)natom * lmx > c->kbt_nsum) {
+    c->kbt_nsum = 0;
     TRY(dregrow(c, &c->d_kbt_sumr, 2 * ts * (size_t)pl.chunk * natom * lmx));
     c->kbt_nsum = (long)natom * lmx;
   }
-  if (npts > c->kbt_cap || !c->d_kbt_mesh) {
+  if (std::max(npts, 1) > c->kbt_cap) {
     const size_t cap = std::max(npts, 1);
+    c->kbt_cap = 0;
     TRY(dregrow(c, &c->d_kbt_mesh, sizeof(int) * cap));
     TRY(dregrow(c, &c->d_kbt_perm, sizeof(int) * cap));
     TRY(dregrow(c, &c->d_kbt_ptatom, sizeof(int) * cap));
     c->kbt_cap = cap;
   }
-  if ((long)npts * lmx > c->kbt_vcap || !c->d_kbt_vnl) {
+  if ((long)std::max(npts, 1) * lmx > c->kbt_vcap) {
     const size_t cap = (size_t)std::max(npts, 1) * lmx;
+    c->kbt_vcap = 0;
     TRY(dregrow(c, &c->d_kbt_vnl, ts * cap));
     TRY(dregrow(c, &c->d_kbt_pvnl, ts * cap));
     c->kbt_vcap = cap;
   }
-  if (!c->d_kbt_ptoff) {
-    TRY(dalloc(c, &c->d_kbt_ptoff, sizeof(int) * (pl.n + 1)));
-    TRY(dalloc(c, &c->d_kbt_clalp, sizeof(double) * QX_KBR_MAX_LMX));
-  }
+  if (!c->d_kbt_ptoff) TRY(dalloc(c, &c->d_kbt_ptoff, sizeof(int) * (pl.n + 1)));
+  if (!c->d_kbt_clalp) TRY(dalloc(c, &c->d_kbt_clalp, sizeof(double) * QX_KBR_MAX_LMX));
   if (!c->d_kbr_bufR) TRY(dalloc(c, &c->d_kbr_bufR, 2 * ts * (size_t)pl.chunk * pl.n));
   CK(cudaMemcpyAsync(c->d_kbt_off, off, sizeof(int) * (natom + 1), cudaMemcpyHostToDevice, c->st));
   CK(cudaMemcpyAsync(c->d_kbt_mesh, mesh, sizeof(int) * npts, cudaMemcpyHostToDevice, c->st));
@@ -1122,7 +1125,10 @@ extern "C" int qx_build_kb_r(qx_ctx *c, int natom, const int *ityp, const double
   const size_t ts = c->tsize();
   const long nlines = (long)pl.k2 * pl.k3;
   bool moved = false;   // a table buffer was (re)allocated: captured graphs hold stale pointers
+  c->have_kbr = false;  // until the tables are whole: a call that fails below may have freed some of them
+  // (a size is zero while its buffers are replaced, so that a replacement that failed is tried again)
   if (natom != c->kbr_natom) {
+    c->kbr_natom = 0;
     TRY(dregrow(c, &c->d_kbr_ityp, sizeof(int) * natom));
     TRY(dregrow(c, &c->d_kbr_satm, sizeof(double) * 3 * natom));
     TRY(dregrow(c, &c->d_kbr_off, sizeof(int) * (natom + 1)));
@@ -1132,14 +1138,15 @@ extern "C" int qx_build_kb_r(qx_ctx *c, int natom, const int *ityp, const double
   }
   const long slabs = (long)natom * (2 * c->kbr_geom.nd[2] + 1);
   if (slabs != c->kbr_slabs) {
+    c->kbr_slabs = 0;
     TRY(dregrow(c, &c->d_kbr_cnt, sizeof(int) * slabs));
     TRY(dregrow(c, &c->d_kbr_soff, sizeof(int) * (slabs + 1)));
     c->kbr_slabs = slabs;
   }
-  if (!c->d_kbr_loff) {
-    TRY(dalloc(c, &c->d_kbr_lcnt, sizeof(int) * nlines));
-    TRY(dalloc(c, &c->d_kbr_loff, sizeof(int) * (nlines + 1)));
-    TRY(dalloc(c, &c->d_kbr_cursor, sizeof(int) * nlines));
+  if (!c->d_kbr_ptoff) {
+    if (!c->d_kbr_lcnt) TRY(dalloc(c, &c->d_kbr_lcnt, sizeof(int) * nlines));
+    if (!c->d_kbr_loff) TRY(dalloc(c, &c->d_kbr_loff, sizeof(int) * (nlines + 1)));
+    if (!c->d_kbr_cursor) TRY(dalloc(c, &c->d_kbr_cursor, sizeof(int) * nlines));
     TRY(dalloc(c, &c->d_kbr_ptoff, sizeof(int) * (pl.n + 1)));
     moved = true;
   }
@@ -1154,6 +1161,7 @@ extern "C" int qx_build_kb_r(qx_ctx *c, int natom, const int *ityp, const double
   CK(cudaStreamSynchronize(c->st));
   if (total > c->kbr_cap) {
     const long cap = (long)(total * 1.25) + 64;
+    c->kbr_cap = 0;
     TRY(dregrow(c, &c->d_kbr_mesh, sizeof(int) * cap));
     TRY(dregrow(c, &c->d_kbr_ptatom, sizeof(int) * cap));
     TRY(dregrow(c, &c->d_kbr_lent, sizeof(int4) * cap));
@@ -1164,6 +1172,7 @@ extern "C" int qx_build_kb_r(qx_ctx *c, int natom, const int *ityp, const double
     moved = true;
   }
   if (c->d_kbr_dtab && c->kbr_dvnl_cap < c->kbr_cap) {
+    c->kbr_dvnl_cap = 0;
     TRY(dregrow(c, &c->d_kbr_dvnl, ts * 3 * c->kbr_lmx * (size_t)c->kbr_cap));
     c->kbr_dvnl_cap = c->kbr_cap;
   }
