@@ -21,10 +21,13 @@
 #include <cmath>
 #include <cstdlib>
 
+#include <cooperative_groups.h>
 #include <mutex>
 #include <type_traits>
 
 #include "qx_internal.h"
+
+namespace cg = cooperative_groups;
 
 // --------------------------------------------------------------------------
 // Small DFTs in registers.  Roots of unity w_R^m = exp(-2 pi i m / R) for
@@ -493,7 +496,11 @@ __global__ void __launch_bounds__(QX_THREADS) k_xinv_r(PipeParams P, const typen
 // and pair, as before, was bound by FP32 to FP64 conversions and by re-reading
 // the table for every pair; at Si64, 160 bands: projections 133 -> 78 us,
 // forces 506 -> 187 us.
-template <typename T, int MT, int NT, bool FORCE>
+// SPLIT: a cluster of CTAs takes an atom's points, a run each, and the first
+// of them adds the sums in order, where atoms and bands alone leave SMs
+// without a CTA (8 atoms, 45^3, 24 bands: 24 CTAs ran 22 k points each; H|psi>
+// FP32 213 -> 68 us, FP64 241 -> 119; Si64 at 16 bands 90 -> 65 and 148 -> 120).
+template <typename T, int MT, int NT, bool FORCE, bool SPLIT>
 __global__ void __launch_bounds__(QX_THREADS) k_ptsum(PipeParams P, const typename c2t<T>::type *__restrict__ R,
                                                        const int *__restrict__ off, const int *__restrict__ mesh,
                                                        const T *__restrict__ vnl, const T *__restrict__ dvnl,
@@ -502,14 +509,21 @@ __global__ void __launch_bounds__(QX_THREADS) k_ptsum(PipeParams P, const typena
                                                        typename c2t<T>::type *__restrict__ sumr,
                                                        double *__restrict__ fpart) {
   constexpr int NW = QX_THREADS / 32, UN = MT * NT <= 8 ? 4 : 2;
-  const int at = blockIdx.x, pg = blockIdx.y * (NT * 4);   // first pair of the CTA
+  const int S = SPLIT ? (int)gridDim.x / natom : 1;         // CTAs an atom, one cluster
+  const int at = blockIdx.x / S, sl = blockIdx.x % S, pg = blockIdx.y * (NT * 4);   // first pair of the CTA
   const int np = min(npl, pair_count(P) - P.pair0);
   if (pg >= np) return;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int row = lane >> 2, kk = lane & 3;                // fragment row (band) and point of this lane
   const int rows = FORCE ? 4 * lmx : lmx;
   const long n = (long)P.k1 * P.k2 * P.k3;
-  const int p0 = off[at], cnt = off[at + 1] - p0;
+  int p0 = off[at], cnt = off[at + 1] - p0;
+  if constexpr (SPLIT) {   // this CTA's run of the atom's points, whole rounds of its warps
+    constexpr int RND = 4 * UN * NW;
+    const int run = ((cnt + S - 1) / S + RND - 1) / RND * RND, lo = min(cnt, sl * run);
+    p0 += lo;
+    cnt = min(cnt - lo, run);
+  }
   double acc[MT][NT][2];
 #pragma unroll
   for (int m = 0; m < MT; ++m)
@@ -575,6 +589,18 @@ __global__ void __launch_bounds__(QX_THREADS) k_ptsum(PipeParams P, const typena
 #pragma unroll
     for (int w = 0; w < NW; ++w) v += red[w][q];
     red[0][q] = v;
+  }
+  if constexpr (SPLIT) {
+    cg::cluster_group cl = cg::this_cluster();
+    cl.sync();
+    if (sl == 0)
+      for (int q = threadIdx.x; q < NQ; q += QX_THREADS) {
+        double v = red[0][q];
+        for (int r = 1; r < S; ++r) v += cl.map_shared_rank(&red[0][0], r)[q];
+        red[0][q] = v;
+      }
+    cl.sync();   // no CTA leaves while the first still reads its sums
+    if (sl) return;
   }
   __syncthreads();
   const double *s = red[0];
@@ -843,15 +869,31 @@ static void z_forward(const PipeParams &P, int npl, const Bufs<T> &bf, const Fft
 // The sums of the chunk's pairs over every atom's points.  Where that fills
 // the GPU a CTA takes 16 bands (projections) or 32 (forces, whose table rows
 // are four times as many; at Si64 16 bands measured 228 us against 198), else 8.
+// An atom's points are split over 2, 4 or 8 CTAs while there are fewer than two
+// CTAs a SM, down to 128 points (a round of its warps) a CTA: at one CTA a SM
+// Si64 with 32 bands took 94 us, at two 80, at four 84.
 template <typename T, bool FORCE>
 static void launch_ptsum(const Plan &pl, const PipeParams &P, int npl, const T *dvnl, const double *wocc,
                          double *fpart, cudaStream_t st) {
   Bufs<T> &bf = pl.bufs<T>();
   auto go = [&](auto mt, auto nt) {
     constexpr int MT = decltype(mt)::value, NT = decltype(nt)::value;
-    k_ptsum<T, MT, NT, FORCE><<<dim3(pl.natom, (npl + NT * 4 - 1) / (NT * 4)), QX_THREADS, 0, st>>>(
-        P, bf.bufR, pl.d_kb_off, pl.d_kb_mesh, bf.kb_vnl, dvnl, pl.d_kb_clalp, pl.rdelv, pl.natom, pl.kb_lmx, npl,
-        wocc, bf.sumr, fpart);
+    const int ny = (npl + NT * 4 - 1) / (NT * 4);
+    int S = 1;
+    while (S < 8 && (long)pl.natom * ny * S < 2 * 148 && pl.npts / pl.natom >= 2 * S * 128) S *= 2;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(pl.natom * S, ny);
+    cfg.blockDim = dim3(QX_THREADS);
+    cfg.stream = st;
+    cudaLaunchAttribute cluster = {};
+    cluster.id = cudaLaunchAttributeClusterDimension;
+    cluster.val.clusterDim.x = S;
+    cluster.val.clusterDim.y = cluster.val.clusterDim.z = 1;
+    cfg.attrs = &cluster;
+    cfg.numAttrs = S > 1 ? 1 : 0;
+    cudaLaunchKernelEx(&cfg, S > 1 ? k_ptsum<T, MT, NT, FORCE, true> : k_ptsum<T, MT, NT, FORCE, false>, P, bf.bufR,
+                       pl.d_kb_off, pl.d_kb_mesh, bf.kb_vnl, dvnl, pl.d_kb_clalp, pl.rdelv, pl.natom, pl.kb_lmx, npl,
+                       wocc, bf.sumr, fpart);
     note_launch();
   };
   using std::integral_constant;
