@@ -760,8 +760,9 @@ static void sgemm_go(dim3 g, int M, int N, int K, float alpha, const float *A, l
 
 // One shape's launch: tile rows MT x NT from the extents (k-contiguous A:
 // both from the band-sized extents; otherwise 64-row tiles down M, or 48- or
-// 32-row ones where 64 leave SMs without a tile (M 4810: 16.2 -> 13.8 us)), and K split to shorten the
-// chain of one CTA: a k-block of 16 costs 0.5 to 1 us, so chunks of about four
+// 32-row ones as long as they stay within a tile a SM (per contraction with 64 /
+// 48 / 32 rows: M 2946, N 100, 94 / 124 / 186 tiles, 6.2 / 5.1 / 6.2 us; M 4166, N 128,
+// 132 / 174 / 262 tiles, 6.2 / 7.7 / 6.7)), and K split to shorten the chain of one CTA: a k-block of 16 costs 0.5 to 1 us, so chunks of about four
 // k-blocks, in whole clusters, as far as two CTAs a SM hold them (cnt: one
 // zeroed counter per tile and slice).  At 65 bands (K 4810) splits summed by
 // the last CTA of a tile cost 30 to 45 us, most of it that CTA's reads;
@@ -777,7 +778,7 @@ static void sgemm_launch(int M, int N, int K, float alpha, const float *A, long 
   const int nt = sgemm_rows(N), tn = (N + 16 * nt - 1) / (16 * nt);
   int mt = TA ? sgemm_rows(M) : 4;
   if (!TA)
-    while (mt > 2 && (long)((M + 16 * mt - 1) / (16 * mt)) * tn < 148) --mt;
+    while (mt > 2 && (long)((M + 16 * (mt - 1) - 1) / (16 * (mt - 1))) * tn <= 148) --mt;
   dim3 g((M + 16 * mt - 1) / (16 * mt), tn);
   const long tiles = (long)g.x * g.y;
   const size_t part = sizeof(float) * (size_t)tiles * 256 * mt * nt;   // one cluster's partial tiles

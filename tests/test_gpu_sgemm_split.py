@@ -4,10 +4,11 @@ threshold and its cluster counts, against the same sums in FP64."""
 import numpy as np
 import pytest
 
+import oracle
 from qxmd_b200 import cell
 from qxmd_b200.lib import Context, QX_NL_GSPACE, QX_PREC_MIXED
 
-from gpu_util import need_gpu
+from gpu_util import need_gpu, relerr
 
 pytestmark = pytest.mark.gpu
 
@@ -24,6 +25,25 @@ def test_many_tiles(monkeypatch, ecut, nb):
     least 1024, fewer than 296 tiles)."""
     monkeypatch.setenv("QX_TC_MIN_FLOPS", "1e18")
     _check(ecut, nb)
+
+
+@pytest.mark.parametrize("nb", [16, 80, 81, 99, 128, 129, 161])
+def test_row_tiles(monkeypatch, nb):
+    """K P of H|psi> (2946 rows) with 32-, 48- and 64-row tiles, against the
+    FP64 oracle."""
+    need_gpu()
+    monkeypatch.setenv("QX_TC_MIN_FLOPS", "1e18")
+    s = cell.build_system(cell.diamond_si((1, 1, 1), seed=1), 30.0, 120.0, nb, with_ewald=False)
+    assert s.gs.nplwex == 2946
+    psi = cell.random_wavefunctions(s.gs.nplwex, nb)
+    psi /= np.linalg.norm(psi, axis=1)[:, None]
+    ctx = Context(s, QX_PREC_MIXED, QX_NL_GSPACE)
+    ctx.put_psi(psi)
+    ctx.enonloc()
+    got = ctx.get_hpsi()
+    ctx.close()
+    # FP32 rounding of the transforms, as the other H|psi> tests of the mixed path
+    assert relerr(got, oracle.Ham(s, QX_NL_GSPACE).hpsi(psi)) < 2e-5
 
 
 def _check(ecut, nb):
