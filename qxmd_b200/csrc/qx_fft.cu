@@ -492,7 +492,8 @@ __global__ void __launch_bounds__(QX_THREADS) k_xinv_r(PipeParams P, const typen
 //     nlkbppr.f90:2024-3120) of each band pair, F = sum_b 2 occ_b / Omega
 //     rdelv^2 sum_l clalp_l P_l D_l in fpart[(pair * natom + atom) * 3 + dim]
 //     (added over pairs in a fixed order afterwards); wocc = occ / Omega.
-// The gathers of psi (32-byte sectors of L2) bound it.  One thread per point
+// The latency of the gathers of psi (32-byte sectors of L2) bounds it, the
+// tensor pipe being active for a third.  One thread per point
 // and pair, as before, was bound by FP32 to FP64 conversions and by re-reading
 // the table for every pair; at Si64, 160 bands: projections 133 -> 78 us,
 // forces 506 -> 187 us.

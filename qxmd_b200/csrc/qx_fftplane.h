@@ -34,10 +34,12 @@ template <int N>
 int zcols2_launch(const PipeParams &P, int npl, const float *cin, long ldc, float2 *bufA, const float2 *src,
                   float2 *zsph, bool inv, cudaStream_t st);
 
-// The k1 x k2 plane shapes with register kernels, X(k1, k2): the square
-// grids of 20 to 64 points built from radices 2, 3, 5 and 7, and the
-// elongated cells of the 48-cell batch (two or three primitive cells along
-// x).  The same list drives the dispatch and the instantiation files.
+// The k1 x k2 plane shapes with register kernels, X(k1, k2): sixteen square
+// ones of 20 to 64 points (36 and 64 for callers with grids of their own; of the
+// lengths that cells give, 35, 56 and 63 have none), and the elongated cells of
+// the 48-cell batch (two or three unit cells along x).  Other planes, 48 x 24 or 49 x 54 say, take the
+// shared-memory stages.  The same list drives the dispatch and the
+// instantiation files.
 #define QX_PLANE_GRIDS(X)                                                                              \
   X(20, 20) X(21, 21) X(24, 24) X(25, 25) X(27, 27) X(30, 30) X(32, 32) X(36, 36) X(40, 40) X(42, 42) \
   X(45, 45) X(48, 48) X(49, 49) X(54, 54) X(60, 60) X(64, 64)                                         \
@@ -47,8 +49,8 @@ int zcols2_launch(const PipeParams &P, int npl, const float *cin, long ldc, floa
 #define QX_ZCOLS_LENGTHS(X) \
   X(20) X(21) X(24) X(25) X(27) X(30) X(32) X(36) X(40) X(42) X(45) X(48) X(49) X(54) X(60) X(64)
 
-// FP64 (qx_fftplane64_kern.cuh): the plane shapes whose lines are even, or odd
-// and at most 32 points.
+// FP64 (qx_fftplane64_kern.cuh): those of the FP32 shapes above whose lines are
+// even, or odd and at most 32 points (not 45 and 49).
 #define QX_PLANE64_GRIDS(X)                                                                            \
   X(20, 20) X(21, 21) X(24, 24) X(25, 25) X(27, 27) X(30, 30) X(32, 32) X(36, 36) X(40, 40) X(42, 42) \
   X(48, 48) X(54, 54) X(60, 60) X(64, 64)                                                             \

@@ -22,8 +22,8 @@
 
 namespace qx {
 
-// Resident CTAs per SM asked of the register allocator: 8 (128 registers)
-// where that needs no spills.
+// Resident CTAs per SM asked of the register allocator: 8 (128 registers) up
+// to 54 points, where that spills nothing or 4 to 32 bytes a thread.
 constexpr int plane_minb(int n) { return n <= 54 ? 8 : 1; }
 
 // Grid rows of the x phase, thread t of a 64-thread CTA: with two planes of
@@ -92,7 +92,8 @@ __device__ __forceinline__ void plane_x_back(const float2 *row, float2 (&x)[NX])
 // zero samples' loads and butterflies and the outputs beyond the sphere are
 // left out at compile time; the tile then has 2 MBX + 1 columns, those beyond
 // the sphere zero.  At Si64 (54 x 54, 160 bands): 88 -> 49 us the pass, and the
-// outputs are the same bit for bit.
+// outputs are the same bit for bit.  The FMA pipe is active for 66 % of it, at
+// 16 warps a SM (the registers' limit); stalls on instruction fetches are few.
 template <int NX, int NY, int PL, int U, bool HALF>
 __global__ void __launch_bounds__(64 * U, (plane_minb(NX > NY ? NX : NY) + U - 1) / U)
     k_plane(PipeParams P, float2 *__restrict__ bufA, const float *__restrict__ vloct, int npl) {
@@ -336,9 +337,9 @@ __global__ void __launch_bounds__(2 * N) k_plane2(PipeParams P, float2 *__restri
 //     bufA.  A grid point's projector points come in grid-point order
 //     (NlPoints), so each thread sums its own points in a fixed order,
 //     for both pairs of the CTA from one read of the projector values.
-// Latency and the L2 traffic of the projector values bound the second (24
-// bytes an entry and CTA, 313 k entries at Si64), hence two pairs a CTA and
-// four grid points in flight a thread.  Against the shared-memory stage
+// The L1 path (70 % busy) and the latency of the projector values' gathers
+// bound the second (24 bytes an entry and CTA, 313 k entries at Si64), hence
+// two pairs a CTA and four grid points in flight a thread.  Against the shared-memory stage
 // kernels and the scatter by float atomics in shared memory that these
 // replace, per 160-band pass at Si64: y and x backward 118 -> 55 us, forward
 // 366 -> 145 us.
