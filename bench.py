@@ -429,7 +429,7 @@ def kb_build_timing(sys_, ctx, R, W, flush):
     ms = t / R
     out = {"ms_per_geometry": ms, "table_bytes_written": nbytes, "gb_per_s": nbytes / (ms * 1e-3) / 1e9,
            "builds_timed": R}
-    # real-space tables (setnlc): point search, values, x-line index; one
+    # real-space tables (setnlc): point search, values, grid-point index; one
     # host read of the point count per build (buffer capacity check)
     br = cell.kbr_builder_tables(sys_.gs, sys_.cell, sys_.pp)
     ctx.set_kb_r_builder(br)

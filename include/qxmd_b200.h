@@ -124,7 +124,10 @@ int qx_get_kb_g(qx_ctx *ctx, double *eqlmr, double *vclalp);
  * zero-based grid index mesh[] and projector values vnl[point*lmx + l];
  * clalp(lmx) = clalp_ncr; rdelv = volume per grid point.  1 <= lmx <=
  * QX_KBR_MAX_LMX; species with fewer projectors than lmx carry zero columns
- * (the reference's lmx(it) differs by species; one stride serves all here). */
+ * (the reference's lmx(it) differs by species; one stride serves all here).
+ * off ascends from 0 on.  May be called again with other tables: the context's
+ * buffers grow on need.  When a call fails after its arguments were accepted
+ * (an allocation), the tables count as unset. */
 int qx_set_kb_r(qx_ctx *ctx, int natom, int lmx, const int *off, const int *mesh, const double *vnl,
                 const double *clalp, double rdelv);
 /* The real-space tables built on the device, for MD steps (setnlc
@@ -155,7 +158,7 @@ int qx_set_kb_r_builder(qx_ctx *ctx, int ntype, int lmx, int mxnl, const double 
 int qx_set_kb_r_channel_radii(qx_ctx *ctx, const double *rcl);
 /* Once per geometry: the points of every atom (species ityp(natom), 0-based,
  * fractional coordinates satm(3, natom)) within its projector radius, their
- * projector values, and the x-line index of the real-space KB kernels.  The
+ * projector values, and the grid-point index of the real-space KB kernels.  The
  * buffers grow by 25 % when the point count outgrows them (captured graphs
  * are then dropped); otherwise they are reused in place. */
 int qx_build_kb_r(qx_ctx *ctx, int natom, const int *ityp, const double *satm);

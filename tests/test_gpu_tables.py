@@ -3,8 +3,8 @@ H|psi> after MD-like moves of the atoms that rebuild the tables in place:
 G space (qx_set_kb_builder once per cell, qx_build_kb_g once per geometry:
 setqlm nlkbpp.f90:2196-2247, setbgq nlkbpp.f90:2135-2187, phases of
 stscfn_pw pwlda.f90:5711-5850) and real space (qx_set_kb_r_builder,
-qx_build_kb_r: setnlc nlkbppr.f90:1010-1560, the points, values and x-line
-index that calnlc's kernels read).
+qx_build_kb_r: setnlc nlkbppr.f90:1010-1560, the points, values and
+grid-point index that calnlc's kernels read).
 
 Tolerances: the FP64 table 1e-13 of its largest entry (the device cos/sin
 and fused multiply-adds against numpy); the FP32 table 2e-7 (one rounding);
